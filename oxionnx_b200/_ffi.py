@@ -40,6 +40,15 @@ class Result(ctypes.Structure):
                 ("shape", ctypes.c_uint64 * MAX_RANK), ("rank", ctypes.c_uint32), ("resident", ctypes.c_void_p)]
 
 
+# the same layouts with plain addresses in place of typed pointers: assigning an integer to such a field is cheap
+class RawOperand(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p if n == "lanes" else t) for n, t in Operand._fields_]
+
+
+class RawResult(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p if n == "lanes" else t) for n, t in Result._fields_]
+
+
 class ValueInfo(ctypes.Structure):
     _fields_ = [("name", ctypes.c_char_p), ("shape", ctypes.POINTER(ctypes.c_uint64)), ("rank", ctypes.c_uint32), ("dtype", ctypes.c_int32)]
 

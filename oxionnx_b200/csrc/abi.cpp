@@ -493,8 +493,7 @@ int oxb200_run(oxb200_ctx* ctx, const oxb200_operand* feeds, uint32_t n_feeds, o
     s.download_async(fetches, n_fetches);
     OXB_CUDA(cudaEventRecord(C.run_ev1, C.stream()));
     s.finish_download();
-    float ms = -1.f;
-    if (cudaEventElapsedTime(&ms, C.run_ev0, C.run_ev1) == cudaSuccess) C.last_run_ms = ms;
+    C.last_run_timed = true;  // the events are read when someone asks (oxb200_last_run_ms)
     return (int)OXB200_OK_HOST;
   });
 }
@@ -521,7 +520,15 @@ int oxb200_run_collect(oxb200_ctx* ctx, oxb200_result* fetches, uint32_t n_fetch
   });
 }
 
-float oxb200_last_run_ms(const oxb200_ctx* ctx) { return ctx ? ctx->impl.last_run_ms : -1.f; }
+float oxb200_last_run_ms(const oxb200_ctx* ctx) {
+  if (!ctx) return -1.f;
+  float ms = -1.f;
+  if (ctx->impl.last_run_timed && cudaEventElapsedTime(&ms, ctx->impl.run_ev0, ctx->impl.run_ev1) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ms = -1.f;
+  }
+  return ms;
+}
 
 // ---- device I/O binding (IoBinding / run_with_binding over device memory) ----
 int oxb200_bind_input_device(oxb200_ctx* ctx, const char* name, const void* device_ptr, int32_t dtype, uint64_t len) {

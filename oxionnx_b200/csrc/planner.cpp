@@ -548,8 +548,7 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
     for (size_t s = 0; s < nodes_[ni].inputs.size(); ++s)
       if (!nodes_[ni].inputs[s].empty()) consumers_[nodes_[ni].inputs[s]].push_back({(int)ni, (int)s});
 
-  OXB_CUDA(cudaMalloc(&S.err_flag_, 256));
-  OXB_CUDA(cudaMemset(S.err_flag_, 0, 256));
+  S.err_flag_ = C.take_error_word();
 
   // graph inputs: raw f32 lanes in logical order, uploaded into persistent staging
   for (auto& in : inputs) {

@@ -170,16 +170,30 @@ class Session {
   std::vector<k::UmmaChain*> umma_chains_;
   std::vector<k::UmmaAttentionPlan*> umma_attentions_;
   size_t n_slots_ = 0;
-  int* err_flag_ = nullptr;
+  int* err_flag_ = nullptr;  // the kernels' error word, in page-locked memory that the device addresses (see check_error_flag)
   std::map<std::string, std::pair<void*, std::pair<DT, Layout>>> external_bind_;
   std::map<std::string, DT> input_types_;
   // device bindings: input index -> caller's buffer (copied into the input's own buffer when a tensor map holds
   // that buffer's address, read in place otherwise); output index -> caller's buffer and capacity
   std::map<int, const void*> bound_in_;
+  std::vector<char> in_tensor_map_;  // per graph input: does a tensor map hold its buffer's address (filled at the first binding)
   std::map<int, std::pair<void*, uint64_t>> bound_out_;
   std::vector<void*> own_in_ptr_;  // the session's own buffer of each graph input (what an unbound input reads)
   bool input_in_tensor_map(int value_index) const;
   void apply_input_bindings();
+  // Host lanes <-> device through page-locked staging (see stage_in / stage_out in runtime.cpp).
+  uint8_t* small_stage_ = nullptr;  // small feeds, then small fetches, of the one synchronous run
+  size_t small_stage_bytes_ = 0, small_stage_used_ = 0;
+  struct PendingCopy {
+    void* dst;
+    const void* src;
+    size_t bytes;
+  };
+  std::vector<PendingCopy> pending_out_;  // fetches that wait in the staging memory for the run's fence
+  void begin_copies();
+  void* small_stage(size_t bytes);
+  void stage_in(void* dst, const void* src, size_t bytes);
+  void stage_out(void* dst, const void* src, size_t bytes);
   std::shared_ptr<void> planner_;  // keeps the objects the step closures refer to alive
   struct Flight {
     bool busy = false;
@@ -188,7 +202,6 @@ class Session {
     std::vector<void*> in_dev;       // this slot's device buffer per graph input
     std::vector<float*> out_host;    // pinned staging per graph output
     std::vector<void*> out_dev;      // device copy of each output, so that the next run need not wait for the download
-    int* err_host = nullptr;         // pinned copy of the kernels' error word
   };
   Flight flight_[2];
   int submit_idx_ = 0, collect_idx_ = 0;
@@ -216,6 +229,8 @@ class Session {
   void allow_graph(bool on) { graph_allowed_ = on; }
 };
 
+struct MovePool;
+
 class Context {
  public:
   Context(int device, const oxb200_config& cfg);
@@ -242,11 +257,20 @@ class Context {
   void release_caches();
   void free_temp_forms();
 
+  // One word of page-locked memory that kernels may write and the host reads after a fence; nullptr-safe to give back.
+  int* take_error_word();
+  void give_error_word(int* word);
+  // Large pageable host buffers: copied in pieces through page-locked buffers by a few host threads, so that the
+  // host copy of one piece runs beside the PCIe transfer of another (host_to_device only enqueues the last
+  // transfers; device_to_host returns when every lane has arrived).
+  void host_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
+  void device_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
   oxb200_counters counters{};
   std::string last_error;
   std::unique_ptr<Session> session;  // the planned session of oxb200_session_plan
   cudaEvent_t run_ev0 = nullptr, run_ev1 = nullptr;
-  float last_run_ms = -1.f;
+  bool last_run_timed = false;  // run_ev0 / run_ev1 bracket a finished run
   std::mutex mu;
 
  private:
@@ -257,7 +281,14 @@ class Context {
   std::map<std::pair<std::string, std::string>, DeviceBuffer> forms_;
   std::set<std::string> resident_names_;
   std::vector<void*> temp_forms_;
+  int* error_words_ = nullptr;  // kErrorWords words, 64 bytes apart
+  std::vector<int*> free_error_words_;
+  std::shared_ptr<MovePool> mover_;  // page-locked pieces and the threads that fill or empty them, made at first use
+  void move_pieces(void* dst, const void* src, size_t bytes, cudaStream_t s, bool to_device);
 };
+
+// Is this host address page-locked (the copy engine can then read it without the driver's staging)?
+bool host_pinned(const void* p);
 
 // Device tensor handed across the ABI (CudaDeviceTensor).
 struct DeviceTensorHandle {

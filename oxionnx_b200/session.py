@@ -364,6 +364,61 @@ class SessionBuilder:
         return Session.from_model(Model.from_file(path), self._device, 1 if level is None else level, self._input_shapes, **self._ctx_kw)
 
 
+class _CallIo:
+    """The operand and result structures of a planned session's calls: names, shapes and extents are filled in once,
+    each call only sets the buffers' addresses (marshalling from scratch was 20 us of a small run)."""
+
+    def __init__(self, session):
+        self.lib = lib = _ffi.lib()
+        graph, planned = session.graph, session._planned_for
+        self.n_in, self.n_out = len(graph.input_names), len(graph.output_names)
+        self.feeds = (_ffi.RawOperand * max(self.n_in, 1))()
+        self.feeds_ptr = ctypes.cast(self.feeds, ctypes.POINTER(_ffi.Operand))
+        self.inputs = []
+        for op, name in zip(self.feeds, graph.input_names):
+            shape = planned[name]
+            op.name = name.encode()
+            op.shape = (ctypes.c_uint64 * max(len(shape), 1))(*shape)
+            op.rank, op.len = len(shape), int(np.prod(shape))
+            self.inputs.append((name, shape, op))
+        self.fetches = (_ffi.RawResult * max(self.n_out, 1))()
+        self.fetches_ptr = ctypes.cast(self.fetches, ctypes.POINTER(_ffi.Result))
+        self.outputs = []
+        for res, name in zip(self.fetches, graph.output_names):
+            r = _ffi.Result()
+            _raise_for(lib.oxb200_fetch_value(session.ctx.handle, name.encode(), ctypes.byref(r)), session.ctx.last_error())
+            shape = tuple(int(r.shape[d]) for d in range(r.rank))
+            res.cap = int(r.len)
+            self.outputs.append((name, shape, res))
+
+    def set_feeds(self, feeds):
+        """Points the operands at the feeds' lanes; the returned arrays must outlive the call."""
+        held = []
+        for name, shape, op in self.inputs:
+            if name not in feeds:
+                raise OnnxError(f"TensorNotFound: missing feed '{name}'")
+            a = feeds[name]
+            typed = _ffi.TYPED.get(a.dtype) if isinstance(a, np.ndarray) else None
+            a = np.ascontiguousarray(a if typed is not None else np.asarray(a, dtype=np.float32))
+            if a.shape != shape and not (shape == () and a.size == 1):
+                raise OnnxError(f"run: feed '{name}' has shape {a.shape}, the plan expects {shape}")
+            held.append(a)
+            if typed is None:
+                op.lanes, op.typed = a.ctypes.data, None
+            else:
+                op.lanes, op.typed, op.dtype = None, a.ctypes.data, typed
+        return held
+
+    def set_fetches(self):
+        """Points the results at fresh arrays, which the call fills."""
+        outs = {}
+        for name, shape, res in self.outputs:
+            a = np.empty(shape, np.float32)
+            res.lanes = a.ctypes.data
+            outs[name] = a
+        return outs
+
+
 class Session:
     """A graph planned once and run device-resident: every intermediate stays in HBM."""
 
@@ -378,7 +433,8 @@ class Session:
         self._input_shapes = dict(input_shapes)
         self._input_types = dict(input_types or {})  # name -> np.uint8 / np.int8 for inputs declared 8-bit
         self._planned_for = None
-        self._out_bufs = None
+        self._io = None
+        self._in_flight = []
 
     @classmethod
     def from_file(cls, path: str, device: int = 0, optimization_level: int = 1, input_shapes: Optional[Dict[str, tuple]] = None, **ctx_kw):
@@ -405,7 +461,8 @@ class Session:
                 self._input_shapes[name] = tuple(shape)
         self._input_types = {name: (np.uint8 if code == _ffi.DT_U8 else np.int8) for name, _, code in model.inputs() if code in (_ffi.DT_U8, _ffi.DT_I8)}
         self._planned_for = None
-        self._out_bufs = None
+        self._io = None
+        self._in_flight = []
         return self
 
     def _plan(self, shapes):
@@ -414,7 +471,7 @@ class Session:
             st, msg = plan_model(self.ctx, self._model, shapes)
             _raise_for(st, msg)
             self._planned_for = {k: tuple(v) for k, v in shapes.items()}
-            self._out_bufs = None
+            self._io = None
             return
         lib = _ffi.lib()
         keep = _ffi.Keep()
@@ -433,9 +490,17 @@ class Session:
                                      len(self.graph.output_names))
         _raise_for(st, self.ctx.last_error())
         self._planned_for = {k: tuple(v) for k, v in shapes.items()}
-        self._out_bufs = None
+        self._io = None
 
     def ensure_planned(self, feeds=None):
+        planned = self._planned_for
+        if planned is not None and feeds is not None:
+            for name, shape in planned.items():
+                v = feeds.get(name)
+                if not isinstance(v, np.ndarray) or v.shape != shape:
+                    break
+            else:
+                return
         shapes = dict(self._input_shapes)
         if feeds is not None:
             shapes.update({k: tuple(np.asarray(v).shape) for k, v in feeds.items()})
@@ -446,62 +511,45 @@ class Session:
         if self._planned_for != {k: tuple(shapes[k]) for k in self.graph.input_names}:
             self._plan({k: tuple(shapes[k]) for k in self.graph.input_names})
 
-    def _operands(self, feeds, keep):
-        ops = keep.add((_ffi.Operand * max(len(self.graph.input_names), 1))())
-        for i, name in enumerate(self.graph.input_names):
-            if name not in feeds:
-                raise OnnxError(f"TensorNotFound: missing feed '{name}'")
-            _ffi.pack_operand(ops[i], name, feeds[name], keep)
-        return ops
-
-    def _results(self, keep, probe=True):
-        lib = _ffi.lib()
-        n_out = len(self.graph.output_names)
-        res = keep.add((_ffi.Result * max(n_out, 1))())
-        if self._out_bufs is None:
-            # learn the output extents from the plan
-            self._out_bufs = []
-            for name in self.graph.output_names:
-                r = _ffi.Result()
-                st = lib.oxb200_fetch_value(self.ctx.handle, name.encode(), ctypes.byref(r))
-                _raise_for(st, self.ctx.last_error())
-                self._out_bufs.append(np.empty(max(int(r.len), 1), np.float32))
-        for i, b in enumerate(self._out_bufs):
-            res[i].lanes = b.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
-            res[i].cap = b.size
-        return res
+    # ---- marshalling of planned runs: the call structures are built once per plan, a run fills in addresses ----
+    def _call_io(self):
+        if self._io is None:
+            self._io = _CallIo(self)
+        return self._io
 
     def run(self, feeds: Dict[str, np.ndarray]) -> Dict[str, np.ndarray]:
         self.ensure_planned(feeds)
-        lib = _ffi.lib()
-        keep = _ffi.Keep()
-        ops = self._operands(feeds, keep)
-        res = self._results(keep)
-        st = lib.oxb200_run(self.ctx.handle, ops, len(self.graph.input_names), res, len(self.graph.output_names))
-        _raise_for(st, self.ctx.last_error())
-        return {name: _ffi.result_array(res[i], self._out_bufs[i]) for i, name in enumerate(self.graph.output_names)}
+        io = self._call_io()
+        held = io.set_feeds(feeds)
+        outs = io.set_fetches()
+        st = io.lib.oxb200_run(self.ctx.handle, io.feeds_ptr, io.n_in, io.fetches_ptr, io.n_out)
+        del held
+        if st:
+            _raise_for(st, self.ctx.last_error())
+        return outs
 
     # ---- pipelined runs: the upload of the next batch overlaps the run of the current one ----
     def submit(self, feeds: Dict[str, np.ndarray]):
         """Enqueues one run (upload, steps, download) and returns at once; at most two may be in flight.
         The feed arrays must stay unchanged until the matching collect()."""
         self.ensure_planned(feeds)
-        keep = _ffi.Keep()
-        ops = self._operands(feeds, keep)
-        _raise_for(_ffi.lib().oxb200_run_submit(self.ctx.handle, ops, len(self.graph.input_names)), self.ctx.last_error())
-        if not hasattr(self, "_in_flight"):
-            self._in_flight = []
-        self._in_flight.append(keep)
+        io = self._call_io()
+        held = io.set_feeds(feeds)
+        st = io.lib.oxb200_run_submit(self.ctx.handle, io.feeds_ptr, io.n_in)
+        if st:
+            _raise_for(st, self.ctx.last_error())
+        self._in_flight.append(held)
 
     def collect(self) -> Dict[str, np.ndarray]:
         """Waits for the oldest submitted run and returns its outputs."""
-        keep = _ffi.Keep()
-        res = self._results(keep)
-        st = _ffi.lib().oxb200_run_collect(self.ctx.handle, res, len(self.graph.output_names))
-        if getattr(self, "_in_flight", None):
+        io = self._call_io()
+        outs = io.set_fetches()
+        st = io.lib.oxb200_run_collect(self.ctx.handle, io.fetches_ptr, io.n_out)
+        if self._in_flight:
             self._in_flight.pop(0)
-        _raise_for(st, self.ctx.last_error())
-        return {name: _ffi.result_array(res[i], self._out_bufs[i]) for i, name in enumerate(self.graph.output_names)}
+        if st:
+            _raise_for(st, self.ctx.last_error())
+        return outs
 
     def run_pipelined(self, batches):
         """Runs a sequence of feed dictionaries with one batch in flight behind the one being awaited."""
@@ -521,11 +569,15 @@ class Session:
     def bind_input_device(self, name: str, device_ptr: int, dtype, count: int):
         """Graph input `name` is read from the caller's device buffer by the following runs."""
         code = _ffi.TYPED.get(np.dtype(dtype), _ffi.DT_F32)
-        _raise_for(_ffi.lib().oxb200_bind_input_device(self.ctx.handle, name.encode(), ctypes.c_void_p(device_ptr), code, count), self.ctx.last_error())
+        st = _ffi.lib().oxb200_bind_input_device(self.ctx.handle, name.encode(), device_ptr, code, count)
+        if st:
+            _raise_for(st, self.ctx.last_error())
 
     def bind_output_device(self, name: str, device_ptr: int, capacity: int):
         """Graph output `name` (f32 lanes, logical order) is also written to the caller's device buffer."""
-        _raise_for(_ffi.lib().oxb200_bind_output_device(self.ctx.handle, name.encode(), ctypes.c_void_p(device_ptr), capacity), self.ctx.last_error())
+        st = _ffi.lib().oxb200_bind_output_device(self.ctx.handle, name.encode(), device_ptr, capacity)
+        if st:
+            _raise_for(st, self.ctx.last_error())
 
     def output_device_ptr(self, name: str):
         """(device address, element count) of the library-owned buffer holding an output's f32 lanes after a run."""
@@ -536,6 +588,12 @@ class Session:
     def run_with_binding(self, feeds: Optional[Dict[str, np.ndarray]] = None, fetch: bool = True) -> Optional[Dict[str, np.ndarray]]:
         """One run with the current bindings: bound inputs are read on the device, unbound ones come from `feeds`;
         with fetch=False nothing is read back (the outputs stay in their device buffers)."""
+        lib = _ffi.lib()
+        if not feeds and not fetch:
+            st = lib.oxb200_run_bound(self.ctx.handle, None, 0, None, 0)
+            if st > _ffi.OK_DEVICE:
+                _raise_for(st, self.ctx.last_error())
+            return None
         feeds = feeds or {}
         keep = _ffi.Keep()
         names = [n for n in self.graph.input_names if n in feeds]
@@ -543,13 +601,12 @@ class Session:
         for i, name in enumerate(names):
             _ffi.pack_operand(ops[i], name, feeds[name], keep)
         if not fetch:
-            st = _ffi.lib().oxb200_run_bound(self.ctx.handle, ops, len(names), None, 0)
-            _raise_for(st, self.ctx.last_error())
+            _raise_for(lib.oxb200_run_bound(self.ctx.handle, ops, len(names), None, 0), self.ctx.last_error())
             return None
-        res = self._results(keep)
-        st = _ffi.lib().oxb200_run_bound(self.ctx.handle, ops, len(names), res, len(self.graph.output_names))
-        _raise_for(st, self.ctx.last_error())
-        return {name: _ffi.result_array(res[i], self._out_bufs[i]) for i, name in enumerate(self.graph.output_names)}
+        io = self._call_io()
+        outs = io.set_fetches()
+        _raise_for(lib.oxb200_run_bound(self.ctx.handle, ops, len(names), io.fetches_ptr, io.n_out), self.ctx.last_error())
+        return outs
 
     def clear_bindings(self):
         _raise_for(_ffi.lib().oxb200_clear_bindings(self.ctx.handle), self.ctx.last_error())
@@ -557,9 +614,10 @@ class Session:
     # ---- measurement helpers: the same run split into stage / resident launches / read ----
     def upload(self, feeds):
         self.ensure_planned(feeds)
-        keep = _ffi.Keep()
-        ops = self._operands(feeds, keep)
-        _raise_for(_ffi.lib().oxb200_upload_feeds(self.ctx.handle, ops, len(self.graph.input_names)), self.ctx.last_error())
+        io = self._call_io()
+        held = io.set_feeds(feeds)
+        _raise_for(io.lib.oxb200_upload_feeds(self.ctx.handle, io.feeds_ptr, io.n_in), self.ctx.last_error())
+        del held
 
     def run_resident(self, iters=1) -> float:
         ms = ctypes.c_float()
@@ -567,10 +625,10 @@ class Session:
         return float(ms.value)
 
     def download(self) -> Dict[str, np.ndarray]:
-        keep = _ffi.Keep()
-        res = self._results(keep)
-        _raise_for(_ffi.lib().oxb200_download_fetches(self.ctx.handle, res, len(self.graph.output_names)), self.ctx.last_error())
-        return {name: _ffi.result_array(res[i], self._out_bufs[i]) for i, name in enumerate(self.graph.output_names)}
+        io = self._call_io()
+        outs = io.set_fetches()
+        _raise_for(io.lib.oxb200_download_fetches(self.ctx.handle, io.fetches_ptr, io.n_out), self.ctx.last_error())
+        return outs
 
     def fetch_value(self, name: str) -> np.ndarray:
         """Any value of the planned graph after a run (keep_intermediates for intermediates)."""
