@@ -213,6 +213,18 @@ def pack_node(node, cnode, keep):
     cnode.attrs, cnode.n_attrs = arr, n
 
 
+def packed_node(node):
+    """(fields, CNode, buffers) of a node, kept on the node itself for as long as its fields stay what they were; hold the
+    tuple for as long as the CNode is used."""
+    now = (node.op, node.name, list(node.inputs), list(node.outputs), {k: list(v) if isinstance(v, (list, tuple)) else v for k, v in (node.attrs or {}).items()})
+    have = node.__dict__.get("_packed")
+    if have is None or any(isinstance(v, np.ndarray) for v in now[4].values()) or have[0] != now:
+        keep, cnode = Keep(), CNode()
+        pack_node(node, cnode, keep)
+        have = node.__dict__["_packed"] = (now, cnode, keep)
+    return have
+
+
 def pack_operand(op, name, array, keep, resident=None):
     op.name = name.encode()
     if resident is not None:

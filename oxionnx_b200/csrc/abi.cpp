@@ -72,6 +72,79 @@ NodeDef to_node(const oxb200_node* n) {
   return d;
 }
 
+// Operand slots whose host lanes a plan never looks at: they can be fed to a kept plan like a graph input.  The
+// integer contractions choose their storage from the lanes, so theirs are not among them.
+bool runtime_lanes(const std::string& op, uint32_t slot) {
+  static const char* unary[] = {"Relu",    "Tanh",    "Sigmoid", "PRelu",   "MaxPool", "GlobalAveragePool", "OxiInstanceNorm", "Resize", "Pad",
+                                "Softmax", "Gelu",    "Erf",     "Silu",    "SiLU",    "Transpose",         "Slice",           "Gemm",   "MatMul",
+                                "Conv",    "ConvAddRelu", "QuantizeLinear", "DequantizeLinear", "LayerNormalization", "LayerNorm"};
+  if (op == "Add" || op == "Sub" || op == "Mul" || op == "Div") return slot <= 1;
+  if (op == "ConvAddRelu" && slot == 3) return true;
+  if (slot != 0) return false;
+  for (const char* u : unary)
+    if (op == u) return true;
+  return false;
+}
+
+void key_bytes(std::string& k, const void* p, size_t n) { k.append((const char*)p, n); }
+template <typename T>
+void key_num(std::string& k, T v) { key_bytes(k, &v, sizeof v); }
+void key_str(std::string& k, const std::string& v) {
+  key_num(k, (uint32_t)v.size());
+  k += v;
+}
+
+// Everything a one-node plan depends on besides the registered weights; empty when some operand's contents are part
+// of the plan, or when the operands are so large that a plan which reads them where they lie is worth its making
+// (a kept plan copies a resident operand whose address a tensor map would hold).
+std::string dispatch_key(Context& C, const NodeDef& nd, const oxb200_operand* operands, uint32_t n, bool to_device) {
+  std::string k;
+  key_str(k, nd.op);
+  key_str(k, nd.name);
+  for (const auto& i : nd.inputs) key_str(k, i);
+  k += '|';
+  for (const auto& o : nd.outputs) key_str(k, o);
+  k += '|';
+  for (const auto& a : nd.attrs.ints) key_str(k, a.first), key_num(k, a.second);
+  k += '|';
+  for (const auto& a : nd.attrs.floats) key_str(k, a.first), key_num(k, a.second);
+  k += '|';
+  for (const auto& a : nd.attrs.strings) key_str(k, a.first), key_str(k, a.second);
+  k += '|';
+  for (const auto& a : nd.attrs.int_lists) key_str(k, a.first), key_num(k, a.second.size()), key_bytes(k, a.second.data(), a.second.size() * sizeof(int64_t));
+  k += '|';
+  for (const auto& a : nd.attrs.float_lists) key_str(k, a.first), key_num(k, a.second.size()), key_bytes(k, a.second.data(), a.second.size() * sizeof(float));
+  k += to_device ? 'D' : 'H';
+  uint64_t elements = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const oxb200_operand& o = operands[i];
+    if (nd.inputs[i].empty()) {
+      k += '-';
+    } else if (o.resident) {
+      k += 'R';
+      key_num(k, (int)o.resident->h.dt), key_num(k, (int)o.resident->h.layout), key_num(k, o.resident->h.shape.size());
+      key_bytes(k, o.resident->h.shape.data(), o.resident->h.shape.size() * sizeof(int64_t));
+      elements += (uint64_t)prod(o.resident->h.shape);
+    } else if (C.weight(nd.inputs[i])) {
+      if (o.typed || (o.lanes && C.weight(nd.inputs[i])->data.size() != o.len)) return std::string();
+      k += 'W';
+    } else if (o.lanes && runtime_lanes(nd.op, i)) {
+      uint64_t count = 1;
+      for (uint32_t d = 0; d < o.rank; ++d) count *= o.shape[d];
+      if (count != o.len) return std::string();
+      for (uint32_t j = 0; j < i; ++j)
+        if (nd.inputs[j] == nd.inputs[i]) return std::string();
+      k += 'L';
+      key_num(k, o.rank);
+      key_bytes(k, o.shape, o.rank * sizeof(uint64_t));
+      elements += o.len;
+    } else {
+      return std::string();
+    }
+  }
+  return elements <= (8u << 20) ? k : std::string();
+}
+
 }  // namespace
 
 extern "C" {
@@ -278,10 +351,18 @@ void oxb200_tensor_release(oxb200_ctx* ctx, oxb200_tensor* t) {
   if (ctx) {
     std::lock_guard<std::mutex> lock(ctx->impl.mu);
     cudaSetDevice(ctx->impl.device());
-    cudaStreamSynchronize(ctx->impl.stream());
+    // an allocation shared with aliases (oxb200_tensor_alias) lives until its last handle is released
+    if (t->h.ptr && t->h.owners.use_count() == 1) {
+      if (t->h.home == &ctx->impl) {
+        ctx->impl.give_block(t->h.ptr, t->h.bytes);
+      } else {
+        cudaStreamSynchronize(ctx->impl.stream());
+        cudaFree(t->h.ptr);
+      }
+    }
+  } else if (t->h.ptr && t->h.owners.use_count() == 1) {
+    cudaFree(t->h.ptr);
   }
-  // an allocation shared with aliases (oxb200_tensor_alias) lives until its last handle is released
-  if (t->h.ptr && t->h.owners.use_count() == 1) cudaFree(t->h.ptr);
   delete t;
 }
 
@@ -341,6 +422,91 @@ int oxb200_dispatch(oxb200_ctx* ctx, const oxb200_node* node, const oxb200_opera
     if (!is_supported_op(nd.op)) raise(OXB200_DECLINED, "operator '%s' is not claimed by this provider", nd.op.c_str());
     if (n_operands != nd.inputs.size()) raise(OXB200_FAILED, "dispatch: %u operands for %zu node inputs", n_operands, nd.inputs.size());
     if (n_results != nd.outputs.size()) raise(OXB200_FAILED, "dispatch: %u result slots for %zu node outputs", n_results, nd.outputs.size());
+    const bool to_device = want_placement == OXB200_PLACE_DEVICE && nd.outputs.size() == 1 && C.cfg().residency != 0;
+    // The device result of a run of `sess`, in a block of the context's pool.
+    auto device_result = [&](Session& sess) {
+      Value* v = sess.find_value(nd.outputs[0]);
+      if (!v || !v->ptr) raise(OXB200_FAILED, "dispatch: output '%s' was not produced", nd.outputs[0].c_str());
+      auto t = std::make_unique<oxb200_tensor>();
+      t->h.home = &C;
+      t->h.dt = v->dt;
+      t->h.layout = v->shape.size() == 4 ? v->layout : Layout::PLAIN;
+      t->h.shape = v->shape;
+      t->h.ptr = C.take_block(v->bytes, &t->h.bytes);
+      try {
+        if (v->bytes) OXB_CUDA(cudaMemcpyAsync(t->h.ptr, v->ptr, v->bytes, cudaMemcpyDeviceToDevice, C.stream()));
+        sess.sync();
+        const int flag = sess.check_error_flag();
+        if (flag) raise(OXB200_FAILED, flag == 20 ? "Gather: an index is out of range (device code %d)" : "a tensor-core kernel gave up on a bounded wait (code %d)", flag);
+      } catch (...) {
+        C.give_block(t->h.ptr, t->h.bytes);
+        throw;
+      }
+      results[0].rank = (uint32_t)v->shape.size();
+      for (size_t d = 0; d < v->shape.size() && d < OXB200_MAX_RANK; ++d) results[0].shape[d] = (uint64_t)v->shape[d];
+      results[0].len = (uint64_t)v->numel();
+      results[0].resident = t.release();
+      return (int)OXB200_OK_DEVICE;
+    };
+    // Host results, positionally aligned with node outputs (elided outputs keep len 0).
+    auto host_results = [&](Session& sess) {
+      std::vector<oxb200_result> fetch;
+      std::vector<uint32_t> slot_of;
+      for (uint32_t i = 0; i < nd.outputs.size(); ++i)
+        if (!nd.outputs[i].empty()) {
+          slot_of.push_back(i);
+          fetch.push_back(results[i]);
+        }
+      sess.download_async(fetch.data(), (uint32_t)fetch.size());
+      sess.finish_download();
+      for (size_t j = 0; j < fetch.size(); ++j) {
+        results[slot_of[j]] = fetch[j];
+        results[slot_of[j]].resident = nullptr;
+      }
+      return (int)OXB200_OK_HOST;
+    };
+    // A host engine dispatches the same nodes over and over: the plan of a node whose operands are registered
+    // weights, resident tensors or plain data lanes is kept (planning anew was 100 us and more per call).
+    const std::string key = dispatch_key(C, nd, operands, n_operands, to_device);
+    if (!key.empty()) {
+      Session* kept = C.find_dispatch_plan(key);
+      std::unique_ptr<Session> fresh;
+      if (!kept) {
+        fresh = std::make_unique<Session>(&C);
+        std::vector<std::pair<std::string, std::vector<int64_t>>> in;
+        for (uint32_t i = 0; i < n_operands; ++i) {
+          const oxb200_operand& o = operands[i];
+          if (nd.inputs[i].empty()) continue;
+          bool known = false;
+          for (const auto& have : in) known = known || have.first == nd.inputs[i];
+          if (o.resident) {
+            if (!accepts_resident_slot(nd.op, i)) raise(OXB200_DECLINED, "%s: operand %u cannot be bound from the device", nd.op.c_str(), i);
+            if (known) continue;
+            in.push_back({nd.inputs[i], o.resident->h.shape});
+            fresh->bind_external(nd.inputs[i], nullptr, o.resident->h.dt, o.resident->h.layout);
+          } else if (!C.weight(nd.inputs[i])) {
+            in.push_back({nd.inputs[i], std::vector<int64_t>(o.shape, o.shape + o.rank)});
+          }
+        }
+        std::vector<std::string> outs;
+        if (!to_device)
+          for (auto& o : nd.outputs)
+            if (!o.empty()) outs.push_back(o);
+        std::map<std::string, const HostTensor*> none;
+        fresh->plan({nd}, in, none, outs);
+        kept = C.keep_dispatch_plan(key, fresh);
+      }
+      Session& sess = kept ? *kept : *fresh;
+      sess.begin_copies();
+      for (uint32_t i = 0; i < n_operands; ++i) {
+        if (nd.inputs[i].empty()) continue;
+        if (operands[i].resident) sess.use_resident(nd.inputs[i], operands[i].resident->h.ptr);
+        else if (!C.weight(nd.inputs[i])) sess.use_host(nd.inputs[i], operands[i].lanes);
+      }
+      sess.run_steps(false);
+      if (to_device) return device_result(sess);
+      return host_results(sess);
+    }
     // operands: registered weights by name, host lanes as plan-time constants, resident tensors as bound inputs
     std::vector<HostTensor> temps;
     temps.reserve(n_operands);
@@ -387,7 +553,6 @@ int oxb200_dispatch(oxb200_ctx* ctx, const oxb200_node* node, const oxb200_opera
       vconsts[nm] = &temps.back();
     }
     std::vector<std::string> outs;
-    const bool to_device = want_placement == OXB200_PLACE_DEVICE && nd.outputs.size() == 1 && C.cfg().residency != 0;
     if (!to_device)
       for (auto& o : nd.outputs)
         if (!o.empty()) outs.push_back(o);
@@ -398,41 +563,8 @@ int oxb200_dispatch(oxb200_ctx* ctx, const oxb200_node* node, const oxb200_opera
     } cleanup{C};
     sess.plan(nodes, inputs, vconsts, outs);
     sess.run_steps(false);
-    if (to_device) {
-      Value* v = sess.find_value(nd.outputs[0]);
-      if (!v || !v->ptr) raise(OXB200_FAILED, "dispatch: output '%s' was not produced", nd.outputs[0].c_str());
-      auto* t = new oxb200_tensor();
-      t->h.bytes = std::max<size_t>(v->bytes, 256);
-      t->h.dt = v->dt;
-      t->h.layout = v->shape.size() == 4 ? v->layout : Layout::PLAIN;
-      t->h.shape = v->shape;
-      t->h.ptr = C.alloc_device(t->h.bytes);
-      if (v->bytes) OXB_CUDA(cudaMemcpyAsync(t->h.ptr, v->ptr, v->bytes, cudaMemcpyDeviceToDevice, C.stream()));
-      sess.sync();
-      int flag = sess.check_error_flag();
-      if (flag) {
-        cudaFree(t->h.ptr);
-        delete t;
-        raise(OXB200_FAILED, flag == 20 ? "Gather: an index is out of range (device code %d)" : "a tensor-core kernel gave up on a bounded wait (code %d)", flag);
-      }
-      results[0].resident = t;
-      results[0].rank = (uint32_t)v->shape.size();
-      for (size_t d = 0; d < v->shape.size() && d < OXB200_MAX_RANK; ++d) results[0].shape[d] = (uint64_t)v->shape[d];
-      results[0].len = (uint64_t)v->numel();
-      return (int)OXB200_OK_DEVICE;
-    }
-    // host results, positionally aligned with node outputs (elided outputs keep len 0)
-    std::vector<oxb200_result> fetch(outs.size());
-    std::vector<uint32_t> slot_of;
-    for (uint32_t i = 0; i < nd.outputs.size(); ++i)
-      if (!nd.outputs[i].empty()) slot_of.push_back(i);
-    for (size_t j = 0; j < outs.size(); ++j) fetch[j] = results[slot_of[j]];
-    sess.download(fetch.data(), (uint32_t)fetch.size());
-    for (size_t j = 0; j < outs.size(); ++j) {
-      results[slot_of[j]] = fetch[j];
-      results[slot_of[j]].resident = nullptr;
-    }
-    return (int)OXB200_OK_HOST;
+    if (to_device) return device_result(sess);
+    return host_results(sess);
   });
 }
 

@@ -563,10 +563,10 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
     if (vc != vconsts_.end()) V(vi).host = vc->second;
     auto eb = S.external_bind_.find(in.first);
     if (eb != S.external_bind_.end()) {
-      V(vi).ptr = eb->second.first;
       V(vi).dt = eb->second.second.first;
       V(vi).layout = eb->second.second.second;
       V(vi).bytes = (size_t)V(vi).numel() * dt_size(V(vi).dt);
+      V(vi).ptr = eb->second.first ? eb->second.first : owned_buffer(std::max<size_t>(V(vi).bytes, 256));
     } else {
       V(vi).ptr = owned_buffer(std::max<size_t>(V(vi).bytes, 256));
     }

@@ -58,6 +58,7 @@ void Context::register_weight(const std::string& name, const float* lanes, uint6
   if ((uint64_t)prod(t.shape) != len) raise(OXB200_FAILED, "weight '%s': %llu lanes do not match its shape", name.c_str(), (unsigned long long)len);
   t.data.assign(lanes, lanes + len);
   weights_[name] = std::move(t);
+  drop_dispatch_plans();
   // a re-registered weight invalidates its packed forms
   for (auto it = forms_.begin(); it != forms_.end();) {
     if (it->first.first == name) {
@@ -126,7 +127,70 @@ uint64_t Context::cached_bytes() const {
   return total;
 }
 
+constexpr size_t kDispatchPlans = 16, kDispatchPlanBytes = 256ull << 20;
+
+Session* Context::find_dispatch_plan(const std::string& key) {
+  for (DispatchEntry& e : dispatch_plans_)
+    if (e.key == key) {
+      e.used = ++dispatch_clock_;
+      return e.plan.get();
+    }
+  return nullptr;
+}
+
+Session* Context::keep_dispatch_plan(const std::string& key, std::unique_ptr<Session>& plan) {
+  const size_t bytes = plan->device_bytes();
+  if (bytes > kDispatchPlanBytes / 4) return nullptr;
+  while (!dispatch_plans_.empty()) {
+    size_t total = bytes, oldest = 0;
+    for (size_t i = 0; i < dispatch_plans_.size(); ++i) {
+      total += dispatch_plans_[i].bytes;
+      if (dispatch_plans_[i].used < dispatch_plans_[oldest].used) oldest = i;
+    }
+    if (total <= kDispatchPlanBytes && dispatch_plans_.size() < kDispatchPlans) break;
+    dispatch_plans_.erase(dispatch_plans_.begin() + oldest);
+  }
+  DispatchEntry e;
+  e.key = key, e.bytes = bytes, e.used = ++dispatch_clock_;
+  e.plan = std::move(plan);
+  dispatch_plans_.push_back(std::move(e));
+  return dispatch_plans_.back().plan.get();
+}
+
+void Context::drop_dispatch_plans() { dispatch_plans_.clear(); }
+
+constexpr size_t kFreeBlocks = 64, kFreeBlockBytes = 256ull << 20;
+
+void* Context::take_block(size_t bytes, size_t* got) {
+  bytes = align_up(std::max<size_t>(bytes, 256), 256);
+  size_t best = free_blocks_.size();
+  for (size_t i = 0; i < free_blocks_.size(); ++i)
+    if (free_blocks_[i].bytes >= bytes && free_blocks_[i].bytes <= bytes + bytes / 4 && (best == free_blocks_.size() || free_blocks_[i].bytes < free_blocks_[best].bytes)) best = i;
+  if (best < free_blocks_.size()) {
+    const Block b = free_blocks_[best];
+    free_blocks_.erase(free_blocks_.begin() + best);
+    free_block_bytes_ -= b.bytes;
+    *got = b.bytes;
+    return b.ptr;
+  }
+  *got = bytes;
+  return alloc_device(bytes);
+}
+
+void Context::give_block(void* ptr, size_t bytes) {
+  if (free_blocks_.size() >= kFreeBlocks || free_block_bytes_ + bytes > kFreeBlockBytes) {
+    cudaFree(ptr);  // waits for whatever still uses it
+    return;
+  }
+  free_blocks_.push_back(Block{ptr, bytes});
+  free_block_bytes_ += bytes;
+}
+
 void Context::release_caches() {
+  drop_dispatch_plans();
+  for (const Block& b : free_blocks_) cudaFree(b.ptr);
+  free_blocks_.clear();
+  free_block_bytes_ = 0;
   for (auto& kv : forms_) cudaFree(kv.second.ptr);
   forms_.clear();
   for (void* p : temp_forms_) cudaFree(p);
@@ -744,6 +808,33 @@ void Session::collect(oxb200_result* fetches, uint32_t n) {
 }
 
 void Session::bind_external(const std::string& name, void* ptr, DT dt, Layout layout) { external_bind_[name] = {ptr, {dt, layout}}; }
+
+void Session::use_resident(const std::string& name, const void* ptr) {
+  if (in_tensor_map_.empty())
+    for (auto& in : input_staging_) in_tensor_map_.push_back(input_in_tensor_map(in.second) ? 1 : 0);
+  for (size_t i = 0; i < input_staging_.size(); ++i) {
+    if (input_staging_[i].first != name) continue;
+    Value& v = values_[input_staging_[i].second];
+    if (in_tensor_map_[i]) OXB_CUDA(cudaMemcpyAsync(v.ptr, ptr, v.bytes, cudaMemcpyDeviceToDevice, ctx_->stream()));
+    else rebind_input(input_staging_[i].second, const_cast<void*>(ptr));
+  }
+}
+
+void Session::use_host(const std::string& name, const void* lanes) {
+  for (auto& in : input_staging_) {
+    if (in.first != name) continue;
+    const size_t bytes = (size_t)values_[in.second].numel() * 4;
+    stage_in(values_[in.second].ptr, lanes, bytes);
+    ctx_->counters.uploads += 1;
+    ctx_->counters.upload_bytes += bytes;
+  }
+}
+
+size_t Session::device_bytes() const {
+  size_t n = arena_.bytes;
+  for (const DeviceBuffer& b : owned_) n += b.bytes;
+  return n;
+}
 
 // ---- device I/O binding -------------------------------------------------------------------------
 bool Session::input_in_tensor_map(int value_index) const {

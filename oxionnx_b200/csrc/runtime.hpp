@@ -133,7 +133,8 @@ class Session {
   const std::vector<std::string>& output_names() const { return outputs_; }
   size_t arena_bytes() const { return arena_.bytes; }
   size_t arena_slots() const { return n_slots_; }
-  // Bind a graph input to storage that already lives on the device (resident dispatch operand).
+  // Bind a graph input to storage that already lives on the device (resident dispatch operand).  With a null `ptr` the
+  // storage's type and order are fixed now and its address is given per run (use_resident).
   void bind_external(const std::string& name, void* ptr, DT dt, Layout layout);
   // Declared element type of a graph input (before plan()): 8-bit inputs are stored and fed as 8-bit lanes.
   void declare_input_type(const std::string& name, DT dt) { input_types_[name] = dt; }
@@ -145,6 +146,11 @@ class Session {
   // run_with_binding: uploads the unbound inputs, runs, copies bound outputs device-to-device, downloads the
   // fetches that have host lanes; one fence
   void run_bound(const oxb200_operand* feeds, uint32_t n, oxb200_result* fetches, uint32_t nf, bool profile);
+  // One node's plan kept by the context (oxb200_dispatch): operands of the next run, then run_steps.
+  void use_resident(const std::string& name, const void* ptr);  // read in place, or copied when a tensor map holds the input's address
+  void use_host(const std::string& name, const void* lanes);
+  size_t device_bytes() const;
+  void begin_copies();
   // After a run, detach the storage of an output so it can outlive the session.
   Value* find_value(const std::string& name);
   int check_error_flag();
@@ -190,7 +196,6 @@ class Session {
     size_t bytes;
   };
   std::vector<PendingCopy> pending_out_;  // fetches that wait in the staging memory for the run's fence
-  void begin_copies();
   void* small_stage(size_t bytes);
   void stage_in(void* dst, const void* src, size_t bytes);
   void stage_out(void* dst, const void* src, size_t bytes);
@@ -231,6 +236,13 @@ class Session {
 
 struct MovePool;
 
+struct DispatchEntry {
+  std::string key;
+  std::unique_ptr<Session> plan;
+  size_t bytes = 0;
+  uint64_t used = 0;
+};
+
 class Context {
  public:
   Context(int device, const oxb200_config& cfg);
@@ -260,6 +272,16 @@ class Context {
   // One word of page-locked memory that kernels may write and the host reads after a fence; nullptr-safe to give back.
   int* take_error_word();
   void give_error_word(int* word);
+  // Plans of single-node dispatches, by everything the plan depends on; at most 16 plans and 256 MB of device memory,
+  // the least recently used goes first.  Registering a weight or releasing the caches drops them all.
+  Session* find_dispatch_plan(const std::string& key);
+  Session* keep_dispatch_plan(const std::string& key, std::unique_ptr<Session>& plan);  // null (and `plan` kept) when it is too large
+  void drop_dispatch_plans();
+  // Storage of device tensors: released blocks wait for the next tensor of about their size (at most 64 blocks and
+  // 256 MB).  Everything rides this context's stream, so reuse needs no fence.
+  void* take_block(size_t bytes, size_t* got);
+  void give_block(void* ptr, size_t bytes);
+
   // Large pageable host buffers: copied in pieces through page-locked buffers by a few host threads, so that the
   // host copy of one piece runs beside the PCIe transfer of another (host_to_device only enqueues the last
   // transfers; device_to_host returns when every lane has arrived).
@@ -284,6 +306,14 @@ class Context {
   int* error_words_ = nullptr;  // kErrorWords words, 64 bytes apart
   std::vector<int*> free_error_words_;
   std::shared_ptr<MovePool> mover_;  // page-locked pieces and the threads that fill or empty them, made at first use
+  std::vector<DispatchEntry> dispatch_plans_;
+  uint64_t dispatch_clock_ = 0;
+  struct Block {
+    void* ptr;
+    size_t bytes;
+  };
+  std::vector<Block> free_blocks_;
+  size_t free_block_bytes_ = 0;
   void move_pieces(void* dst, const void* src, size_t bytes, cudaStream_t s, bool to_device);
 };
 
@@ -294,6 +324,7 @@ bool host_pinned(const void* p);
 struct DeviceTensorHandle {
   // handles that alias one allocation share this count; the last one released frees the memory
   std::shared_ptr<int> owners = std::make_shared<int>(0);
+  Context* home = nullptr;  // the context whose pool the allocation came from
   void* ptr = nullptr;
   size_t bytes = 0;
   DT dt = DT::F32;

@@ -14,6 +14,7 @@ Errors keep the reference's three-way meaning: `Declined` (Ok(None): let the nex
 try), `OnnxError` (Err: log and fall back) and `VerifyMismatch` (proved wrong: fail the run).
 """
 import ctypes
+import threading
 from dataclasses import dataclass
 from typing import Dict, List, Optional
 
@@ -226,6 +227,20 @@ class CudaContext:
         _raise_for(st, self.last_error())
 
 
+_scratch_bufs = threading.local()
+
+
+def _scratch(slot, lanes):
+    """Host lanes that a dispatch writes and its caller copies out at once: kept per thread up to 16 MB a slot, because
+    the pages of a fresh buffer cost more than the copy."""
+    if lanes > 1 << 22 or slot >= 4:
+        return np.empty(lanes, np.float32)
+    bufs = _scratch_bufs.__dict__.setdefault("bufs", {})
+    if slot not in bufs or bufs[slot].size < lanes:
+        bufs[slot] = np.empty(lanes, np.float32)
+    return bufs[slot]
+
+
 def try_cuda_dispatch_resident(node: Node, weights: Dict[str, np.ndarray], intermediates: Dict[str, object], placement: str,
                                ctx: CudaContext):
     """One node through the provider.  `intermediates` maps names to numpy arrays (host) or
@@ -233,8 +248,8 @@ def try_cuda_dispatch_resident(node: Node, weights: Dict[str, np.ndarray], inter
     (placement "device"), or None when the provider declines."""
     lib = _ffi.lib()
     keep = _ffi.Keep()
-    cnode = _ffi.CNode()
-    _ffi.pack_node(node, cnode, keep)
+    packed = _ffi.packed_node(node)
+    cnode = packed[1]
     n_in = len(node.inputs)
     ops = keep.add((_ffi.Operand * max(n_in, 1))())
     for i, name in enumerate(node.inputs):
@@ -262,7 +277,7 @@ def try_cuda_dispatch_resident(node: Node, weights: Dict[str, np.ndarray], inter
     guess = max([int(np.asarray(v).size) for v in intermediates.values() if isinstance(v, np.ndarray)] + [1])
     guess = min(max(guess * 64, 1 << 16, cap), 1 << 26)
     for i in range(n_out):
-        b = np.empty(guess, np.float32)
+        b = _scratch(i, guess)
         bufs.append(b)
         res[i].lanes = b.ctypes.data_as(ctypes.POINTER(ctypes.c_float))
         res[i].cap = b.size
