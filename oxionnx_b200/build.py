@@ -26,6 +26,8 @@ SOURCES = {
     "umma_i8.cu": [f for f in COMMON if f != "--fmad=false"],
     "umma_tf32.cu": [f for f in COMMON if f != "--fmad=false"],
     "umma_f16.cu": [f for f in COMMON if f != "--fmad=false"],
+    "umma_small_i8.cu": [f for f in COMMON if f != "--fmad=false"],
+    "umma_small_float.cu": [f for f in COMMON if f != "--fmad=false"],
     "umma_probe.cu": [f for f in COMMON if f != "--fmad=false"],
     "umma_chain.cu": [f for f in COMMON if f != "--fmad=false"],
     "umma_attention.cu": [f for f in COMMON if f != "--fmad=false"],
@@ -35,7 +37,7 @@ SOURCES = {
     "onnx_model.cpp": COMMON,
     "model_abi.cpp": COMMON,
 }
-HEADERS = ["common.hpp", "kernels.hpp", "runtime.hpp", "umma_kernel.cuh", "umma_launch.cuh", "umma_chain.cuh", "model.hpp", "abi_internal.hpp", os.path.join("..", "..", "include", "oxb200.h")]
+HEADERS = ["common.hpp", "kernels.hpp", "runtime.hpp", "umma_kernel.cuh", "umma_launch.cuh", "umma_small.cuh", "pdl.cuh", "umma_chain.cuh", "model.hpp", "abi_internal.hpp", os.path.join("..", "..", "include", "oxb200.h")]
 
 
 def _nvcc():

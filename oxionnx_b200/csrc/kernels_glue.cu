@@ -11,6 +11,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 
 namespace oxb {
 namespace k {
@@ -96,6 +97,7 @@ __device__ __forceinline__ float round_tf32(float v) {
 
 // ---------------------------------------------------------------------------------------
 __global__ void convert_kernel(const void* src, DT sdt, Layout sl, void* dst, DT ddt, Layout dl, Dims4 d, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t si = o;
     if (sl != dl) si = encode(decode(o, dl, d), sl, d);
@@ -109,6 +111,7 @@ __global__ void convert_kernel(const void* src, DT sdt, Layout sl, void* dst, DT
 // View: [outer, A, B] -> [outer, B, A]; 32x32 tiles.
 template <typename TS, typename TD>
 __global__ void transpose_tiles(const TS* __restrict__ src, TD* __restrict__ dst, int64_t A, int64_t B) {
+  pdl_enter();
   __shared__ float tile[32][33];
   int64_t outer = blockIdx.z;
   int64_t a0 = (int64_t)blockIdx.y * 32, b0 = (int64_t)blockIdx.x * 32;
@@ -128,6 +131,7 @@ __global__ void transpose_tiles(const TS* __restrict__ src, TD* __restrict__ dst
 // ---------------------------------------------------------------------------------------
 __global__ void quantize_kernel(const void* x, DT xdt, Layout xl, void* y, DT ydt, Layout yl, Dims4 d, const float* scale, int64_t ns,
                                 const float* zp, int64_t nz, float lo, float hi, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(o, yl, d);
     int64_t xi = xl == yl ? o : encode(q, xl, d);
@@ -144,6 +148,7 @@ __global__ void quantize_kernel(const void* x, DT xdt, Layout xl, void* y, DT yd
 // four 16-byte loads and one 16-byte store.
 __global__ void quantize_vec16_kernel(const float4* __restrict__ x, uint4* __restrict__ y, float scale, float zp, float lo, float hi,
                                       int64_t n16) {
+  pdl_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x) {
     uint32_t packed[4];
 #pragma unroll
@@ -165,6 +170,7 @@ __global__ void quantize_vec16_kernel(const float4* __restrict__ x, uint4* __res
 
 __global__ void dequantize_kernel(const void* x, DT xdt, Layout xl, void* y, Layout yl, Dims4 d, const float* scale, int64_t ns,
                                   const float* zp, int64_t nz, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(o, yl, d);
     int64_t xi = xl == yl ? o : encode(q, xl, d);
@@ -180,6 +186,7 @@ __global__ void dequantize_kernel(const void* x, DT xdt, Layout xl, void* y, Lay
 // without the conversion pipe); (v - zp) * scale is rounded as in the generic kernel.
 __global__ void dequantize_vec4_kernel(const uint32_t* __restrict__ x, bool is_signed, float4* __restrict__ y, const float* __restrict__ scale,
                                        const float* __restrict__ zp, int64_t n4) {
+  pdl_enter();
   const float s = scale[0], z = zp ? zp[0] : 0.f;
   const uint32_t flip = is_signed ? 0x80808080u : 0u;
   const float off = is_signed ? 8388736.0f : 8388608.0f;  // 2^23 (+ 128 for the flipped sign bit)
@@ -208,12 +215,14 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 __global__ void minmax_init_kernel(uint32_t* keys) {
+  pdl_enter();
   keys[0] = 0xffffffffu;  // running min key
   keys[1] = 0u;           // running max key
 }
 
 // `vec` = 0: x is not 16-byte aligned, every lane goes through the scalar loop.
 __global__ void minmax_kernel(const float* __restrict__ x, int64_t n, uint32_t* keys, int vec) {
+  pdl_enter();
   float mn = INFINITY, mx = -INFINITY;
   int64_t n4 = vec ? n / 4 : 0;
   const float4* x4 = (const float4*)x;
@@ -253,6 +262,7 @@ __global__ void minmax_kernel(const float* __restrict__ x, int64_t n, uint32_t* 
 
 // params[0] = y_scale, params[1] = y_zero_point
 __global__ void dynq_params_kernel(const uint32_t* keys, float* params) {
+  pdl_enter();
   float max_x = fmaxf(key_float(keys[1]), 0.f);
   float min_x = fminf(key_float(keys[0]), 0.f);
   float span = (max_x == min_x) ? 1.0f : __fsub_rn(max_x, min_x);
@@ -264,6 +274,7 @@ __global__ void dynq_params_kernel(const uint32_t* keys, float* params) {
 }
 
 __global__ void dynq_apply_kernel(const float* __restrict__ x, uint8_t* __restrict__ y, const float* params, int64_t n) {
+  pdl_enter();
   float s = params[0], z = params[1];
   int64_t n4 = n / 4;  // the entry point that launches this kernel has checked the alignment of x (16) and y (4)
   const float4* x4 = (const float4*)x;
@@ -291,6 +302,7 @@ __global__ void dynq_apply_kernel(const float* __restrict__ x, uint8_t* __restri
 // consumers, and the last block to finish puts the keys back to their identity values for the next call: two
 // launches per DynamicQuantizeLinear instead of four.  keys[2] is the arrival counter.
 __global__ void dynq_apply_fused_kernel(const float* __restrict__ x, uint8_t* __restrict__ y, uint32_t* keys, float* params, int64_t n, int vec) {
+  pdl_enter();
   const float max_x = fmaxf(key_float(keys[1]), 0.f);
   const float min_x = fminf(key_float(keys[0]), 0.f);
   const float span = (max_x == min_x) ? 1.0f : __fsub_rn(max_x, min_x);
@@ -333,6 +345,7 @@ __global__ void dynq_apply_fused_kernel(const float* __restrict__ x, uint8_t* __
 // ---- DynamicQuantizeLinear, session path: wide passes ---------------------------------------------------
 // First pass: four independent 16-byte loads per thread and iteration, one pair of atomics per block.
 __global__ void __launch_bounds__(kThreads) minmax_wide_kernel(const float* __restrict__ x, int64_t n, uint32_t* keys) {
+  pdl_enter();
   float mn = INFINITY, mx = -INFINITY;
   const int64_t n4 = n / 4;
   const float4* x4 = (const float4*)x;
@@ -408,6 +421,7 @@ __device__ __forceinline__ uint32_t dynq_byte(float x, float s, float r, float z
 // consecutive lanes per iteration: four coalesced 16-byte loads and four coalesced 4-byte stores per thread.
 __global__ void __launch_bounds__(kThreads) dynq_apply_wide_kernel(const float* __restrict__ x, uint8_t* __restrict__ y, uint32_t* keys, float* params,
                                                                    int64_t n) {
+  pdl_enter();
   const float max_x = fmaxf(key_float(keys[1]), 0.f);
   const float min_x = fminf(key_float(keys[0]), 0.f);
   const float span = (max_x == min_x) ? 1.0f : __fsub_rn(max_x, min_x);
@@ -464,6 +478,7 @@ __device__ __forceinline__ float apply_bin(int op, float a, float b) {
 
 __global__ void binary_kernel(const void* a, DT adt, Layout al, Dims4 ad, const void* b, DT bdt, Layout bl, Dims4 bd, void* out, DT odt,
                               Layout ol, Dims4 od, int op, int relu_after, int rtf32, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(o, ol, od);
     float av = load_as_f32(a, adt, encode_bcast(q, al, ad));
@@ -478,6 +493,7 @@ __global__ void binary_kernel(const void* a, DT adt, Layout al, Dims4 ad, const 
 // Same shape, same order, f32: four elements per thread with 16-byte accesses.
 __global__ void binary_vec4_kernel(const float4* __restrict__ a, const float4* __restrict__ b, float4* __restrict__ out, int op,
                                    int relu_after, int rtf32, int64_t n4) {
+  pdl_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
     float4 x = a[i], y = b[i];
     float r[4] = {apply_bin(op, x.x, y.x), apply_bin(op, x.y, y.y), apply_bin(op, x.z, y.z), apply_bin(op, x.w, y.w)};
@@ -494,6 +510,7 @@ __global__ void binary_vec4_kernel(const float4* __restrict__ a, const float4* _
 // sample), f32 in the logical order; 16-byte accesses, 32-bit index arithmetic.
 __global__ void binary_suffix_vec4_kernel(const float4* __restrict__ a, const float4* __restrict__ b, float4* __restrict__ out, int op, int relu_after,
                                           int rtf32, uint32_t n4, uint32_t nb4) {
+  pdl_enter();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
     const float4 x = a[i], y = __ldg(b + i % nb4);
     float r[4] = {apply_bin(op, x.x, y.x), apply_bin(op, x.y, y.y), apply_bin(op, x.z, y.z), apply_bin(op, x.w, y.w)};
@@ -520,6 +537,7 @@ __device__ __forceinline__ float erf_poly(float x) {
 }
 
 __global__ void unary_kernel(const void* x, DT xdt, void* y, DT ydt, int op, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     float v = load_as_f32(x, xdt, o);
     float r;
@@ -542,6 +560,7 @@ __global__ void unary_kernel(const void* x, DT xdt, void* y, DT ydt, int op, int
 }
 
 __global__ void prelu_kernel(const float* x, Layout xl, float* y, Dims4 d, const float* slope, int64_t ns, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(o, xl, d);
     float v = x[o];
@@ -553,6 +572,7 @@ __global__ void prelu_kernel(const float* x, Layout xl, float* y, Dims4 d, const
 // ---- pooling ----------------------------------------------------------------------------
 template <typename T>
 __global__ void max_pool_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y, Dims4 xd, PoolShape ps, int64_t total, T lowest) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t c = o % xd.C;
     int64_t t = o / xd.C;
@@ -579,6 +599,7 @@ __global__ void max_pool_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y,
 // (x - zp) * scale with each operation rounded, and added in (h, w) order as the f32 kernel adds.
 __global__ void global_avg_pool_nhwc_q_kernel(const uint32_t* __restrict__ x, bool is_signed, float scale, float zp, float4* __restrict__ y, Dims4 d,
                                               int rtf32) {
+  pdl_enter();
   const int64_t c4n = d.C / 4, total = d.N * c4n, hw = d.H * d.W;
   const uint32_t flip = is_signed ? 0x80808080u : 0u;
   const float off = is_signed ? 8388736.0f : 8388608.0f;
@@ -621,6 +642,7 @@ __global__ void global_avg_pool_nhwc_q_kernel(const uint32_t* __restrict__ x, bo
 // byte-max instructions.  KIND 0 = f32, 1 = u8, 2 = i8.
 template <int KIND>
 __global__ void max_pool_nhwc_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, Dims4 xd, PoolShape ps, int64_t cvec, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t c = o % cvec;
     int64_t t = o / cvec;
@@ -660,6 +682,7 @@ __global__ void max_pool_nhwc_vec_kernel(const uint4* __restrict__ x, uint4* __r
 // window are issued together (clamped coordinates), 32-bit index arithmetic.  KIND 0 = f32, 1 = u8, 2 = i8.
 template <int KIND>
 __global__ void max_pool_3x3s2_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, int H, int W, int P, int Q, int cvec, int total) {
+  pdl_enter();
   for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < total; o += gridDim.x * blockDim.x) {
     const int c = o % cvec;
     int t = o / cvec;
@@ -711,6 +734,7 @@ __global__ void max_pool_3x3s2_kernel(const uint4* __restrict__ x, uint4* __rest
 // One thread per (n, c): the sum runs over the plane in (h, w) order exactly like the
 // reference loop; consecutive threads read consecutive channels, so loads are coalesced.
 __global__ void global_avg_pool_nhwc_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, int rtf32) {
+  pdl_enter();
   int64_t total = d.N * d.C;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t c = o % d.C, n = o / d.C;
@@ -736,6 +760,7 @@ __global__ void global_avg_pool_nhwc_kernel(const float* __restrict__ x, float* 
 // (coalesced 128-byte rows), 8 warps striding over the pixels.
 __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps, const float* scale_nc,
                                           const float* shift_nc, int relu, int round_tf32_flag) {
+  pdl_enter();
   int64_t cgroups = (d.C + 31) / 32;
   int64_t n = blockIdx.x / cgroups, cg = blockIdx.x % cgroups;
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -785,6 +810,7 @@ __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __
 // each; the per-warp partial sums are added in warp order as above.
 __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps,
                                                                         const float* scale_nc, const float* shift_nc, int relu, int round_tf32_flag) {
+  pdl_enter();
   extern __shared__ float slab[];  // [pixel][32 channels]
   __shared__ float red[32][33];
   const int64_t cgroups = (d.C + 31) / 32;
@@ -866,6 +892,7 @@ __device__ __forceinline__ int64_t nearest_index(int rule, float s, int64_t in_s
 
 __global__ void resize_nhwc_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 xd, Dims4 yd, int mode, int coord, int rule,
                                    float sh, float sw, int64_t total, int rtf32) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t c = o % yd.C;
     int64_t t = o / yd.C;
@@ -896,6 +923,7 @@ __global__ void resize_nhwc_kernel(const float* __restrict__ x, float* __restric
 template <typename I>  // index type: 32-bit divisions where the tensor allows them
 __global__ void resize_nhwc_vec4_kernel(const float4* __restrict__ x, float4* __restrict__ y, Dims4 xd, Dims4 yd, int mode, int coord, int rule,
                                         float sh, float sw, int64_t total4, int rtf32) {
+  pdl_enter();
   const I c4n = (I)(yd.C / 4), yW = (I)yd.W, yH = (I)yd.H;
   for (I o = (I)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x); o < (I)total4; o += (I)((int64_t)gridDim.x * blockDim.x)) {
     const I c4 = o % c4n;
@@ -943,6 +971,7 @@ __device__ __forceinline__ int64_t pad_src(int64_t idx, int64_t ext, int mode, b
 
 __global__ void pad_kernel(const void* x, void* y, DT dt, Layout L, Dims4 xd, Dims4 yd, int mode, float value, int pn, int pc, int ph, int pw,
                            int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(o, L, yd);
     bool outside = false;
@@ -960,6 +989,7 @@ __global__ void pad_kernel(const void* x, void* y, DT dt, Layout L, Dims4 xd, Di
 template <typename I>  // index type: 32-bit divisions where the tensor allows them
 __global__ void pad_nhwc_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, Dims4 xd, Dims4 yd, int64_t vec_per_pixel, int mode, uint4 fill,
                                     int ph, int pw, int64_t total) {
+  pdl_enter();
   const I vpp = (I)vec_per_pixel, yW = (I)yd.W, yH = (I)yd.H;
   for (I o = (I)(blockIdx.x * (int64_t)blockDim.x + threadIdx.x); o < (I)total; o += (I)((int64_t)gridDim.x * blockDim.x)) {
     const int64_t v = o % vpp;
@@ -975,6 +1005,7 @@ __global__ void pad_nhwc_vec_kernel(const uint4* __restrict__ x, uint4* __restri
 }
 
 __global__ void concat_kernel(const void* x, void* y, DT dt, Layout L, Dims4 xd, Dims4 yd, int axis, int64_t offset, int64_t total) {
+  pdl_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     Coord q = decode(i, L, xd);
     if (axis == 0) q.n += offset;
@@ -1121,6 +1152,7 @@ __device__ __forceinline__ uint4 residual_vec(const uint4 av, const uint4 bv, bo
 template <int MODE>
 __global__ void residual_requant_kernel(const uint4* __restrict__ a, bool a_signed, const uint4* __restrict__ b, bool b_signed, uint4* __restrict__ y,
                                         int64_t n16, ResidualParams rp) {
+  pdl_enter();
   const float off_a = 8388608.0f + rp.a_zp + (a_signed ? 128.f : 0.f), off_b = 8388608.0f + rp.b_zp + (b_signed ? 128.f : 0.f);
   const uint32_t flip_a = a_signed ? 0x80808080u : 0u, flip_b = b_signed ? 0x80808080u : 0u;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n16; i += (int64_t)gridDim.x * blockDim.x)
@@ -1129,6 +1161,7 @@ __global__ void residual_requant_kernel(const uint4* __restrict__ a, bool a_sign
 
 __global__ void residual_requant_tail_kernel(const uint8_t* a, bool a_signed, const uint8_t* b, bool b_signed, uint8_t* y, int64_t begin, int64_t n,
                                              ResidualParams rp) {
+  pdl_enter();
   for (int64_t i = begin + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float av = a_signed ? (float)(int8_t)a[i] : (float)a[i];
     float bv = b_signed ? (float)(int8_t)b[i] : (float)b[i];
@@ -1138,6 +1171,7 @@ __global__ void residual_requant_tail_kernel(const uint8_t* a, bool a_signed, co
 
 // Four consecutive packed channels per thread, written as one 4-byte or 16-byte store.
 __global__ void s2d_pack_kernel(const void* src, DT sdt, Layout sl, Dims4 d, void* dst, DT ddt, int c_pad, int sub, int64_t total4) {
+  pdl_enter();
   const int64_t H2 = d.H / 2, W2 = d.W / 2;
   const int c4n = c_pad / 4;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total4; o += (int64_t)gridDim.x * blockDim.x) {
@@ -1190,6 +1224,7 @@ __device__ __forceinline__ void s2d_store_pair(void* dst, uint4 block, int64_t n
 
 __global__ void s2d_window_pack_kernel(const void* src, DT sdt, Layout sl, Dims4 d, void* dst, DT ddt, int pad_left, int wp, int sub, S2dQuant q,
                                        int64_t total, int pair_top, int rows_phys) {
+  pdl_enter();
   const int64_t H2 = d.H / 2, W2 = d.W / 2;
   const int c4 = 4 * (int)d.C;
   const int64_t rows = pair_top >= 0 ? rows_phys + 1 : H2;
@@ -1256,6 +1291,7 @@ __device__ __forceinline__ float quotient_rint(float x, float s, float r, bool s
 template <int C>
 __global__ void s2d_window_pack_nchw_f32_kernel(const float* __restrict__ src, Dims4 d, void* dst, DT ddt, int pad_left, int wp, int sub, S2dQuant q,
                                                 float rcp, bool safe, int64_t total, int pair_top, int rows_phys) {
+  pdl_enter();
   const int64_t H2 = d.H / 2, W2 = d.W / 2;
   const int64_t rows = pair_top >= 0 ? rows_phys + 1 : H2;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
@@ -1310,6 +1346,7 @@ __global__ void s2d_window_pack_nchw_f32_kernel(const float* __restrict__ src, D
 template <int C, bool SIGNED>
 __global__ void s2d_window_pack_nchw_q8_kernel(const uint8_t* __restrict__ src, Dims4 d, void* dst, DT ddt, int pad_left, int wp, int sub, int64_t total,
                                                int pair_top, int rows_phys) {
+  pdl_enter();
   const int64_t H2 = d.H / 2, W2 = d.W / 2;
   const int64_t rows = pair_top >= 0 ? rows_phys + 1 : H2;
   const int lo = ddt == DT::U8 ? 0 : -128, hi = ddt == DT::U8 ? 255 : 127;
@@ -1345,6 +1382,7 @@ __global__ void s2d_window_pack_nchw_q8_kernel(const uint8_t* __restrict__ src, 
 
 // y = x[start0 : start0 + Y0, start1 : ..., ...] over up to four logical (row-major) axes, unit steps.
 __global__ void slice_kernel(const void* x, void* y, int es, Dims4 xd, Dims4 yd, Dims4 start, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = o;
     const int64_t i3 = t % yd.W;
@@ -1365,6 +1403,7 @@ __global__ void slice_kernel(const void* x, void* y, int es, Dims4 xd, Dims4 yd,
 // every row and zeros behind it.  One pixel (16 bytes) per thread.
 __global__ void window_pack_f32_kernel(const float* __restrict__ src, Layout sl, Dims4 d, float4* __restrict__ dst, int pad_left, int wp,
                                        int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     const int64_t xw = o % wp;
     int64_t t = o / wp;
@@ -1390,6 +1429,7 @@ __global__ void window_pack_f32_kernel(const float* __restrict__ src, Layout sl,
 // an integer; negative values count from the end).  An index outside the table records code 20.
 __global__ void gather_rows_kernel(const float* __restrict__ table, const float* __restrict__ idx, float* __restrict__ out, int64_t n_idx, int64_t rows,
                                    int64_t inner, int* err) {
+  pdl_enter();
   const int64_t total = n_idx * inner;
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = o / inner, j = o - i * inner;
@@ -1406,6 +1446,7 @@ __global__ void gather_rows_kernel(const float* __restrict__ table, const float*
 
 // Permutation of up to four logical axes: yd is the output shape, xstride[d] the input stride of output axis d.
 __global__ void transpose_perm_kernel(const uint32_t* __restrict__ x, uint32_t* __restrict__ y, Dims4 yd, Dims4 xstride, int64_t total) {
+  pdl_enter();
   for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = o;
     const int64_t i3 = t % yd.W;
@@ -1422,6 +1463,7 @@ __global__ void transpose_perm_kernel(const uint32_t* __restrict__ x, uint32_t* 
 // pieces of the inner rows, 32-bit index arithmetic.
 __global__ void transpose_perm_vec4_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint32_t d1, uint32_t d2, uint32_t w4, uint32_t s0, uint32_t s1,
                                            uint32_t s2, uint32_t total4) {
+  pdl_enter();
   for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total4; o += gridDim.x * blockDim.x) {
     uint32_t t = o;
     const uint32_t i3 = t % w4;
@@ -1437,6 +1479,7 @@ __global__ void transpose_perm_vec4_kernel(const uint4* __restrict__ x, uint4* _
 // The same permutation when the input's contiguous axis becomes the output's second-to-last one (V -> V^T per head):
 // 32 x 32 tiles through shared memory, 128-byte reads along the input rows and 128-byte writes along the output rows.
 __global__ void transpose_tiled_kernel(const uint32_t* __restrict__ x, uint32_t* __restrict__ y, Dims4 yd, Dims4 xs, int64_t blocks) {
+  pdl_enter();
   __shared__ uint32_t tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 256 threads: 8 rows of a tile per pass
   const int64_t th = (yd.H + 31) / 32, tw = (yd.W + 31) / 32;
@@ -1464,6 +1507,7 @@ __global__ void transpose_tiled_kernel(const uint32_t* __restrict__ x, uint32_t*
 // 32 output rows (the input's contiguous axis) x 128 output columns with 16-byte loads along the input rows and
 // 16-byte stores along the output rows.
 __global__ void transpose_tiled_vec4_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 yd, Dims4 xs, int64_t blocks) {
+  pdl_enter();
   __shared__ float tile[128][33];  // [output column][output row]
   const int64_t th = (yd.H + 31) / 32, tw = (yd.W + 127) / 128;
   for (int64_t b = blockIdx.x; b < blocks; b += gridDim.x) {
@@ -1511,6 +1555,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // (nn/normalization.rs softmax_into; the sums are reassociated across lanes: float tolerance).
 __global__ void softmax_rows_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t rows, int64_t n, const float* __restrict__ scale,
                                     const float* __restrict__ mask, int64_t rows_per_mask, int round_tf32_flag) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -1549,6 +1594,7 @@ __global__ void softmax_rows_kernel(const float* __restrict__ x, float* __restri
 template <int NV4>
 __global__ void softmax_rows_reg_kernel(const float4* __restrict__ x, float4* __restrict__ y, int64_t rows, const float* __restrict__ scale,
                                         const float4* __restrict__ mask, int64_t rows_per_mask, int round_tf32_flag) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const float sc = scale ? scale[0] : 1.f;
@@ -1598,6 +1644,7 @@ __global__ void softmax_rows_reg_kernel(const float4* __restrict__ x, float4* __
 template <int NV4>
 __global__ void layer_norm_rows_reg_kernel(const float4* __restrict__ x, const float4* __restrict__ x2, float4* __restrict__ y, int64_t rows,
                                            const float4* __restrict__ scale, const float4* __restrict__ bias, float eps, uint32_t* minmax_keys) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   const float n = (float)(128 * NV4);
   float mn = INFINITY, mx = -INFINITY;
@@ -1673,6 +1720,7 @@ __global__ void layer_norm_rows_reg_kernel(const float4* __restrict__ x, const f
 // mean = sum / n, var = sum((x - mean)^2) / n, inv_std = 1 / sqrt(var + eps), (x - mean) * inv_std * scale [+ bias].
 __global__ void layer_norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ x2, float* __restrict__ y, int64_t rows, int64_t n,
                                        const float* __restrict__ scale, const float* __restrict__ bias, float eps, uint32_t* minmax_keys) {
+  pdl_enter();
   const int lane = threadIdx.x & 31;
   float mn = INFINITY, mx = -INFINITY;  // extrema of what this thread writes (for a DynamicQuantizeLinear reader)
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1746,24 +1794,25 @@ void convert(const TensorRef& src, const TensorRef& dst, cudaStream_t s) {
     dim3 block(32, 8), grid((unsigned)ceil_div(B, 32), (unsigned)ceil_div(A, 32), (unsigned)d.N);
     if (grid.y <= 65535) {
       if (src.dt == DT::F32 && dst.dt == DT::F32) {
-        transpose_tiles<float, float><<<grid, block, 0, s>>>((const float*)src.ptr, (float*)dst.ptr, A, B);
+        launch(transpose_tiles<float, float>, grid, block, 0, s, (const float*)src.ptr, (float*)dst.ptr, A, B);
         return;
       }
       if (src.dt == DT::U8 && dst.dt == DT::F32) {
-        transpose_tiles<uint8_t, float><<<grid, block, 0, s>>>((const uint8_t*)src.ptr, (float*)dst.ptr, A, B);
+        launch(transpose_tiles<uint8_t, float>, grid, block, 0, s, (const uint8_t*)src.ptr, (float*)dst.ptr, A, B);
         return;
       }
       if (src.dt == DT::I8 && dst.dt == DT::F32) {
-        transpose_tiles<int8_t, float><<<grid, block, 0, s>>>((const int8_t*)src.ptr, (float*)dst.ptr, A, B);
+        launch(transpose_tiles<int8_t, float>, grid, block, 0, s, (const int8_t*)src.ptr, (float*)dst.ptr, A, B);
         return;
       }
     }
   }
-  convert_kernel<<<grid_for(total), kThreads, 0, s>>>(src.ptr, src.dt, src.layout, dst.ptr, dst.dt, dst.layout, d, total);
+  launch(convert_kernel, grid_for(total), kThreads, 0, s, src.ptr, src.dt, src.layout, dst.ptr, dst.dt, dst.layout, d, total);
 }
 
 // Eight lanes per thread: two 16-byte loads, one 16-byte store; the tail runs lane by lane.
 __global__ void f32_to_half_kernel(const float* __restrict__ src, void* __restrict__ dst, bool bf16, int64_t n8, int64_t n) {
+  pdl_enter();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += stride) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(src) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(src) + 2 * i + 1);
@@ -1784,6 +1833,7 @@ __global__ void f32_to_half_kernel(const float* __restrict__ src, void* __restri
 }
 
 __global__ void round_to_tf32_kernel(const float* __restrict__ src, float* __restrict__ dst, int64_t n4, int64_t n) {
+  pdl_enter();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += stride) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(src) + i);
@@ -1795,14 +1845,14 @@ __global__ void round_to_tf32_kernel(const float* __restrict__ src, float* __res
 void round_to_tf32_copy(const float* src, float* dst, int64_t n, cudaStream_t s) {
   if (n == 0) return;
   const int64_t n4 = ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) ? n / 4 : 0;
-  round_to_tf32_kernel<<<grid_for(std::max<int64_t>(n4, n - n4 * 4)), kThreads, 0, s>>>(src, dst, n4, n);
+  launch(round_to_tf32_kernel, grid_for(std::max<int64_t>(n4, n - n4 * 4)), kThreads, 0, s, src, dst, n4, n);
 }
 
 void convert_f32_to_half(const float* src, void* dst, DT dst_dt, int64_t n, cudaStream_t s) {
   if (n == 0) return;
   if (!(dst_dt == DT::F16 || dst_dt == DT::BF16)) OXB_FAIL("convert_f32_to_half: destination is not a 16-bit float type");
   const int64_t n8 = ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) ? n / 8 : 0;
-  f32_to_half_kernel<<<grid_for(std::max<int64_t>(n8, n - n8 * 8)), kThreads, 0, s>>>(src, dst, dst_dt == DT::BF16, n8, n);
+  launch(f32_to_half_kernel, grid_for(std::max<int64_t>(n8, n - n8 * 8)), kThreads, 0, s, src, dst, dst_dt == DT::BF16, n8, n);
 }
 
 void residual_requant(const void* a, DT a_dt, const void* b, DT b_dt, void* y, DT y_dt, int64_t n, const ResidualParams& rp, cudaStream_t s) {
@@ -1812,12 +1862,12 @@ void residual_requant(const void* a, DT a_dt, const void* b, DT b_dt, void* y, D
   int64_t n16 = 0;
   if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) & 15) == 0) n16 = n / 16;
   if (n16 > 0) {
-    if (rp.proven_fast == 2) residual_requant_kernel<2><<<grid_for(n16), kThreads, 0, s>>>((const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
-    else if (rp.proven_fast == 1) residual_requant_kernel<1><<<grid_for(n16), kThreads, 0, s>>>((const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
-    else residual_requant_kernel<0><<<grid_for(n16), kThreads, 0, s>>>((const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
+    if (rp.proven_fast == 2) launch(residual_requant_kernel<2>, grid_for(n16), kThreads, 0, s, (const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
+    else if (rp.proven_fast == 1) launch(residual_requant_kernel<1>, grid_for(n16), kThreads, 0, s, (const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
+    else launch(residual_requant_kernel<0>, grid_for(n16), kThreads, 0, s, (const uint4*)a, as, (const uint4*)b, bs, (uint4*)y, n16, rp);
   }
   if (n16 * 16 < n)
-    residual_requant_tail_kernel<<<grid_for(n - n16 * 16), kThreads, 0, s>>>((const uint8_t*)a, as, (const uint8_t*)b, bs, (uint8_t*)y, n16 * 16, n, rp);
+    launch(residual_requant_tail_kernel, grid_for(n - n16 * 16), kThreads, 0, s, (const uint8_t*)a, as, (const uint8_t*)b, bs, (uint8_t*)y, n16 * 16, n, rp);
 }
 
 // Host restatement of both device formulas (IEEE single precision, one rounding per operation,
@@ -1873,7 +1923,7 @@ void s2d_pack(const TensorRef& src, void* dst, DT dst_dt, int c_pad, int sub, cu
   int64_t total4 = src.d.N * (src.d.H / 2) * (src.d.W / 2) * (c_pad / 4);
   if (total4 == 0) return;
   if (!(dst_dt == DT::F32 || dst_dt == DT::U8 || dst_dt == DT::I8)) OXB_FAIL("s2d_pack: unsupported storage type");
-  s2d_pack_kernel<<<grid_for(total4), kThreads, 0, s>>>(src.ptr, src.dt, src.layout, src.d, dst, dst_dt, c_pad, sub, total4);
+  launch(s2d_pack_kernel, grid_for(total4), kThreads, 0, s, src.ptr, src.dt, src.layout, src.d, dst, dst_dt, c_pad, sub, total4);
 }
 
 void s2d_window_pack(const TensorRef& src, void* dst, DT dst_dt, int pad_left, int wp, int sub, const S2dQuant& q, int pair_top, int rows_phys,
@@ -1889,10 +1939,10 @@ void s2d_window_pack(const TensorRef& src, void* dst, DT dst_dt, int pad_left, i
     const int g = grid_for(total);
     const float* x = (const float*)src.ptr;
     switch ((int)src.d.C) {
-      case 1: s2d_window_pack_nchw_f32_kernel<1><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
-      case 2: s2d_window_pack_nchw_f32_kernel<2><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
-      case 3: s2d_window_pack_nchw_f32_kernel<3><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
-      default: s2d_window_pack_nchw_f32_kernel<4><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
+      case 1: launch(s2d_window_pack_nchw_f32_kernel<1>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
+      case 2: launch(s2d_window_pack_nchw_f32_kernel<2>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
+      case 3: launch(s2d_window_pack_nchw_f32_kernel<3>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
+      default: launch(s2d_window_pack_nchw_f32_kernel<4>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, q, rcp, safe, total, pair_top, rows_phys); break;
     }
     return;
   }
@@ -1901,8 +1951,8 @@ void s2d_window_pack(const TensorRef& src, void* dst, DT dst_dt, int pad_left, i
     const int g = grid_for(total);
     const uint8_t* x = (const uint8_t*)src.ptr;
 #define OXB_Q8_PACK(CC)                                                                                                                          \
-  if (src.dt == DT::I8) s2d_window_pack_nchw_q8_kernel<CC, true><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, total, pair_top, rows_phys); \
-  else s2d_window_pack_nchw_q8_kernel<CC, false><<<g, kThreads, 0, s>>>(x, src.d, dst, dst_dt, pad_left, wp, sub, total, pair_top, rows_phys);
+  if (src.dt == DT::I8) launch(s2d_window_pack_nchw_q8_kernel<CC, true>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, total, pair_top, rows_phys); \
+  else launch(s2d_window_pack_nchw_q8_kernel<CC, false>, g, kThreads, 0, s, x, src.d, dst, dst_dt, pad_left, wp, sub, total, pair_top, rows_phys);
     switch ((int)src.d.C) {
       case 1: OXB_Q8_PACK(1) break;
       case 2: OXB_Q8_PACK(2) break;
@@ -1912,21 +1962,21 @@ void s2d_window_pack(const TensorRef& src, void* dst, DT dst_dt, int pad_left, i
 #undef OXB_Q8_PACK
     return;
   }
-  s2d_window_pack_kernel<<<grid_for(total), kThreads, 0, s>>>(src.ptr, src.dt, src.layout, src.d, dst, dst_dt, pad_left, wp, sub, q, total, pair_top, rows_phys);
+  launch(s2d_window_pack_kernel, grid_for(total), kThreads, 0, s, src.ptr, src.dt, src.layout, src.d, dst, dst_dt, pad_left, wp, sub, q, total, pair_top, rows_phys);
 }
 
 void window_pack_f32(const TensorRef& src, void* dst, int pad_left, int wp, cudaStream_t s) {
   const int64_t total = src.d.N * src.d.H * wp;
   if (total == 0) return;
   if (src.dt != DT::F32 || src.d.C > 4) OXB_FAIL("window_pack_f32: unsupported operand");
-  window_pack_f32_kernel<<<grid_for(total), kThreads, 0, s>>>((const float*)src.ptr, src.layout, src.d, (float4*)dst, pad_left, wp, total);
+  launch(window_pack_f32_kernel, grid_for(total), kThreads, 0, s, (const float*)src.ptr, src.layout, src.d, (float4*)dst, pad_left, wp, total);
 }
 
 void quantize_linear(const TensorRef& x, const TensorRef& y, const float* scale, int64_t n_scale, const float* zp, int64_t n_zp, float lo,
                      float hi, cudaStream_t s) {
   int64_t total = y.d.numel();
   if (total == 0) return;
-  quantize_kernel<<<grid_for(total), kThreads, 0, s>>>(x.ptr, x.dt, x.layout, y.ptr, y.dt, y.layout, y.d, scale, n_scale, zp, n_zp, lo, hi,
+  launch(quantize_kernel, grid_for(total), kThreads, 0, s, x.ptr, x.dt, x.layout, y.ptr, y.dt, y.layout, y.d, scale, n_scale, zp, n_zp, lo, hi,
                                                        total);
 }
 
@@ -1941,7 +1991,7 @@ bool quantize_linear_scalar_ok(const TensorRef& x, const TensorRef& y) {
 void quantize_linear_scalar(const TensorRef& x, const TensorRef& y, float scale, float zp, float lo, float hi, cudaStream_t s) {
   int64_t total = y.d.numel();
   if (quantize_linear_scalar_ok(x, y)) {
-    quantize_vec16_kernel<<<grid_for(total / 16), kThreads, 0, s>>>((const float4*)x.ptr, (uint4*)y.ptr, scale, zp, lo, hi, total / 16);
+    launch(quantize_vec16_kernel, grid_for(total / 16), kThreads, 0, s, (const float4*)x.ptr, (uint4*)y.ptr, scale, zp, lo, hi, total / 16);
     return;
   }
   OXB_FAIL("quantize_linear_scalar: no vector path for this operand");
@@ -1954,10 +2004,10 @@ void dequantize_linear(const TensorRef& x, const TensorRef& y, const float* scal
   const bool same_order = x.layout == y.layout || y.d.C == 1 || y.d.H * y.d.W == 1;
   if ((x.dt == DT::U8 || x.dt == DT::I8) && n_scale == 1 && n_zp <= 1 && same_order && total % 4 == 0 && ((uintptr_t)x.ptr & 3) == 0 &&
       ((uintptr_t)y.ptr & 15) == 0) {
-    dequantize_vec4_kernel<<<grid_for(total / 4), kThreads, 0, s>>>((const uint32_t*)x.ptr, x.dt == DT::I8, (float4*)y.ptr, scale, zp, total / 4);
+    launch(dequantize_vec4_kernel, grid_for(total / 4), kThreads, 0, s, (const uint32_t*)x.ptr, x.dt == DT::I8, (float4*)y.ptr, scale, zp, total / 4);
     return;
   }
-  dequantize_kernel<<<grid_for(total), kThreads, 0, s>>>(x.ptr, x.dt, x.layout, y.ptr, y.layout, y.d, scale, n_scale, zp, n_zp, total);
+  launch(dequantize_kernel, grid_for(total), kThreads, 0, s, x.ptr, x.dt, x.layout, y.ptr, y.layout, y.d, scale, n_scale, zp, n_zp, total);
 }
 
 void dynamic_quantize_linear(const TensorRef& x, const TensorRef& y, float* params, float* scratch, cudaStream_t s, bool have_minmax) {
@@ -1967,15 +2017,15 @@ void dynamic_quantize_linear(const TensorRef& x, const TensorRef& y, float* para
   uint32_t* keys = (uint32_t*)scratch;
   if ((((uintptr_t)x.ptr) & 15) != 0 || (((uintptr_t)y.ptr) & 3) != 0) {
     // operands that are not aligned for 16-byte loads / 4-byte stores: the same arithmetic, one lane per access
-    if (!have_minmax) minmax_kernel<<<grid_for(n), kThreads, 0, s>>>((const float*)x.ptr, n, keys, 0);
-    dynq_apply_fused_kernel<<<grid_for(n), kThreads, 0, s>>>((const float*)x.ptr, (uint8_t*)y.ptr, keys, params, n, 0);
+    if (!have_minmax) launch(minmax_kernel, grid_for(n), kThreads, 0, s, (const float*)x.ptr, n, keys, 0);
+    launch(dynq_apply_fused_kernel, grid_for(n), kThreads, 0, s, (const float*)x.ptr, (uint8_t*)y.ptr, keys, params, n, 0);
     return;
   }
   const int64_t cap = 148 * 8;
   const int64_t b_mm = std::min<int64_t>(cap, std::max<int64_t>(1, (n / 4 + kThreads * 4 - 1) / (kThreads * 4)));
   const int64_t b_ap = std::min<int64_t>(cap, std::max<int64_t>(1, (n / 4 + (kThreads / 32) * 128 - 1) / ((kThreads / 32) * 128)));
-  if (!have_minmax) minmax_wide_kernel<<<(int)b_mm, kThreads, 0, s>>>((const float*)x.ptr, n, keys);
-  dynq_apply_wide_kernel<<<(int)b_ap, kThreads, 0, s>>>((const float*)x.ptr, (uint8_t*)y.ptr, keys, params, n);
+  if (!have_minmax) launch(minmax_wide_kernel, (int)b_mm, kThreads, 0, s, (const float*)x.ptr, n, keys);
+  launch(dynq_apply_wide_kernel, (int)b_ap, kThreads, 0, s, (const float*)x.ptr, (uint8_t*)y.ptr, keys, params, n);
 }
 
 void dynamic_quantize_scratch_init(float* scratch) {
@@ -1989,7 +2039,7 @@ void binary(const TensorRef& a, const TensorRef& b, const TensorRef& out, int op
   bool same = a.d.numel() == total && b.d.numel() == total && a.layout == out.layout && b.layout == out.layout && a.dt == DT::F32 &&
               b.dt == DT::F32 && out.dt == DT::F32 && total % 4 == 0;
   if (same) {
-    binary_vec4_kernel<<<grid_for(total / 4), kThreads, 0, s>>>((const float4*)a.ptr, (const float4*)b.ptr, (float4*)out.ptr, op, relu_after,
+    launch(binary_vec4_kernel, grid_for(total / 4), kThreads, 0, s, (const float4*)a.ptr, (const float4*)b.ptr, (float4*)out.ptr, op, relu_after,
                                                                round_tf32_flag, total / 4);
     return;
   }
@@ -2005,25 +2055,25 @@ void binary(const TensorRef& a, const TensorRef& b, const TensorRef& out, int op
       nb *= bd[j];
     }
     if (suffix && nb % 4 == 0) {
-      binary_suffix_vec4_kernel<<<grid_for(total / 4), kThreads, 0, s>>>((const float4*)a.ptr, (const float4*)b.ptr, (float4*)out.ptr, op, relu_after,
+      launch(binary_suffix_vec4_kernel, grid_for(total / 4), kThreads, 0, s, (const float4*)a.ptr, (const float4*)b.ptr, (float4*)out.ptr, op, relu_after,
                                                                          round_tf32_flag, (uint32_t)(total / 4), (uint32_t)(nb / 4));
       return;
     }
   }
-  binary_kernel<<<grid_for(total), kThreads, 0, s>>>(a.ptr, a.dt, a.layout, a.d, b.ptr, b.dt, b.layout, b.d, out.ptr, out.dt, out.layout,
+  launch(binary_kernel, grid_for(total), kThreads, 0, s, a.ptr, a.dt, a.layout, a.d, b.ptr, b.dt, b.layout, b.d, out.ptr, out.dt, out.layout,
                                                      out.d, op, relu_after, round_tf32_flag, total);
 }
 
 void unary(const TensorRef& x, const TensorRef& y, int op, cudaStream_t s) {
   int64_t total = y.d.numel();
   if (total == 0) return;
-  unary_kernel<<<grid_for(total), kThreads, 0, s>>>(x.ptr, x.dt, y.ptr, y.dt, op, total);
+  launch(unary_kernel, grid_for(total), kThreads, 0, s, x.ptr, x.dt, y.ptr, y.dt, op, total);
 }
 
 void prelu(const TensorRef& x, const TensorRef& y, const float* slope, int64_t n_slope, cudaStream_t s) {
   int64_t total = y.d.numel();
   if (total == 0) return;
-  prelu_kernel<<<grid_for(total), kThreads, 0, s>>>((const float*)x.ptr, x.layout, (float*)y.ptr, x.d, slope, n_slope, total);
+  launch(prelu_kernel, grid_for(total), kThreads, 0, s, (const float*)x.ptr, x.layout, (float*)y.ptr, x.d, slope, n_slope, total);
 }
 
 void max_pool(const TensorRef& x, const TensorRef& y, const PoolShape& ps, cudaStream_t s) {
@@ -2036,20 +2086,20 @@ void max_pool(const TensorRef& x, const TensorRef& y, const PoolShape& ps, cudaS
     if (ps.kh == 3 && ps.kw == 3 && ps.sh == 2 && ps.sw == 2 && ps.dh == 1 && ps.dw == 1 && ps.pt == 1 && ps.pl == 1 && tv < 0x7fffffffLL &&
         x.d.numel() / per < 0x7fffffffLL) {
       const int H = (int)x.d.H, W = (int)x.d.W, cv = (int)cvec, n = (int)tv;
-      if (x.dt == DT::F32) max_pool_3x3s2_kernel<0><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
-      else if (x.dt == DT::U8) max_pool_3x3s2_kernel<1><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
-      else max_pool_3x3s2_kernel<2><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
+      if (x.dt == DT::F32) launch(max_pool_3x3s2_kernel<0>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
+      else if (x.dt == DT::U8) launch(max_pool_3x3s2_kernel<1>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
+      else launch(max_pool_3x3s2_kernel<2>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, H, W, ps.P, ps.Q, cv, n);
       return;
     }
-    if (x.dt == DT::F32) max_pool_nhwc_vec_kernel<0><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
-    else if (x.dt == DT::U8) max_pool_nhwc_vec_kernel<1><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
-    else max_pool_nhwc_vec_kernel<2><<<gv, kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
+    if (x.dt == DT::F32) launch(max_pool_nhwc_vec_kernel<0>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
+    else if (x.dt == DT::U8) launch(max_pool_nhwc_vec_kernel<1>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
+    else launch(max_pool_nhwc_vec_kernel<2>, gv, kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, x.d, ps, cvec, tv);
     return;
   }
   int g = grid_for(total);
-  if (x.dt == DT::F32) max_pool_nhwc_kernel<float><<<g, kThreads, 0, s>>>((const float*)x.ptr, (float*)y.ptr, x.d, ps, total, -INFINITY);
-  else if (x.dt == DT::U8) max_pool_nhwc_kernel<uint8_t><<<g, kThreads, 0, s>>>((const uint8_t*)x.ptr, (uint8_t*)y.ptr, x.d, ps, total, 0);
-  else if (x.dt == DT::I8) max_pool_nhwc_kernel<int8_t><<<g, kThreads, 0, s>>>((const int8_t*)x.ptr, (int8_t*)y.ptr, x.d, ps, total, -128);
+  if (x.dt == DT::F32) launch(max_pool_nhwc_kernel<float>, g, kThreads, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, ps, total, -INFINITY);
+  else if (x.dt == DT::U8) launch(max_pool_nhwc_kernel<uint8_t>, g, kThreads, 0, s, (const uint8_t*)x.ptr, (uint8_t*)y.ptr, x.d, ps, total, 0);
+  else if (x.dt == DT::I8) launch(max_pool_nhwc_kernel<int8_t>, g, kThreads, 0, s, (const int8_t*)x.ptr, (int8_t*)y.ptr, x.d, ps, total, -128);
   else OXB_FAIL("max_pool: unsupported storage type");
 }
 
@@ -2058,13 +2108,13 @@ void global_avg_pool_dequant(const TensorRef& x, const TensorRef& y, float scale
     OXB_FAIL("global_avg_pool_dequant: unsupported operand");
   const int64_t total4 = x.d.N * x.d.C / 4;
   if (total4 == 0) return;
-  global_avg_pool_nhwc_q_kernel<<<grid_for(total4, 128), 128, 0, s>>>((const uint32_t*)x.ptr, x.dt == DT::I8, scale, zp, (float4*)y.ptr, x.d, round_tf32_flag);
+  launch(global_avg_pool_nhwc_q_kernel, grid_for(total4, 128), 128, 0, s, (const uint32_t*)x.ptr, x.dt == DT::I8, scale, zp, (float4*)y.ptr, x.d, round_tf32_flag);
 }
 
 void global_avg_pool(const TensorRef& x, const TensorRef& y, int round_tf32_flag, cudaStream_t s) {
   int64_t total = x.d.N * x.d.C;
   if (total == 0) return;
-  global_avg_pool_nhwc_kernel<<<grid_for(total, 128), 128, 0, s>>>((const float*)x.ptr, (float*)y.ptr, x.d, round_tf32_flag);
+  launch(global_avg_pool_nhwc_kernel, grid_for(total, 128), 128, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, round_tf32_flag);
 }
 
 void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, const float* shift_nc, int relu, int round_tf32_flag,
@@ -2088,11 +2138,11 @@ void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const floa
         h = slab;
       }
     }
-    instance_norm_nhwc_smem_kernel<<<(unsigned)blocks, 1024, slab, s>>>((const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu,
+    launch(instance_norm_nhwc_smem_kernel, (unsigned)blocks, 1024, slab, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu,
                                                                         round_tf32_flag);
     return;
   }
-  instance_norm_nhwc_kernel<<<(unsigned)blocks, 256, 0, s>>>((const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu, round_tf32_flag);
+  launch(instance_norm_nhwc_kernel, (unsigned)blocks, 256, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu, round_tf32_flag);
 }
 
 void resize(const TensorRef& x, const TensorRef& y, int mode, int coord, int nearest_rule, float scale_h, float scale_w, int round_tf32_flag,
@@ -2101,14 +2151,14 @@ void resize(const TensorRef& x, const TensorRef& y, int mode, int coord, int nea
   if (total == 0) return;
   if (y.d.C % 4 == 0 && ((uintptr_t)x.ptr & 15) == 0 && ((uintptr_t)y.ptr & 15) == 0) {
     if (total / 4 + (int64_t)148 * 64 * kThreads < (int64_t)1 << 31)
-      resize_nhwc_vec4_kernel<uint32_t><<<grid_for(total / 4), kThreads, 0, s>>>((const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, mode, coord, nearest_rule,
+      launch(resize_nhwc_vec4_kernel<uint32_t>, grid_for(total / 4), kThreads, 0, s, (const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, mode, coord, nearest_rule,
                                                                                 scale_h, scale_w, total / 4, round_tf32_flag);
     else
-      resize_nhwc_vec4_kernel<int64_t><<<grid_for(total / 4), kThreads, 0, s>>>((const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, mode, coord, nearest_rule,
+      launch(resize_nhwc_vec4_kernel<int64_t>, grid_for(total / 4), kThreads, 0, s, (const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, mode, coord, nearest_rule,
                                                                                scale_h, scale_w, total / 4, round_tf32_flag);
     return;
   }
-  resize_nhwc_kernel<<<grid_for(total), kThreads, 0, s>>>((const float*)x.ptr, (float*)y.ptr, x.d, y.d, mode, coord, nearest_rule, scale_h,
+  launch(resize_nhwc_kernel, grid_for(total), kThreads, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, y.d, mode, coord, nearest_rule, scale_h,
                                                           scale_w, total, round_tf32_flag);
 }
 
@@ -2135,26 +2185,26 @@ void pad(const TensorRef& x, const TensorRef& y, int mode, float value, int pn, 
     const int64_t vpp = (int64_t)(x.d.C * es / 16);
     const int64_t total_v = y.d.N * y.d.H * y.d.W * vpp;
     if (total_v + (int64_t)148 * 64 * kThreads < (int64_t)1 << 31)
-      pad_nhwc_vec_kernel<uint32_t><<<grid_for(total_v), kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, x.d, y.d, vpp, mode,
+      launch(pad_nhwc_vec_kernel<uint32_t>, grid_for(total_v), kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, x.d, y.d, vpp, mode,
                                                                           make_uint4(word, word, word, word), ph, pw, total_v);
     else
-      pad_nhwc_vec_kernel<int64_t><<<grid_for(total_v), kThreads, 0, s>>>((const uint4*)x.ptr, (uint4*)y.ptr, x.d, y.d, vpp, mode,
+      launch(pad_nhwc_vec_kernel<int64_t>, grid_for(total_v), kThreads, 0, s, (const uint4*)x.ptr, (uint4*)y.ptr, x.d, y.d, vpp, mode,
                                                                          make_uint4(word, word, word, word), ph, pw, total_v);
     return;
   }
-  pad_kernel<<<grid_for(total), kThreads, 0, s>>>(x.ptr, y.ptr, x.dt, x.layout, x.d, y.d, mode, value, pn, pc, ph, pw, total);
+  launch(pad_kernel, grid_for(total), kThreads, 0, s, x.ptr, y.ptr, x.dt, x.layout, x.d, y.d, mode, value, pn, pc, ph, pw, total);
 }
 
 void slice_rows(const void* x, void* y, DT dt, const Dims4& xd, const Dims4& yd, const Dims4& start, cudaStream_t s) {
   const int64_t total = yd.numel();
   if (total == 0) return;
   const int es = dt == DT::F32 || dt == DT::I32 ? 4 : (dt == DT::I16 ? 2 : 1);
-  slice_kernel<<<grid_for(total), kThreads, 0, s>>>(x, y, es, xd, yd, start, total);
+  launch(slice_kernel, grid_for(total), kThreads, 0, s, x, y, es, xd, yd, start, total);
 }
 
 void gather_rows(const float* table, const float* idx, float* out, int64_t n_idx, int64_t rows, int64_t inner, int* err, cudaStream_t s) {
   if (n_idx * inner == 0) return;
-  gather_rows_kernel<<<grid_for(n_idx * inner), kThreads, 0, s>>>(table, idx, out, n_idx, rows, inner, err);
+  launch(gather_rows_kernel, grid_for(n_idx * inner), kThreads, 0, s, table, idx, out, n_idx, rows, inner, err);
 }
 
 void transpose_perm(const void* x, void* y, const Dims4& yd, const Dims4& xstride, cudaStream_t s) {
@@ -2163,22 +2213,22 @@ void transpose_perm(const void* x, void* y, const Dims4& yd, const Dims4& xstrid
   if (xstride.W == 1 && yd.W % 4 == 0 && xstride.N % 4 == 0 && xstride.C % 4 == 0 && xstride.H % 4 == 0 && total < (int64_t)1 << 31 &&
       ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0) {
     const uint32_t total4 = (uint32_t)(total / 4);
-    transpose_perm_vec4_kernel<<<grid_for(total4), kThreads, 0, s>>>((const uint4*)x, (uint4*)y, (uint32_t)yd.C, (uint32_t)yd.H, (uint32_t)(yd.W / 4),
+    launch(transpose_perm_vec4_kernel, grid_for(total4), kThreads, 0, s, (const uint4*)x, (uint4*)y, (uint32_t)yd.C, (uint32_t)yd.H, (uint32_t)(yd.W / 4),
                                                                      (uint32_t)(xstride.N / 4), (uint32_t)(xstride.C / 4), (uint32_t)(xstride.H / 4), total4);
     return;
   }
   if (xstride.H == 1 && xstride.W != 1 && yd.H % 4 == 0 && yd.W % 4 == 0 && yd.H >= 8 && yd.W >= 32 && xstride.W % 4 == 0 && xstride.N % 4 == 0 &&
       xstride.C % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0) {
     const int64_t blocks = yd.N * yd.C * ((yd.H + 31) / 32) * ((yd.W + 127) / 128);
-    transpose_tiled_vec4_kernel<<<(unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s>>>((const float*)x, (float*)y, yd, xstride, blocks);
+    launch(transpose_tiled_vec4_kernel, (unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s, (const float*)x, (float*)y, yd, xstride, blocks);
     return;
   }
   if (xstride.H == 1 && xstride.W != 1 && yd.H >= 8 && yd.W >= 8) {
     const int64_t blocks = yd.N * yd.C * ((yd.H + 31) / 32) * ((yd.W + 31) / 32);
-    transpose_tiled_kernel<<<(unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s>>>((const uint32_t*)x, (uint32_t*)y, yd, xstride, blocks);
+    launch(transpose_tiled_kernel, (unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s, (const uint32_t*)x, (uint32_t*)y, yd, xstride, blocks);
     return;
   }
-  transpose_perm_kernel<<<grid_for(total), kThreads, 0, s>>>((const uint32_t*)x, (uint32_t*)y, yd, xstride, total);
+  launch(transpose_perm_kernel, grid_for(total), kThreads, 0, s, (const uint32_t*)x, (uint32_t*)y, yd, xstride, total);
 }
 
 void softmax_rows(const float* x, float* y, int64_t rows, int64_t n, const float* scale, const float* mask, int64_t rows_per_mask, int round_tf32_flag,
@@ -2188,12 +2238,12 @@ void softmax_rows(const float* x, float* y, int64_t rows, int64_t n, const float
   if (n % 128 == 0 && n <= 512 && n != 384 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)mask) & 15) == 0) {
     const int g = grid_for(rows * 32);
     const float4 *x4 = (const float4*)x, *m4 = (const float4*)mask;
-    if (n == 128) softmax_rows_reg_kernel<1><<<g, kThreads, 0, s>>>(x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
-    else if (n == 256) softmax_rows_reg_kernel<2><<<g, kThreads, 0, s>>>(x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
-    else softmax_rows_reg_kernel<4><<<g, kThreads, 0, s>>>(x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
+    if (n == 128) launch(softmax_rows_reg_kernel<1>, g, kThreads, 0, s, x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
+    else if (n == 256) launch(softmax_rows_reg_kernel<2>, g, kThreads, 0, s, x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
+    else launch(softmax_rows_reg_kernel<4>, g, kThreads, 0, s, x4, (float4*)y, rows, scale, m4, rpm, round_tf32_flag);
     return;
   }
-  softmax_rows_kernel<<<grid_for(rows * 32), kThreads, 0, s>>>(x, y, rows, n, scale, mask, rpm, round_tf32_flag);
+  launch(softmax_rows_kernel, grid_for(rows * 32), kThreads, 0, s, x, y, rows, n, scale, mask, rpm, round_tf32_flag);
 }
 
 void layer_norm_rows(const float* x, float* y, int64_t rows, int64_t n, const float* scale, const float* bias, float eps, cudaStream_t s,
@@ -2202,19 +2252,19 @@ void layer_norm_rows(const float* x, float* y, int64_t rows, int64_t n, const fl
   if (n % 256 == 0 && n <= 1024 && (((uintptr_t)x | (uintptr_t)x2 | (uintptr_t)y | (uintptr_t)scale | (uintptr_t)bias) & 15) == 0) {
     const int g = grid_for(rows * 32);
     const float4 *x4 = (const float4*)x, *x24 = (const float4*)x2, *s4 = (const float4*)scale, *b4 = (const float4*)bias;
-    if (n == 256) layer_norm_rows_reg_kernel<2><<<g, kThreads, 0, s>>>(x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
-    else if (n == 512) layer_norm_rows_reg_kernel<4><<<g, kThreads, 0, s>>>(x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
-    else if (n == 768) layer_norm_rows_reg_kernel<6><<<g, kThreads, 0, s>>>(x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
-    else layer_norm_rows_reg_kernel<8><<<g, kThreads, 0, s>>>(x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
+    if (n == 256) launch(layer_norm_rows_reg_kernel<2>, g, kThreads, 0, s, x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
+    else if (n == 512) launch(layer_norm_rows_reg_kernel<4>, g, kThreads, 0, s, x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
+    else if (n == 768) launch(layer_norm_rows_reg_kernel<6>, g, kThreads, 0, s, x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
+    else launch(layer_norm_rows_reg_kernel<8>, g, kThreads, 0, s, x4, x24, (float4*)y, rows, s4, b4, eps, minmax_keys);
     return;
   }
-  layer_norm_rows_kernel<<<grid_for(rows * 32), kThreads, 0, s>>>(x, x2, y, rows, n, scale, bias, eps, minmax_keys);
+  launch(layer_norm_rows_kernel, grid_for(rows * 32), kThreads, 0, s, x, x2, y, rows, n, scale, bias, eps, minmax_keys);
 }
 
 void concat_into(const TensorRef& x, const TensorRef& y, int axis, int64_t offset, cudaStream_t s) {
   int64_t total = x.d.numel();
   if (total == 0) return;
-  concat_kernel<<<grid_for(total), kThreads, 0, s>>>(x.ptr, y.ptr, x.dt, x.layout, x.d, y.d, axis, offset, total);
+  launch(concat_kernel, grid_for(total), kThreads, 0, s, x.ptr, y.ptr, x.dt, x.layout, x.d, y.d, axis, offset, total);
 }
 
 // =========================================================================================
@@ -2291,10 +2341,10 @@ extern "C" int oxb200_dynamic_quantize_linear_noalloc(int device_ordinal, const 
   }
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const int64_t count = (int64_t)n;
-  minmax_init_kernel<<<1, 1, 0, s>>>(scratch);  // the shared words start every call from their identity values
-  minmax_kernel<<<grid_for(count / 4 + 1), kThreads, 0, s>>>(x_device, count, scratch, 1);
-  dynq_params_kernel<<<1, 1, 0, s>>>(scratch, scale_zp_device);
-  dynq_apply_kernel<<<grid_for(count / 4 + 1), kThreads, 0, s>>>(x_device, y_device, scale_zp_device, count);
+  launch(minmax_init_kernel, 1, 1, 0, s, scratch);  // the shared words start every call from their identity values
+  launch(minmax_kernel, grid_for(count / 4 + 1), kThreads, 0, s, x_device, count, scratch, 1);
+  launch(dynq_params_kernel, 1, 1, 0, s, scratch, scale_zp_device);
+  launch(dynq_apply_kernel, grid_for(count / 4 + 1), kThreads, 0, s, x_device, y_device, scale_zp_device, count);
   e = cudaGetLastError();
   if (previous >= 0 && previous != device_ordinal) cudaSetDevice(previous);
   if (e != cudaSuccess) return fail(std::string("dynamic_quantize_linear_noalloc: launch failed: ") + cudaGetErrorString(e));

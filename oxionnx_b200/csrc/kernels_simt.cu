@@ -5,6 +5,7 @@
 // oxionnx-ops/src/registry/quant_ops/conv_kernel.rs:205-249.  They are the path for nodes
 // the tensor-core kernel is not eligible for; the hot layers go through kernels_umma.cu.
 #include "kernels.hpp"
+#include "pdl.cuh"
 
 namespace oxb {
 namespace k {
@@ -99,6 +100,7 @@ __device__ __forceinline__ void finish_int(const EpiDev& e, void* out, int64_t i
 template <typename TX, typename TW, bool IS_INT>
 __global__ void conv_direct_kernel(const TX* __restrict__ x, const TW* __restrict__ w, void* __restrict__ out, ConvShape cs, EpiDev e,
                                    int x_plain_nchw, int64_t total) {
+  pdl_enter();
   const int cg = cs.C / cs.group, ocg = cs.OC / cs.group;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
     int oc = (int)(idx % cs.OC);
@@ -163,6 +165,7 @@ __global__ void conv_direct_kernel(const TX* __restrict__ x, const TW* __restric
 
 __global__ void matmul_f32_direct_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ c, int64_t M, int64_t K,
                                          int64_t N, int64_t a_bs, int64_t b_bs) {
+  pdl_enter();
   // 32x32 output tile per block, K stepped through shared memory in slabs of 32.
   __shared__ float As[32][33], Bs[32][33];
   int64_t batch = blockIdx.z;
@@ -201,7 +204,7 @@ void launch_conv(const void* x, const void* w, void* out, const ConvShape& cs, c
   if (total == 0) return;
   int64_t blocks = (total + 255) / 256;
   if (blocks > 148 * 256) blocks = 148 * 256;
-  conv_direct_kernel<TX, TW, IS_INT><<<(unsigned)blocks, 256, 0, s>>>((const TX*)x, (const TW*)w, out, cs, e, x_plain_nchw, total);
+  launch(conv_direct_kernel<TX, TW, IS_INT>, (unsigned)blocks, 256, 0, s, (const TX*)x, (const TW*)w, out, cs, e, x_plain_nchw, total);
 }
 
 }  // namespace
@@ -238,7 +241,7 @@ void matmul_f32_direct(const float* a, const float* b, float* c, int64_t batch, 
                        int64_t b_bstride, cudaStream_t s) {
   if (batch * M * N == 0) return;
   dim3 block(32, 8), grid((unsigned)ceil_div(N, 32), (unsigned)ceil_div(M, 32), (unsigned)batch);
-  matmul_f32_direct_kernel<<<grid, block, 0, s>>>(a, b, c, M, K, N, a_bstride, b_bstride);
+  launch(matmul_f32_direct_kernel, grid, block, 0, s, a, b, c, M, K, N, a_bstride, b_bstride);
 }
 
 }  // namespace k

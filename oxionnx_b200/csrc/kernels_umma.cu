@@ -123,6 +123,7 @@ struct UmmaPlan {
   int bn;
   int kind;
   int pair;
+  int small;  // the small-problem kernel (umma_small.cuh)
   int grid;
   int device;
   size_t smem;
@@ -194,6 +195,65 @@ size_t warp_row_bytes(int bn, int kind, size_t oes, bool one_run) {
   return std::min<size_t>(128, (size_t)cpw * 32 * oes);
 }
 
+// The small-problem kernel's geometry for a problem that cannot fill the chip with the persistent kernel's tiles, or
+// bn = 0 when the problem is not small.
+struct SmallShape {
+  int bn = 0, splits = 1, k_per = 0;
+  int a_rows = 0, kpb = 1, stages = 1;
+  size_t stage_bytes = 0, smem = 0;
+  double us = 0.0;  // estimated time
+};
+
+// Ring and receive slots of a candidate: [ring | slots for the slices' accumulators], and room for the activation
+// rows an MMA reads past a short box.  A stage is at most 32 KB, so that its MMAs start early.  Two CTAs share an SM
+// (this layer's and the next one's prologue) unless the slice is at least six blocks longer than such a ring: a slot's
+// round trip is near 2 us, so a slice that outlives the ring runs at the ring's depth, which costs more than the prologue.
+void layout_small(SmallShape& c, int swz) {
+  const int64_t block = (int64_t)(c.a_rows + c.bn) * swz;
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(16, (32 * 1024) / block));
+  c.kpb = (int)ceil_div(c.k_per, ceil_div(c.k_per, most));
+  c.stage_bytes = (size_t)block * c.kpb;
+  const int chunks = (int)ceil_div(c.k_per, c.kpb);
+  const size_t slots = c.splits > 1 ? (size_t)ceil_div(4 * (c.bn / 32), c.splits) * c.splits * 4096 : 0;
+  const size_t fixed = slots + (size_t)(BLOCK_M - c.a_rows) * swz + 1024;
+  auto depth = [&](int64_t budget) { return (int)std::min<int64_t>((budget - (int64_t)fixed) / (int64_t)c.stage_bytes, chunks); };
+  int stages = depth(110 * 1024);
+  if (stages < std::min(2, chunks) || c.k_per >= stages * c.kpb + 6) stages = depth(SMALL_SMEM_MAX);
+  c.stages = std::min(std::max(stages, 1), 16);
+  c.smem = c.stages * c.stage_bytes + fixed;
+}
+
+// Tile width and slices by a model fitted to sweeps of both over sixteen layer shapes: 3 us from one layer to the next,
+// 0.12 us per K block that the ring holds, 1.7 us over the ring's depth per block beyond it, 0.7 us per further
+// 32-channel run a warp finishes, 1.1 us for the slices' meeting.  Clusters are placed whole, beside those of the layer
+// before and behind: with more than 148 / 128 / 64 CTAs in clusters of 2 / 4 / 8 some wait for a place (3x3 512 at 7x7,
+// i8: 5.9 us with 64 CTAs in clusters of 4, 15.6 us with 128 in clusters of 8).
+SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, int max_split) {
+  SmallShape best;
+  const int64_t m_tiles = ceil_div(M, BLOCK_M);
+  for (int bn : {32, 64, 128}) {
+    if (bn > 32 && OC <= bn / 2) break;
+    const int64_t tiles = m_tiles * ceil_div(OC, bn);
+    for (int sp : {1, 2, 4, 8}) {
+      if (sp > max_split || sp > k_iters) break;
+      SmallShape c;
+      c.bn = bn, c.splits = sp, c.k_per = (int)ceil_div(k_iters, (int64_t)sp);
+      if (sp > 1 && (sp - 1) * (int64_t)c.k_per >= k_iters) continue;  // a slice would be empty
+      c.a_rows = (int)std::min<int64_t>(BLOCK_M, align_up((size_t)M, 32));
+      const int64_t ctas = tiles * sp;
+      if (ctas > (sp == 1 ? 2 * sms : (sp == 2 ? sms : (sp == 4 ? 128 : 64)))) continue;
+      layout_small(c, swz);
+      if (ctas > sms && c.smem > 112 * 1024) continue;
+      const double ring = c.stages * c.kpb;
+      const double share = ctas > sms ? 2.0 : 1.0;  // CTAs of this layer on one SM
+      c.us = 3.0 + share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring)) +
+             0.7 * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
+      if (best.bn == 0 || c.us < best.us) best = c;
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt, void* out, const ConvShape& cs, const Epilogue& e, int kind,
@@ -250,6 +310,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   const int bn_max = cs.OC <= 32 ? 32 : (cs.OC <= 64 ? 64 : (cs.OC <= 128 ? 128 : 256));
   const int64_t k_iters_host = (int64_t)cs.R * cs.S * (cs.C / cb);
   int bn = bn_max, splits = 1;
+  SmallShape small;
   {
     const double k_bytes = (double)cs.K() * es;
     const double k_steps = k_bytes / 32.0;
@@ -279,6 +340,16 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
         }
       }
     }
+    // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
+    // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
+    if (tune.cta_pairs != 2) {
+      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split);
+      if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
+      if (small.bn > 0) {
+        bn = small.bn;
+        splits = 1;
+      }
+    }
   }
   // CTA pairs: two CTAs share a 256 x 256 tile and each stages 128 rows of A and 128 rows of B per K block (32 KB
   // at 128-byte K blocks instead of the 48 KB of a lone CTA's 128 x 256 tile), which relieves both the L2 -> shared
@@ -289,7 +360,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     bn = 256;
     splits = 1;
   }
-  if (tune.cta_pairs != 1 && bn == 256 && splits == 1 && cs.OC >= 256) {
+  if (tune.cta_pairs != 1 && small.bn == 0 && bn == 256 && splits == 1 && cs.OC >= 256) {
     const int64_t pair_tiles = ceil_div(M, 2 * BLOCK_M) * ceil_div(cs.OC, 256);
     const double k_bytes = (double)cs.K() * es;
     // Measured: with 2 KB of K or more per row a pair wins once every pair has at least two tiles (3x3 256->256,
@@ -315,7 +386,17 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   };
   const CUtensorMapDataType dtype = operand_map_type(kind);
   CUresult rc;
-  if (gemm_like) {
+  const int a_rows = small.bn > 0 ? small.a_rows : BLOCK_M;
+  // Small problems: one three-dimensional box [blocks][rows][block] brings a ring stage with one instruction.
+  if (gemm_like && small.bn > 0) {
+    cuuint64_t gdim[3] = {(cuuint64_t)cb, (cuuint64_t)M, (cuuint64_t)k_iters_host};
+    cuuint64_t gstr[2] = {(cuuint64_t)cs.C * es, (cuuint64_t)swz};
+    cuuint32_t box[3] = {(cuuint32_t)cb, (cuuint32_t)a_rows, (cuuint32_t)small.kpb};
+    cuuint32_t estr[3] = {1, 1, 1};
+    rc = g_encode_tiled(&kp.tmA, dtype, 3, const_cast<void*>(x), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    kp.a_im2col = 0;
+  } else if (gemm_like) {
     cuuint64_t gdim[2] = {(cuuint64_t)cs.C, (cuuint64_t)M};
     cuuint64_t gstr[1] = {(cuuint64_t)cs.C * es};
     cuuint32_t box[2] = {(cuuint32_t)cb, (cuuint32_t)BLOCK_M};
@@ -330,7 +411,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     int lower[2] = {-cs.pl, -cs.pt};
     int upper[2] = {cs.pr - (cs.S - 1) * cs.dw, cs.pb - (cs.R - 1) * cs.dh};
     cuuint32_t estr[4] = {1, (cuuint32_t)cs.sw, (cuuint32_t)cs.sh, 1};
-    rc = g_encode_im2col(&kp.tmA, dtype, 4, const_cast<void*>(x), gdim, gstr, lower, upper, (cuuint32_t)cb, (cuuint32_t)BLOCK_M, estr,
+    rc = g_encode_im2col(&kp.tmA, dtype, 4, const_cast<void*>(x), gdim, gstr, lower, upper, (cuuint32_t)cb, (cuuint32_t)a_rows, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     kp.a_im2col = 1;
@@ -343,7 +424,15 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     }
   }
   if (rc != CUDA_SUCCESS) return fail("activation tensor map rejected by the driver");
-  {
+  if (small.bn > 0) {
+    cuuint64_t gdim[3] = {(cuuint64_t)cb, (cuuint64_t)cs.OC, (cuuint64_t)k_iters_host};
+    cuuint64_t gstr[2] = {(cuuint64_t)cs.K() * es, (cuuint64_t)swz};
+    cuuint32_t box[3] = {(cuuint32_t)cb, (cuuint32_t)bn, (cuuint32_t)small.kpb};
+    cuuint32_t estr[3] = {1, 1, 1};
+    rc = g_encode_tiled(&kp.tmB, dtype, 3, const_cast<void*>(w_packed), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return fail("weight tensor map rejected by the driver");
+  } else {
     const int64_t ktot = cs.K();
     cuuint64_t gdim[2] = {(cuuint64_t)ktot, (cuuint64_t)cs.OC};
     cuuint64_t gstr[1] = {(cuuint64_t)ktot * es};
@@ -395,7 +484,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   {
     const size_t b_total = (size_t)k_iters_host * bn * swz;
     // Measured (i8, M=802816): 3x3 64->64 125.1 us against 137.6 us, 1x1 256->64 53.6 against 55.6, 1x1 256->128 215.4 against 221.6.
-    if (!pair && splits == 1 && n_tiles == 1 && b_total <= 48 * 1024 && m_tiles >= 2 * sms) kp.b_resident_bytes = (uint32_t)b_total;
+    if (!pair && small.bn == 0 && splits == 1 && n_tiles == 1 && b_total <= 48 * 1024 && m_tiles >= 2 * sms) kp.b_resident_bytes = (uint32_t)b_total;
   }
   const size_t kb_bytes = (size_t)(BLOCK_M + (kp.b_resident_bytes ? 0 : (pair ? bn / 2 : bn))) * swz;
   int kpb = 1;
@@ -425,7 +514,18 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // the staged row was sized for one run per store; the unsplit loop stores a warp's whole share at once
     if (!have_ws && kp.out_tma && (int)warp_row_bytes(bn, kind, dt_size(e.out_dt), false) != kp.out_row_bytes) kp.out_tma = 0;
   }
-  layout_smem(kp, bn, kind, pair, &pl->smem);
+  if (small.bn > 0) {
+    kp.small_bn = bn;
+    kp.a_rows = a_rows;
+    kp.splits = small.splits;
+    kp.k_per = small.k_per;
+    kp.kpb = small.kpb;
+    kp.stages = small.stages;
+    kp.stage_off = (uint32_t)(small.stages * small.stage_bytes);
+    pl->smem = small.smem;
+  } else {
+    layout_smem(kp, bn, kind, pair, &pl->smem);
+  }
   kp.mode = e.mode;
   if (e.mode == EPI_F32) kp.variant = (e.residual ? V_F32_RES : V_F32_BASE) + e.act * 2 + (e.round_tf32 ? 1 : 0);
   else if (e.mode == EPI_REQUANT) {
@@ -464,7 +564,10 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   pl->kind = kind;
   pl->device = device;
   pl->pair = pair ? 1 : 0;
-  if (pair) {
+  pl->small = small.bn > 0 ? 1 : 0;
+  if (pl->small) {
+    pl->grid = (int)(m_tiles * n_tiles * kp.splits);
+  } else if (pair) {
     // as many pairs as the device can hold at once (an odd SM of a cluster-scheduling group stays idle)
     int max_pairs = 0;
     try {
@@ -482,7 +585,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   char split_note[24] = "";
   if (kp.splits > 1) snprintf(split_note, sizeof split_note, " splitK=%d", kp.splits);
   snprintf(pl->desc, sizeof pl->desc, "umma_%s M=%lld N=%d K=%lld tile=%dx%dx%dB stages=%dx%d %s%s%s", kname, (long long)M, cs.OC, (long long)cs.K(),
-           pair ? 256 : 128, bn, swz, kp.stages, kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? " cta-pair" : "");
+           pair ? 256 : a_rows, bn, swz, kp.stages, kp.kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? " cta-pair" : (pl->small ? " small" : ""));
   return pl;
 }
 
@@ -582,6 +685,7 @@ UmmaPlan* umma_plan_create_batched(const BatchedGemm& g, std::string* why) {
   pl->bn = bn;
   pl->kind = KIND_TF32;
   pl->pair = 0;
+  pl->small = 0;
   pl->device = current_device();
   pl->grid = (int)std::min<int64_t>(items * m_tiles * n_tiles, sm_count(pl->device));
   snprintf(pl->desc, sizeof pl->desc, "umma_tf32 batched %lldx(M=%d N=%d K=%d) tile=128x%dx%dB stages=%dx%d", (long long)items, g.M, g.N, g.K, bn, swz, kp.stages, kpb);
@@ -833,7 +937,11 @@ bool umma_chain_launch(const UmmaChain* c, int* err_flag, const float* head_x, c
 void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s) {
   KParams kp = p->kp;
   kp.err_flag = err_flag;
-  if (p->kind == KIND_I8) launch_kind_i8(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
+  if (p->small) {
+    if (p->kind == KIND_I8) launch_small_i8(kp, p->grid, p->smem, p->device, s);
+    else if (p->kind == KIND_TF32) launch_small_tf32(kp, p->grid, p->smem, p->device, s);
+    else launch_small_f16(kp, p->grid, p->smem, p->device, s);
+  } else if (p->kind == KIND_I8) launch_kind_i8(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   else if (p->kind == KIND_TF32) launch_kind_tf32(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   else launch_kind_f16(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   OXB_CUDA(cudaGetLastError());

@@ -18,6 +18,7 @@
 #include <mutex>
 #include <string>
 
+#include "pdl.cuh"
 #include "umma_kernel.cuh"
 
 namespace oxb {
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_s = tmem_base_slot, tmem_o = tmem_base_slot + 128u;
+  pdl_enter();
   auto give_up = [&](int code) {
     if (!*abortp) {
       *abortp = 1;
@@ -396,8 +398,7 @@ void umma_attention_launch(const UmmaAttentionPlan* p, int* err_flag, cudaStream
   }
   AttnParams ap = p->ap;
   ap.err_flag = err_flag;
-  umma_attention_kernel<<<p->grid, ATT_THREADS, ATT_SMEM, s>>>(ap);
-  OXB_CUDA(cudaGetLastError());
+  launch(umma_attention_kernel, p->grid, ATT_THREADS, ATT_SMEM, s, ap);
 }
 
 }  // namespace k

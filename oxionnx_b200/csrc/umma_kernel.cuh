@@ -94,6 +94,7 @@ struct alignas(64) KParams {
   // > 0: the layer has one channel tile and its whole packed weight matrix (this many bytes) stays in shared memory
   // in front of the ring for the life of the CTA; ring stages then hold activation blocks only
   uint32_t b_resident_bytes;
+  int small_bn, a_rows;  // small-problem kernel only: the tile's channels, the rows of an activation box
   // epilogue
   int mode;
   int variant;  // which epilogue_math instantiation runs
@@ -659,11 +660,10 @@ __device__ __forceinline__ void math_dequant(const KParams& p, const uint32_t (&
 // the whole tile loop of an epilogue warp is instantiated per variant, so the code a warp runs
 // is one straight body without a dispatch inside the loop.
 template <int KIND, int VARIANT>
-__device__ __forceinline__ void epilogue_chunk(const KParams& p, const uint32_t (&v)[32], int xz, int oc, size_t esz, const float* res, uint32_t (&w)[32]) {
+__device__ __forceinline__ void epilogue_chunk(const KParams& p, const uint32_t (&v)[32], int xz, float xs, int oc, size_t esz, const float* res, uint32_t (&w)[32]) {
   if constexpr (VARIANT < V_F32_RES) math_f32<KIND, VARIANT / 2, VARIANT & 1, false>(p, v, p.bias_f + oc, p.slope + oc, nullptr, w);
   else if constexpr (VARIANT < V_REQUANT) math_f32<KIND, (VARIANT - V_F32_RES) / 2, (VARIANT - V_F32_RES) & 1, true>(p, v, p.bias_f + oc, p.slope + oc, res, w);
   else if constexpr (VARIANT >= V_DEQUANT) {
-    const float xs = __ldg(p.dq_x_scale);
     math_dequant<((VARIANT - V_DEQUANT) & 1) != 0, (VARIANT - V_DEQUANT) / 2>(p, v, p.bias_i + oc, p.wsum + oc, p.dq_w_scale + oc, p.dq_bias + oc, xz, xs, w);
   } else if constexpr (VARIANT == V_REQUANT) math_int<true, false>(p, v, p.bias_i + oc, nullptr, p.combined + oc, xz, esz, w);
   else if constexpr (VARIANT == V_REQUANT_DYN) math_int<true, true>(p, v, p.bias_i + oc, p.wsum + oc, p.combined + oc, xz, esz, w);
@@ -783,6 +783,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
   const int first = (slot % ES::WPQ) * CPW;
   int xz = 0;
   if (p.x_zp_dev) xz = __float2int_rn(*p.x_zp_dev);
+  const float xs = VARIANT >= V_DEQUANT ? *p.dq_x_scale : 0.f;
   const size_t esz = (p.out_dt == (int)DT::F32 || p.out_dt == (int)DT::I32) ? 4 : ((p.out_dt == (int)DT::I16 || p.out_dt == (int)DT::F16 || p.out_dt == (int)DT::BF16) ? 2 : 1);
   const int chunk_bytes = 32 * (int)esz;
   const int pitch = p.out_row_bytes;  // staged row length: 32, 64 or 128 bytes, at most one warp's share of a row
@@ -835,7 +836,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
     };
     auto math = [&](const uint32_t(&v)[32], int ch) {
       const float* res = (VARIANT >= V_F32_RES && VARIANT < V_REQUANT && row_ok) ? p.residual + (size_t)m * p.OC + oc0 + ch * 32 : nullptr;
-      epilogue_chunk<KIND, VARIANT>(p, v, xz, oc0 + ch * 32, esz, res, w);
+      epilogue_chunk<KIND, VARIANT>(p, v, xz, xs, oc0 + ch * 32, esz, res, w);
       if (track && row_ok) {
         const int valid = p.OC - (oc0 + ch * 32);  // lanes of a ragged last run hold no output
         if (valid >= 32) {
@@ -1309,6 +1310,11 @@ constexpr int kMaxDevices = 64;
 void launch_kind_i8(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
 void launch_kind_tf32(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
 void launch_kind_f16(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
+// The small-problem kernel (umma_small.cuh): one tile, or one K slice of a tile, per CTA.
+constexpr int SMALL_SMEM_MAX = 220 * 1024;
+void launch_small_i8(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
+void launch_small_tf32(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
+void launch_small_f16(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
 // How many CTA pairs of the 256-wide kernel of this kind can be resident at once on `device`.
 int max_pairs_kind_i8(size_t smem, int device);
 int max_pairs_kind_tf32(size_t smem, int device);

@@ -28,3 +28,55 @@ def test_dispatch_plans_follow_their_operands():
             assert np.array_equal(z, np.maximum(want, 0))
             y.release()
     ctx.close()
+
+
+def _run(graph, weights, feeds, **tuning):
+    b = Session.builder()
+    if "kernel_path" in tuning:
+        b = b.with_kernel_path(tuning.pop("kernel_path"))
+    sess = b.with_tuning(**tuning).build_from_graph(graph, weights)
+    out = sess.run(feeds)
+    kernels = [s["kernel"] for s in sess.steps()]
+    sess.close()
+    return out, kernels
+
+
+# batch, channels, height, width, filters, kernel, stride: ragged row and channel tiles, slices of uneven length
+SHAPES = [(1, 32, 1, 1, 32, 1, 1), (1, 64, 5, 7, 40, 3, 1), (1, 128, 13, 11, 96, 1, 1), (1, 512, 7, 7, 512, 3, 1), (2, 256, 9, 9, 1000, 1, 1), (1, 2048, 1, 1, 1000, 1, 1),
+          (1, 64, 17, 16, 64, 3, 2), (3, 384, 7, 7, 130, 3, 1)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("requant", ["packed", "f64", "union"])
+def test_small_integer_convolutions_match_the_direct_kernel(shape, requant):
+    n, c, h, w, oc, k, stride = shape
+    rng = np.random.default_rng([n, c, h, oc, k])
+    weights = {"w": rng.integers(-127, 128, (oc, c, k, k)).astype(np.float32), "ws": rng.uniform(0.001, 0.01, oc).astype(np.float32),
+               "wz": np.zeros(oc, np.float32), "b": rng.integers(-1000, 1001, oc).astype(np.float32), "xs": np.float32([0.02]), "z0": np.float32([0]),
+               "ys": np.float32([0.05 * np.sqrt(c * k * k)]), "yz": np.float32([0 if requant == "union" else 128])}
+    nodes = [Node("QuantizeLinear", "q", ["x", "xs", "z0"], ["xq"], {}),
+             Node("QLinearConv", "conv", ["xq", "xs", "z0", "w", "ws", "wz", "ys", "yz", "b"], ["yq"], {"strides": [stride] * 2, "pads": [k // 2] * 4}),
+             Node("DequantizeLinear", "dq", ["yq", "ys", "yz"], ["y"], {})]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds, requant_f64=1 if requant == "f64" else 0)
+    assert any("small" in s for s in kernels), kernels
+    want, _ = _run(graph, weights, feeds, kernel_path="direct")
+    assert np.array_equal(got["y"], want["y"])
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("precision", ["tf32", "bf16"])
+def test_small_float_convolutions_match_the_direct_kernel(shape, precision):
+    n, c, h, w, oc, k, stride = shape
+    rng = np.random.default_rng([n, c, h, oc, k, 1])
+    weights = {"w1": (rng.standard_normal((oc, c, k, k)) / np.sqrt(c * k * k)).astype(np.float32), "b1": rng.standard_normal(oc).astype(np.float32)}
+    attrs = {"strides": [stride] * 2, "pads": [k // 2] * 4}
+    nodes = [Node("Relu", "pre", ["x"], ["x1"], {}), Node("Conv", "c1", ["x1", "w1", "b1"], ["y"], dict(attrs, activation="relu"))]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds, float_precision=precision)
+    assert any("small" in s for s in kernels), kernels
+    want, _ = _run(graph, weights, feeds, kernel_path="direct")
+    tol = 2e-3 if precision == "tf32" else 2e-2
+    assert np.all(np.abs(got["y"] - want["y"]) <= tol * np.abs(want["y"]) + tol * np.abs(want["y"]).max())
