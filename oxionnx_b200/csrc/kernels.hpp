@@ -313,6 +313,7 @@ struct FusedAttention {
   const float* q = nullptr;
   const float* k = nullptr;
   const float* vt = nullptr;
+  const float* v = nullptr;  // attention_f32: V as it is, [B * S, H * D]
   float* out = nullptr;
   int64_t o_rows = 0, o_cols = 0;
   int o_rb = 0, o_rh = 0, o_ch = 0;
@@ -322,6 +323,10 @@ struct FusedAttention {
   int round_probs = 1;                  // the probabilities feed a TF32 product
   unsigned int* minmax_keys = nullptr;  // as Epilogue::minmax_keys, for the context
 };
+// The same chain in f32 on the CUDA cores for any S up to this and D = 64, reading V in place and writing
+// [B * S, H * D]; bit for bit what transposes, matmul_f32_direct and softmax_rows give.
+constexpr int kAttentionF32MaxS = 1024;
+void attention_f32(const FusedAttention& a, cudaStream_t s);
 struct UmmaAttentionPlan;
 UmmaAttentionPlan* umma_attention_create(const FusedAttention& a, std::string* why);
 void umma_attention_destroy(UmmaAttentionPlan* p);

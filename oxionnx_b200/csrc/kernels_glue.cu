@@ -1640,6 +1640,146 @@ __global__ void softmax_rows_reg_kernel(const float4* __restrict__ x, float4* __
   }
 }
 
+// An attention layer's f32 side (scores, scale + mask + softmax, context) for heads of 64 lanes and any number of
+// positions the tensor-core kernel does not take, in one launch that reads Q, K and V as column windows of their
+// [B * S, H * 64] matrices and writes the context merged.  It replaces three transposes, two 32 x 32-tile products
+// and a softmax (eight launches a layer with the head merge), and gives their results bit for bit: every score and
+// every context lane is one chain of fused multiply-adds in ascending k, and a row's exponentials are summed by the
+// lanes of one warp in the order softmax_rows uses.
+//
+// Bound by the FMA pipe for long sequences (4 * S * S * 64 per head) and by latency for short ones.  A block takes TM
+// query rows of one head, so that short batches still fill the chip; a thread holds RM x 4 results, which takes one
+// 16-byte read of each operand per RM x 4 FMAs, and K is kept transposed so that both are conflict free.  The
+// block's score rows stay in shared memory.  A layer of 2 x 77 positions, 12 heads: 60 us in eight launches -> 15 us.
+template <int TM>
+__global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ kk, const float* __restrict__ v,
+                                                            float* __restrict__ out, int S, int H, const float* __restrict__ scale,
+                                                            const float* __restrict__ mask, unsigned int* minmax_keys) {
+  pdl_enter();
+  constexpr int D = 64, RM = TM / 8, KP = 68, QP = TM + 4;
+  extern __shared__ __align__(16) float att_smem[];
+  float* qs = att_smem;          // [64][QP], transposed
+  float* kv = qs + D * QP;       // K tile [64 lanes][KP keys], then V tile [64 keys][64 lanes]
+  float* ps = kv + D * KP;       // [TM][pitch] scores, then probabilities
+  const int pitch = ((S + 63) & ~63) + 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.y / H, h = blockIdx.y - b * H;
+  const int row0 = blockIdx.x * TM;
+  const int64_t ld = (int64_t)H * D;
+  const float* qb = q + ((int64_t)b * S + row0) * ld + h * D;
+  const float* kb = kk + (int64_t)b * S * ld + h * D;
+  const float* vb = v + (int64_t)b * S * ld + h * D;
+  const int rows = min(TM, S - row0);
+  for (int i = tid; i < TM * 16; i += 128) {  // 16 rows x 32 bytes per warp and pass
+    const int r = (i & 15) + ((i >> 8) << 4), d4 = ((i >> 4) & 15) * 4;
+    const float4 t = r < rows ? *reinterpret_cast<const float4*>(qb + (int64_t)r * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    qs[(d4 + 0) * QP + r] = t.x, qs[(d4 + 1) * QP + r] = t.y, qs[(d4 + 2) * QP + r] = t.z, qs[(d4 + 3) * QP + r] = t.w;
+  }
+  const int kg = (tid & 15) * 4, rg = (tid >> 4) * RM;  // this thread's four keys (or lanes) and RM rows
+  for (int k0 = 0; k0 < S; k0 += 64) {
+    for (int i = tid; i < 64 * 16; i += 128) {
+      const int key = (i & 15) + ((i >> 8) << 4), d4 = ((i >> 4) & 15) * 4;
+      const float4 t = k0 + key < S ? *reinterpret_cast<const float4*>(kb + (int64_t)(k0 + key) * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      kv[(d4 + 0) * KP + key] = t.x, kv[(d4 + 1) * KP + key] = t.y, kv[(d4 + 2) * KP + key] = t.z, kv[(d4 + 3) * KP + key] = t.w;
+    }
+    __syncthreads();
+    float acc[RM][4];
+#pragma unroll
+    for (int r = 0; r < RM; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+#pragma unroll 8
+    for (int d = 0; d < D; ++d) {
+      const float4 kf = *reinterpret_cast<const float4*>(kv + d * KP + kg);
+      float qf[RM];
+      if (RM == 4) *reinterpret_cast<float4*>(qf) = *reinterpret_cast<const float4*>(qs + d * QP + rg);
+      else *reinterpret_cast<float2*>(qf) = *reinterpret_cast<const float2*>(qs + d * QP + rg);
+#pragma unroll
+      for (int r = 0; r < RM; ++r) {
+        acc[r][0] = fmaf(qf[r], kf.x, acc[r][0]);
+        acc[r][1] = fmaf(qf[r], kf.y, acc[r][1]);
+        acc[r][2] = fmaf(qf[r], kf.z, acc[r][2]);
+        acc[r][3] = fmaf(qf[r], kf.w, acc[r][3]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RM; ++r) *reinterpret_cast<float4*>(ps + (rg + r) * pitch + k0 + kg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    __syncthreads();
+  }
+  const float sc = scale ? scale[0] : 1.f;
+  const float* pm = mask ? mask + (int64_t)b * S : nullptr;
+  for (int r = warp; r < TM; r += 4) {
+    float* row = ps + r * pitch;
+    float mx = -INFINITY;
+    for (int k = lane; k < S; k += 32) {
+      float x = row[k];
+      if (scale) x = __fmul_rn(x, sc);
+      if (pm) x = __fadd_rn(x, pm[k]);
+      row[k] = x;
+      mx = fmaxf(mx, x);
+    }
+    mx = warp_max(mx);
+    float sum = 0.f;
+    for (int k = lane; k < S; k += 32) {
+      const float e = expf(__fsub_rn(row[k], mx));
+      row[k] = e;
+      sum += e;
+    }
+    const float inv = __frcp_rn(warp_sum(sum));
+    for (int k = lane; k < S; k += 32) row[k] = round_tf32(__fmul_rn(row[k], inv));  // the probabilities feed a contraction
+    for (int k = S + lane; k < pitch; k += 32) row[k] = 0.f;
+  }
+  float acc[RM][4];
+#pragma unroll
+  for (int r = 0; r < RM; ++r)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+  for (int k0 = 0; k0 < S; k0 += 64) {
+    __syncthreads();
+    const int n = min(64, S - k0);
+    for (int i = tid; i < 64 * 16; i += 128) {
+      const int key = i >> 4, d4 = (i & 15) * 4;
+      *reinterpret_cast<float4*>(kv + key * D + d4) =
+          key < n ? *reinterpret_cast<const float4*>(vb + (int64_t)(k0 + key) * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int k4 = 0; k4 < n; k4 += 4) {  // lanes past the last position multiply zeros, as the padded slabs of the plain product do
+      float pf[RM][4];
+#pragma unroll
+      for (int r = 0; r < RM; ++r) *reinterpret_cast<float4*>(pf[r]) = *reinterpret_cast<const float4*>(ps + (rg + r) * pitch + k0 + k4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 vf = *reinterpret_cast<const float4*>(kv + (k4 + j) * D + kg);
+#pragma unroll
+        for (int r = 0; r < RM; ++r) {
+          acc[r][0] = fmaf(pf[r][j], vf.x, acc[r][0]);
+          acc[r][1] = fmaf(pf[r][j], vf.y, acc[r][1]);
+          acc[r][2] = fmaf(pf[r][j], vf.z, acc[r][2]);
+          acc[r][3] = fmaf(pf[r][j], vf.w, acc[r][3]);
+        }
+      }
+    }
+  }
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int r = 0; r < RM; ++r) {
+    if (rg + r >= rows) continue;
+    *reinterpret_cast<float4*>(out + ((int64_t)b * S + row0 + rg + r) * ld + h * D + kg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) lo = fminf(lo, acc[r][e]), hi = fmaxf(hi, acc[r][e]);
+  }
+  if (minmax_keys) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = warp_max(hi);
+    if (lane == 0 && lo != INFINITY) {
+      atomicMin(minmax_keys, float_key(lo));
+      atomicMax(minmax_keys + 1, float_key(hi));
+    }
+  }
+}
+
 // LayerNormalization for rows of 128 * NV4 lanes, the row kept in registers (read once, in 16-byte pieces).
 template <int NV4>
 __global__ void layer_norm_rows_reg_kernel(const float4* __restrict__ x, const float4* __restrict__ x2, float4* __restrict__ y, int64_t rows,
@@ -2244,6 +2384,37 @@ void softmax_rows(const float* x, float* y, int64_t rows, int64_t n, const float
     return;
   }
   launch(softmax_rows_kernel, grid_for(rows * 32), kThreads, 0, s, x, y, rows, n, scale, mask, rpm, round_tf32_flag);
+}
+
+namespace {
+template <int TM>
+size_t attention_f32_smem(int S) {
+  return (size_t)(64 * (TM + 4) + 64 * 68 + TM * (((S + 63) & ~63) + 4)) * sizeof(float);
+}
+
+template <int TM>
+void attention_f32_launch(const FusedAttention& a, cudaStream_t s) {
+  // the opt-in for more than 48 KB of dynamic shared memory is a per-device property of the kernel
+  static std::mutex mu;
+  static bool have[64] = {};
+  int device = 0;
+  OXB_CUDA(cudaGetDevice(&device));
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!have[device & 63]) {
+      OXB_CUDA(cudaFuncSetAttribute(attention_f32_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_f32_smem<TM>(kAttentionF32MaxS)));
+      have[device & 63] = true;
+    }
+  }
+  launch(attention_f32_kernel<TM>, dim3((unsigned)ceil_div(a.S, TM), (unsigned)(a.B * a.H)), 128, attention_f32_smem<TM>(a.S), s, a.q, a.k, a.v, a.out, a.S, a.H,
+         a.scale, a.mask, a.minmax_keys);
+}
+}  // namespace
+
+// 16 query rows per block while 32 would leave SMs without two (2 sequences of 77: 120 blocks instead of 72).
+void attention_f32(const FusedAttention& a, cudaStream_t s) {
+  if ((int64_t)a.B * a.H * ceil_div(a.S, 32) < 2 * 148) attention_f32_launch<16>(a, s);
+  else attention_f32_launch<32>(a, s);
 }
 
 void layer_norm_rows(const float* x, float* y, int64_t rows, int64_t n, const float* scale, const float* bias, float eps, cudaStream_t s,

@@ -1004,7 +1004,7 @@ void Planner::plan_dynamic_quantize(const NodeDef& n) {
   // is built when the arena is laid out and reads the value's keys then).
   if (!C.cfg().keep_intermediates && V(xi).alias_of < 0 && V(xi).producer >= 0 && V(xi).producer < (int)S.steps_.size() &&
       (S.steps_[V(xi).producer].kernel == "layer_norm_rows" || S.steps_[V(xi).producer].kernel == "add+layer_norm_rows" ||
-       (S.steps_[V(xi).producer].kernel == "umma" && S.steps_[V(xi).producer].family == 0)) &&
+       S.steps_[V(xi).producer].kernel == "attention_f32" || (S.steps_[V(xi).producer].kernel == "umma" && S.steps_[V(xi).producer].family == 0)) &&
       V(xi).minmax_keys == nullptr) {
     V(xi).minmax_keys = scratch;
     have_minmax = true;
@@ -2685,7 +2685,8 @@ void Planner::plan_transpose(const NodeDef& n) {
     auto it = consumers_.find(n.outputs[0]);
     const bool to_matmul = it != consumers_.end() && it->second.size() == 1 && nodes_[it->second[0].first].op == "MatMul";
     const int64_t B = xv.shape[0], Sq = xv.shape[1], H = xv.shape[2], D = xv.shape[3];
-    if ((p0 || p1) && to_matmul && root != xi && V(root).shape == std::vector<int64_t>{B * Sq, H * D} && V(root).host == nullptr && Sq % 128 == 0 && D % 8 == 0) {
+    if ((p0 || p1) && to_matmul && root != xi && V(root).shape == std::vector<int64_t>{B * Sq, H * D} && V(root).host == nullptr &&
+        ((Sq % 128 == 0 && D % 8 == 0) || (D == 64 && Sq <= k::kAttentionF32MaxS))) {
       lazy_heads_[yi] = LazyHeads{xi, root, B, Sq, H, D, p0 ? 0 : 1, cur_node_, perm, false};
       return;
     }
@@ -2740,6 +2741,7 @@ bool Planner::try_plan_attention_product(const NodeDef& n, int ai, int bi) {
   std::string label;
   if (a_lazy && la->second.kind == 0 && hb.kind == 1 && la->second.B == B && la->second.S == Sq && la->second.H == H && la->second.D == D) {
     if (try_plan_fused_attention(n, ai, bi)) return true;
+    if (Sq % 128 != 0) return false;
     // scores
     g.M = (int)Sq, g.N = (int)Sq, g.K = (int)D;
     g.a_rows = B * Sq, g.a_cols = H * D, g.a_rb = (int)Sq, g.a_rh = 0, g.a_ch = (int)D;
@@ -2749,7 +2751,7 @@ bool Planner::try_plan_attention_product(const NodeDef& n, int ai, int bi) {
     g.round_tf32 = feeds_contraction(n.outputs[0]) ? 1 : 0;
     reads = {la->second.root_vi, hb.root_vi};
     label = "scores";
-  } else if (!a_lazy && hb.kind == 0 && V(ai).dt == DT::F32 && V(ai).shape == std::vector<int64_t>{B, H, Sq, Sq} && V(ai).layout == Layout::PLAIN &&
+  } else if (!a_lazy && Sq % 128 == 0 && hb.kind == 0 && V(ai).dt == DT::F32 && V(ai).shape == std::vector<int64_t>{B, H, Sq, Sq} && V(ai).layout == Layout::PLAIN &&
              V(ai).host == nullptr) {
     // context: V^T per head first
     const int vt = add_value(V(hb.src_vi).name + "@heads_t", {B, H, D, Sq}, DT::F32, Layout::PLAIN);
@@ -2824,7 +2826,9 @@ bool Planner::try_plan_fused_attention(const NodeDef& n, int qi, int ki) {
   if (C.cfg().keep_intermediates || C.cfg().kernel_path != 0 || !k::umma_available()) return false;
   const LazyHeads hq = lazy_heads_.find(qi)->second, hk = lazy_heads_.find(ki)->second;
   const int64_t B = hq.B, Sq = hq.S, H = hq.H, D = hq.D;
-  if (Sq != 128 || D != 64 || B * H > 0x3fffffffLL) return false;
+  // 128 positions: on the tensor cores; a number the tensor-core products do not take: in f32 on the CUDA cores
+  const bool simt = Sq % 128 != 0;
+  if (!(Sq == 128 || (simt && Sq <= k::kAttentionF32MaxS && B * H <= 65535)) || D != 64 || B * H > 0x3fffffffLL) return false;
   auto only_user = [&](const std::string& name, const char* opn) -> int {
     if (graph_outputs_.count(name)) return -1;
     auto it = consumers_.find(name);
@@ -2883,16 +2887,41 @@ bool Planner::try_plan_fused_attention(const NodeDef& n, int qi, int ki) {
   } else {
     t_i = -1;
   }
+  if (simt && r_i < 0) return false;  // writes the merged form only
   // from here on the plan is committed
   const float* dscale = (const float*)C.resident_form(mul.inputs[s_slot], "raw_f32", 4, [sc](void* p) { std::memcpy(p, sc->data.data(), 4); },
                                                       cacheable_const(mul.inputs[s_slot]));
-  const int vt = add_value(V(hv.src_vi).name + "@heads_t", {B, H, D, Sq}, DT::F32, Layout::PLAIN);
-  emit_transpose(nodes_[hv.node], hv.src_vi, {0, 2, 3, 1}, vt);
+  int vt = -1;
+  if (!simt) {
+    vt = add_value(V(hv.src_vi).name + "@heads_t", {B, H, D, Sq}, DT::F32, Layout::PLAIN);
+    emit_transpose(nodes_[hv.node], hv.src_vi, {0, 2, 3, 1}, vt);
+  }
   skipped_[mul_i] = skipped_[add_i] = skipped_[sm_i] = skipped_[av_i] = 1;
   if (t_i >= 0) skipped_[t_i] = skipped_[r_i] = 1;
   lazy_heads_.find(qi)->second.materialised = lazy_heads_.find(ki)->second.materialised = lv->second.materialised = true;
   const int out_vi = add_value(out_name, oshape, DT::F32, Layout::PLAIN);
   const int q_root = hq.root_vi, k_root = hk.root_vi;
+  if (simt) {
+    const int v_root = hv.root_vi;
+    Step& st = add_step(av, "attention_f32", 1, {q_root, k_root, v_root, mi}, {out_vi});
+    st.work = 4.0 * (double)B * H * Sq * Sq * D;
+    st.work_is_bytes = false;
+    st.launch = [this, q_root, k_root, v_root, mi, out_vi, dscale, B, H, Sq, D](cudaStream_t s) {
+      k::FusedAttention fa;
+      fa.q = (const float*)V(q_root).ptr;
+      fa.k = (const float*)V(k_root).ptr;
+      fa.v = (const float*)V(v_root).ptr;
+      fa.out = (float*)V(out_vi).ptr;
+      fa.B = (int)B, fa.H = (int)H, fa.S = (int)Sq, fa.D = (int)D;
+      fa.scale = dscale;
+      fa.mask = (const float*)V(mi).ptr;
+      fa.minmax_keys = (unsigned int*)V(out_vi).minmax_keys;
+      k::attention_f32(fa, s);
+      C.counters.simt_launches++;
+      C.counters.kernel_launches++;
+    };
+    return true;
+  }
   Step& st = add_step(av, "umma", 0, {q_root, k_root, vt, mi}, {out_vi});
   st.work = 4.0 * (double)B * H * Sq * Sq * D;
   st.work_is_bytes = false;

@@ -80,3 +80,15 @@ def test_small_float_convolutions_match_the_direct_kernel(shape, precision):
     want, _ = _run(graph, weights, feeds, kernel_path="direct")
     tol = 2e-3 if precision == "tf32" else 2e-2
     assert np.all(np.abs(got["y"] - want["y"]) <= tol * np.abs(want["y"]) + tol * np.abs(want["y"]).max())
+
+
+@pytest.mark.parametrize("batch,seq", [(1, 1), (1, 16), (2, 33), (3, 63), (2, 65), (1, 127), (4, 129), (2, 320), (1, 513)])
+def test_attention_at_ragged_lengths_is_the_separate_nodes_bit_for_bit(batch, seq):
+    graph, weights, feeds, _ = models.build_bert_dynamic_int8(batch=batch, seq=seq, hidden=128, heads=2, ffn=128, layers=2, vocab=100)
+    f = feeds()
+    f["attention_mask"][:, (seq + 1) // 2:] = 0
+    f["attention_mask"][0] = 1
+    got, kernels = _run(graph, weights, f)
+    assert kernels.count("attention_f32") == 2, kernels
+    want, _ = _run(graph, weights, f, keep_intermediates=True)
+    assert np.array_equal(got["hidden"], want["hidden"])
