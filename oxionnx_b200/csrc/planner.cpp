@@ -588,12 +588,22 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
     int vi = it->second;
     V(vi).is_graph_output = true;
     out_node.name = o;
-    bool direct = V(vi).dt == DT::F32 && (effective_layout(V(vi)) == Layout::PLAIN || order_free(V(vi))) && V(vi).alias_of < 0 &&
-                  !V(vi).is_graph_input && V(vi).host == nullptr;
-    if (direct) {
-      // give the value its own persistent storage instead of an arena slot
-      V(vi).external = true;
-      V(vi).ptr = owned_buffer(std::max<size_t>(V(vi).bytes, 256));
+    // An output whose storage already holds the lanes in the logical order is handed out as it is, and so is a view of
+    // such a value (Reshape, Flatten): the storage moves out of the arena into a persistent buffer.
+    int root = vi;
+    bool plain = true;
+    while (plain) {
+      const Value& rv = V(root);
+      plain = rv.dt == DT::F32 && (effective_layout(rv) == Layout::PLAIN || order_free(rv)) && rv.numel() == V(vi).numel();
+      if (rv.alias_of < 0) break;
+      root = rv.alias_of;
+    }
+    if (plain && !V(root).is_graph_input && V(root).host == nullptr && V(root).producer >= 0) {
+      if (!V(root).external) {
+        V(root).external = true;
+        V(root).ptr = owned_buffer(std::max<size_t>(V(root).bytes, 256));
+      }
+      V(vi).ptr = V(root).ptr;
       S.output_staging_.push_back({o, vi});
       continue;
     }
@@ -624,6 +634,7 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
 // value, so other readers and kept intermediates see what the separate kernels would have produced.
 void Planner::link_chains() {
   size_t i = 0;
+  if (getenv("OXB_NOCHAIN")) return;
   while (i < chain_links_.size()) {
     size_t j = i + 1;
     while (j < chain_links_.size() && j - i < 4 && chain_links_[j].step == chain_links_[j - 1].step + 1 && chain_links_[j].rows == chain_links_[i].rows &&
