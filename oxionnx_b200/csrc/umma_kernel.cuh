@@ -54,6 +54,7 @@ namespace umma {
 constexpr int BLOCK_M = 128;
 constexpr int MAX_STAGES = 12;
 constexpr int MAX_ACC = 8;
+constexpr int MAX_RES_BUFS = 4;
 constexpr long long WAIT_CYCLES = 2000000000LL;  // ~1 s at 2 GHz
 
 // Kinds of the contraction: operand storage and tensor-core instruction.
@@ -67,6 +68,7 @@ struct alignas(64) KParams {
   CUtensorMap tmA;
   CUtensorMap tmB;
   CUtensorMap tmO;
+  CUtensorMap tmR;  // the residual in the boxes of tmO (res_bufs > 0)
   int out_tma, out_row_bytes;
   int a_im2col;
   int M, OC;
@@ -99,7 +101,14 @@ struct alignas(64) KParams {
   int mode;
   int variant;  // which epilogue_math instantiation runs
   const float* bias_f;
-  const float* residual;  // f32 [M, OC] added after the bias, or null
+  const void* residual;  // [M, OC] f32 added after the bias, or the 8-bit operand of a join; or null
+  // > 0: epilogue warps keep this many staging buffers each, fetch the residual's box for the store res_bufs - 2 (at
+  // least one) stores ahead into the buffer it will be stored from, and combine in place
+  int res_bufs;
+  // join variant: clamp((acc requantised and clamped to [lo, hi]) * join_a + residual * join_b + join_c) rounded to
+  // even, bounds join_lo .. join_hi; join_flip: the residual's lanes are signed
+  float join_a, join_b, join_c;
+  int join_lo, join_hi, join_flip;
   const float* slope;     // PRelu: per-channel slope, padded like the bias
   int act;
   float clip_lo, clip_hi;
@@ -332,8 +341,10 @@ enum {
   V_REQUANT_LEAN_DYN = 27,
   V_REQUANT_FBIAS = 28,  // LEAN with the bias added as a float after the conversion
   V_REQUANT_PACKED = 29, // FBIAS with the saturation done on packed 16-bit lanes (8-bit outputs of bounded magnitude)
-  V_DEQUANT = 30         // 30..35: dequantising variants, + (dynamic zero point ? 1 : 0) + 2 * activation
+  V_DEQUANT = 30,        // 30..35: dequantising variants, + (dynamic zero point ? 1 : 0) + 2 * activation
+  V_JOIN = 36            // PACKED, then joined with a quantised residual
 };
+__host__ __device__ constexpr bool variant_has_residual(int v) { return (v >= V_F32_RES && v < V_REQUANT) || v == V_JOIN; }
 
 __device__ __forceinline__ float act_f32(int act, float f, float slope, float lo, float hi) {
   if (act == 1) return fmaxf(f, 0.f);
@@ -369,20 +380,13 @@ __device__ __forceinline__ void pack_float(const float (&f)[4], int j4, int out_
 
 template <int KIND, int ACT, int RT, bool RES>
 __device__ __forceinline__ void math_f32(const KParams& p, const uint32_t (&v)[32], const float* __restrict__ bias, const float* __restrict__ slope,
-                                         const float* __restrict__ res, uint32_t (&w)[32]) {
-  // this pixel's 32 channels of the residual: one full 128-byte line per thread, all eight loads in flight
-  // together before the first is used
-  float4 rv[RES ? 8 : 1];
-  if (RES) {
-#pragma unroll
-    for (int j4 = 0; j4 < 8; ++j4) rv[j4] = res != nullptr ? __ldg(reinterpret_cast<const float4*>(res) + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+                                         const uint4 (&rv)[8], uint32_t (&w)[32]) {
 #pragma unroll
   for (int j4 = 0; j4 < 8; ++j4) {
     const float4 b = __ldg(reinterpret_cast<const float4*>(bias) + j4);
     const float bb[4] = {b.x, b.y, b.z, b.w};
     float rr[4] = {0.f, 0.f, 0.f, 0.f};
-    if (RES) rr[0] = rv[j4].x, rr[1] = rv[j4].y, rr[2] = rv[j4].z, rr[3] = rv[j4].w;
+    if (RES) rr[0] = __uint_as_float(rv[j4].x), rr[1] = __uint_as_float(rv[j4].y), rr[2] = __uint_as_float(rv[j4].z), rr[3] = __uint_as_float(rv[j4].w);
     float ss[4] = {0.f, 0.f, 0.f, 0.f};
     if (ACT == 4) {
       const float4 s = __ldg(reinterpret_cast<const float4*>(slope) + j4);
@@ -571,6 +575,16 @@ __device__ __forceinline__ void fma2(float& x0, float& x1, float y0, float y1, f
   asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(d));
 }
 
+// x = x * y + z, lane by lane with one factor
+__device__ __forceinline__ void fma2v(float& x0, float& x1, float y, float z0, float z1) {
+  uint64_t a, b, c, d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x0), "f"(x1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(b) : "f"(y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(c) : "f"(z0), "f"(z1));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(d));
+}
+
 // The one-FMA requantisation (see math_requant_fma; the float-bias form) for 8-bit outputs whose magnitude the
 // host has bounded below 2^15 from the weights and the scales: the rounded result sits in the low mantissa bits
 // of s = fma(a, c, 1.5 * 2^23 + zp), and because 1.5 * 2^23 has sixteen zero low bits, the low half-word of s is
@@ -602,6 +616,50 @@ __device__ __forceinline__ void math_requant_packed(const KParams& p, const uint
       p01 = __vmins2(__vmaxs2(p01, lo2), hi2);
       p23 = __vmins2(__vmaxs2(p23, lo2), hi2);
     }
+    w[j4] = __byte_perm(p01, p23, 0x6420);
+  }
+}
+
+// The requantisation above followed by the residual join of a quantised network, y = Q(relu?(DQ(a) + DQ(b))): the
+// requantised lane stays a float (clamped to its own range, which is what its 8-bit storage would have held), the
+// residual's bytes become floats through the mantissa of 2^23, and the join is a * join_a + b * join_b + join_c, rounded
+// to even and clamped as packed int16.  The host finds constants for which that equals the separate nodes' lane for
+// every one of the 256 x 256 input pairs (residual_join_constants), or the join stays a kernel of its own.
+__device__ __forceinline__ void math_join(const KParams& p, const uint32_t (&v)[32], const float* __restrict__ bias_f, const float* __restrict__ comb,
+                                          const uint4 (&rv)[8], uint32_t (&w)[32]) {
+  const float magic = 12582912.0f;
+  const float magic_zp = magic + (float)p.y_zp, flo = magic + (float)p.lo, fhi = magic + (float)p.hi;
+  const float b_off = p.join_flip ? -8388736.0f : -8388608.0f;
+  const uint32_t flip = p.join_flip ? 0x80808080u : 0u;
+  const uint32_t lo2 = ((uint32_t)p.join_lo & 0xffffu) * 0x00010001u, hi2 = ((uint32_t)p.join_hi & 0xffffu) * 0x00010001u;
+  const float jc = p.join_c, ja = p.join_a, jb = p.join_b;
+  const uint32_t rw[8] = {rv[0].x, rv[0].y, rv[0].z, rv[0].w, rv[1].x, rv[1].y, rv[1].z, rv[1].w};
+#pragma unroll
+  for (int j4 = 0; j4 < 8; ++j4) {
+    const float4 bi = __ldg(reinterpret_cast<const float4*>(bias_f) + j4);
+    const float4 c = __ldg(reinterpret_cast<const float4*>(comb) + j4);
+    float a0 = __int2float_rn((int32_t)v[4 * j4]), a1 = __int2float_rn((int32_t)v[4 * j4 + 1]);
+    float a2 = __int2float_rn((int32_t)v[4 * j4 + 2]), a3 = __int2float_rn((int32_t)v[4 * j4 + 3]);
+    add2(a0, a1, bi.x, bi.y);
+    add2(a2, a3, bi.z, bi.w);
+    fma2(a0, a1, c.x, c.y, magic_zp);
+    fma2(a2, a3, c.z, c.w, magic_zp);
+    a0 = fminf(fmaxf(a0, flo), fhi), a1 = fminf(fmaxf(a1, flo), fhi), a2 = fminf(fmaxf(a2, flo), fhi), a3 = fminf(fmaxf(a3, flo), fhi);
+    add2(a0, a1, -magic, -magic);
+    add2(a2, a3, -magic, -magic);
+    const uint32_t r = rw[j4] ^ flip;
+    float b0 = __uint_as_float(__byte_perm(r, 0x4B000000u, 0x7440)), b1 = __uint_as_float(__byte_perm(r, 0x4B000000u, 0x7441));
+    float b2 = __uint_as_float(__byte_perm(r, 0x4B000000u, 0x7442)), b3 = __uint_as_float(__byte_perm(r, 0x4B000000u, 0x7443));
+    add2(b0, b1, b_off, b_off);
+    add2(b2, b3, b_off, b_off);
+    fma2(b0, b1, jb, jb, jc);
+    fma2(b2, b3, jb, jb, jc);
+    fma2v(a0, a1, ja, b0, b1);
+    fma2v(a2, a3, ja, b2, b3);
+    add2(a0, a1, magic, magic);
+    add2(a2, a3, magic, magic);
+    const uint32_t p01 = __vmins2(__vmaxs2(__byte_perm(__float_as_uint(a0), __float_as_uint(a1), 0x5410), lo2), hi2);
+    const uint32_t p23 = __vmins2(__vmaxs2(__byte_perm(__float_as_uint(a2), __float_as_uint(a3), 0x5410), lo2), hi2);
     w[j4] = __byte_perm(p01, p23, 0x6420);
   }
 }
@@ -660,9 +718,11 @@ __device__ __forceinline__ void math_dequant(const KParams& p, const uint32_t (&
 // the whole tile loop of an epilogue warp is instantiated per variant, so the code a warp runs
 // is one straight body without a dispatch inside the loop.
 template <int KIND, int VARIANT>
-__device__ __forceinline__ void epilogue_chunk(const KParams& p, const uint32_t (&v)[32], int xz, float xs, int oc, size_t esz, const float* res, uint32_t (&w)[32]) {
-  if constexpr (VARIANT < V_F32_RES) math_f32<KIND, VARIANT / 2, VARIANT & 1, false>(p, v, p.bias_f + oc, p.slope + oc, nullptr, w);
-  else if constexpr (VARIANT < V_REQUANT) math_f32<KIND, (VARIANT - V_F32_RES) / 2, (VARIANT - V_F32_RES) & 1, true>(p, v, p.bias_f + oc, p.slope + oc, res, w);
+__device__ __forceinline__ void epilogue_chunk(const KParams& p, const uint32_t (&v)[32], int xz, float xs, int oc, size_t esz, const uint4 (&rv)[8],
+                                               uint32_t (&w)[32]) {
+  if constexpr (VARIANT < V_F32_RES) math_f32<KIND, VARIANT / 2, VARIANT & 1, false>(p, v, p.bias_f + oc, p.slope + oc, rv, w);
+  else if constexpr (VARIANT < V_REQUANT) math_f32<KIND, (VARIANT - V_F32_RES) / 2, (VARIANT - V_F32_RES) & 1, true>(p, v, p.bias_f + oc, p.slope + oc, rv, w);
+  else if constexpr (VARIANT == V_JOIN) math_join(p, v, p.bias_if + oc, p.combined + oc, rv, w);
   else if constexpr (VARIANT >= V_DEQUANT) {
     math_dequant<((VARIANT - V_DEQUANT) & 1) != 0, (VARIANT - V_DEQUANT) / 2>(p, v, p.bias_i + oc, p.wsum + oc, p.dq_w_scale + oc, p.dq_bias + oc, xz, xs, w);
   } else if constexpr (VARIANT == V_REQUANT) math_int<true, false>(p, v, p.bias_i + oc, nullptr, p.combined + oc, xz, esz, w);
@@ -677,6 +737,18 @@ __device__ __forceinline__ void epilogue_chunk(const KParams& p, const uint32_t 
   else {
     if (p.lo == 0) math_requant_packed<true>(p, v, p.bias_if + oc, p.combined + oc, w);
     else math_requant_packed<false>(p, v, p.bias_if + oc, p.combined + oc, w);
+  }
+}
+
+// This pixel's 32 channels of the residual straight from memory, all loads in flight together: 128 bytes of f32, or 32
+// bytes of 8-bit lanes (rv[0], rv[1]).
+template <int VARIANT>
+__device__ __forceinline__ void load_residual(const KParams& p, long long m, int oc, bool row_ok, uint4 (&rv)[8]) {
+  if constexpr (variant_has_residual(VARIANT)) {
+    constexpr int N = VARIANT == V_JOIN ? 2 : 8;
+    const uint4* src = reinterpret_cast<const uint4*>((const uint8_t*)p.residual + ((size_t)m * p.OC + oc) * (VARIANT == V_JOIN ? 1 : 4));
+#pragma unroll
+    for (int j = 0; j < N; ++j) rv[j] = row_ok ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 
@@ -771,8 +843,8 @@ struct EpiShape {
 // CTA's own, or the even CTA's for a pair (a shared::cluster address).
 template <int BN, int KIND, int VARIANT, bool SPLIT, bool PAIR>
 __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int lane, uint32_t tmem_base, uint64_t* bar_acc_full,
-                                              uint64_t* bar_acc_empty, uint32_t stage_addr, volatile int* abortp, int total_tiles, int tile0, int tile_step,
-                                              int pair_rank) {
+                                              uint64_t* bar_acc_empty, uint64_t* bar_res, uint32_t stage_addr, volatile int* abortp, int total_tiles,
+                                              int tile0, int tile_step, int pair_rank) {
   constexpr int EW = epi_warps(KIND);
   using ES = EpiShape<BN, EW>;
   constexpr int CPW = ES::CPW;
@@ -788,14 +860,44 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
   const int chunk_bytes = 32 * (int)esz;
   const int pitch = p.out_row_bytes;  // staged row length: 32, 64 or 128 bytes, at most one warp's share of a row
   const int cpg = p.out_tma ? pitch / chunk_bytes : 1;  // runs per staged store: 1, 2 or 4
-  const uint32_t stage_row_addr = stage_addr + (uint32_t)(lane * pitch);
+  uint32_t stage_base = stage_addr, stage_row_addr = stage_addr + (uint32_t)(lane * pitch);
   const uint32_t stage_xor = ((uint32_t)(lane * pitch) >> 7) & (uint32_t)(pitch / 16 - 1);
   uint32_t local = 0;
+  bool lost = false;  // a residual box did not arrive
   const bool plain = !p.batched && p.splits == 1;
   // extrema of the f32 lanes this thread writes, when a DynamicQuantizeLinear reads the output next
   const bool track = p.minmax_keys != nullptr && esz == 4 && (VARIANT < V_REQUANT || VARIANT >= V_DEQUANT);
   float seen_min = INFINITY, seen_max = -INFINITY;
   TileWalk walk(tile0, tile_step, p.n_tiles);
+  // residual boxes fetched ahead (res_bufs > 0; never with split K or batched products): `ahead` walks the stores that
+  // this warp will make, `fetched` and `used` count them
+  constexpr bool kRes = variant_has_residual(VARIANT) && !SPLIT;
+  const int nb = kRes ? p.res_bufs : 0;
+  const uint32_t buf_bytes = (uint32_t)(32 * pitch);
+  TileWalk ahead = walk;
+  int ahead_t = tile0, ahead_ch = first;
+  uint32_t ahead_local = 0, fetched = 0, used = 0;
+  auto fetch_next = [&]() {  // the residual of the next store not yet fetched, if there is one
+    while (ahead_t < total_tiles) {
+      const int a_end = min(first + CPW, min(BN, p.OC - ahead.n * BN + 31) / 32);
+      if ((ES::NG == 1 || (int)(ahead_local % ES::NG) == group) && ahead_ch < a_end) break;
+      ahead_t += tile_step;
+      ++ahead_local;
+      ahead.next();
+      ahead_ch = first;
+    }
+    if (ahead_t >= total_tiles) return;
+    if (lane == 0) {
+      const uint32_t b = fetched % (uint32_t)nb, bar = smem_u32(&bar_res[b]);
+      mbar_expect_tx(bar, buf_bytes);
+      tma_load_2d(stage_addr + b * buf_bytes, &p.tmR, bar, ahead.n * BN + ahead_ch * 32,
+                  ahead.m * (PAIR ? 2 * BLOCK_M : BLOCK_M) + (PAIR ? pair_rank * BLOCK_M : 0) + quarter * 32);
+    }
+    ++fetched;
+    ahead_ch += cpg;
+  };
+  if (kRes && nb > 0)
+    for (int i = 0; i < (nb > 2 ? nb - 2 : 1); ++i) fetch_next();
   for (int t = tile0; t < total_tiles; t += tile_step, ++local, walk.next()) {
     if (ES::NG > 1 && (int)(local % ES::NG) != group) continue;
     int tt = t, o_row0 = 0, o_col0 = 0;
@@ -825,6 +927,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
     const int n_chunks = min(BN, p.OC - oc0 + 31) / 32;  // uniform across the CTA
     const int end = min(first + CPW, n_chunks);           // this warp's runs: [first, end)
     uint32_t va[32], w[32];
+    uint4 rv[8];
 
     auto release = [&]() {  // every TMEM read of this warp for this tile has landed
       tc_fence_before();
@@ -835,8 +938,17 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
       }
     };
     auto math = [&](const uint32_t(&v)[32], int ch) {
-      const float* res = (VARIANT >= V_F32_RES && VARIANT < V_REQUANT && row_ok) ? p.residual + (size_t)m * p.OC + oc0 + ch * 32 : nullptr;
-      epilogue_chunk<KIND, VARIANT>(p, v, xz, xs, oc0 + ch * 32, esz, res, w);
+      if (kRes && nb > 0) {
+        const uint32_t byte_off = (uint32_t)(((ch - first) & (cpg - 1)) * chunk_bytes);
+#pragma unroll
+        for (int j = 0; j < (VARIANT == V_JOIN ? 2 : 8); ++j)
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(rv[j].x), "=r"(rv[j].y), "=r"(rv[j].z), "=r"(rv[j].w)
+                       : "r"(stage_row_addr + ((((byte_off >> 4) + (uint32_t)j) ^ stage_xor) << 4)));
+      } else {
+        load_residual<VARIANT>(p, m, oc0 + ch * 32, row_ok, rv);
+      }
+      epilogue_chunk<KIND, VARIANT>(p, v, xz, xs, oc0 + ch * 32, esz, rv, w);
       if (track && row_ok) {
         const int valid = p.OC - (oc0 + ch * 32);  // lanes of a ragged last run hold no output
         if (valid >= 32) {
@@ -864,7 +976,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
     auto store = [&](int ch) {
       if (p.out_tma) {
         const int in_group = (ch - first) & (cpg - 1);
-        if (in_group == 0) {
+        if (in_group == 0 && !(kRes && nb > 0)) {
           // the staging rows are rewritten: their previous store must have read them
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
@@ -874,7 +986,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(&p.tmO, stage_addr, o_col0 + oc0 + (ch - in_group) * 32, o_row0 + m0 + quarter * 32);
+            tma_store_2d(&p.tmO, stage_base, o_col0 + oc0 + (ch - in_group) * 32, o_row0 + m0 + quarter * 32);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -943,12 +1055,36 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
       // conditional read costs register moves at the loop's join.
 #pragma unroll 1
       for (int c = first; c < end; ++c) {
+        if (kRes && nb > 0 && ((c - first) & (cpg - 1)) == 0) {
+          // The buffer of the store to fetch for was last stored from `nb` stores before it: with nb - 2 stores fetched
+          // ahead only the newest store may still be reading (with a single one ahead, none of two buffers' may).
+          if (lane == 0) {
+            if (nb > 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          }
+          __syncwarp();
+          fetch_next();
+          const uint32_t b = used % (uint32_t)nb;
+          bool here = mbar_wait(smem_u32(&bar_res[b]), (used / (uint32_t)nb) & 1u, abortp);
+          if (!here && !*abortp) {
+            *abortp = 1;
+            atomicExch(p.err_flag, 7);
+          }
+          if (!__all_sync(0xffffffffu, here)) {
+            lost = true;
+            break;
+          }
+          stage_base = stage_addr + b * buf_bytes;
+          stage_row_addr = stage_base + (uint32_t)(lane * pitch);
+          ++used;
+        }
         tmem_ld32_nowait(taddr + (uint32_t)c * 32u, va);
         tmem_ld_wait_for(va);
         if (c + 1 == end) release();
         math(va, c);
         store(c);
       }
+      if (lost) break;
     }
   }
   if (p.out_tma && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -981,6 +1117,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
   __shared__ __align__(8) uint64_t bar_acc_full[MAX_ACC];
   __shared__ __align__(8) uint64_t bar_acc_empty[MAX_ACC];
   __shared__ __align__(8) uint64_t bar_b_resident;
+  __shared__ __align__(8) uint64_t bar_res[EW][MAX_RES_BUFS];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
@@ -1009,6 +1146,8 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
       mbar_init(smem_u32(&bar_empty[i]), 1);
     }
     mbar_init(smem_u32(&bar_b_resident), 1);
+    if (p.res_bufs > 0)
+      for (int i = 0; i < EW * MAX_RES_BUFS; ++i) mbar_init(smem_u32(&bar_res[0][0] + i), 1);
     for (int i = 0; i < ES::NACC; ++i) {
       mbar_init(smem_u32(&bar_acc_full[i]), 1);
       // one arrival per epilogue warp of the group that drains it (of both CTAs for a pair)
@@ -1229,12 +1368,12 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
     }
   } else {
     // ---------------- epilogue ----------------
-    const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * (uint32_t)(32 * p.out_row_bytes);
+    const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));
     const bool split = !p.batched && p.splits > 1;
 #define OXB_EPI(V)                                                                                                                                    \
   case V:                                                                                                                                             \
-    if (!PAIR && split) epilogue_role<BN, KIND, V, !PAIR, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
-    else epilogue_role<BN, KIND, V, false, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
+    if (!PAIR && split) epilogue_role<BN, KIND, V, !PAIR, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, bar_res[warp - 2], stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
+    else epilogue_role<BN, KIND, V, false, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, bar_res[warp - 2], stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
     break;
     if constexpr (KIND == KIND_I8) {
       switch (p.variant) {
@@ -1254,6 +1393,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         OXB_EPI(33)
         OXB_EPI(34)
         OXB_EPI(35)
+        OXB_EPI(V_JOIN)
         default: break;
       }
     } else {

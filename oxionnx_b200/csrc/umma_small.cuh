@@ -114,8 +114,9 @@ __device__ __forceinline__ void small_finish(const KParams& p, const uint32_t (&
                                              float& seen_min, float& seen_max) {
   const bool row_ok = m < p.M;
   uint32_t w[32];
-  const float* res = (VARIANT >= V_F32_RES && VARIANT < V_REQUANT && row_ok) ? p.residual + (size_t)m * p.OC + oc : nullptr;
-  epilogue_chunk<KIND, VARIANT>(p, acc, xz, xs, oc, esz, res, w);
+  uint4 rv[8];
+  load_residual<VARIANT>(p, m, oc, row_ok, rv);
+  epilogue_chunk<KIND, VARIANT>(p, acc, xz, xs, oc, esz, rv, w);
   const int valid = min(32, p.OC - oc);
   if (!row_ok) return;
   if (p.minmax_keys != nullptr && esz == 4 && (VARIANT < V_REQUANT || VARIANT >= V_DEQUANT)) {
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
         OXB_SMALL(33)
         OXB_SMALL(34)
         OXB_SMALL(35)
+        OXB_SMALL(V_JOIN)
         default: break;
       }
     } else {
