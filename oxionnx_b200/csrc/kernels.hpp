@@ -73,6 +73,13 @@ struct ResidualParams {
 };
 // Decides once, at plan time, whether the fast kernel may be used for these parameters.
 void residual_requant_prepare(ResidualParams& rp, DT a_dt, DT b_dt);
+// Constants of the join inside a contraction's epilogue: lane = clamp(rne(fma(a, ca, fma(b, cb, cc))), lo, hi) with the
+// ReLU in the lower bound.  False when none were found that give the reference's lane for every pair of inputs.
+struct JoinConstants {
+  float ca = 0.f, cb = 0.f, cc = 0.f;
+  int lo = 0, hi = 255;
+};
+bool residual_join_constants(const ResidualParams& rp, DT a_dt, DT b_dt, JoinConstants* out);
 void residual_requant(const void* a, DT a_dt, const void* b, DT b_dt, void* y, DT y_dt, int64_t n, const ResidualParams& rp, cudaStream_t s);
 
 // ---- element-wise -----------------------------------------------------------------------
@@ -179,7 +186,11 @@ struct Epilogue {
   int round_tf32 = 0;
   // EPI_F32 with a fused residual: out = act((acc + bias_f[oc]) + residual[m * OC + oc]); the two
   // additions round as the separate Conv and Add nodes do
-  const float* residual = nullptr;
+  const void* residual = nullptr;
+  // EPI_REQUANT on the tensor cores, packed form only: the requantised lane is joined with the 8-bit `residual`,
+  // out = clamp(rne(lane * join_a + residual * join_b + join_c), join_lo, join_hi); lo / hi / y_zp stay the lane's own
+  int join = 0, join_signed = 0, join_lo = 0, join_hi = 255;
+  float join_a = 0.f, join_b = 0.f, join_c = 0.f;
   // integer modes.  Direct kernels subtract zero points per element; the tensor-core kernel
   // computes raw = sum(x*w) and applies acc = raw + bias_i[oc] - x_zp * wsum[oc].
   const int32_t* bias_i = nullptr;

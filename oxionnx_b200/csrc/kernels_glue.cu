@@ -6,6 +6,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -2057,6 +2058,63 @@ void residual_requant_prepare(ResidualParams& rp, DT a_dt, DT b_dt) {
   }
   rp.y_rcp = y_rcp;
   rp.proven_fast = packed_ok ? 2 : 1;
+}
+
+bool residual_join_constants(const ResidualParams& rp, DT a_dt, DT b_dt, JoinConstants* out) {
+  auto sane = [](float v) { return std::isfinite(v) && std::fabs(v) >= 9.5367431640625e-07f && std::fabs(v) <= 1048576.0f; };
+  if (!sane(rp.a_scale) || !sane(rp.b_scale) || !sane(rp.y_scale) || rp.y_scale <= 0.f) return false;
+  if (!(std::fabs(rp.a_zp) <= 255.f && std::fabs(rp.b_zp) <= 255.f && std::fabs(rp.y_zp) <= 255.f)) return false;
+  const int a_lo = a_dt == DT::I8 ? -128 : 0, b_lo = b_dt == DT::I8 ? -128 : 0;
+  const float magic = 12582912.0f, lo_eff = rp.relu ? std::fmax(rp.lo, rp.y_zp) : rp.lo;
+  // the separate nodes' lane of every pair
+  std::vector<int16_t> want(65536);
+  for (int i = 0; i < 256; ++i) {
+    volatile float va = ((float)(i + a_lo) - rp.a_zp) * rp.a_scale;
+    for (int j = 0; j < 256; ++j) {
+      volatile float vb = ((float)(j + b_lo) - rp.b_zp) * rp.b_scale;
+      volatile float sum = va + vb;
+      if (rp.relu) sum = std::fmax(sum, 0.f);
+      volatile float quot = sum / rp.y_scale;
+      volatile float ref = std::nearbyintf(quot) + rp.y_zp;
+      want[i * 256 + j] = (int16_t)std::fmin(std::fmax(ref, rp.lo), rp.hi);
+    }
+  }
+  // The one real quotient is rounded in other places here than there, so a pair within some 1e-5 of a tie may come out on
+  // the other side; neighbours of the constants move those few pairs.
+  const double ca = (double)rp.a_scale / rp.y_scale, cb = (double)rp.b_scale / rp.y_scale;
+  auto step = [](float v, int n) {
+    for (; n > 0; --n) v = std::nextafterf(v, INFINITY);
+    for (; n < 0; ++n) v = std::nextafterf(v, -INFINITY);
+    return v;
+  };
+  static const int order[] = {0, 1, -1, 2, -2, 3, -3, 4, -4};
+  int hint = 0;  // the pair that refuted the last candidate is tried first
+  for (int sa = 0; sa < 3; ++sa)
+    for (int sb = 0; sb < 3; ++sb)
+      for (int sc : order) {
+        JoinConstants k;
+        k.ca = step((float)ca, order[sa]), k.cb = step((float)cb, order[sb]);
+        k.cc = step((float)((double)rp.y_zp - (double)rp.a_zp * k.ca - (double)rp.b_zp * k.cb), sc);
+        k.lo = (int)lo_eff, k.hi = (int)rp.hi;
+        auto holds = [&](int pair) {
+          const float a = (float)((pair >> 8) + a_lo), b = (float)((pair & 255) + b_lo);
+          const float t = std::fmaf(a, k.ca, std::fmaf(b, k.cb, k.cc));
+          volatile float m = t + magic;
+          const float r = m - magic;
+          return std::fabs(r) <= 32000.f && std::fmin(std::fmax(r, lo_eff), rp.hi) == (float)want[pair];
+        };
+        bool ok = holds(hint);
+        for (int pair = 0; pair < 65536 && ok; ++pair)
+          if (!holds(pair)) {
+            ok = false;
+            hint = pair;
+          }
+        if (ok) {
+          *out = k;
+          return true;
+        }
+      }
+  return false;
 }
 
 void s2d_pack(const TensorRef& src, void* dst, DT dst_dt, int c_pad, int sub, cudaStream_t s) {

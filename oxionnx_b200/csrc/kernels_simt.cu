@@ -211,7 +211,7 @@ void launch_conv(const void* x, const void* w, void* out, const ConvShape& cs, c
 
 void conv_direct(const void* x, DT x_dt, int x_plain_nchw, const void* w, DT w_dt, void* out, const ConvShape& cs, const Epilogue& ep,
                  cudaStream_t s) {
-  EpiDev e{ep.mode,     ep.bias_f,    ep.act,  ep.clip_lo, ep.clip_hi,  ep.slope, ep.round_tf32, ep.residual, ep.bias_i, ep.x_zp, ep.x_zp_dev,
+  EpiDev e{ep.mode,     ep.bias_f,    ep.act,  ep.clip_lo, ep.clip_hi,  ep.slope, ep.round_tf32, (const float*)ep.residual, ep.bias_i, ep.x_zp, ep.x_zp_dev,
            ep.x_zp_rows, ep.w_zp,     ep.n_w_zp, ep.combined, ep.y_zp,  ep.relu_fused && ep.lo < 0 ? 0 : ep.lo, ep.hi, ep.out_dt, ep.dq_w_scale, ep.dq_x_scale_dev, ep.dq_bias, ep.dq_act};
   if (ep.mode == EPI_F32) {
     if (x_dt != DT::F32 || w_dt != DT::F32) OXB_FAIL("conv_direct: float epilogue needs f32 operands");

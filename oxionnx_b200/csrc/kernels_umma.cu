@@ -175,7 +175,7 @@ void layout_smem(KParams& kp, int bn, int kind, bool pair, size_t* smem_total) {
   const size_t resident = kp.b_resident_bytes;
   const size_t kb_bytes = (size_t)(BLOCK_M + (resident ? 0 : (pair ? bn / 2 : bn))) * kp.swizzle_bytes;
   const size_t stage_bytes = kb_bytes * kp.kpb;
-  const size_t staging = kp.out_tma ? (size_t)ew * 32 * kp.out_row_bytes : 0;
+  const size_t staging = kp.out_tma ? (size_t)ew * 32 * kp.out_row_bytes * std::max(kp.res_bufs, 1) : 0;
   // one persistent CTA per SM: the ring may use most of the shared memory and runs on across tiles
   const size_t budget = std::min<size_t>(192 * 1024, kSmemBudget - staging) - resident;
   int stages = (int)(budget / stage_bytes);
@@ -240,6 +240,9 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
       c.bn = bn, c.splits = sp, c.k_per = (int)ceil_div(k_iters, (int64_t)sp);
       if (sp > 1 && (sp - 1) * (int64_t)c.k_per >= k_iters) continue;  // a slice would be empty
       c.a_rows = (int)std::min<int64_t>(BLOCK_M, align_up((size_t)M, 32));
+      // a longer slice is the persistent kernel's: sixteen epilogue warps and a longer ring win from there on (i8
+      // 1500 x 1024, K = 4096: 24.7 us here, 20.6 there; TF32 6272 x 256, K = 2304: 39 and 34)
+      if (c.k_per > 20) continue;
       const int64_t ctas = tiles * sp;
       if (ctas > (sp == 1 ? 2 * sms : (sp == 2 ? sms : (sp == 4 ? 128 : 64)))) continue;
       layout_small(c, swz);
@@ -292,6 +295,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   }
   if (e.x_zp_rows || e.n_w_zp > 0) return no("per-row or weight zero points need the direct kernel");
   if (e.mode == EPI_F32 ? e.bias_f == nullptr : e.bias_i == nullptr) return no("the tensor-core epilogue needs a (padded) bias vector");
+  if (e.join && (!e.residual || !e.bias_if || dt_size(e.out_dt) != 1 || cs.OC % 32 != 0)) return no("the join needs an 8-bit residual, the float bias and whole channel runs");
   if (e.mode == EPI_F32 && e.act == 4 && e.slope == nullptr) return no("the PRelu epilogue needs a (padded) slope vector");
 
   // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles
@@ -527,10 +531,27 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     kp.stage_off = (uint32_t)(small.stages * small.stage_bytes);
     pl->smem = small.smem;
   } else {
+    // A residual is fetched through the staging rows of the store it is combined for: four buffers per epilogue warp
+    // where the ring keeps three stages beside them, else three or two.
+    if (e.residual && kp.out_tma && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0) {
+      const size_t oes = dt_size(e.out_dt);
+      cuuint64_t gdim[2] = {(cuuint64_t)cs.OC, (cuuint64_t)M};
+      cuuint64_t gstr[1] = {(cuuint64_t)cs.OC * oes};
+      cuuint32_t box[2] = {(cuuint32_t)(kp.out_row_bytes / oes), 32};
+      cuuint32_t estr[2] = {1, 1};
+      if (g_encode_tiled(&kp.tmR, output_map_type(e.out_dt), 2, const_cast<void*>(e.residual), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         swizzle_enum(kp.out_row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
+        const size_t per_buf = (size_t)epi_warps(kind) * 32 * kp.out_row_bytes;
+        auto fits = [&](int bufs, int stages) { return kSmemBudget >= bufs * per_buf + kp.b_resident_bytes + stages * kb_bytes * kp.kpb; };
+        while (kp.kpb > 1 && !fits(3, 2)) kp.kpb /= 2;
+        kp.res_bufs = fits(4, 3) ? 4 : (fits(3, 2) ? 3 : (fits(2, 2) ? 2 : 0));
+      }
+    }
     layout_smem(kp, bn, kind, pair, &pl->smem);
   }
   kp.mode = e.mode;
-  if (e.mode == EPI_F32) kp.variant = (e.residual ? V_F32_RES : V_F32_BASE) + e.act * 2 + (e.round_tf32 ? 1 : 0);
+  if (e.join) kp.variant = V_JOIN;
+  else if (e.mode == EPI_F32) kp.variant = (e.residual ? V_F32_RES : V_F32_BASE) + e.act * 2 + (e.round_tf32 ? 1 : 0);
   else if (e.mode == EPI_REQUANT) {
     const bool fma = e.combined_fma_ok && tune.requant_f64 != 1;
     const bool lean = fma && e.acc_abs_bound > 0 && e.acc_abs_bound < 16777216;
@@ -544,6 +565,8 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   kp.bias_f = e.bias_f;
   kp.slope = e.slope;
   kp.residual = e.residual;
+  kp.join_a = e.join_a, kp.join_b = e.join_b, kp.join_c = e.join_c;
+  kp.join_lo = e.join_lo, kp.join_hi = e.join_hi, kp.join_flip = e.join_signed;
   kp.dq_w_scale = e.dq_w_scale;
   kp.dq_x_scale = e.dq_x_scale_dev;
   kp.dq_bias = e.dq_bias;

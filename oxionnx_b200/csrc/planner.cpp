@@ -496,7 +496,7 @@ class Planner {
 
   struct Contraction {
     k::ConvShape cs;
-    int x_vi, out_vi;
+    int x_vi, out_vi = -1;
     bool x_plain_nchw = false;
     // weights in ONNX order [OC][C/g][R][S] as exact values
     const HostTensor* w = nullptr;
@@ -519,9 +519,17 @@ class Planner {
     std::vector<float> combined;  // OC
     float w_scale_mul = 1.0f;     // Gemm alpha folded into the packed weights
     double algorithmic_ops = 0;   // ops of the node as written (a rewritten stem pads its reduction)
+    // a quantised residual join behind the node (match_join); dropped when the node cannot take it into its epilogue
+    bool join = false;
+    k::ResidualParams join_rp{};
+    int join_other = -1;
+    std::vector<int> join_nodes;
+    std::string join_out, out_name;
+    std::vector<int64_t> out_shape;
     int w_cacheable = -1;         // whether the packed weights may stay resident (-1: decide from the name)
   };
   void emit_contraction(const NodeDef& n, Contraction& c);
+  void match_join(Contraction& c);
 
   void finalize_lifetimes_and_arena();
   struct LastAdd {
@@ -1118,6 +1126,27 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
     }
   epi.acc_abs_bound = acc_abs_bound;
 
+  if (c.out_vi < 0) {  // a QLinearConv: with the residual join behind it, or without
+    k::JoinConstants jc;
+    bool take = c.join && want_umma && C.cfg().requant_f64 == 0 && c.x_zp_static && acc_abs_bound > 0 && acc_abs_bound < 16777216 && cs.OC % 32 == 0;
+    double cmax = 0.0;
+    for (float v : c.combined) {
+      const float a = std::fabs(v);
+      take = take && (a == 0.f || (a >= 4.76837158203125e-07f && a <= 1099511627776.0f));
+      cmax = std::max(cmax, (double)a);
+    }
+    take = take && (double)acc_abs_bound * cmax * 1.0001 + std::fabs((double)epi.y_zp) + 1.0 < 32000.0;
+    if (take) take = k::residual_join_constants(c.join_rp, epi.out_dt, V(c.join_other).dt, &jc);
+    if (take) {
+      for (int i : c.join_nodes) skipped_[i] = 1;
+      epi.join = 1;
+      epi.join_a = jc.ca, epi.join_b = jc.cb, epi.join_c = jc.cc, epi.join_lo = jc.lo, epi.join_hi = jc.hi;
+      epi.join_signed = V(c.join_other).dt == DT::I8 ? 1 : 0;
+      epi.out_dt = c.join_rp.lo < 0.f ? DT::I8 : DT::U8;
+      c.res_vi = c.join_other;
+    }
+    c.out_vi = add_value(take ? c.join_out : c.out_name, c.out_shape, epi.out_dt, Layout::NHWC);
+  }
   const int x_vi = c.x_vi, out_vi = c.out_vi, xzp_vi = c.x_zp_vi, res_vi = c.res_vi, dq_vi = c.dq_xs_vi;
   std::vector<int> reads = {x_vi};
   if (xzp_vi >= 0) reads.push_back(xzp_vi);
@@ -1226,7 +1255,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
     st.finalize = [this, step_index, x_vi = x_op_vi, out_vi, xzp_vi, res_vi, dq_vi, wdev, xdt, wdt, cs, epi, kind, n]() mutable {
       k::Epilogue e = epi;
       if (xzp_vi >= 0) e.x_zp_dev = (const float*)V(xzp_vi).ptr;
-      if (res_vi >= 0) e.residual = (const float*)V(res_vi).ptr;
+      if (res_vi >= 0) e.residual = V(res_vi).ptr;
       if (dq_vi >= 0) e.dq_x_scale_dev = (const float*)V(dq_vi).ptr;
       e.minmax_keys = (unsigned int*)V(out_vi).minmax_keys;
       std::string why2;
@@ -1238,7 +1267,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       if (!plan) OXB_FAIL("%s '%s': tensor-core plan rejected after selection: %s", n.op.c_str(), n.name.c_str(), why2.c_str());
       S.umma_plans_.push_back(plan);
       Step& me = S.steps_[step_index];
-      me.kernel = std::string(k::umma_plan_desc(plan)) + (res_vi >= 0 ? " +residual" : "") + (dq_vi >= 0 ? " +dequant" : "");
+      me.kernel = std::string(k::umma_plan_desc(plan)) + (res_vi >= 0 ? (e.join ? " +join" : " +residual") : "") + (dq_vi >= 0 ? " +dequant" : "");
       // a quantised linear layer over few rows may become a link of a one-kernel chain (link_chains)
       if (kind == 0 && e.mode == k::EPI_REQUANT && xzp_vi < 0 && res_vi < 0 && dq_vi < 0 && cs.R == 1 && cs.S == 1 && cs.sh == 1 && cs.sw == 1 &&
           cs.pt == 0 && cs.pl == 0 && cs.pb == 0 && cs.pr == 0 && cs.group == 1 && cs.x_pixel_stride == 0 && cs.M() <= 64 && cs.C % 128 == 0 &&
@@ -1329,7 +1358,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
     st.launch = [this, x_vi, out_vi, xzp_vi, res_vi, dq_vi, wdev, xdt, wdt, cs, epi, plain](cudaStream_t s) {
       k::Epilogue e = epi;
       if (xzp_vi >= 0) e.x_zp_dev = (const float*)V(xzp_vi).ptr;
-      if (res_vi >= 0) e.residual = (const float*)V(res_vi).ptr;
+      if (res_vi >= 0) e.residual = V(res_vi).ptr;
       if (dq_vi >= 0) e.dq_x_scale_dev = (const float*)V(dq_vi).ptr;
       k::conv_direct(V(x_vi).ptr, xdt, plain, wdev, wdt, V(out_vi).ptr, cs, e, s);
       C.counters.simt_launches++;
@@ -1840,7 +1869,9 @@ void Planner::plan_conv_family(const NodeDef& n, int ni) {
     r.lo = std::max(r.lo, 0);
   }
   c.epi.out_dt = narrowest_int(r.lo, r.hi);
-  c.out_vi = add_value(out_name, out_shape, c.epi.out_dt, Layout::NHWC);
+  c.out_name = out_name;
+  c.out_shape = out_shape;
+  if (!C.cfg().keep_intermediates && C.cfg().kernel_path == 0 && dt_size(c.epi.out_dt) == 1) match_join(c);
   emit_contraction(n, c);
 }
 
@@ -3175,6 +3206,65 @@ void Planner::plan_alias(const NodeDef& n) {
 // parameters: the residual join of a quantised ResNet.  One kernel performs the same f32
 // operations in the same order, so the lanes equal the unfused chain's bit for bit; the
 // float intermediates never reach memory.
+// The join behind a quantised convolution, DequantizeLinear -> Add(., DequantizeLinear(other)) -> [Relu] ->
+// QuantizeLinear, when the other operand is already on the device: its parameters, nodes and output (see
+// try_plan_residual_chain, which runs the same chain as a kernel of its own).
+void Planner::match_join(Contraction& c) {
+  auto only_consumer = [&](const std::string& name) -> int {
+    if (graph_outputs_.count(name)) return -1;
+    auto it = consumers_.find(name);
+    if (it == consumers_.end() || it->second.size() != 1 || skipped_[it->second[0].first]) return -1;
+    return it->second[0].first;
+  };
+  auto per_tensor = [&](const NodeDef& d, float* scale, float* zp, bool* has_zp) -> bool {
+    for (const std::string& a : d.attrs.names())
+      if (a != "axis") return false;
+    const HostTensor* sc = const_in(d, 1);
+    if (!sc || sc->data.size() != 1 || !std::isfinite(sc->data[0]) || sc->data[0] == 0.f) return false;
+    *scale = sc->data[0];
+    *zp = 0.f;
+    *has_zp = has_in(d, 2);
+    if (*has_zp) {
+      const HostTensor* z = const_in(d, 2);
+      if (!z || z->data.size() != 1 || !std::isfinite(z->data[0]) || z->data[0] != std::nearbyint(z->data[0])) return false;
+      *zp = z->data[0];
+    }
+    return true;
+  };
+  k::ResidualParams rp{};
+  bool has_zp;
+  const int dq_i = only_consumer(c.out_name);
+  if (dq_i < 0 || nodes_[dq_i].op != "DequantizeLinear" || in_name(nodes_[dq_i], 0) != c.out_name || !per_tensor(nodes_[dq_i], &rp.a_scale, &rp.a_zp, &has_zp)) return;
+  const int add_i = only_consumer(nodes_[dq_i].outputs[0]);
+  if (add_i < 0 || nodes_[add_i].op != "Add" || nodes_[add_i].inputs.size() != 2 || !nodes_[add_i].attrs.names().empty()) return;
+  const NodeDef& add = nodes_[add_i];
+  const std::string& other = add.inputs[add.inputs[0] == nodes_[dq_i].outputs[0] ? 1 : 0];
+  if (S.index_.count(other) || only_consumer(other) != add_i) return;
+  int d2_i = -1;
+  for (int j = 0; j < add_i; ++j)
+    if (!skipped_[j] && nodes_[j].op == "DequantizeLinear" && !nodes_[j].outputs.empty() && nodes_[j].outputs[0] == other) d2_i = j;
+  if (d2_i < 0 || d2_i == dq_i || !per_tensor(nodes_[d2_i], &rp.b_scale, &rp.b_zp, &has_zp)) return;
+  auto x2 = S.index_.find(in_name(nodes_[d2_i], 0));
+  if (x2 == S.index_.end()) return;
+  const Value& vb = V(x2->second);
+  if (!(vb.dt == DT::U8 || vb.dt == DT::I8) || vb.shape != c.out_shape || (!order_free(vb) && vb.layout != Layout::NHWC)) return;
+  std::string cur = add.outputs[0];
+  const int relu_i = sole_consumer(cur, "Relu");
+  rp.relu = relu_i >= 0 ? 1 : 0;
+  if (relu_i >= 0) cur = nodes_[relu_i].outputs[0];
+  const int q_i = only_consumer(cur);
+  if (q_i < 0 || nodes_[q_i].op != "QuantizeLinear" || in_name(nodes_[q_i], 0) != cur || !per_tensor(nodes_[q_i], &rp.y_scale, &rp.y_zp, &has_zp)) return;
+  const bool u8 = !has_zp || rp.y_zp > 127.0f;  // saturation_range (oxionnx-ops src/indexing/quantize.rs:58-64)
+  rp.lo = u8 ? 0.f : -128.f;
+  rp.hi = u8 ? 255.f : 127.f;
+  c.join = true;
+  c.join_rp = rp;
+  c.join_other = x2->second;
+  c.join_out = nodes_[q_i].outputs[0];
+  c.join_nodes = {dq_i, d2_i, add_i, q_i};
+  if (relu_i >= 0) c.join_nodes.push_back(relu_i);
+}
+
 bool Planner::try_plan_residual_chain(const NodeDef& n, int ni) {
   // per-tensor parameters held by initializers: scale at slot 1, optional zero point at slot 2
   auto per_tensor = [&](const NodeDef& d, float* scale, float* zp, bool* has_zp) -> bool {
