@@ -1080,7 +1080,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
   // ---- can the tensor-core kernel take it? ----
   std::string why;
   bool want_umma = C.cfg().kernel_path == 0 && k::umma_available() && !c.x_plain_nchw;
-  Value& xv = V(c.x_vi);
+  const Value xv = V(c.x_vi);  // a copy: values are added below
   if (want_umma && c.is_int) {
     bool w_zp_zero = true;
     for (int32_t z : c.w_zp) w_zp_zero &= z == 0;
