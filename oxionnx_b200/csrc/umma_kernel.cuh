@@ -178,24 +178,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (clock64() - start > WAIT_CYCLES) return false;
   }
 }
-// The wait of a role that the epilogue holds up: after eight attempts it sleeps between them.  A parked attempt comes
-// back after some 70 cycles, and the fifteen instructions around it cost a scheduler that also runs four epilogue
-// warps a fifth of its issue slots; nothing is lost by noticing 0.2 us late, ring and accumulators are buffered.
-__device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-#pragma unroll 1
-  for (int attempt = 0; attempt < 8; ++attempt)
-    if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  while (true) {
-#pragma unroll 1
-    for (int attempt = 0; attempt < 32; ++attempt) {
-      __nanosleep(200);
-      if (mbar_try_wait(bar, parity)) return true;
-    }
-    if (*abort_flag) return false;
-    if (clock64() - start > WAIT_CYCLES) return false;
-  }
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // arrival on a barrier of any CTA of the cluster (address from mapa)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -1242,7 +1224,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
       // order of a hundred cycles, whatever the box size: a stage carries several K blocks when
       // they are small, so that those costs are paid once per stage.
       for (int it = it_begin; it < it_end; it += p.kpb) {
-        bool got = mbar_wait_idle(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp);
+        bool got = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0 && !*abortp) {
             *abortp = 1;
@@ -1321,7 +1303,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         const uint32_t buf = local % (uint32_t)ES::NACC;
         const uint32_t acc_phase = (local / (uint32_t)ES::NACC) & 1u;
         // the epilogue must have drained this accumulator (free on its first use)
-        bool got = mbar_wait_idle(smem_u32(&bar_acc_empty[buf]), acc_phase ^ 1u, abortp);
+        bool got = mbar_wait(smem_u32(&bar_acc_empty[buf]), acc_phase ^ 1u, abortp);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0 && !*abortp) {
             *abortp = 1;
