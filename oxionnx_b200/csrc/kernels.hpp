@@ -106,7 +106,8 @@ void global_avg_pool(const TensorRef& x, const TensorRef& y, int round_tf32, cud
 void global_avg_pool_dequant(const TensorRef& x, const TensorRef& y, float scale, float zp, int round_tf32, cudaStream_t s);
 // OxiInstanceNorm over (n, c) planes, two-pass variance about the mean; optional fused
 // per-sample modulation y = norm * scale[n,c] + shift[n,c] (both may be NULL).
-void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, const float* shift_nc, int relu, int round_tf32,
+// The modulators' lanes of sample n start at n * stride.
+void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32,
                    cudaStream_t s);
 
 // ---- spatial glue -----------------------------------------------------------------------

@@ -760,7 +760,7 @@ __global__ void global_avg_pool_nhwc_kernel(const float* __restrict__ x, float* 
 // Instance norm on NHWC: one block per (n, 32-channel group); 32 lanes across channels
 // (coalesced 128-byte rows), 8 warps striding over the pixels.
 __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps, const float* scale_nc,
-                                          const float* shift_nc, int relu, int round_tf32_flag) {
+                                          int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32_flag) {
   pdl_enter();
   int64_t cgroups = (d.C + 31) / 32;
   int64_t n = blockIdx.x / cgroups, cg = blockIdx.x % cgroups;
@@ -794,8 +794,8 @@ __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __
   float inv_std = 1.0f / sqrtf(var + eps);
   float sc = 1.f, sf = 0.f;
   bool mod = scale_nc != nullptr || shift_nc != nullptr;
-  if (valid && scale_nc) sc = scale_nc[n * d.C + c];
-  if (valid && shift_nc) sf = shift_nc[n * d.C + c];
+  if (valid && scale_nc) sc = scale_nc[n * scale_stride + c];
+  if (valid && shift_nc) sf = shift_nc[n * shift_stride + c];
   if (valid)
     for (int64_t i = warp; i < hw; i += nwarps) {
       float v = (px[i * d.C] - mean) * inv_std;
@@ -810,7 +810,8 @@ __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __
 // the tensor is read from HBM once instead of three times.  32 warps stride over the pixels, four loads in flight
 // each; the per-warp partial sums are added in warp order as above.
 __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps,
-                                                                        const float* scale_nc, const float* shift_nc, int relu, int round_tf32_flag) {
+                                                                        const float* scale_nc, int64_t scale_stride, const float* shift_nc,
+                                                                        int64_t shift_stride, int relu, int round_tf32_flag) {
   pdl_enter();
   extern __shared__ float slab[];  // [pixel][32 channels]
   __shared__ float red[32][33];
@@ -858,8 +859,8 @@ __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const flo
   const float inv_std = 1.0f / sqrtf(var + eps);
   float sc = 1.f, sf = 0.f;
   const bool mod = scale_nc != nullptr || shift_nc != nullptr;
-  if (valid && scale_nc) sc = scale_nc[n * d.C + c];
-  if (valid && shift_nc) sf = shift_nc[n * d.C + c];
+  if (valid && scale_nc) sc = scale_nc[n * scale_stride + c];
+  if (valid && shift_nc) sf = shift_nc[n * shift_stride + c];
   if (valid)
     for (int j = warp; j < hw; j += 32) {
       float v = (slab[j * 32 + lane] - mean) * inv_std;
@@ -2315,8 +2316,8 @@ void global_avg_pool(const TensorRef& x, const TensorRef& y, int round_tf32_flag
   launch(global_avg_pool_nhwc_kernel, grid_for(total, 128), 128, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, round_tf32_flag);
 }
 
-void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, const float* shift_nc, int relu, int round_tf32_flag,
-                   cudaStream_t s) {
+void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc,
+                   int64_t shift_stride, int relu, int round_tf32_flag, cudaStream_t s) {
   int64_t cgroups = (x.d.C + 31) / 32;
   int64_t blocks = x.d.N * cgroups;
   if (blocks == 0) return;
@@ -2336,11 +2337,12 @@ void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const floa
         h = slab;
       }
     }
-    launch(instance_norm_nhwc_smem_kernel, (unsigned)blocks, 1024, slab, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu,
-                                                                        round_tf32_flag);
+    launch(instance_norm_nhwc_smem_kernel, (unsigned)blocks, 1024, slab, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, scale_stride, shift_nc,
+           shift_stride, relu, round_tf32_flag);
     return;
   }
-  launch(instance_norm_nhwc_kernel, (unsigned)blocks, 256, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, shift_nc, relu, round_tf32_flag);
+  launch(instance_norm_nhwc_kernel, (unsigned)blocks, 256, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, scale_stride, shift_nc, shift_stride, relu,
+         round_tf32_flag);
 }
 
 void resize(const TensorRef& x, const TensorRef& y, int mode, int coord, int nearest_rule, float scale_h, float scale_w, int round_tf32_flag,

@@ -486,6 +486,19 @@ class Planner {
   };
   std::map<int, LazyHeads> lazy_heads_;
   void materialise_heads(int yi);
+  // A Slice of the columns of a [rows, width] f32 value: a reader that takes a row stride reads the source itself
+  // (view_of), and a slice that nothing else reads is not run (drop_unread_slices).
+  struct SliceView {
+    int src_vi, step;
+    int64_t offset, stride, rows, cols;
+  };
+  std::map<int, SliceView> slice_views_;
+  const SliceView* view_of(int vi) {
+    while (V(vi).alias_of >= 0) vi = V(vi).alias_of;
+    auto it = slice_views_.find(vi);
+    return it == slice_views_.end() ? nullptr : &it->second;
+  }
+  void drop_unread_slices();
   bool try_plan_attention_product(const NodeDef& n, int ai, int bi);
   void plan_softmax(const NodeDef& n);
   bool try_plan_scaled_masked_softmax(const NodeDef& n);
@@ -630,6 +643,7 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
     S.output_staging_.push_back({o, so});
   }
 
+  drop_unread_slices();
   finalize_lifetimes_and_arena();
   for (auto& st : S.steps_)
     if (st.finalize) st.finalize();
@@ -2473,13 +2487,25 @@ void Planner::plan_instance_norm(const NodeDef& n) {
   TensorRef xr = ref_of(xi), yr = ref_of(yi);
   xr.layout = yr.layout = Layout::NHWC;
   std::vector<int> reads = {xi};
-  if (scale_vi >= 0) reads.push_back(scale_vi);
-  if (shift_vi >= 0) reads.push_back(shift_vi);
+  // the modulators' lanes of sample n start at n * stride + offset: C and 0, or those of the slices they are
+  struct Lanes {
+    int vi = -1;
+    int64_t offset = 0, stride = 0;
+  };
+  auto lanes_of = [&](int vi) {
+    Lanes l{vi, 0, xv.shape[1]};
+    if (vi < 0) return l;
+    const SliceView* sv = view_of(vi);
+    if (sv != nullptr && sv->rows == xv.shape[0] && sv->cols == xv.shape[1]) l = Lanes{sv->src_vi, sv->offset, sv->stride};
+    reads.push_back(l.vi);
+    return l;
+  };
+  const Lanes scale = lanes_of(scale_vi), shift = lanes_of(shift_vi);
   Step& st = add_step(n, scale_vi >= 0 ? "instance_norm+adain" : "instance_norm", 2, reads, {yi});
   st.work = 3.0 * (double)xv.bytes;
-  st.launch = [this, xr, yr, xi, yi, eps, scale_vi, shift_vi, relu, rt](cudaStream_t s) {
-    k::instance_norm(bound(xr, xi), bound(yr, yi), eps, scale_vi >= 0 ? (const float*)V(scale_vi).ptr : nullptr,
-                     shift_vi >= 0 ? (const float*)V(shift_vi).ptr : nullptr, relu, rt, s);
+  st.launch = [this, xr, yr, xi, yi, eps, scale, shift, relu, rt](cudaStream_t s) {
+    k::instance_norm(bound(xr, xi), bound(yr, yi), eps, scale.vi >= 0 ? (const float*)V(scale.vi).ptr + scale.offset : nullptr, scale.stride,
+                     shift.vi >= 0 ? (const float*)V(shift.vi).ptr + shift.offset : nullptr, shift.stride, relu, rt, s);
     C.counters.glue_launches++;
     C.counters.kernel_launches++;
   };
@@ -2661,6 +2687,8 @@ void Planner::plan_slice(const NodeDef& n) {
   };
   const Dims4 xd = pad4(xv.shape, 1), yd = pad4(os, 1), sd = pad4(ds, 0);
   const DT dt = xv.dt;
+  if (rank == 2 && dt == DT::F32 && os[0] == xv.shape[0] && xv.host == nullptr && !C.cfg().keep_intermediates && !graph_outputs_.count(n.outputs[0]))
+    slice_views_[yi] = SliceView{xi, (int)S.steps_.size(), ds[1], xv.shape[1], os[0], os[1]};
   Step& stp = add_step(n, "slice", 2, {xi}, {yi});
   stp.work = 2.0 * (double)V(yi).bytes;
   stp.launch = [this, xi, yi, dt, xd, yd, sd](cudaStream_t s) {
@@ -2668,6 +2696,27 @@ void Planner::plan_slice(const NodeDef& n) {
     C.counters.glue_launches++;
     C.counters.kernel_launches++;
   };
+}
+
+void Planner::drop_unread_slices() {
+  for (auto& sv : slice_views_) {
+    bool read = V(sv.first).is_graph_output;
+    for (const Value& v : S.values_) {
+      int root = v.alias_of;
+      while (root >= 0 && V(root).alias_of >= 0) root = V(root).alias_of;
+      read = read || (root == sv.first && v.is_graph_output);
+    }
+    for (const Step& st : S.steps_)
+      for (int r : st.reads) {
+        while (V(r).alias_of >= 0) r = V(r).alias_of;
+        read = read || r == sv.first;
+      }
+    if (read) continue;
+    Step& st = S.steps_[sv.second.step];
+    st.kernel = "slice (read in place)";
+    st.work = 0;
+    st.launch = [](cudaStream_t) {};
+  }
 }
 
 // Gather along axis 0 of a rank-2 initializer (an embedding table) with device-resident index lanes

@@ -92,3 +92,25 @@ def test_attention_at_ragged_lengths_is_the_separate_nodes_bit_for_bit(batch, se
     assert kernels.count("attention_f32") == 2, kernels
     want, _ = _run(graph, weights, f, keep_intermediates=True)
     assert np.array_equal(got["hidden"], want["hidden"])
+
+
+@pytest.mark.parametrize("reader", ["modulators", "other"])
+def test_slices_read_in_place_by_the_normalisation(reader):
+    n, c, hw = 3, 40, 6
+    rng = np.random.default_rng(11)
+    weights = {"g": (rng.standard_normal((16, 2 * c)) * 0.3).astype(np.float32), "s0": np.float32([0]), "s1": np.float32([c]), "s2": np.float32([2 * c]),
+               "ax": np.float32([1]), "shape": np.float32([n, c, 1, 1])}
+    nodes = [Node("MatMul", "mm", ["l", "g"], ["style"], {}), Node("Slice", "sa", ["style", "s0", "s1", "ax"], ["a"], {}),
+             Node("Slice", "sb", ["style", "s1", "s2", "ax"], ["b"], {}), Node("Reshape", "ra", ["a", "shape"], ["a4"], {}),
+             Node("Reshape", "rb", ["b", "shape"], ["b4"], {}), Node("OxiInstanceNorm", "in", ["x"], ["xn"], {"epsilon": 1e-5}),
+             Node("Mul", "mul", ["xn", "a4"], ["xm"], {}), Node("Add", "add", ["xm", "b4"], ["y"], {})]
+    outs = ["y"]
+    if reader == "other":
+        nodes.append(Node("Sigmoid", "sg", ["a"], ["z"], {}))
+        outs.append("z")
+    graph = Graph(nodes=nodes, input_names=["x", "l"], output_names=outs)
+    feeds = {"x": rng.standard_normal((n, c, hw, hw)).astype(np.float32), "l": rng.standard_normal((n, 16)).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds)
+    assert kernels.count("slice (read in place)") == (2 if reader == "modulators" else 1), kernels
+    want, _ = _run(graph, weights, feeds, keep_intermediates=True)
+    assert all(np.array_equal(got[o], want[o]) for o in outs)
