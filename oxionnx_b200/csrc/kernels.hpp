@@ -106,6 +106,13 @@ void global_avg_pool(const TensorRef& x, const TensorRef& y, int round_tf32, cud
 void global_avg_pool_dequant(const TensorRef& x, const TensorRef& y, float scale, float zp, int round_tf32, cudaStream_t s);
 // OxiInstanceNorm over (n, c) planes, two-pass variance about the mean; optional fused
 // per-sample modulation y = norm * scale[n,c] + shift[n,c] (both may be NULL).
+// Second pass of a convolution run as R x 1 filters: y[row][q][oc] = relu?(sum_s x[row][q + s - pl][s * OC + oc] + bias[oc]) over
+// x [rows][W][OCp] and y [rows][Q][OC]; positions outside 0 .. W - 1 add nothing.
+struct RowSums {
+  int64_t rows = 0;
+  int W = 0, Q = 0, OC = 0, OCp = 0, S = 0, pl = 0, relu = 0, round_tf32 = 0;
+};
+void row_sums(const float* x, const float* bias, float* y, const RowSums& r, cudaStream_t s);
 // The modulators' lanes of sample n start at n * stride.
 void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32,
                    cudaStream_t s);

@@ -871,6 +871,38 @@ __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const flo
     }
 }
 
+// Second pass of a convolution run as R x 1 filters.  Bound by reading the partials once (4 x 128 x 134 rows of 32 floats:
+// 8.8 MB).  A block stages kRowSumTile + S - 1 pixels of one row in shared memory with 16-byte loads (pixel pitch
+// OCp + 1: neighbouring outputs read S * OC lanes apart without bank conflicts), then every thread adds S partials of
+// one (pixel, filter).
+constexpr int kRowSumTile = 64;
+__global__ void __launch_bounds__(256) row_sums_kernel(const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ y, RowSums r,
+                                                       int tiles) {
+  pdl_enter();
+  extern __shared__ float px[];
+  const int64_t row = blockIdx.x / tiles;
+  const int q0 = (int)(blockIdx.x % tiles) * kRowSumTile;
+  const int span = kRowSumTile + r.S - 1, pitch = r.OCp + 1, quads = r.OCp / 4;
+  for (int i = threadIdx.x; i < span * quads; i += 256) {
+    const int p = i / quads, l = (i % quads) * 4, w = q0 + p - r.pl;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (w >= 0 && w < r.W) v = *reinterpret_cast<const float4*>(x + (row * r.W + w) * r.OCp + l);
+    float* d = px + p * pitch + l;
+    d[0] = v.x, d[1] = v.y, d[2] = v.z, d[3] = v.w;
+  }
+  __syncthreads();
+  const int count = min(kRowSumTile, r.Q - q0) * r.OC;
+  float* out = y + (row * r.Q + q0) * r.OC;
+  for (int i = threadIdx.x; i < count; i += 256) {
+    const int p = i / r.OC, oc = i % r.OC;
+    float sum = 0.f;
+    for (int k = 0; k < r.S; ++k) sum += px[(p + k) * pitch + k * r.OC + oc];
+    sum += bias[oc];
+    if (r.relu) sum = fmaxf(sum, 0.f);
+    out[i] = r.round_tf32 ? round_tf32(sum) : sum;
+  }
+}
+
 // ---- resize / pad / concat --------------------------------------------------------------
 __device__ __forceinline__ float src_coord(int coord, int64_t o, float scale, int64_t in_size, int64_t out_size) {
   switch (coord) {
@@ -2314,6 +2346,13 @@ void global_avg_pool(const TensorRef& x, const TensorRef& y, int round_tf32_flag
   int64_t total = x.d.N * x.d.C;
   if (total == 0) return;
   launch(global_avg_pool_nhwc_kernel, grid_for(total, 128), 128, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, round_tf32_flag);
+}
+
+void row_sums(const float* x, const float* bias, float* y, const RowSums& r, cudaStream_t s) {
+  const int tiles = (r.Q + kRowSumTile - 1) / kRowSumTile;
+  const size_t smem = (size_t)(kRowSumTile + r.S - 1) * (r.OCp + 1) * sizeof(float);  // S <= 64: 33 KB at most
+  if (r.rows * tiles == 0) return;
+  launch(row_sums_kernel, (unsigned)(r.rows * tiles), 256, smem, s, x, bias, y, r, tiles);
 }
 
 void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc,

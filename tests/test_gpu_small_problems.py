@@ -94,6 +94,25 @@ def test_attention_at_ragged_lengths_is_the_separate_nodes_bit_for_bit(batch, se
     assert np.array_equal(got["hidden"], want["hidden"])
 
 
+# batch, channels, height, width, filters, kernel, pad: ragged tiles of the second pass, the fewest and the most columns
+@pytest.mark.parametrize("shape", [(1, 32, 134, 140, 3, 7, 0), (2, 64, 100, 101, 2, 5, 2), (1, 32, 129, 128, 9, 7, 3), (3, 128, 90, 67, 1, 3, 1)])
+@pytest.mark.parametrize("activation", ["", "relu"])
+def test_row_summed_convolutions_match_the_direct_kernel(shape, activation):
+    n, c, h, w, oc, k, pad = shape
+    rng = np.random.default_rng([n, c, h, oc, k, 2])
+    weights = {"w1": (rng.standard_normal((oc, c, k, k)) / np.sqrt(c * k * k)).astype(np.float32), "b1": rng.standard_normal(oc).astype(np.float32)}
+    attrs = {"pads": [pad] * 4}
+    if activation:
+        attrs["activation"] = activation
+    nodes = [Node("Relu", "pre", ["x"], ["x1"], {}), Node("Conv", "c1", ["x1", "w1", "b1"], ["y"], attrs)]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds)
+    assert "row_sums" in kernels, kernels
+    want, _ = _run(graph, weights, feeds, kernel_path="direct")
+    assert np.all(np.abs(got["y"] - want["y"]) <= 2e-3 * np.abs(want["y"]) + 2e-3 * np.abs(want["y"]).max())
+
+
 @pytest.mark.parametrize("reader", ["modulators", "other"])
 def test_slices_read_in_place_by_the_normalisation(reader):
     n, c, hw = 3, 40, 6
