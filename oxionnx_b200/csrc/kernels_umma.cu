@@ -383,7 +383,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   if (m_tiles * n_tiles > 0x7fffffffLL) return no("grid too large");
 
   UmmaPlan* pl = new UmmaPlan();
-  std::memset(&pl->kp, 0, sizeof(KParams));
+  pl->kp = KParams();
   KParams& kp = pl->kp;
   auto fail = [&](const char* msg) -> UmmaPlan* {
     if (pl->ws) cudaFree(pl->ws);
@@ -641,7 +641,7 @@ UmmaPlan* umma_plan_create_batched(const BatchedGemm& g, std::string* why) {
   const int64_t items = (int64_t)g.outer * g.inner, m_tiles = g.M / BLOCK_M, n_tiles = g.N / bn;
   if (items * m_tiles * n_tiles > 0x7fffffffLL) return no("grid too large");
   UmmaPlan* pl = new UmmaPlan();
-  std::memset(&pl->kp, 0, sizeof(KParams));
+  pl->kp = KParams();
   KParams& kp = pl->kp;
   const CUtensorMapDataType dtype = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   cuuint32_t estr[2] = {1, 1};
