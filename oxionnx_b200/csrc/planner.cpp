@@ -3337,6 +3337,10 @@ void Planner::match_join(Contraction& c) {
     }
     return true;
   };
+  // A short K over a tensor that does not stay in L2 keeps the join a pass of its own: that pass runs at the memory's
+  // rate, while here the join doubles the instructions of an epilogue that already bounds the layer (1x1 64 -> 256 at
+  // M = 3211264: 788 us joined, 334 + 407 apart; 1x1 128 -> 512 at M = 802816: 352 joined, 178 + 207 apart).
+  if (c.cs.K() < 128 && prod(c.out_shape) > (64ll << 20)) return;
   k::ResidualParams rp{};
   bool has_zp;
   const int dq_i = only_consumer(c.out_name);
