@@ -113,8 +113,17 @@ struct RowSums {
   int W = 0, Q = 0, OC = 0, OCp = 0, S = 0, pl = 0, relu = 0, round_tf32 = 0;
 };
 void row_sums(const float* x, const float* bias, float* y, const RowSums& r, cudaStream_t s);
-// The modulators' lanes of sample n start at n * stride.
-void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32,
+// What follows the normalisation's modulation in its third pass: a residual [pixels][C] added, and a copy of the result padded in its
+// plane (mode as in `pad`).  `y.ptr` may be NULL when only the padded copy is read.  The modulators' lanes of sample n start
+// at n * stride.
+struct NormTail {
+  const float* residual = nullptr;
+  float* padded = nullptr;
+  int pad_h = 0, pad_w = 0, mode = 0;  // extent of the padded plane; 0: constant fill, 1: reflect, 2: edge
+  int pt = 0, pl = 0;
+  float value = 0.f;
+};
+void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32, const NormTail& tail,
                    cudaStream_t s);
 
 // ---- spatial glue -----------------------------------------------------------------------

@@ -757,10 +757,96 @@ __global__ void global_avg_pool_nhwc_kernel(const float* __restrict__ x, float* 
   }
 }
 
+// Four channels of a pixel: one 16-byte access where the channel count allows it, else those that exist.
+__device__ __forceinline__ float4 load_quad(const float* p, bool vec, int have) {
+  if (vec) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(have > 0 ? p[0] : 0.f, have > 1 ? p[1] : 0.f, have > 2 ? p[2] : 0.f, have > 3 ? p[3] : 0.f);
+}
+__device__ __forceinline__ void store_quad(float* p, const float (&v)[4], bool vec, int have) {
+  if (vec) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    return;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (e < have) p[e] = v[e];
+}
+
+// Third pass of the normalisation for the 32 channels of a block: modulation, residual, Relu, and the result written to
+// its plane, to a padded plane or to both (a separate pad reads the plane again and writes it a second time).  A
+// warp takes four pixels of eight float4 lanes: with a pixel a warp the pass was bound by its index arithmetic
+// (4 x 1024 x 32 x 32 padded to 34 x 34: 15.3 + 12.7 us apart, 26.8 us with a pixel a warp, 18.5 us with four).
+template <typename Load>
+__device__ __forceinline__ void norm_write(Load load, const float* x, float* y, const Dims4& d, int64_t n, int64_t c0, int warp, int nwarps, int lane, float mean_l, float inv_l,
+                                           bool mod, float sc_l, float sf_l, int relu, int rtf32, const NormTail& tail) {
+  const int W = (int)d.W, q = (lane & 7) * 4, sub = lane >> 3;
+  const int64_t hw = d.H * d.W, C = d.C;
+  const int have = (int)(C - c0) - q;  // channels of this lane's quad that exist
+  const bool vec = (C & 3) == 0 && (((uintptr_t)x | (uintptr_t)y | (uintptr_t)tail.padded | (uintptr_t)tail.residual) & 15) == 0;
+  float mean[4], inv[4], sc[4], sf[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    mean[e] = __shfl_sync(0xffffffffu, mean_l, q + e), inv[e] = __shfl_sync(0xffffffffu, inv_l, q + e);
+    sc[e] = __shfl_sync(0xffffffffu, sc_l, q + e), sf[e] = __shfl_sync(0xffffffffu, sf_l, q + e);
+  }
+  if (have <= 0) return;
+  const float* res = tail.residual ? tail.residual + n * hw * C + c0 + q : nullptr;
+  float* py = y ? y + n * hw * C + c0 + q : nullptr;
+  auto quad = [&](int64_t j, const float4& r4, float (&v)[4]) {
+    const float4 x4 = load(j, q, vec, have);
+    const float x[4] = {x4.x, x4.y, x4.z, x4.w}, r[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      v[e] = (x[e] - mean[e]) * inv[e];
+      if (mod) v[e] = v[e] * sc[e] + sf[e];  // two roundings, as the separate Mul and Add nodes (this file is built without contraction)
+      if (res) v[e] = v[e] + r[e];
+      if (relu) v[e] = fmaxf(v[e], 0.f);
+      if (rtf32) v[e] = round_tf32(v[e]);
+    }
+  };
+  const int step = 4 * nwarps;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tail.padded == nullptr) {
+#pragma unroll 2
+    for (int64_t j = warp * 4 + sub; j < hw; j += step) {
+      float v[4];
+      quad(j, res ? load_quad(res + j * C, vec, have) : zero, v);
+      store_quad(py + j * C, v, vec, have);
+    }
+    return;
+  }
+  // a lane's pixels of the padded plane are `step` apart: row and column advance without a division
+  const int H = (int)d.H, total = tail.pad_h * tail.pad_w;
+  float* pp = tail.padded + n * total * C + c0 + q;
+  int oh = (warp * 4 + sub) / tail.pad_w, ow = (warp * 4 + sub) - oh * tail.pad_w;
+  const int step_h = step / tail.pad_w, step_w = step - step_h * tail.pad_w;
+#pragma unroll 2
+  for (int o = warp * 4 + sub; o < total; o += step) {
+    int ih = oh - tail.pt, iw = ow - tail.pl;
+    const bool self = (unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W;
+    float v[4] = {tail.value, tail.value, tail.value, tail.value};
+    if (self || tail.mode != 0) {
+      if (tail.mode == 1) {
+        ih = ih < 0 ? -ih : (ih >= H ? 2 * (H - 1) - ih : ih);
+        iw = iw < 0 ? -iw : (iw >= W ? 2 * (W - 1) - iw : iw);
+      } else {
+        ih = min(max(ih, 0), H - 1), iw = min(max(iw, 0), W - 1);
+      }
+      const int64_t j = ih * W + iw;
+      quad(j, res ? load_quad(res + j * C, vec, have) : zero, v);
+      if (py && self) store_quad(py + j * C, v, vec, have);
+    }
+    store_quad(pp + o * C, v, vec, have);
+    oh += step_h, ow += step_w;
+    if (ow >= tail.pad_w) ow -= tail.pad_w, ++oh;
+  }
+}
+
 // Instance norm on NHWC: one block per (n, 32-channel group); 32 lanes across channels
 // (coalesced 128-byte rows), 8 warps striding over the pixels.
 __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps, const float* scale_nc,
-                                          int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32_flag) {
+                                          int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32_flag,
+                                          const __grid_constant__ NormTail tail) {
   pdl_enter();
   int64_t cgroups = (d.C + 31) / 32;
   int64_t n = blockIdx.x / cgroups, cg = blockIdx.x % cgroups;
@@ -769,7 +855,6 @@ __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __
   bool valid = c < d.C;
   int64_t hw = d.H * d.W;
   const float* px = x + n * hw * d.C + c;
-  float* py = y + n * hw * d.C + c;
   __shared__ float red[32][33];
   float sum = 0.f;
   if (valid)
@@ -796,24 +881,20 @@ __global__ void instance_norm_nhwc_kernel(const float* __restrict__ x, float* __
   bool mod = scale_nc != nullptr || shift_nc != nullptr;
   if (valid && scale_nc) sc = scale_nc[n * scale_stride + c];
   if (valid && shift_nc) sf = shift_nc[n * shift_stride + c];
-  if (valid)
-    for (int64_t i = warp; i < hw; i += nwarps) {
-      float v = (px[i * d.C] - mean) * inv_std;
-      if (mod) v = v * sc + sf;  // two roundings, as the separate Mul and Add nodes (this file is built without contraction)
-      if (relu) v = fmaxf(v, 0.f);
-      if (round_tf32_flag) v = round_tf32(v);
-      py[i * d.C] = v;
-    }
+  const float* base = x + n * hw * d.C + cg * 32;
+  norm_write([&](int64_t j, int q, bool vec, int have) { return load_quad(base + j * d.C + q, vec, have); }, x, y, d, n, cg * 32, warp, nwarps, lane, mean,
+             inv_std, mod, sc, sf, relu, round_tf32_flag, tail);
 }
 
 // The same normalisation with the block's slab (all pixels x 32 channels) staged in shared memory by the first pass:
-// the tensor is read from HBM once instead of three times.  32 warps stride over the pixels, four loads in flight
+// the tensor is read from HBM once instead of three times.  32 warps stride over the pixels, eight loads in flight
 // each; the per-warp partial sums are added in warp order as above.
 __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const float* __restrict__ x, float* __restrict__ y, Dims4 d, float eps,
                                                                         const float* scale_nc, int64_t scale_stride, const float* shift_nc,
-                                                                        int64_t shift_stride, int relu, int round_tf32_flag) {
+                                                                        int64_t shift_stride, int relu, int round_tf32_flag,
+                                          const __grid_constant__ NormTail tail) {
   pdl_enter();
-  extern __shared__ float slab[];  // [pixel][32 channels]
+  extern __shared__ __align__(16) float slab[];  // [pixel][32 channels]
   __shared__ float red[32][33];
   const int64_t cgroups = (d.C + 31) / 32;
   const int64_t n = blockIdx.x / cgroups, cg = blockIdx.x % cgroups;
@@ -822,15 +903,14 @@ __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const flo
   const bool valid = c < d.C;
   const int hw = (int)(d.H * d.W);
   const float* px = x + n * hw * d.C + c;
-  float* py = y + n * hw * d.C + c;
   float sum = 0.f;
   int i = warp;
-  for (; i + 96 < hw; i += 128) {
-    float v[4];
+  for (; i + 224 < hw; i += 256) {
+    float v[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = valid ? px[(int64_t)(i + 32 * k) * d.C] : 0.f;
+    for (int k = 0; k < 8; ++k) v[k] = valid ? px[(int64_t)(i + 32 * k) * d.C] : 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 8; ++k) {
       slab[(i + 32 * k) * 32 + lane] = v[k];
       sum += v[k];
     }
@@ -861,14 +941,8 @@ __global__ void __launch_bounds__(1024) instance_norm_nhwc_smem_kernel(const flo
   const bool mod = scale_nc != nullptr || shift_nc != nullptr;
   if (valid && scale_nc) sc = scale_nc[n * scale_stride + c];
   if (valid && shift_nc) sf = shift_nc[n * shift_stride + c];
-  if (valid)
-    for (int j = warp; j < hw; j += 32) {
-      float v = (slab[j * 32 + lane] - mean) * inv_std;
-      if (mod) v = v * sc + sf;  // two roundings, as the separate Mul and Add nodes (this file is built without contraction)
-      if (relu) v = fmaxf(v, 0.f);
-      if (round_tf32_flag) v = round_tf32(v);
-      py[(int64_t)j * d.C] = v;
-    }
+  norm_write([&](int64_t j, int q, bool, int) { return *reinterpret_cast<const float4*>(&slab[(int)j * 32 + q]); }, x, y, d, n, cg * 32, warp, 32, lane, mean,
+             inv_std, mod, sc, sf, relu, round_tf32_flag, tail);
 }
 
 // Second pass of a convolution run as R x 1 filters.  Bound by reading the partials once (4 x 128 x 134 rows of 32 floats:
@@ -2356,7 +2430,7 @@ void row_sums(const float* x, const float* bias, float* y, const RowSums& r, cud
 }
 
 void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc,
-                   int64_t shift_stride, int relu, int round_tf32_flag, cudaStream_t s) {
+                   int64_t shift_stride, int relu, int round_tf32_flag, const NormTail& tail, cudaStream_t s) {
   int64_t cgroups = (x.d.C + 31) / 32;
   int64_t blocks = x.d.N * cgroups;
   if (blocks == 0) return;
@@ -2377,11 +2451,11 @@ void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const floa
       }
     }
     launch(instance_norm_nhwc_smem_kernel, (unsigned)blocks, 1024, slab, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, scale_stride, shift_nc,
-           shift_stride, relu, round_tf32_flag);
+           shift_stride, relu, round_tf32_flag, tail);
     return;
   }
   launch(instance_norm_nhwc_kernel, (unsigned)blocks, 256, 0, s, (const float*)x.ptr, (float*)y.ptr, x.d, eps, scale_nc, scale_stride, shift_nc, shift_stride, relu,
-         round_tf32_flag);
+         round_tf32_flag, tail);
 }
 
 void resize(const TensorRef& x, const TensorRef& y, int mode, int coord, int nearest_rule, float scale_h, float scale_w, int round_tf32_flag,

@@ -468,6 +468,12 @@ class Planner {
   void plan_global_avg_pool(const NodeDef& n);
   void plan_instance_norm(const NodeDef& n);
   void plan_resize(const NodeDef& n);
+  struct PadSpec {
+    std::vector<int64_t> pads, shape;  // shape: the padded tensor's
+    int mode = 0;
+    float value = 0.f;
+  };
+  PadSpec pad_spec(const NodeDef& n, const std::vector<int64_t>& shape);
   void plan_pad(const NodeDef& n);
   void plan_concat(const NodeDef& n);
   void plan_slice(const NodeDef& n);
@@ -2536,8 +2542,48 @@ void Planner::plan_instance_norm(const NodeDef& n) {
       }
     }
   }
+  // Behind the modulation: the addition of a residual that is already on the device, and a spatial Pad of the result, whose
+  // plane the third pass writes itself (beside the unpadded one only if something else reads that).
+  int res_vi = -1, pad_vi = -1, pad_i = -1;
+  bool plain_read = true;
+  if (scale_vi >= 0 && relu == 0 && !graph_outputs_.count(out_name)) {
+    auto it = consumers_.find(out_name);
+    if (it != consumers_.end() && it->second.size() == 1 && it->second[0].second <= 1) {
+      const int add_i = it->second[0].first;
+      const NodeDef& add = nodes_[add_i];
+      if (!skipped_[add_i] && add.op == "Add" && add.inputs.size() == 2 && add.attrs.names().empty() && add.inputs[0] != add.inputs[1]) {
+        auto other = S.index_.find(add.inputs[1 - it->second[0].second]);
+        if (other != S.index_.end()) {
+          const Value& ov = V(other->second);
+          if (ov.dt == DT::F32 && ov.shape == xv.shape && ov.layout == Layout::NHWC && ov.host == nullptr) {
+            res_vi = other->second;
+            skipped_[add_i] = 1;
+            out_name = add.outputs[0];
+          }
+        }
+      }
+    }
+  }
   const int rt = scale_vi >= 0 && feeds_contraction(out_name) ? 1 : 0;
-  int yi = add_value(out_name, xv.shape, DT::F32, Layout::NHWC);
+  k::NormTail tail;
+  if (scale_vi >= 0) {
+    auto it = consumers_.find(out_name);
+    if (it != consumers_.end())
+      for (auto& use : it->second) {
+        const NodeDef& pad = nodes_[use.first];
+        if (use.second != 0 || pad.op != "Pad" || skipped_[use.first] || pad_i >= 0) continue;
+        const PadSpec ps = pad_spec(pad, xv.shape);
+        if (ps.pads[0] || ps.pads[1] || ps.pads[4] || ps.pads[5] || ps.shape[2] * ps.shape[3] >= 1 << 30) continue;
+        pad_i = use.first;
+        tail.pad_h = (int)ps.shape[2], tail.pad_w = (int)ps.shape[3], tail.mode = ps.mode;
+        tail.pt = (int)ps.pads[2], tail.pl = (int)ps.pads[3], tail.value = ps.value;
+        plain_read = it->second.size() > 1 || graph_outputs_.count(out_name) > 0;
+        skipped_[pad_i] = 1;
+        pad_vi = add_value(pad.outputs[0], ps.shape, DT::F32, Layout::NHWC);
+        if (rt) tf32_rounded_names_.insert(pad.outputs[0]);
+      }
+  }
+  int yi = plain_read ? add_value(out_name, xv.shape, DT::F32, Layout::NHWC) : pad_vi;
   TensorRef xr = ref_of(xi), yr = ref_of(yi);
   xr.layout = yr.layout = Layout::NHWC;
   std::vector<int> reads = {xi};
@@ -2555,11 +2601,22 @@ void Planner::plan_instance_norm(const NodeDef& n) {
     return l;
   };
   const Lanes scale = lanes_of(scale_vi), shift = lanes_of(shift_vi);
-  Step& st = add_step(n, scale_vi >= 0 ? "instance_norm+adain" : "instance_norm", 2, reads, {yi});
+  if (res_vi >= 0) reads.push_back(res_vi);
+  std::vector<int> writes = {yi};
+  if (pad_vi >= 0 && plain_read) writes.push_back(pad_vi);
+  std::string kernel = scale_vi >= 0 ? "instance_norm+adain" : "instance_norm";
+  if (res_vi >= 0) kernel += "+residual";
+  if (pad_vi >= 0) kernel += "+pad";
+  Step& st = add_step(n, kernel.c_str(), 2, reads, writes);
   st.work = 3.0 * (double)xv.bytes;
-  st.launch = [this, xr, yr, xi, yi, eps, scale, shift, relu, rt](cudaStream_t s) {
-    k::instance_norm(bound(xr, xi), bound(yr, yi), eps, scale.vi >= 0 ? (const float*)V(scale.vi).ptr + scale.offset : nullptr, scale.stride,
-                     shift.vi >= 0 ? (const float*)V(shift.vi).ptr + shift.offset : nullptr, shift.stride, relu, rt, s);
+  st.launch = [this, xr, yr, xi, yi, eps, scale, shift, relu, rt, tail, res_vi, pad_vi, plain_read](cudaStream_t s) {
+    k::NormTail tl = tail;
+    if (res_vi >= 0) tl.residual = (const float*)V(res_vi).ptr;
+    if (pad_vi >= 0) tl.padded = (float*)V(pad_vi).ptr;
+    k::TensorRef y = bound(yr, yi);
+    if (!plain_read) y.ptr = nullptr;
+    k::instance_norm(bound(xr, xi), y, eps, scale.vi >= 0 ? (const float*)V(scale.vi).ptr + scale.offset : nullptr, scale.stride,
+                     shift.vi >= 0 ? (const float*)V(shift.vi).ptr + shift.offset : nullptr, shift.stride, relu, rt, tl, s);
     C.counters.glue_launches++;
     C.counters.kernel_launches++;
   };
@@ -2613,11 +2670,9 @@ void Planner::plan_resize(const NodeDef& n) {
   };
 }
 
-void Planner::plan_pad(const NodeDef& n) {
+Planner::PadSpec Planner::pad_spec(const NodeDef& n, const std::vector<int64_t>& shape) {
   check_attrs(n, {"mode", "pads", "value"});
-  int xi = value_of(in_name(n, 0));
-  const Value xv = V(xi);
-  if (xv.shape.size() != 4) OXB_DECLINE("Pad '%s': only rank-4 inputs are claimed", n.name.c_str());
+  if (shape.size() != 4) OXB_DECLINE("Pad '%s': only rank-4 inputs are claimed", n.name.c_str());
   std::vector<int64_t> pads;
   if (has_in(n, 1)) {
     const HostTensor* p = const_in(n, 1);
@@ -2637,12 +2692,22 @@ void Planner::plan_pad(const NodeDef& n) {
   std::string mode = n.attrs.s("mode");
   int m = (mode.empty() || mode == "constant") ? 0 : (mode == "reflect" ? 1 : (mode == "edge" ? 2 : -1));
   if (m < 0) OXB_DECLINE("Pad '%s': mode '%s'", n.name.c_str(), mode.c_str());
-  std::vector<int64_t> os = xv.shape;
+  std::vector<int64_t> os = shape;
   for (int d = 0; d < 4; ++d) {
     if (pads[d] < 0 || pads[d + 4] < 0) OXB_DECLINE("Pad '%s': negative pads", n.name.c_str());
-    if (m == 1 && (pads[d] >= xv.shape[d] || pads[d + 4] >= xv.shape[d]) && (pads[d] > 0 || pads[d + 4] > 0)) OXB_DECLINE("Pad: reflect pad must be smaller than the axis extent");
+    if (m == 1 && (pads[d] >= shape[d] || pads[d + 4] >= shape[d]) && (pads[d] > 0 || pads[d + 4] > 0)) OXB_DECLINE("Pad: reflect pad must be smaller than the axis extent");
     os[d] += pads[d] + pads[d + 4];
   }
+  return PadSpec{pads, os, m, value};
+}
+
+void Planner::plan_pad(const NodeDef& n) {
+  int xi = value_of(in_name(n, 0));
+  const Value xv = V(xi);
+  const PadSpec ps = pad_spec(n, xv.shape);
+  const std::vector<int64_t>&pads = ps.pads, &os = ps.shape;
+  const int m = ps.mode;
+  const float value = ps.value;
   int yi = add_value(n.outputs[0], os, xv.dt, xv.layout);
   TensorRef xr = ref_of(xi), yr = ref_of(yi);
   int pn = (int)pads[0], pc = (int)pads[1], ph = (int)pads[2], pw = (int)pads[3];

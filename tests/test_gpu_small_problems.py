@@ -133,3 +133,29 @@ def test_slices_read_in_place_by_the_normalisation(reader):
     assert kernels.count("slice (read in place)") == (2 if reader == "modulators" else 1), kernels
     want, _ = _run(graph, weights, feeds, keep_intermediates=True)
     assert all(np.array_equal(got[o], want[o]) for o in outs)
+
+
+@pytest.mark.parametrize("h,w", [(4, 5), (17, 19), (45, 40)])  # planes of both kernels, the largest past shared memory
+@pytest.mark.parametrize("mode,plain", [("reflect", True), ("edge", False), ("constant", True)])
+def test_normalisation_adds_the_residual_and_pads(h, w, mode, plain):
+    n, c = 2, 40 if plain else 42
+    rng = np.random.default_rng([h, w, len(mode)])
+    weights = {"g": (rng.standard_normal((16, 2 * c)) * 0.3).astype(np.float32), "s0": np.float32([0]), "s1": np.float32([c]), "s2": np.float32([2 * c]),
+               "ax": np.float32([1]), "shape": np.float32([n, c, 1, 1]), "pads": np.float32([0, 0, 1, 2, 0, 0, 3, 0]), "fill": np.float32([0.5])}
+    nodes = [Node("MatMul", "mm", ["l", "g"], ["style"], {}), Node("Slice", "sa", ["style", "s0", "s1", "ax"], ["a"], {}),
+             Node("Slice", "sb", ["style", "s1", "s2", "ax"], ["b"], {}), Node("Reshape", "ra", ["a", "shape"], ["a4"], {}),
+             Node("Reshape", "rb", ["b", "shape"], ["b4"], {}), Node("Relu", "rx", ["x"], ["x1"], {}),
+             Node("MaxPool", "rr", ["x1"], ["r1"], {"kernel_shape": [3, 3], "strides": [1, 1], "pads": [1] * 4}),
+             Node("OxiInstanceNorm", "in", ["r1"], ["xn"], {"epsilon": 1e-5}),
+             Node("Mul", "mul", ["xn", "a4"], ["xm"], {}), Node("Add", "add", ["xm", "b4"], ["xa"], {}), Node("Add", "res", ["xa", "r1"], ["xr"], {}),
+             Node("Pad", "pad", ["xr", "pads", "fill"] if mode == "constant" else ["xr", "pads"], ["y"], {"mode": mode})]
+    outs = ["y"]
+    if plain:
+        nodes.append(Node("Sigmoid", "sg", ["xr"], ["z"], {}))
+        outs.append("z")
+    graph = Graph(nodes=nodes, input_names=["x", "l"], output_names=outs)
+    feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32), "l": rng.standard_normal((n, 16)).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds)
+    assert "instance_norm+adain+residual+pad" in kernels, kernels
+    want, _ = _run(graph, weights, feeds, keep_intermediates=True)
+    assert all(np.array_equal(got[o], want[o]) for o in outs)
