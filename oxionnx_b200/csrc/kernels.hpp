@@ -292,6 +292,12 @@ void umma_plan_destroy(UmmaPlan* p);
 // next launch does not inherit a half-counted tile.  A no-op for plans that do not split K.
 void umma_plan_reset_after_error(UmmaPlan* p);
 void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s);
+// May the plan run beside its predecessors in the stream, as far as its own state goes (no workspace, no extrema keys)?
+bool umma_plan_stands_alone(const UmmaPlan* p);
+// late_trigger: dependents of this launch start only once its predecessors are complete.  late_wait: this launch follows
+// such a launch (or another late_wait one behind it) directly in the stream, reads and overwrites nothing that those
+// write or read, and waits for them only before it ends.
+void umma_plan_set_order(UmmaPlan* p, bool late_trigger, bool late_wait);
 const char* umma_plan_desc(const UmmaPlan* p);
 // Re-point a plan at new buffers (arena moved) is not supported: plans are rebuilt.
 

@@ -730,6 +730,11 @@ void umma_plan_reset_after_error(UmmaPlan* p) {
   (void)cudaMemset(p->ws_count, 0, cnt * sizeof(unsigned int));
 }
 const char* umma_plan_desc(const UmmaPlan* p) { return p->desc; }
+bool umma_plan_stands_alone(const UmmaPlan* p) { return !p->ws && !p->ws_count && p->kp.minmax_keys == nullptr; }
+void umma_plan_set_order(UmmaPlan* p, bool late_trigger, bool late_wait) {
+  p->kp.late_trigger = late_trigger ? 1 : 0;
+  p->kp.late_wait = late_wait ? 1 : 0;
+}
 
 // ---- chain of quantised linear layers over few rows ------------------------------------------------------------
 struct UmmaChain {

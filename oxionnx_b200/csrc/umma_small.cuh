@@ -152,7 +152,7 @@ __device__ __forceinline__ void small_epilogue(const KParams& p, int warp, int l
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
       // the predecessor may still read what this grid overwrites, and write what the lines below read
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
       if (p.x_zp_dev) xz = __float2int_rn(*p.x_zp_dev);
       if (VARIANT >= V_DEQUANT) xs = *p.dq_x_scale;
       bool ok = mbar_spin(bar_acc, 0u, abortp);
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int* abortp = &abort_flag;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---------------- TMA producer: weights of the first ring, then the wait, then everything else ----------------
@@ -311,7 +311,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
         mbar_expect_tx(smem_u32(&bar_full[i]), expect(i));
         tma_load_3d(ring + (uint32_t)i * stage_bytes + kpb * a_bytes, &p.tmB, smem_u32(&bar_full[i]), 0, oc0, it_begin + i * p.kpb);
       }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       uint32_t stage = 0, phase = 0;
       for (int c = 0, it = it_begin; c < chunks; ++c, it += p.kpb) {
         const uint32_t full = smem_u32(&bar_full[stage]), dst = ring + stage * stage_bytes;
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      asm volatile("griddepcontrol.wait;" ::: "memory");  // the bounded waits below must not time the predecessor
+      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");  // the bounded waits below must not time the predecessor
       const uint64_t desc = make_smem_desc(0, swz);
       uint32_t stage = 0, phase = 0;
       for (int it = it_begin; it < it_end; it += p.kpb) {
@@ -450,6 +451,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   }
   __syncthreads();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+  if (p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // The opt-in for more than 48 KB of dynamic shared memory, per kernel and device (see ensure_smem_attr).  The split

@@ -159,3 +159,27 @@ def test_normalisation_adds_the_residual_and_pads(h, w, mode, plain):
     assert "instance_norm+adain+residual+pad" in kernels, kernels
     want, _ = _run(graph, weights, feeds, keep_intermediates=True)
     assert all(np.array_equal(got[o], want[o]) for o in outs)
+
+
+# rows and the three products' widths: all small, the persistent kernel's, split K beside unsplit, one after the other's memory
+@pytest.mark.parametrize("rows,k,widths", [(5, 256, (96, 512, 40)), (154, 768, (768, 768, 768)), (3000, 512, (512, 1024, 256)), (64, 2048, (64, 2048, 1000))])
+@pytest.mark.parametrize("graph_replay", [False, True])
+def test_products_that_run_side_by_side(rows, k, widths, graph_replay):
+    rng = np.random.default_rng([rows, k, *widths])
+    weights, nodes, outs = {}, [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {})], []
+    for i, n in enumerate(widths):
+        weights[f"w{i}"] = rng.integers(-127, 128, (k, n)).astype(np.float32)
+        nodes.append(Node("MatMulInteger", f"mm{i}", ["xq", f"w{i}", "xz"], [f"acc{i}"], {}))
+    for i, n in enumerate(widths):
+        nodes.append(Node("Relu", f"r{i}", [f"acc{i}"], [f"y{i}"], {}))
+        outs.append(f"y{i}")
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=outs)
+    sess = Session.builder().with_cuda_graph(graph_replay).build_from_graph(graph, weights)
+    ref = Session.builder().with_kernel_path("direct").build_from_graph(graph, weights)
+    for _ in range(6):
+        feeds = {"x": rng.standard_normal((rows, k)).astype(np.float32)}
+        got, want = sess.run(feeds), ref.run(feeds)
+        assert all(np.array_equal(got[o], want[o]) for o in outs)
+    assert sum("umma_i8" in s["kernel"] for s in sess.steps()) == 3
+    sess.close()
+    ref.close()
