@@ -549,6 +549,7 @@ class Planner {
   };
   void emit_contraction(const NodeDef& n, Contraction& c);
   void match_join(Contraction& c);
+  void plan_siblings(int ni);
 
   void finalize_lifetimes_and_arena();
   struct PlanStep {
@@ -611,6 +612,7 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
     if (skipped_[ni]) continue;
     cur_node_ = (int)ni;
     plan_node((int)ni);
+    plan_siblings((int)ni);
   }
 
   // graph outputs: f32 lanes in logical order in persistent staging
@@ -695,6 +697,27 @@ void Planner::link_independent() {
     if (j > i + 1)
       for (size_t m = i; m < j; ++m) k::umma_plan_set_order(plan_steps_[m].plan, m == i, m > i);
     i = j;
+  }
+}
+
+// A convolution that reads what node `ni`, a convolution too, reads and otherwise only initializers (the projection
+// shortcut of a residual block) is planned right behind it, so that the two run side by side (link_independent) and the
+// shortcut's sum joins the branch's last convolution instead.  For inputs of up to 16 MB, where a layer leaves part of
+// the chip idle; beyond, a layer fills it and the shortcut's output would only be kept for longer (one frame: INT8 326 -> 316 us, f32 436 -> 417 us).
+void Planner::plan_siblings(int ni) {
+  const NodeDef& n = nodes_[ni];
+  if ((n.op != "Conv" && n.op != "QLinearConv") || C.cfg().keep_intermediates || n.inputs.empty()) return;
+  auto x = S.index_.find(n.inputs[0]);
+  auto it = consumers_.find(n.inputs[0]);
+  if (x == S.index_.end() || it == consumers_.end() || V(x->second).bytes > (16u << 20)) return;
+  for (auto& use : it->second) {
+    const int si = use.first;
+    if (si <= ni || skipped_[si] || nodes_[si].op != n.op || use.second != 0) continue;
+    bool ready = true;
+    for (size_t i = 1; i < nodes_[si].inputs.size(); ++i) ready = ready && (nodes_[si].inputs[i].empty() || const_of(nodes_[si].inputs[i]) != nullptr);
+    if (!ready) continue;
+    plan_node(si);
+    skipped_[si] = 1;
   }
 }
 
