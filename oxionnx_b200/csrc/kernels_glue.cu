@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(kThreads) dynq_apply_wide_kernel(const float* 
   uint32_t* y4 = (uint32_t*)y;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-  for (int64_t base = ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)) * 128; base < n4; base += warps * 128) {
+  // from the end: what the producer wrote last is still in L2 (100 MB: 33.1 -> 31.0 us)
+  for (int64_t base = ((n4 + 127) / 128 - 1 - ((int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5))) * 128; base >= 0; base -= warps * 128) {
     float4 v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
