@@ -1094,6 +1094,47 @@ __global__ void pad_kernel(const void* x, void* y, DT dt, Layout L, Dims4 xd, Di
   }
 }
 
+// Linear resize of many channels (C % 4 == 0, C >= 128): the pixel-by-pixel form above is bound by its index divisions and
+// coordinates, which four channels cannot pay for.  A block takes kResizeSpan pixels of one output row, so the row's
+// coordinates are found once, a warp takes a pixel and its lanes the channels.  Same arithmetic per lane
+// (4 x 512 x 64 x 64 doubled: 78.4 -> 55.6 us; 4 x 1024 x 32 x 32: 43.3 -> 29.0 us).
+constexpr int kResizeSpan = 32;
+__global__ void __launch_bounds__(256) resize_linear_rows_kernel(const float4* __restrict__ x, float4* __restrict__ y, Dims4 xd, Dims4 yd, int coord, float sh,
+                                                                 float sw, int rtf32) {
+  pdl_enter();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c4n = (int)(yd.C / 4);
+  const int64_t n = blockIdx.x / yd.H, oy = blockIdx.x - n * yd.H;
+  const float cy = fminf(fmaxf(src_coord(coord, oy, sh, xd.H, yd.H), 0.f), (float)(xd.H - 1));
+  const int64_t y0 = (int64_t)floorf(cy), y1 = y0 + 1 < xd.H ? y0 + 1 : xd.H - 1;
+  const float fy = __fsub_rn(cy, (float)y0), gy = __fsub_rn(1.f, fy);
+  const float4 *row0 = x + (n * xd.H + y0) * xd.W * c4n, *row1 = x + (n * xd.H + y1) * xd.W * c4n;
+  float4* out = y + (int64_t)blockIdx.x * yd.W * c4n;
+  const int64_t last = min((int64_t)(blockIdx.y + 1) * kResizeSpan, yd.W);
+  for (int64_t ox = (int64_t)blockIdx.y * kResizeSpan + warp; ox < last; ox += 8) {
+    const float cx = fminf(fmaxf(src_coord(coord, ox, sw, xd.W, yd.W), 0.f), (float)(xd.W - 1));
+    const int64_t x0 = (int64_t)floorf(cx), x1 = x0 + 1 < xd.W ? x0 + 1 : xd.W - 1;
+    const float fx = __fsub_rn(cx, (float)x0), gx = __fsub_rn(1.f, fx);
+    const float4 *p00 = row0 + x0 * c4n, *p01 = row0 + x1 * c4n, *p10 = row1 + x0 * c4n, *p11 = row1 + x1 * c4n;
+    float4* o = out + ox * c4n;
+#pragma unroll 2
+    for (int c = lane; c < c4n; c += 32) {
+      const float4 v00 = p00[c], v01 = p01[c], v10 = p10[c], v11 = p11[c];
+      float4 r;
+#define OXB_LERP(f)                                                                          \
+  {                                                                                          \
+    const float top = __fadd_rn(__fmul_rn(v00.f, gx), __fmul_rn(v01.f, fx));                 \
+    const float bot = __fadd_rn(__fmul_rn(v10.f, gx), __fmul_rn(v11.f, fx));                 \
+    r.f = __fadd_rn(__fmul_rn(top, gy), __fmul_rn(bot, fy));                                 \
+  }
+      OXB_LERP(x) OXB_LERP(y) OXB_LERP(z) OXB_LERP(w)
+#undef OXB_LERP
+      if (rtf32) r = make_float4(round_tf32(r.x), round_tf32(r.y), round_tf32(r.z), round_tf32(r.w));  // the lanes feed a TF32 product
+      o[c] = r;
+    }
+  }
+}
+
 // Spatial padding of an NHWC tensor in 16-byte pieces (any storage type whose pixel is a multiple of 16 bytes).
 template <typename I>  // index type: 32-bit divisions where the tensor allows them
 __global__ void pad_nhwc_vec_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, Dims4 xd, Dims4 yd, int64_t vec_per_pixel, int mode, uint4 fill,
@@ -2464,7 +2505,11 @@ void resize(const TensorRef& x, const TensorRef& y, int mode, int coord, int nea
   int64_t total = y.d.numel();
   if (total == 0) return;
   if (y.d.C % 4 == 0 && ((uintptr_t)x.ptr & 15) == 0 && ((uintptr_t)y.ptr & 15) == 0) {
-    if (total / 4 + (int64_t)148 * 64 * kThreads < (int64_t)1 << 31)
+    const int64_t rows = y.d.N * y.d.H, spans = (y.d.W + kResizeSpan - 1) / kResizeSpan;
+    if (mode != 0 && y.d.C >= 128 && y.d.C < (int64_t)1 << 31 && rows < (int64_t)1 << 31 && spans < 65536)  // fewer channels leave lanes of a warp idle
+      launch(resize_linear_rows_kernel, dim3((unsigned)rows, (unsigned)spans), 256, 0, s, (const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, coord, scale_h, scale_w,
+             round_tf32_flag);
+    else if (total / 4 + (int64_t)148 * 64 * kThreads < (int64_t)1 << 31)
       launch(resize_nhwc_vec4_kernel<uint32_t>, grid_for(total / 4), kThreads, 0, s, (const float4*)x.ptr, (float4*)y.ptr, x.d, y.d, mode, coord, nearest_rule,
                                                                                 scale_h, scale_w, total / 4, round_tf32_flag);
     else

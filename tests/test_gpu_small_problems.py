@@ -183,3 +183,17 @@ def test_products_that_run_side_by_side(rows, k, widths, graph_replay):
     assert sum("umma_i8" in s["kernel"] for s in sess.steps()) == 3
     sess.close()
     ref.close()
+
+
+@pytest.mark.parametrize("channels,h,w,scale", [(128, 5, 7, 2.0), (132, 9, 33, 1.5), (320, 1, 70, 3.0)])
+@pytest.mark.parametrize("coord", ["half_pixel", "align_corners", "asymmetric"])
+def test_linear_resize_of_many_channels_is_the_one_of_few(channels, h, w, scale, coord):
+    rng = np.random.default_rng([channels, h, w])
+    weights = {"s": np.float32([1, 1, scale, scale])}
+    nodes = [Node("Relu", "r", ["x"], ["x1"], {}), Node("Resize", "up", ["x1", "", "s"], ["y"], {"mode": "linear", "coordinate_transformation_mode": coord})]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    x = rng.standard_normal((2, channels, h, w)).astype(np.float32)
+    got, _ = _run(graph, weights, {"x": x})
+    for c in range(0, channels, 64):
+        want, _ = _run(graph, weights, {"x": np.ascontiguousarray(x[:, c:c + 64])})
+        assert np.array_equal(got["y"][:, c:c + 64], want["y"])
