@@ -126,6 +126,9 @@ struct NormTail {
 void instance_norm(const TensorRef& x, const TensorRef& y, float eps, const float* scale_nc, int64_t scale_stride, const float* shift_nc, int64_t shift_stride, int relu, int round_tf32, const NormTail& tail,
                    cudaStream_t s);
 
+// A copy between device memory and page-locked host memory (either way) by a kernel.
+void copy_bytes(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
 // ---- spatial glue -----------------------------------------------------------------------
 // mode 0 nearest, 1 linear; coord 0 half_pixel, 1 pytorch_half_pixel, 2 asymmetric,
 // 3 align_corners; nearest_rule 0 round_prefer_floor, 1 floor, 2 ceil, 3 round_prefer_ceil
