@@ -1814,7 +1814,7 @@ __global__ void softmax_rows_reg_kernel(const float4* __restrict__ x, float4* __
 // Bound by the FMA pipe for long sequences (4 * S * S * 64 per head) and by latency for short ones.  A block takes TM
 // query rows of one head, so that short batches still fill the chip; a thread holds RM x 4 results, which takes one
 // 16-byte read of each operand per RM x 4 FMAs, and K is kept transposed so that both are conflict free.  The
-// block's score rows stay in shared memory.  A layer of 2 x 77 positions, 12 heads: 60 us in eight launches -> 15 us.
+// block's score rows stay in shared memory.  A layer of 2 x 77 positions, 12 heads: 60 us in eight launches -> 18 us.
 template <int TM>
 __global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ kk, const float* __restrict__ v,
                                                             float* __restrict__ out, int S, int H, const float* __restrict__ scale,
