@@ -379,9 +379,23 @@ class SessionBuilder:
         return Session.from_model(Model.from_file(path), self._device, 1 if level is None else level, self._input_shapes, **self._ctx_kw)
 
 
+def _lanes(feeds, names):
+    """The feeds of `names` as arrays the library reads in place: contiguous, 8-bit lanes as they are, anything else as
+    f32."""
+    lanes = {}
+    for name in names:
+        if name in feeds:
+            a = feeds[name]
+            typed = isinstance(a, np.ndarray) and a.dtype in _ffi.TYPED
+            lanes[name] = np.ascontiguousarray(a if typed else np.asarray(a, dtype=np.float32))
+    return lanes
+
+
 class _CallIo:
     """The operand and result structures of a planned session's calls: names, shapes and extents are filled in once,
-    each call only sets the buffers' addresses (marshalling from scratch was 20 us of a small run)."""
+    each call only sets the buffers' addresses (marshalling from scratch was 20 us of a small run).  One set per session:
+    from the first address set until the library has returned, a call holds the session's lock, or a call of another
+    thread would put its own addresses in their place."""
 
     def __init__(self, session):
         self.lib = lib = _ffi.lib()
@@ -406,23 +420,19 @@ class _CallIo:
             res.cap = int(r.len)
             self.outputs.append((name, shape, res))
 
-    def set_feeds(self, feeds):
-        """Points the operands at the feeds' lanes; the returned arrays must outlive the call."""
-        held = []
+    def set_feeds(self, lanes):
+        """Points the operands at the feeds' lanes (see _lanes), which must outlive the call."""
         for name, shape, op in self.inputs:
-            if name not in feeds:
+            if name not in lanes:
                 raise OnnxError(f"TensorNotFound: missing feed '{name}'")
-            a = feeds[name]
-            typed = _ffi.TYPED.get(a.dtype) if isinstance(a, np.ndarray) else None
-            a = np.ascontiguousarray(a if typed is not None else np.asarray(a, dtype=np.float32))
+            a = lanes[name]
             if a.shape != shape and not (shape == () and a.size == 1):
                 raise OnnxError(f"run: feed '{name}' has shape {a.shape}, the plan expects {shape}")
-            held.append(a)
+            typed = _ffi.TYPED.get(a.dtype)
             if typed is None:
                 op.lanes, op.typed = a.ctypes.data, None
             else:
                 op.lanes, op.typed, op.dtype = None, a.ctypes.data, typed
-        return held
 
     def set_fetches(self):
         """Points the results at fresh arrays, which the call fills."""
@@ -450,6 +460,7 @@ class Session:
         self._planned_for = None
         self._io = None
         self._in_flight = []
+        self._lock = threading.RLock()
 
     @classmethod
     def from_file(cls, path: str, device: int = 0, optimization_level: int = 1, input_shapes: Optional[Dict[str, tuple]] = None, **ctx_kw):
@@ -478,6 +489,7 @@ class Session:
         self._planned_for = None
         self._io = None
         self._in_flight = []
+        self._lock = threading.RLock()
         return self
 
     def _plan(self, shapes):
@@ -516,54 +528,61 @@ class Session:
                     break
             else:
                 return
-        shapes = dict(self._input_shapes)
-        if feeds is not None:
-            shapes.update({k: tuple(np.asarray(v).shape) for k, v in feeds.items()})
-            if self._planned_for is None:  # a feed that arrives as 8-bit lanes declares its input 8-bit
-                for k, v in feeds.items():
-                    if isinstance(v, np.ndarray) and v.dtype in _ffi.TYPED:
-                        self._input_types.setdefault(k, v.dtype)
-        if self._planned_for != {k: tuple(shapes[k]) for k in self.graph.input_names}:
-            self._plan({k: tuple(shapes[k]) for k in self.graph.input_names})
+        with self._lock:
+            shapes = dict(self._input_shapes)
+            if feeds is not None:
+                shapes.update({k: tuple(np.asarray(v).shape) for k, v in feeds.items()})
+                if self._planned_for is None:  # a feed that arrives as 8-bit lanes declares its input 8-bit
+                    for k, v in feeds.items():
+                        if isinstance(v, np.ndarray) and v.dtype in _ffi.TYPED:
+                            self._input_types.setdefault(k, v.dtype)
+            if self._planned_for != {k: tuple(shapes[k]) for k in self.graph.input_names}:
+                self._plan({k: tuple(shapes[k]) for k in self.graph.input_names})
 
     # ---- marshalling of planned runs: the call structures are built once per plan, a run fills in addresses ----
+    # Threads may share a session: each converts its feeds for itself, then holds the lock from planning until the library
+    # has returned and the message of a failure has been read.
     def _call_io(self):
         if self._io is None:
             self._io = _CallIo(self)
         return self._io
 
     def run(self, feeds: Dict[str, np.ndarray]) -> Dict[str, np.ndarray]:
-        self.ensure_planned(feeds)
-        io = self._call_io()
-        held = io.set_feeds(feeds)
-        outs = io.set_fetches()
-        st = io.lib.oxb200_run(self.ctx.handle, io.feeds_ptr, io.n_in, io.fetches_ptr, io.n_out)
-        del held
-        if st:
-            _raise_for(st, self.ctx.last_error())
+        lanes = _lanes(feeds, self.graph.input_names)
+        with self._lock:
+            self.ensure_planned(feeds)
+            io = self._call_io()
+            io.set_feeds(lanes)
+            outs = io.set_fetches()
+            st = io.lib.oxb200_run(self.ctx.handle, io.feeds_ptr, io.n_in, io.fetches_ptr, io.n_out)
+            if st:
+                _raise_for(st, self.ctx.last_error())
         return outs
 
     # ---- pipelined runs: the upload of the next batch overlaps the run of the current one ----
     def submit(self, feeds: Dict[str, np.ndarray]):
         """Enqueues one run (upload, steps, download) and returns at once; at most two may be in flight.
         The feed arrays must stay unchanged until the matching collect()."""
-        self.ensure_planned(feeds)
-        io = self._call_io()
-        held = io.set_feeds(feeds)
-        st = io.lib.oxb200_run_submit(self.ctx.handle, io.feeds_ptr, io.n_in)
-        if st:
-            _raise_for(st, self.ctx.last_error())
-        self._in_flight.append(held)
+        lanes = _lanes(feeds, self.graph.input_names)
+        with self._lock:
+            self.ensure_planned(feeds)
+            io = self._call_io()
+            io.set_feeds(lanes)
+            st = io.lib.oxb200_run_submit(self.ctx.handle, io.feeds_ptr, io.n_in)
+            if st:
+                _raise_for(st, self.ctx.last_error())
+            self._in_flight.append(lanes)
 
     def collect(self) -> Dict[str, np.ndarray]:
         """Waits for the oldest submitted run and returns its outputs."""
-        io = self._call_io()
-        outs = io.set_fetches()
-        st = io.lib.oxb200_run_collect(self.ctx.handle, io.fetches_ptr, io.n_out)
-        if self._in_flight:
-            self._in_flight.pop(0)
-        if st:
-            _raise_for(st, self.ctx.last_error())
+        with self._lock:
+            io = self._call_io()
+            outs = io.set_fetches()
+            st = io.lib.oxb200_run_collect(self.ctx.handle, io.fetches_ptr, io.n_out)
+            if self._in_flight:
+                self._in_flight.pop(0)
+            if st:
+                _raise_for(st, self.ctx.last_error())
         return outs
 
     def run_pipelined(self, batches):
@@ -618,9 +637,10 @@ class Session:
         if not fetch:
             _raise_for(lib.oxb200_run_bound(self.ctx.handle, ops, len(names), None, 0), self.ctx.last_error())
             return None
-        io = self._call_io()
-        outs = io.set_fetches()
-        _raise_for(lib.oxb200_run_bound(self.ctx.handle, ops, len(names), io.fetches_ptr, io.n_out), self.ctx.last_error())
+        with self._lock:
+            io = self._call_io()
+            outs = io.set_fetches()
+            _raise_for(lib.oxb200_run_bound(self.ctx.handle, ops, len(names), io.fetches_ptr, io.n_out), self.ctx.last_error())
         return outs
 
     def clear_bindings(self):
@@ -628,11 +648,12 @@ class Session:
 
     # ---- measurement helpers: the same run split into stage / resident launches / read ----
     def upload(self, feeds):
-        self.ensure_planned(feeds)
-        io = self._call_io()
-        held = io.set_feeds(feeds)
-        _raise_for(io.lib.oxb200_upload_feeds(self.ctx.handle, io.feeds_ptr, io.n_in), self.ctx.last_error())
-        del held
+        lanes = _lanes(feeds, self.graph.input_names)
+        with self._lock:
+            self.ensure_planned(feeds)
+            io = self._call_io()
+            io.set_feeds(lanes)
+            _raise_for(io.lib.oxb200_upload_feeds(self.ctx.handle, io.feeds_ptr, io.n_in), self.ctx.last_error())
 
     def run_resident(self, iters=1) -> float:
         ms = ctypes.c_float()
@@ -640,9 +661,10 @@ class Session:
         return float(ms.value)
 
     def download(self) -> Dict[str, np.ndarray]:
-        io = self._call_io()
-        outs = io.set_fetches()
-        _raise_for(io.lib.oxb200_download_fetches(self.ctx.handle, io.fetches_ptr, io.n_out), self.ctx.last_error())
+        with self._lock:
+            io = self._call_io()
+            outs = io.set_fetches()
+            _raise_for(io.lib.oxb200_download_fetches(self.ctx.handle, io.fetches_ptr, io.n_out), self.ctx.last_error())
         return outs
 
     def fetch_value(self, name: str) -> np.ndarray:
