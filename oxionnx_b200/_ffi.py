@@ -5,6 +5,8 @@ import os
 
 import numpy as np
 
+from .graph import Node
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("OXB200_LIBRARY") or os.path.join(HERE, "_lib", "liboxb200.so")
 
@@ -215,13 +217,16 @@ def pack_node(node, cnode, keep):
 
 def packed_node(node):
     """(fields, CNode, buffers) of a node, kept on the node itself for as long as its fields stay what they were; hold the
-    tuple for as long as the CNode is used."""
+    tuple for as long as the CNode is used.  Only a graph.Node leaves it out when it is copied or pickled, so any other
+    object is packed anew."""
     now = (node.op, node.name, list(node.inputs), list(node.outputs), {k: list(v) if isinstance(v, (list, tuple)) else v for k, v in (node.attrs or {}).items()})
-    have = node.__dict__.get("_packed")
+    have = getattr(node, "_packed", None)
     if have is None or any(isinstance(v, np.ndarray) for v in now[4].values()) or have[0] != now:
         keep, cnode = Keep(), CNode()
         pack_node(node, cnode, keep)
-        have = node.__dict__["_packed"] = (now, cnode, keep)
+        have = (now, cnode, keep)
+        if isinstance(node, Node):
+            node.__dict__["_packed"] = have
     return have
 
 

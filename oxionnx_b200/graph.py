@@ -20,6 +20,10 @@ class Node:
     outputs: List[str]
     attrs: Dict[str, object] = field(default_factory=dict)
 
+    def __getstate__(self):
+        # what a dispatch keeps on the node (_ffi.packed_node) holds addresses: copies and pickles go without it
+        return {k: v for k, v in self.__dict__.items() if k != "_packed"}
+
 
 @dataclass
 class Graph:
