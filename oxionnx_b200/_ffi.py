@@ -215,13 +215,20 @@ def pack_node(node, cnode, keep):
     cnode.attrs, cnode.n_attrs = arr, n
 
 
+def _attr_key(value):
+    """An attribute's value with its type and its elements' types: 1 and 1.0 are equal but travel as different kinds."""
+    if isinstance(value, (list, tuple)):
+        return [(type(v), v) for v in value]
+    return (type(value), value)
+
+
 def packed_node(node):
     """(fields, CNode, buffers) of a node, kept on the node itself for as long as its fields stay what they were; hold the
     tuple for as long as the CNode is used.  Only a graph.Node leaves it out when it is copied or pickled, so any other
     object is packed anew."""
-    now = (node.op, node.name, list(node.inputs), list(node.outputs), {k: list(v) if isinstance(v, (list, tuple)) else v for k, v in (node.attrs or {}).items()})
+    now = (node.op, node.name, list(node.inputs), list(node.outputs), {k: _attr_key(v) for k, v in (node.attrs or {}).items()})
     have = getattr(node, "_packed", None)
-    if have is None or any(isinstance(v, np.ndarray) for v in now[4].values()) or have[0] != now:
+    if have is None or any(isinstance(v, np.ndarray) for v in (node.attrs or {}).values()) or have[0] != now:
         keep, cnode = Keep(), CNode()
         pack_node(node, cnode, keep)
         have = (now, cnode, keep)
