@@ -295,12 +295,14 @@ void umma_plan_destroy(UmmaPlan* p);
 // next launch does not inherit a half-counted tile.  A no-op for plans that do not split K.
 void umma_plan_reset_after_error(UmmaPlan* p);
 void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s);
-// May the plan run beside its predecessors in the stream, as far as its own state goes (no workspace, no extrema keys)?
-bool umma_plan_stands_alone(const UmmaPlan* p);
-// late_trigger: dependents of this launch start only once its predecessors are complete.  late_wait: this launch follows
-// such a launch (or another late_wait one behind it) directly in the stream, reads and overwrites nothing that those
-// write or read, and waits for them only before it ends.
-void umma_plan_set_order(UmmaPlan* p, bool late_trigger, bool late_wait);
+// One to kGroupMax small problems that read and overwrite nothing of one another, as one launch.  Null when the plans are not
+// all small ones of one kind.  The group keeps what it needs of the plans.
+struct UmmaGroup;
+constexpr int kGroupMax = 3;
+bool umma_plans_group(const UmmaPlan* a, const UmmaPlan* b);  // may the two be members of one group?
+UmmaGroup* umma_group_create(UmmaPlan* const* plans, int n);
+void umma_group_destroy(UmmaGroup* g);
+void umma_group_launch(const UmmaGroup* g, int* err_flag, cudaStream_t s);
 const char* umma_plan_desc(const UmmaPlan* p);
 // Re-point a plan at new buffers (arena moved) is not supported: plans are rebuilt.
 

@@ -118,12 +118,20 @@ constexpr size_t kSmemBudget = 227 * 1024 - 2048;
 
 }  // namespace
 
+// A launch of the small-problem kernel.
+struct UmmaGroup {
+  SmallGroup g;
+  int kind = 0, grid = 0, device = 0;
+  size_t smem = 0;
+};
+
 struct UmmaPlan {
   KParams kp;
   int bn;
   int kind;
   int pair;
   int small;  // the small-problem kernel (umma_small.cuh)
+  UmmaGroup* alone = nullptr;  // ... and its launch by itself
   int grid;
   int device;
   size_t smem;
@@ -615,6 +623,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   if (kp.splits > 1) snprintf(split_note, sizeof split_note, " splitK=%d", kp.splits);
   snprintf(pl->desc, sizeof pl->desc, "umma_%s M=%lld N=%d K=%lld tile=%dx%dx%dB stages=%dx%d %s%s%s", kname, (long long)M, cs.OC, (long long)cs.K(),
            pair ? 256 : a_rows, bn, swz, kp.stages, kp.kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? " cta-pair" : (pl->small ? " small" : ""));
+  if (pl->small) pl->alone = umma_group_create(&pl, 1);
   return pl;
 }
 
@@ -723,6 +732,7 @@ UmmaPlan* umma_plan_create_batched(const BatchedGemm& g, std::string* why) {
 
 void umma_plan_destroy(UmmaPlan* p) {
   if (!p) return;
+  umma_group_destroy(p->alone);
   if (p->ws) cudaFree(p->ws);
   if (p->ws_count) cudaFree(p->ws_count);
   delete p;
@@ -733,10 +743,40 @@ void umma_plan_reset_after_error(UmmaPlan* p) {
   (void)cudaMemset(p->ws_count, 0, cnt * sizeof(unsigned int));
 }
 const char* umma_plan_desc(const UmmaPlan* p) { return p->desc; }
-bool umma_plan_stands_alone(const UmmaPlan* p) { return !p->ws && !p->ws_count && p->kp.minmax_keys == nullptr; }
-void umma_plan_set_order(UmmaPlan* p, bool late_trigger, bool late_wait) {
-  p->kp.late_trigger = late_trigger ? 1 : 0;
-  p->kp.late_wait = late_wait ? 1 : 0;
+
+// ---- small problems, alone or side by side ------------------------------------------------------------------------
+static_assert(kGroupMax == GROUP_MAX, "one limit");
+
+bool umma_plans_group(const UmmaPlan* a, const UmmaPlan* b) {
+  const int ka = a->kind == KIND_BF16 ? KIND_F16 : a->kind, kb = b->kind == KIND_BF16 ? KIND_F16 : b->kind;
+  return a->small && b->small && ka == kb && a->device == b->device;
+}
+UmmaGroup* umma_group_create(UmmaPlan* const* plans, int n) {
+  if (n < 1 || n > GROUP_MAX) return nullptr;
+  for (int i = 0; i < n; ++i)
+    if (!umma_plans_group(plans[0], plans[i])) return nullptr;
+  UmmaGroup* u = new UmmaGroup();
+  u->kind = plans[0]->kind, u->device = plans[0]->device;
+  SmallGroup& g = u->g;
+  g.width = 1;
+  for (int i = 0; i < n; ++i) g.width = std::max(g.width, plans[i]->kp.splits);
+  for (int i = 0; i < GROUP_MAX; ++i) {
+    g.first[i] = i < n ? u->grid : 0x7fffffff;
+    if (i >= n) continue;
+    g.m[i] = plans[i]->kp;
+    u->grid += (int)ceil_div((int64_t)plans[i]->grid, g.width) * g.width;  // splits are powers of two: whole tiles
+    u->smem = std::max(u->smem, plans[i]->smem);
+  }
+  return u;
+}
+void umma_group_destroy(UmmaGroup* u) { delete u; }
+void umma_group_launch(const UmmaGroup* u, int* err_flag, cudaStream_t s) {
+  SmallGroup g = u->g;
+  for (KParams& m : g.m) m.err_flag = err_flag;
+  if (u->kind == KIND_I8) launch_small_i8(g, u->grid, u->smem, u->device, s);
+  else if (u->kind == KIND_TF32) launch_small_tf32(g, u->grid, u->smem, u->device, s);
+  else launch_small_f16(g, u->grid, u->smem, u->device, s);
+  OXB_CUDA(cudaGetLastError());
 }
 
 // ---- chain of quantised linear layers over few rows ------------------------------------------------------------
@@ -969,13 +1009,10 @@ bool umma_chain_launch(const UmmaChain* c, int* err_flag, const float* head_x, c
 }
 
 void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s) {
+  if (p->alone) return umma_group_launch(p->alone, err_flag, s);
   KParams kp = p->kp;
   kp.err_flag = err_flag;
-  if (p->small) {
-    if (p->kind == KIND_I8) launch_small_i8(kp, p->grid, p->smem, p->device, s);
-    else if (p->kind == KIND_TF32) launch_small_tf32(kp, p->grid, p->smem, p->device, s);
-    else launch_small_f16(kp, p->grid, p->smem, p->device, s);
-  } else if (p->kind == KIND_I8) launch_kind_i8(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
+  if (p->kind == KIND_I8) launch_kind_i8(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   else if (p->kind == KIND_TF32) launch_kind_tf32(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   else launch_kind_f16(kp, p->bn, p->pair != 0, p->grid, p->smem, p->device, s);
   OXB_CUDA(cudaGetLastError());

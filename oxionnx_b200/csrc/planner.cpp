@@ -666,12 +666,13 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
   link_independent();
 }
 
-// Neighbouring contractions that depend on nothing of one another (the Q, K and V products of an attention layer, a
-// style's Gemm behind a convolution) run side by side: the first opens the stream when its predecessors are complete, the
-// others do not wait for it.  Small ones then share the chip, large ones start in the last, partly empty wave of the
-// one before (an encoder layer with three 768 -> 768 products, M=154: 100 -> 84 us; M=8192: 299 -> 295 us).  A member
-// may overwrite nothing that the others read or write, so memory that the arena hands on between them ends a run, and
-// so does an output that outlives the pass.
+// Neighbouring small contractions that depend on nothing of one another (the Q, K and V products of an attention layer, a
+// residual block's first convolution and its shortcut) run side by side as one launch of the first of them; the others
+// keep their place in the plan and launch nothing (each by itself -> side by side: encoder of 2x77 tokens 1153 -> 1016 us,
+// one frame through the INT8 network 323 -> 306 us, through the f32 network 439 -> 420 us).  Large ones keep a launch each:
+// a product may only start beside another, ahead of its own wait, where the two are one grid, since a grid sees what
+// was written before its predecessor through that wait alone.  A member may overwrite nothing that the others read or
+// write, so memory that the arena hands on between them ends a run, and so does an output that outlives the pass.
 void Planner::link_independent() {
   auto overlap = [&](const std::vector<int>& a, const std::vector<int>& b) {
     for (int i : a)
@@ -681,21 +682,40 @@ void Planner::link_independent() {
       }
     return false;
   };
-  auto own_launch = [&](const PlanStep& t) { return S.steps_[t.step].kernel.find("chain") == std::string::npos; };
+  auto own_launch = [&](const PlanStep& t) {
+    const Step& st = S.steps_[t.step];
+    bool ok = st.kernel.find("chain") == std::string::npos;
+    for (int w : st.writes) ok = ok && !V(w).external && !V(w).is_graph_output;
+    return ok;
+  };
   for (size_t i = 0; i < plan_steps_.size();) {
     size_t j = i + 1;
-    for (; own_launch(plan_steps_[i]) && j < plan_steps_.size(); ++j) {
+    for (; own_launch(plan_steps_[i]) && j < plan_steps_.size() && j - i < (size_t)k::kGroupMax; ++j) {
       const Step& st = S.steps_[plan_steps_[j].step];
-      bool ok = plan_steps_[j].step == plan_steps_[j - 1].step + 1 && own_launch(plan_steps_[j]) && k::umma_plan_stands_alone(plan_steps_[j].plan);
-      for (int w : st.writes) ok = ok && !V(w).external && !V(w).is_graph_output;
+      bool ok = plan_steps_[j].step == plan_steps_[j - 1].step + 1 && own_launch(plan_steps_[j]) && k::umma_plans_group(plan_steps_[i].plan, plan_steps_[j].plan);
       for (size_t m = i; m < j && ok; ++m) {
         const Step& ms = S.steps_[plan_steps_[m].step];
         ok = !overlap(st.writes, ms.reads) && !overlap(st.writes, ms.writes) && !overlap(st.reads, ms.writes);
       }
       if (!ok) break;
     }
-    if (j > i + 1)
-      for (size_t m = i; m < j; ++m) k::umma_plan_set_order(plan_steps_[m].plan, m == i, m > i);
+    std::vector<k::UmmaPlan*> members;
+    for (size_t m = i; m < j; ++m) members.push_back(plan_steps_[m].plan);
+    if (k::UmmaGroup* group = members.size() > 1 ? k::umma_group_create(members.data(), (int)members.size()) : nullptr) {
+      S.umma_groups_.push_back(group);
+      Step& first = S.steps_[plan_steps_[i].step];
+      int* err = S.err_flag_;
+      first.launch = [this, group, err](cudaStream_t s) {
+        k::umma_group_launch(group, err, s);
+        C.counters.umma_launches++;
+        C.counters.kernel_launches++;
+      };
+      for (size_t m = i + 1; m < j; ++m) {
+        Step& st = S.steps_[plan_steps_[m].step];
+        st.kernel.insert(st.kernel.find(" small") + 6, " (inside the launch of '" + first.node_name + "')");
+        st.launch = [](cudaStream_t) {};
+      }
+    }
     i = j;
   }
 }
@@ -703,7 +723,9 @@ void Planner::link_independent() {
 // A convolution that reads what node `ni`, a convolution too, reads and otherwise only initializers (the projection
 // shortcut of a residual block) is planned right behind it, so that the two run side by side (link_independent) and the
 // shortcut's sum joins the branch's last convolution instead.  For inputs of up to 16 MB, where a layer leaves part of
-// the chip idle; beyond, a layer fills it and the shortcut's output would only be kept for longer (one frame: INT8 326 -> 316 us, f32 436 -> 417 us).
+// the chip idle (one frame: INT8 294 -> 276 us, f32 437 -> 421 us; INT8 batch 4 411 -> 395 us); from about that size on the
+// two are launches of their own and nothing is gained (INT8 batch 16 and 37, f32 batch 4 and 16: within 0.3 % either
+// way), and the shortcut's output would only be kept for longer.
 void Planner::plan_siblings(int ni) {
   const NodeDef& n = nodes_[ni];
   if ((n.op != "Conv" && n.op != "QLinearConv") || C.cfg().keep_intermediates || n.inputs.empty()) return;

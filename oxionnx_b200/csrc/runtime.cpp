@@ -372,6 +372,7 @@ Session::~Session() {
   cudaSetDevice(ctx_->device());
   cudaStreamSynchronize(ctx_->stream());
   for (auto* p : umma_plans_) k::umma_plan_destroy(p);
+  for (auto* g : umma_groups_) k::umma_group_destroy(g);
   for (auto* c : umma_chains_) k::umma_chain_destroy(c);
   for (auto* a : umma_attentions_) k::umma_attention_destroy(a);
   for (auto& s : steps_) {

@@ -173,6 +173,7 @@ class Session {
   DeviceBuffer arena_;
   std::vector<DeviceBuffer> owned_;  // staging + parameter buffers
   std::vector<k::UmmaPlan*> umma_plans_;
+  std::vector<k::UmmaGroup*> umma_groups_;
   std::vector<k::UmmaChain*> umma_chains_;
   std::vector<k::UmmaAttentionPlan*> umma_attentions_;
   size_t n_slots_ = 0;

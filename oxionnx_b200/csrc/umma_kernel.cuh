@@ -70,10 +70,6 @@ struct alignas(64) KParams {
   CUtensorMap tmO;
   CUtensorMap tmR;  // the residual in the boxes of tmO (res_bufs > 0)
   uint64_t neg_zero2 = 0x8000000080000000ull;  // two negative zeros (see gelu_erf2)
-  // A run of launches that read nothing of one another (umma_plan_set_order): the first lets its dependents start only
-  // when its own predecessors are complete, the others start without waiting and wait before they end instead, so
-  // that the completion of the last is the completion of all.
-  int late_trigger, late_wait;
   int out_tma, out_row_bytes;
   int a_im2col;
   int M, OC;
@@ -1220,9 +1216,8 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
   const uint32_t tmem_base = tmem_base_slot;
   volatile int* abortp = &abort_flag;
   // let the next grid in the stream start its own prologue, then wait for the previous grid's results
-  if (!p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // The producer and the MMA issuer run their loops with the whole warp (every lane polls the
   // barrier, one lane issues): a lone lane looping while its 31 siblings sit at the teardown
@@ -1489,7 +1484,6 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
     if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(ES::TMEM_COLS) : "memory");
     else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(ES::TMEM_COLS) : "memory");
   }
-  if (p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---- launch -----------------------------------------------------------------------------------
@@ -1500,11 +1494,19 @@ constexpr int kMaxDevices = 64;
 void launch_kind_i8(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
 void launch_kind_tf32(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
 void launch_kind_f16(const KParams& kp, int bn, bool pair, int grid, size_t smem, int device, cudaStream_t s);
-// The small-problem kernel (umma_small.cuh): one tile, or one K slice of a tile, per CTA.
+// The small-problem kernel (umma_small.cuh): one tile, or one K slice of a tile, per CTA.  Up to GROUP_MAX problems of one
+// kind that depend on nothing of one another are one grid: member i has the CTAs from first[i] on, whole clusters of
+// `width` CTAs each.
 constexpr int SMALL_SMEM_MAX = 220 * 1024;
-void launch_small_i8(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
-void launch_small_tf32(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
-void launch_small_f16(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s);
+constexpr int GROUP_MAX = 3;
+struct SmallGroup {
+  KParams m[GROUP_MAX];
+  int first[GROUP_MAX];  // members that are not there begin past the grid
+  int width;
+};
+void launch_small_i8(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s);
+void launch_small_tf32(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s);
+void launch_small_f16(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s);
 // How many CTA pairs of the 256-wide kernel of this kind can be resident at once on `device`.
 int max_pairs_kind_i8(size_t smem, int device);
 int max_pairs_kind_tf32(size_t smem, int device);

@@ -132,7 +132,7 @@ __device__ __forceinline__ void small_finish(const KParams& p, const uint32_t (&
 
 template <int KIND, int VARIANT>
 __device__ __forceinline__ void small_epilogue(const KParams& p, int warp, int lane, uint32_t tmem_base, uint32_t bar_acc, uint32_t bar_recv, uint32_t recv,
-                                               volatile int* abortp, int slice, int m0, int oc0) {
+                                               volatile int* abortp, int slice, int rank0, int m0, int oc0) {
   const int quarter = warp & 3;
   const int runs = p.small_bn / 32, splits = p.splits;
   const long long m = (long long)m0 + quarter * 32 + lane;
@@ -152,7 +152,7 @@ __device__ __forceinline__ void small_epilogue(const KParams& p, int warp, int l
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
       // the predecessor may still read what this grid overwrites, and write what the lines below read
-      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       if (p.x_zp_dev) xz = __float2int_rn(*p.x_zp_dev);
       if (VARIANT >= V_DEQUANT) xs = *p.dq_x_scale;
       bool ok = mbar_spin(bar_acc, 0u, abortp);
@@ -176,7 +176,7 @@ __device__ __forceinline__ void small_epilogue(const KParams& p, int warp, int l
             for (int j = 0; j < 8; ++j)
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(place + (uint32_t)j * 512u), "r"(v[4 * j]), "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3]) : "memory");
           } else {
-            const uint32_t dst = mapa(place, (uint32_t)owner), bar = mapa(bar_recv, (uint32_t)owner);
+            const uint32_t dst = mapa(place, (uint32_t)(rank0 + owner)), bar = mapa(bar_recv, (uint32_t)(rank0 + owner));
 #pragma unroll
             for (int j = 0; j < 8; ++j) st_async_v4(dst + (uint32_t)j * 512u, bar, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           }
@@ -235,8 +235,10 @@ __device__ __forceinline__ void small_epilogue(const KParams& p, int warp, int l
   }
 }
 
+// CTA `cta` of a problem whose launch has clusters of `width` CTAs: a cluster holds width / splits tiles, the slices of a
+// tile side by side; the CTAs that the last cluster has too many do nothing.
 template <int KIND>
-__global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __grid_constant__ KParams p) {
+__device__ __forceinline__ void small_tile(const KParams& p, int cta, int width) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[SMALL_MAX_STAGES];
   __shared__ __align__(8) uint64_t bar_empty[SMALL_MAX_STAGES];
@@ -252,8 +254,12 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   const uint32_t stage_bytes = kpb * (a_bytes + b_bytes);
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t recv = ring + p.stage_off;
-  const int slice = splits > 1 ? (int)cluster_ctarank() : 0;
-  const int tile = (int)blockIdx.x / splits;
+  const int tile = cta / splits, slice = splits > 1 ? cta - tile * splits : 0;
+  const int rank0 = splits < width ? cta % width - slice : 0;  // the cluster rank of the tile's first slice
+  if (tile >= p.m_tiles * p.n_tiles) {
+    if (splits > 1) cluster_sync_all();
+    return;
+  }
   const int tile_m = tile / p.n_tiles, tile_n = tile - tile_m * p.n_tiles;
   const int m0 = tile_m * BLOCK_M, oc0 = tile_n * bn;
   const int it_begin = slice * p.k_per, it_end = min(p.taps * p.cblocks, it_begin + p.k_per);
@@ -287,7 +293,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   volatile int* abortp = &abort_flag;
-  if (!p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---------------- TMA producer: weights of the first ring, then the wait, then everything else ----------------
@@ -311,8 +317,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
         mbar_expect_tx(smem_u32(&bar_full[i]), expect(i));
         tma_load_3d(ring + (uint32_t)i * stage_bytes + kpb * a_bytes, &p.tmB, smem_u32(&bar_full[i]), 0, oc0, it_begin + i * p.kpb);
       }
-      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-      if (p.late_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       uint32_t stage = 0, phase = 0;
       for (int c = 0, it = it_begin; c < chunks; ++c, it += p.kpb) {
         const uint32_t full = smem_u32(&bar_full[stage]), dst = ring + stage * stage_bytes;
@@ -352,7 +357,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      if (!p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");  // the bounded waits below must not time the predecessor
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // the bounded waits below must not time the predecessor
       const uint64_t desc = make_smem_desc(0, swz);
       uint32_t stage = 0, phase = 0;
       for (int it = it_begin; it < it_end; it += p.kpb) {
@@ -388,7 +393,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   } else {
     // ---------------- epilogue ----------------
 #define OXB_SMALL(V)                                                                                                                                   \
-  case V: small_epilogue<KIND, V>(p, warp, lane, tmem_base, smem_u32(&bar_acc), smem_u32(&bar_recv), recv, abortp, slice, m0, oc0); break;
+  case V: small_epilogue<KIND, V>(p, warp, lane, tmem_base, smem_u32(&bar_acc), smem_u32(&bar_recv), recv, abortp, slice, rank0, m0, oc0); break;
     if constexpr (KIND == KIND_I8) {
       switch (p.variant) {
         OXB_SMALL(V_REQUANT)
@@ -451,7 +456,21 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __gr
   }
   __syncthreads();
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
-  if (p.late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Independent problems side by side (the Q, K and V products of an attention layer, a residual block's first convolution
+// and its shortcut): each leaves most of the chip idle, and one after the other each would wait for the one before.  In
+// one grid they share one griddepcontrol.wait, which orders every member behind everything before the grid.  A lone
+// problem is a group of one: a kernel of its own for groups would evict this one's instructions and find its own cold
+// (encoder of 2x77 tokens 1048 us with two kernels, 1016 us with one).  The cluster is the widest that a member's slices
+// need, also where the members together are more than are resident at once (INT8 frame: 303 us, against 308 us when such
+// members are launched one after the other).
+template <int KIND>
+__global__ void __launch_bounds__(SMALL_THREADS, 2) umma_small_kernel(const __grid_constant__ SmallGroup g) {
+  int i = 0;
+#pragma unroll
+  for (int j = 1; j < GROUP_MAX; ++j) i += (int)blockIdx.x >= g.first[j] ? 1 : 0;
+  small_tile<KIND>(g.m[i], (int)blockIdx.x - g.first[i], g.width);
 }
 
 // The opt-in for more than 48 KB of dynamic shared memory, per kernel and device (see ensure_smem_attr).  The split
@@ -469,7 +488,7 @@ void ensure_small_attr(int device) {
 }
 
 template <int KIND>
-void launch_small_kind(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s) {
+void launch_small_kind(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s) {
   ensure_small_attr<KIND>(device);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -480,11 +499,11 @@ void launch_small_kind(const KParams& kp, int grid, size_t smem, int device, cud
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)kp.splits;
+  attr[1].val.clusterDim.x = (unsigned)g.width;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = kp.splits > 1 ? 2 : 1;
-  OXB_CUDA(cudaLaunchKernelEx(&cfg, umma_small_kernel<KIND>, kp));
+  cfg.numAttrs = g.width > 1 ? 2 : 1;
+  OXB_CUDA(cudaLaunchKernelEx(&cfg, umma_small_kernel<KIND>, g));
 }
 
 }  // namespace umma

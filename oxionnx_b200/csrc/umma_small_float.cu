@@ -5,8 +5,8 @@ namespace oxb {
 namespace k {
 namespace umma {
 
-void launch_small_tf32(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_TF32>(kp, grid, smem, device, s); }
-void launch_small_f16(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_F16>(kp, grid, smem, device, s); }
+void launch_small_tf32(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_TF32>(g, grid, smem, device, s); }
+void launch_small_f16(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_F16>(g, grid, smem, device, s); }
 
 }  // namespace umma
 }  // namespace k

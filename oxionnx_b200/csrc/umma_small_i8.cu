@@ -5,7 +5,7 @@ namespace oxb {
 namespace k {
 namespace umma {
 
-void launch_small_i8(const KParams& kp, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_I8>(kp, grid, smem, device, s); }
+void launch_small_i8(const SmallGroup& g, int grid, size_t smem, int device, cudaStream_t s) { launch_small_kind<KIND_I8>(g, grid, smem, device, s); }
 
 }  // namespace umma
 }  // namespace k

@@ -185,6 +185,59 @@ def test_products_that_run_side_by_side(rows, k, widths, graph_replay):
     ref.close()
 
 
+# input channels, height, width, filters of the first convolution and of the shortcut: one slice each, unequal slices (four and
+# one, eight and four), a last cluster with CTAs too many, ragged tiles
+@pytest.mark.parametrize("c,h,w,oc1,oc2", [(64, 9, 7, 64, 256), (1024, 14, 14, 512, 2048), (1024, 14, 14, 512, 968), (2048, 5, 5, 40, 200)])
+@pytest.mark.parametrize("kind", ["int8", "tf32", "bf16"])
+def test_a_shortcut_beside_its_first_convolution(c, h, w, oc1, oc2, kind):
+    rng = np.random.default_rng([c, h, oc1, oc2])
+    conv, first, sc = {"strides": [2, 2]}, {"strides": [1, 1]}, {"strides": [2, 2]}
+    feeds = {"x": rng.standard_normal((1, c, h, w)).astype(np.float32)}
+    if kind == "int8":
+        weights = {"s": np.float32([0.02]), "z": np.float32([128]), "z0": np.float32([0]), "j": np.float32([0.04])}
+        nodes = [Node("QuantizeLinear", "q", ["x", "s", "z"], ["xq"], {})]
+        for name, x, oc, k, attrs in (("c1", "xq", oc1, c, first), ("c2", "c1q", oc2, oc1, conv), ("sc", "xq", oc2, c, sc)):
+            weights.update({name + "w": rng.integers(-127, 128, (oc, k, 1, 1)).astype(np.float32), name + "ws": rng.uniform(2e-4, 4e-4, oc).astype(np.float32),
+                            name + "b": rng.integers(-1000, 1001, oc).astype(np.float32)})
+            nodes.append(Node("QLinearConv", name, [x, "s", "z", name + "w", name + "ws", "z0", "s", "z", name + "b"], [name + "q"], attrs))
+        nodes += [Node("DequantizeLinear", "d1", ["c2q", "s", "z"], ["a"], {}), Node("DequantizeLinear", "d2", ["scq", "s", "z"], ["b"], {}),
+                  Node("Add", "add", ["a", "b"], ["sum"], {}), Node("Relu", "relu", ["sum"], ["r"], {}), Node("QuantizeLinear", "qj", ["r", "j", "z0"], ["yq"], {}),
+                  Node("DequantizeLinear", "dq", ["yq", "j", "z0"], ["y"], {})]
+        tuning, tol = {}, 0.0
+    else:
+        weights, nodes = {}, [Node("Relu", "pre", ["x"], ["x1"], {})]
+        for name, x, oc, k, attrs in (("c1", "x1", oc1, c, dict(first, activation="relu")), ("c2", "c1y", oc2, oc1, conv), ("sc", "x1", oc2, c, sc)):
+            weights.update({name + "w": (rng.standard_normal((oc, k, 1, 1)) / np.sqrt(k)).astype(np.float32), name + "b": rng.standard_normal(oc).astype(np.float32)})
+            nodes.append(Node("Conv", name, [x, name + "w", name + "b"], [name + "y"], attrs))
+        nodes += [Node("Add", "add", ["c2y", "scy"], ["sum"], {}), Node("Relu", "relu", ["sum"], ["y"], {})]
+        # two products after one another, 11 (TF32) or 8 (bf16) significant bits each
+        tuning, tol = {"float_precision": kind}, 4e-3 if kind == "tf32" else 4e-2
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    got, kernels = _run(graph, weights, feeds, **tuning)
+    beside = [s for s in kernels if "inside the launch of 'c1'" in s]
+    assert len(beside) == 1 and ("im2col" in beside[0]), kernels
+    want, _ = _run(graph, weights, feeds, kernel_path="direct")
+    assert np.all(np.abs(got["y"] - want["y"]) <= tol * np.abs(want["y"]).max())
+
+
+def test_side_by_side_products_are_one_launch():
+    rng = np.random.default_rng(5)
+    weights, nodes, outs = {}, [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {})], []
+    for i in range(5):  # more than one launch takes
+        weights[f"w{i}"] = rng.integers(-127, 128, (256, 96)).astype(np.float32)
+        nodes.append(Node("MatMulInteger", f"mm{i}", ["xq", f"w{i}", "xz"], [f"acc{i}"], {}))
+    for i in range(5):
+        nodes.append(Node("Relu", f"r{i}", [f"acc{i}"], [f"y{i}"], {}))
+        outs.append(f"y{i}")
+    sess = Session.builder().build_from_graph(Graph(nodes=nodes, input_names=["x"], output_names=outs), weights)
+    feeds = {"x": rng.standard_normal((33, 256)).astype(np.float32)}
+    sess.run(feeds)
+    before = sess.cuda_cache_counters()["umma_launches"]
+    sess.run(feeds)
+    assert sess.cuda_cache_counters()["umma_launches"] - before == 2
+    sess.close()
+
+
 @pytest.mark.parametrize("channels,h,w,scale", [(128, 5, 7, 2.0), (132, 9, 33, 1.5), (320, 1, 70, 3.0)])
 @pytest.mark.parametrize("coord", ["half_pixel", "align_corners", "asymmetric"])
 def test_linear_resize_of_many_channels_is_the_one_of_few(channels, h, w, scale, coord):
