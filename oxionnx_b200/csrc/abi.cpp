@@ -497,6 +497,11 @@ int oxb200_dispatch(oxb200_ctx* ctx, const oxb200_node* node, const oxb200_opera
         kept = C.keep_dispatch_plan(key, fresh);
       }
       Session& sess = kept ? *kept : *fresh;
+      struct InUse {
+        Context& c;
+        ~InUse() { c.plan_in_use = nullptr; }
+      } in_use{C};
+      C.plan_in_use = kept;
       sess.begin_copies();
       for (uint32_t i = 0; i < n_operands; ++i) {
         if (nd.inputs[i].empty()) continue;

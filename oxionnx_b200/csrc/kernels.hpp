@@ -3,6 +3,8 @@
 // synchronises.
 #pragma once
 
+#include <functional>
+
 #include "common.hpp"
 
 namespace oxb {
@@ -283,10 +285,13 @@ struct UmmaPlan;
 // Choices a context may override (oxb200_config): `requant_f64` 1 keeps the two-pass f64 requantisation even where
 // the one-FMA form is proven, 2 keeps the one-FMA form without the packed 16-bit saturation; `split_k_max` bounds the slices of a split reduction (0: the default of 8, 1: never
 // split); `cta_pairs` 0 lets the tile model decide, 1 never pairs CTAs, 2 pairs them wherever the shape allows.
+// `alloc` gives the device memory of workspaces, null when there is none (the plan then does without).
+typedef std::function<void*(size_t)> DeviceAlloc;
 struct UmmaTuning {
   int requant_f64 = 0;
   int split_k_max = 0;
   int cta_pairs = 0;
+  DeviceAlloc alloc;
 };
 UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt, void* out, const ConvShape& cs, const Epilogue& e, int kind,
                            const UmmaTuning& tune, std::string* why);
@@ -334,7 +339,7 @@ struct UmmaChainEnds {
   int tail_signed = 0;
 };
 struct UmmaChain;
-UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int rows, const UmmaChainEnds& ends, std::string* why);
+UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int rows, const UmmaChainEnds& ends, const DeviceAlloc& alloc, std::string* why);
 void umma_chain_destroy(UmmaChain* c);
 // After a launch that gave up: clears the arrival counters and the grid barrier's counter.
 void umma_chain_reset_after_error(UmmaChain* c);

@@ -515,7 +515,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     if (eff > 1) {
       const size_t ws_words = (size_t)m_tiles * n_tiles * eff * BLOCK_M * bn;
       const size_t cnt = (size_t)m_tiles * n_tiles * epi_warps(kind) * 4;
-      if (cudaMalloc(&pl->ws, ws_words * 4) == cudaSuccess && cudaMalloc(&pl->ws_count, cnt * sizeof(unsigned int)) == cudaSuccess &&
+      if ((pl->ws = tune.alloc(ws_words * 4)) && (pl->ws_count = tune.alloc(cnt * sizeof(unsigned int))) &&
           cudaMemset(pl->ws_count, 0, cnt * sizeof(unsigned int)) == cudaSuccess) {
         kp.splits = (int)eff;
         kp.k_per = (int)k_per;
@@ -853,7 +853,7 @@ bool chain_layout(UmmaChain* c, const UmmaChainLayer* layers, int n_layers, int 
 
 void umma_chain_destroy(UmmaChain* c);
 
-UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int rows, const UmmaChainEnds& ends, std::string* why) {
+UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int rows, const UmmaChainEnds& ends, const DeviceAlloc& alloc, std::string* why) {
   auto no = [&](const char* msg) -> UmmaChain* {
     if (why) *why = msg;
     return nullptr;
@@ -901,7 +901,7 @@ UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int row
     }
     if (cluster > 1) {
       // one empty launch with this geometry: cooperative and cluster attributes together
-      if (!probe_bar && (cudaMalloc(&probe_bar, 256) != cudaSuccess || cudaMemset(probe_bar, 0, 256) != cudaSuccess)) {
+      if (!probe_bar && (!(probe_bar = (uint64_t*)alloc(256)) || cudaMemset(probe_bar, 0, 256) != cudaSuccess)) {
         (void)cudaGetLastError();
         continue;
       }
@@ -933,7 +933,7 @@ UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int row
   }
   const size_t bar_off = off;
   off += 256;
-  if (cudaMalloc(&c->scratch, off) != cudaSuccess || cudaMemset(c->scratch, 0, off) != cudaSuccess) {
+  if (!(c->scratch = alloc(off)) || cudaMemset(c->scratch, 0, off) != cudaSuccess) {
     (void)cudaGetLastError();
     if (c->scratch) cudaFree(c->scratch);
     delete c;
@@ -947,7 +947,7 @@ UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int row
     cuuint32_t estr[2] = {1, 1};
     const size_t w_rows = (size_t)P.n_tiles * (L.K / 128) * 128;  // rows of 128 bytes
     CUresult rc = CUDA_ERROR_OUT_OF_MEMORY;
-    if (cudaMalloc(&c->w_tiles[l], w_rows * 128) == cudaSuccess) {
+    if ((c->w_tiles[l] = alloc(w_rows * 128))) {
       chain_repack(L.w, c->w_tiles[l], L.N, L.K, nullptr);
       if (cudaStreamSynchronize(nullptr) == cudaSuccess) {
         cuuint64_t wdim[2] = {128, (cuuint64_t)w_rows}, wstr[1] = {128};

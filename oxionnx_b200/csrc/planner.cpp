@@ -800,7 +800,7 @@ void Planner::link_chains() {
         }
       }
       std::string why;
-      k::UmmaChain* chain = k::umma_chain_create(layers.data(), (int)layers.size(), chain_links_[i].rows, ends, &why);
+      k::UmmaChain* chain = k::umma_chain_create(layers.data(), (int)layers.size(), chain_links_[i].rows, ends, [this](size_t bytes) { return C.try_alloc_device(bytes); }, &why);
       if (chain) {
         S.umma_chains_.push_back(chain);
         Step& first = S.steps_[chain_links_[i].step];
@@ -922,7 +922,7 @@ void Planner::finalize_lifetimes_and_arena() {
   S.n_slots_ = slots.size();
   S.arena_.bytes = total;
   if (total > 0) {
-    OXB_CUDA(cudaMalloc(&S.arena_.ptr, total));
+    S.arena_.ptr = C.alloc_device(total);
   }
   for (int i : order) V(i).ptr = (uint8_t*)S.arena_.ptr + offs[V(i).slot];
   for (int i = 0; i < (int)S.values_.size(); ++i)
@@ -1373,6 +1373,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       tune.requant_f64 = C.cfg().requant_f64;
       tune.split_k_max = C.cfg().split_k_max;
       tune.cta_pairs = C.cfg().cta_pairs;
+      tune.alloc = [this](size_t bytes) { return C.try_alloc_device(bytes); };
       k::UmmaPlan* plan = k::umma_plan_create(V(x_vi).ptr, xdt, wdev, wdt, V(out_vi).ptr, cs, e, kind, tune, &why2);
       if (!plan) OXB_FAIL("%s '%s': tensor-core plan rejected after selection: %s", n.op.c_str(), n.name.c_str(), why2.c_str());
       S.umma_plans_.push_back(plan);

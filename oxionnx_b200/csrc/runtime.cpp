@@ -79,10 +79,30 @@ const HostTensor* Context::weight(const std::string& name) const {
 
 bool Context::weight_resident(const std::string& name) const { return resident_names_.count(name) != 0; }
 
-void* Context::alloc_device(size_t bytes) {
+// Memory that this context only holds for reuse is given back before an allocation fails: first the free blocks, then the
+// kept plans but the one in use.
+void* Context::try_alloc_device(size_t bytes, cudaError_t* error) {
   void* p = nullptr;
-  if (bytes == 0) bytes = 256;
-  OXB_CUDA(cudaMalloc(&p, align_up(bytes, 256)));
+  bytes = align_up(std::max<size_t>(bytes, 256), 256);
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && drop_free_blocks()) {
+    (void)cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && drop_dispatch_plans()) {
+    (void)cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+  }
+  if (error) *error = e;
+  if (e == cudaSuccess) return p;
+  (void)cudaGetLastError();
+  return nullptr;
+}
+
+void* Context::alloc_device(size_t bytes) {
+  cudaError_t e = cudaSuccess;
+  void* p = try_alloc_device(bytes, &e);
+  OXB_CUDA(e);
   return p;
 }
 
@@ -157,7 +177,12 @@ Session* Context::keep_dispatch_plan(const std::string& key, std::unique_ptr<Ses
   return dispatch_plans_.back().plan.get();
 }
 
-void Context::drop_dispatch_plans() { dispatch_plans_.clear(); }
+bool Context::drop_dispatch_plans() {
+  const size_t before = dispatch_plans_.size();
+  dispatch_plans_.erase(std::remove_if(dispatch_plans_.begin(), dispatch_plans_.end(), [&](const DispatchEntry& e) { return e.plan.get() != plan_in_use; }),
+                        dispatch_plans_.end());
+  return dispatch_plans_.size() != before;
+}
 
 constexpr size_t kFreeBlocks = 64, kFreeBlockBytes = 256ull << 20;
 
@@ -186,11 +211,17 @@ void Context::give_block(void* ptr, size_t bytes) {
   free_block_bytes_ += bytes;
 }
 
-void Context::release_caches() {
-  drop_dispatch_plans();
+bool Context::drop_free_blocks() {
+  if (free_blocks_.empty()) return false;
   for (const Block& b : free_blocks_) cudaFree(b.ptr);
   free_blocks_.clear();
   free_block_bytes_ = 0;
+  return true;
+}
+
+void Context::release_caches() {
+  drop_dispatch_plans();
+  drop_free_blocks();
   for (auto& kv : forms_) cudaFree(kv.second.ptr);
   forms_.clear();
   for (void* p : temp_forms_) cudaFree(p);
@@ -712,16 +743,14 @@ void Session::prepare_pipeline() {
     OXB_CUDA(cudaEventCreateWithFlags(&fl.down, cudaEventDisableTiming));
     for (auto& in : input_staging_) {
       void* p = values_[in.second].ptr;
-      if (f == 1 && pipe_double_) OXB_CUDA(cudaMalloc(&p, std::max<size_t>((size_t)values_[in.second].numel() * dt_size(values_[in.second].dt), 256)));
+      if (f == 1 && pipe_double_) p = ctx_->alloc_device((size_t)values_[in.second].numel() * dt_size(values_[in.second].dt));
       fl.in_dev.push_back(p);
     }
     for (auto& out : output_staging_) {
       float* p = nullptr;
       OXB_CUDA(cudaMallocHost(&p, std::max<size_t>((size_t)values_[out.second].numel() * 4, 4)));
       fl.out_host.push_back(p);
-      void* d = nullptr;
-      OXB_CUDA(cudaMalloc(&d, std::max<size_t>((size_t)values_[out.second].numel() * 4, 256)));
-      fl.out_dev.push_back(d);
+      fl.out_dev.push_back(ctx_->alloc_device((size_t)values_[out.second].numel() * 4));
     }
   }
   pipe_ready_ = true;

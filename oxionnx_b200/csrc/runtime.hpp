@@ -266,6 +266,7 @@ class Context {
   void* resident_form(const std::string& name, const std::string& form, size_t bytes, const std::function<void(void*)>& fill_host,
                       bool cacheable);
   void* alloc_device(size_t bytes);
+  void* try_alloc_device(size_t bytes, cudaError_t* error = nullptr);  // null when there is no memory
   void free_device(void* p);
   void release_caches();
   void free_temp_forms();
@@ -274,14 +275,18 @@ class Context {
   int* take_error_word();
   void give_error_word(int* word);
   // Plans of single-node dispatches, by everything the plan depends on; at most 16 plans and 256 MB of device memory,
-  // the least recently used goes first.  Registering a weight or releasing the caches drops them all.
+  // the least recently used goes first.  Registering a weight or releasing the caches drops them all; an allocation
+  // that finds no memory drops all but `plan_in_use`.
   Session* find_dispatch_plan(const std::string& key);
   Session* keep_dispatch_plan(const std::string& key, std::unique_ptr<Session>& plan);  // null (and `plan` kept) when it is too large
-  void drop_dispatch_plans();
+  bool drop_dispatch_plans();  // did any go?
+  const Session* plan_in_use = nullptr;  // the kept plan that the dispatch under way runs
   // Storage of device tensors: released blocks wait for the next tensor of about their size (at most 64 blocks and
-  // 256 MB).  Everything rides this context's stream, so reuse needs no fence.
+  // 256 MB).  Everything rides this context's stream, so reuse needs no fence.  An allocation that finds no memory
+  // gives them all back.
   void* take_block(size_t bytes, size_t* got);
   void give_block(void* ptr, size_t bytes);
+  bool drop_free_blocks();  // were there any?
 
   // Large pageable host buffers: copied in pieces through page-locked buffers by a few host threads, so that the
   // host copy of one piece runs beside the PCIe transfer of another (host_to_device only enqueues the last
