@@ -2392,6 +2392,7 @@ void dynamic_quantize_linear(const TensorRef& x, const TensorRef& y, float* para
 void dynamic_quantize_scratch_init(float* scratch) {
   const uint32_t init[3] = {0xffffffffu, 0u, 0u};
   OXB_CUDA(cudaMemcpy(scratch, init, sizeof init, cudaMemcpyHostToDevice));
+  OXB_CUDA(cudaStreamSynchronize(nullptr));  // a copy of so few bytes may return before they have landed
 }
 
 void binary(const TensorRef& a, const TensorRef& b, const TensorRef& out, int op, int relu_after, int round_tf32_flag, cudaStream_t s) {

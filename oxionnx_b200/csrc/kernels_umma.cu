@@ -113,6 +113,10 @@ uint32_t make_idesc(int kind, bool a_signed, bool b_signed, int bn, int m) {
   return d;
 }
 
+// Zeroes device memory before anything that is enqueued after this call, on whatever stream: a memset returns before it has
+// run, and the contexts' streams do not wait for the default stream.
+bool zero_now(void* p, size_t bytes) { return cudaMemset(p, 0, bytes) == cudaSuccess && cudaStreamSynchronize(nullptr) == cudaSuccess; }
+
 // Shared memory of one CTA: 227 KB less the kernel's static part (barriers) and alignment slack.
 constexpr size_t kSmemBudget = 227 * 1024 - 2048;
 
@@ -516,7 +520,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
       const size_t ws_words = (size_t)m_tiles * n_tiles * eff * BLOCK_M * bn;
       const size_t cnt = (size_t)m_tiles * n_tiles * epi_warps(kind) * 4;
       if ((pl->ws = tune.alloc(ws_words * 4)) && (pl->ws_count = tune.alloc(cnt * sizeof(unsigned int))) &&
-          cudaMemset(pl->ws_count, 0, cnt * sizeof(unsigned int)) == cudaSuccess) {
+          zero_now(pl->ws_count, cnt * sizeof(unsigned int))) {
         kp.splits = (int)eff;
         kp.k_per = (int)k_per;
         kp.ws = (uint32_t*)pl->ws;
@@ -740,7 +744,7 @@ void umma_plan_destroy(UmmaPlan* p) {
 void umma_plan_reset_after_error(UmmaPlan* p) {
   if (!p || !p->ws_count) return;
   const size_t cnt = (size_t)p->kp.m_tiles * p->kp.n_tiles * epi_warps(p->kind) * 4;
-  (void)cudaMemset(p->ws_count, 0, cnt * sizeof(unsigned int));
+  (void)zero_now(p->ws_count, cnt * sizeof(unsigned int));
 }
 const char* umma_plan_desc(const UmmaPlan* p) { return p->desc; }
 
@@ -901,7 +905,7 @@ UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int row
     }
     if (cluster > 1) {
       // one empty launch with this geometry: cooperative and cluster attributes together
-      if (!probe_bar && (!(probe_bar = (uint64_t*)alloc(256)) || cudaMemset(probe_bar, 0, 256) != cudaSuccess)) {
+      if (!probe_bar && (!(probe_bar = (uint64_t*)alloc(256)) || !zero_now(probe_bar, 256))) {
         (void)cudaGetLastError();
         continue;
       }
@@ -933,7 +937,7 @@ UmmaChain* umma_chain_create(const UmmaChainLayer* layers, int n_layers, int row
   }
   const size_t bar_off = off;
   off += 256;
-  if (!(c->scratch = alloc(off)) || cudaMemset(c->scratch, 0, off) != cudaSuccess) {
+  if (!(c->scratch = alloc(off)) || !zero_now(c->scratch, off)) {
     (void)cudaGetLastError();
     if (c->scratch) cudaFree(c->scratch);
     delete c;
@@ -995,7 +999,7 @@ void umma_chain_destroy(UmmaChain* c) {
   delete c;
 }
 void umma_chain_reset_after_error(UmmaChain* c) {
-  if (c && c->scratch) (void)cudaMemset(c->scratch, 0, c->scratch_bytes);
+  if (c && c->scratch) (void)zero_now(c->scratch, c->scratch_bytes);
 }
 const char* umma_chain_desc(const UmmaChain* c) { return c->desc; }
 bool umma_chain_launch(const UmmaChain* c, int* err_flag, const float* head_x, cudaStream_t s) {

@@ -122,3 +122,37 @@ def test_u8_declared_input_is_fed_as_bytes_and_gives_the_same_lanes():
     assert all(np.array_equal(o["logits"], want) for o in outs)
     s8.close()
     s32.close()
+
+
+@pytest.mark.parametrize("kind", ["split_k", "dynamic_quantize", "chain"])
+def test_a_plan_made_while_the_default_stream_is_busy(kind):
+    """Counters and keys that a plan's kernels start from are set before its first run, whatever else the default stream
+    has queued up."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(7)
+    if kind == "split_k":  # more K blocks than the small-problem kernel takes: the slices meet through counters
+        weights = {"w": (rng.standard_normal((256, 256, 3, 3)) / 48).astype(np.float32), "b": np.zeros(256, np.float32)}
+        graph = Graph(nodes=[Node("Conv", "c", ["x", "w", "b"], ["y"], {"pads": [1] * 4})], input_names=["x"], output_names=["y"])
+        feeds = {"x": rng.standard_normal((32, 256, 14, 14)).astype(np.float32)}
+    elif kind == "dynamic_quantize":
+        weights = {"w": rng.integers(-127, 128, (256, 64)).astype(np.float32)}
+        graph = Graph(nodes=[Node("DynamicQuantizeLinear", "q", ["x"], ["xq", "xs", "xz"], {}), Node("MatMulInteger", "m", ["xq", "w", "xz"], ["y"], {})],
+                      input_names=["x"], output_names=["y"])
+        feeds = {"x": rng.standard_normal((16, 256)).astype(np.float32)}
+    else:
+        graph, weights, make, _ = models.build_int8_mlp(rows=16, dims=(256, 512, 256))
+        feeds = make()
+
+    def first_run(busy):
+        if busy:
+            torch.cuda._sleep(200_000_000)  # 0.1 s
+        session = Session.builder().with_input_shapes({"x": feeds["x"].shape}).build_from_graph(graph, weights)
+        out = session.run(feeds)["y"]
+        kernels = [s["kernel"] for s in session.steps()]
+        session.close()
+        return out, kernels
+
+    want, kernels = first_run(False)
+    assert any({"split_k": "splitK", "dynamic_quantize": "dynamic_quantize", "chain": "chain"}[kind] in k and "small" not in k for k in kernels), kernels
+    got, _ = first_run(True)
+    assert np.array_equal(got, want)
