@@ -176,7 +176,9 @@ int oxb200_device_count(void);
  * context are serialised by the context's own lock. */
 int oxb200_ctx_create(int device_ordinal, const oxb200_config* cfg, oxb200_ctx** out);
 void oxb200_ctx_destroy(oxb200_ctx* ctx);
-const char* oxb200_last_error(const oxb200_ctx* ctx); /* ctx may be NULL: last error of the calling thread */
+/* The message of the last failed or declined call on ctx, whatever its thread; with ctx NULL, of the calling thread's last.
+ * Valid until the calling thread's next oxb200_last_error. */
+const char* oxb200_last_error(const oxb200_ctx* ctx);
 /* CudaContext::cache_counters (src/context.rs:394-430) */
 void oxb200_get_counters(const oxb200_ctx* ctx, oxb200_counters* out);
 /* CudaContext::release_device_caches */

@@ -29,11 +29,7 @@ const char kVerifyPrefix[] = "CUDA VERIFY MISMATCH: ";
 
 int fail_with(oxb200_ctx* ctx, int code, const std::string& msg) {
   g_thread_error = msg;
-  if (ctx) {
-    ctx->impl.last_error = msg;
-    if (code == OXB200_DECLINED) ctx->impl.counters.declines++;
-    else ctx->impl.counters.failures++;
-  }
+  if (ctx) ctx->impl.set_last_error(code, msg);
   return code;
 }
 
@@ -222,7 +218,12 @@ int oxb200_ctx_create(int device_ordinal, const oxb200_config* cfg, oxb200_ctx**
 
 void oxb200_ctx_destroy(oxb200_ctx* ctx) { delete ctx; }
 
-const char* oxb200_last_error(const oxb200_ctx* ctx) { return ctx ? ctx->impl.last_error.c_str() : g_thread_error.c_str(); }
+const char* oxb200_last_error(const oxb200_ctx* ctx) {
+  if (!ctx) return g_thread_error.c_str();
+  static thread_local std::string copy;  // another thread may fail, and replace the message, while the caller reads
+  copy = ctx->impl.last_error();
+  return copy.c_str();
+}
 
 void oxb200_get_counters(const oxb200_ctx* ctx, oxb200_counters* out) {
   if (ctx && out) *out = ctx->impl.counters;

@@ -218,9 +218,7 @@ int oxb200_model_initializer(oxb200_model* m, uint32_t index, oxb200_operand* ou
 int oxb200_session_plan_model(oxb200_ctx* ctx, oxb200_model* m, const oxb200_value_info* shapes, uint32_t n_shapes) {
   if (!ctx || !m) return model_fail(OXB200_FAILED, "session_plan_model: NULL argument");
   auto fail_ctx = [&](int code, const std::string& msg) {
-    ctx->impl.last_error = msg;
-    if (code == OXB200_DECLINED) ctx->impl.counters.declines++;
-    else ctx->impl.counters.failures++;
+    ctx->impl.set_last_error(code, msg);
     return model_fail(code, msg);
   };
   try {

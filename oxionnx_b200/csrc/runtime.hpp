@@ -295,13 +295,25 @@ class Context {
   void device_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
   oxb200_counters counters{};
-  std::string last_error;
+  // The message of the last failed or declined call, from whichever thread; calls report it after they have let go of `mu`.
+  void set_last_error(int code, const std::string& message) {
+    std::lock_guard<std::mutex> lock(error_mu_);
+    last_error_ = message;
+    if (code == OXB200_DECLINED) counters.declines++;
+    else counters.failures++;
+  }
+  std::string last_error() const {
+    std::lock_guard<std::mutex> lock(error_mu_);
+    return last_error_;
+  }
   std::unique_ptr<Session> session;  // the planned session of oxb200_session_plan
   cudaEvent_t run_ev0 = nullptr, run_ev1 = nullptr;
   bool last_run_timed = false;  // run_ev0 / run_ev1 bracket a finished run
   std::mutex mu;
 
  private:
+  mutable std::mutex error_mu_;
+  std::string last_error_;
   int device_;
   oxb200_config cfg_;
   cudaStream_t stream_ = nullptr;

@@ -82,3 +82,28 @@ def test_threads_share_a_planned_session():
     for got, w in zip(_in_threads([lambda b=b: many(b) for b in batches]), want):
         assert all(np.array_equal(g, w) for g in got)
     session.close()
+
+
+@pytest.mark.gpu
+def test_messages_of_failing_threads_are_whole():
+    """Threads that share a context and are refused all the time: every message read is one that some call left."""
+    ctx = S.CudaContext(0)
+    lib = _ffi.lib()
+    expected = {f"attribute '{c * 60}' has a kind this provider does not handle" for c in "abcd"}
+
+    def refused(letter):
+        attr = (_ffi.Attr * 1)()
+        attr[0].name, attr[0].kind = (letter * 60).encode(), 99
+        node, keep = _ffi.CNode(), _ffi.Keep()
+        node.op_type, node.attrs, node.n_attrs = b"Relu", attr, 1
+        results = (_ffi.Result * 1)()
+        seen = set()
+        for _ in range(2000):
+            assert lib.oxb200_dispatch(ctx.handle, ctypes.byref(node), None, 0, 0, results, 0) == _ffi.DECLINED
+            seen.add(ctx.last_error())
+        return seen
+
+    for seen in _in_threads([lambda c=c: refused(c) for c in "abcd"]):
+        assert seen <= expected
+    assert ctx.cache_counters()["declines"] == 8000
+    ctx.close()
