@@ -689,9 +689,11 @@ __device__ __forceinline__ uint64_t both(float x) { return pack2(x, x); }
 // Exact Gelu of two lanes, y * 0.5 * (1 + erf(y / sqrt 2)), with the reference's polynomial for erf (Abramowitz-Stegun
 // 7.1.26, nn_ops/activations.rs:578) in its operation order, so that the lanes are those of the separate node bit for
 // bit.  1 / d is one Newton step with fused residual (Markstein) on the approximate reciprocal: for 1 <= d <= 2^100 it is
-// the correctly rounded quotient for every float; beyond, the capped d gives a t that the underflown exponential
-// multiplies away.  The epilogue is bound by instruction issue: two lanes an instruction and no range branch took
-// M=8192 N=3072 K=768 from 92.4 us to 70.2 us (M=154: 24.8 -> 18.8 us).
+// the correctly rounded quotient whatever approximation the documented unit in the last place allows, but for significands
+// of all ones, of which no x gives the one that would matter (tests/host_checks/newton_reciprocal_check.c tries them all).
+// Beyond 2^100 the capped d gives a t that the underflown exponential multiplies away.  The epilogue is bound by
+// instruction issue: two lanes an instruction and no range branch took M=8192 N=3072 K=768 from 92.4 us to 70.2 us
+// (M=154: 24.8 -> 18.8 us).
 __device__ __forceinline__ uint64_t gelu_erf2(uint64_t y, uint64_t neg_zero) {
   auto mulp = [neg_zero](uint64_t a, uint64_t b) { return fmap(a, b, neg_zero); };
   const uint64_t g = mulp(y, both(0.70710678118654752440f));

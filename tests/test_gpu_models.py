@@ -154,6 +154,45 @@ def test_contraction_hands_its_extrema_to_the_next_dynamic_quantize_linear(rows,
     assert np.max(np.abs(got["yq"].astype(np.int32) - ref["yq"].astype(np.int32))) <= 1  # the oracle's Gelu may differ in the last place
 
 
+def _gelu_arguments(n):
+    """n values for the exact Gelu: those around the end of a binade of its polynomial's denominator (1 + 0.3275911 |y| / sqrt 2
+    = 2), the ends of the range, and a dense rest."""
+    f = np.float32
+    special = np.arange(f(4.3165).view(np.int32), f(4.3175).view(np.int32), dtype=np.int32).view(f)
+    d = f(1) + special * f(0.70710678118654752440) * f(0.3275911)
+    assert d[0] < 2 < d[-1]
+    ends = np.float32([0.0, 1e-45, 1e-38, 1e-20, 1e-7, 14.3, 14.5, 18.0, 40.0, 1e10, 1e30, 3.4e38])
+    rest = np.random.default_rng(8).uniform(0, 15, n // 2 - special.size - ends.size).astype(f)
+    half = np.concatenate([special, ends, rest])
+    return np.concatenate([half, -half])
+
+
+@pytest.mark.parametrize("pairs", ["auto", "always"])  # the small-problem kernel, the persistent one
+def test_gelu_in_the_epilogue_is_the_separate_node_at_its_hardest_arguments(pairs):
+    """The bias carries the argument (every weight is zero), so each is met exactly."""
+    from oxionnx_b200.graph import Graph, Node
+    n, k = 30000, 64
+    y = _gelu_arguments(n)
+    w = {"w": np.zeros((k, n), np.float32), "ws": np.full(n, 0.01, np.float32), "bias": y}
+    nodes = [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {}), Node("MatMulInteger", "mmi", ["xq", "w", "xz"], ["acc"], {}),
+             Node("Cast", "cast", ["acc"], ["accf"], {"to": 1}), Node("Mul", "scales", ["xs", "ws"], ["sc"], {}),
+             Node("Mul", "rescale", ["accf", "sc"], ["scaled"], {}), Node("Add", "addb", ["scaled", "bias"], ["lin"], {}),
+             Node("Gelu", "act", ["lin"], ["y"], {}), Node("Relu", "keep", ["y"], ["r"], {}), Node("Sub", "neg", ["y", "r"], ["m"], {})]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["r", "m"])
+    feeds = {"x": np.random.default_rng(9).standard_normal((2, k)).astype(np.float32)}
+    fused = Session.builder().with_tuning(cta_pairs=pairs).build_from_graph(graph, w)
+    got = fused.run(feeds)
+    kernels = [s["kernel"] for s in fused.steps()]
+    assert any(s.startswith("umma_i8") and "+dequant" in s and ("small" in s) == (pairs == "auto") for s in kernels), kernels
+    fused.close()
+    apart = Session.builder().with_keep_intermediates(True).build_from_graph(graph, w)
+    want = apart.run(feeds)
+    assert np.array_equal(apart.fetch_value("lin")[1], y)
+    apart.close()
+    for name in ("r", "m"):
+        assert np.array_equal(got[name], want[name])
+
+
 @pytest.mark.parametrize("shape", [(5, 37, 768), (64, 96), (3, 130, 1024)])
 def test_layer_norm_absorbs_the_residual_add_in_front_of_it(shape):
     """Add -> LayerNormalization with the sum read by nothing else is one kernel (the sum is never written); the
