@@ -623,8 +623,9 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     pl->grid = (int)std::min<int64_t>(m_tiles * n_tiles * kp.splits, sms);
   }
   const char* kname = kind == KIND_I8 ? "i8" : (kind == KIND_TF32 ? "tf32" : (kind == KIND_F16 ? "f16" : "bf16"));
-  char split_note[24] = "";
+  char split_note[40] = "";
   if (kp.splits > 1) snprintf(split_note, sizeof split_note, " splitK=%d", kp.splits);
+  else if (kp.res_bufs > 0) snprintf(split_note, sizeof split_note, " residual-buffers=%d", kp.res_bufs);
   snprintf(pl->desc, sizeof pl->desc, "umma_%s M=%lld N=%d K=%lld tile=%dx%dx%dB stages=%dx%d %s%s%s", kname, (long long)M, cs.OC, (long long)cs.K(),
            pair ? 256 : a_rows, bn, swz, kp.stages, kp.kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? " cta-pair" : (pl->small ? " small" : ""));
   if (pl->small) pl->alone = umma_group_create(&pl, 1);

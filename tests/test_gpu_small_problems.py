@@ -220,6 +220,52 @@ def test_a_shortcut_beside_its_first_convolution(c, h, w, oc1, oc2, kind):
     assert np.all(np.abs(got["y"] - want["y"]) <= tol * np.abs(want["y"]).max())
 
 
+# storage of the convolution's lanes, of the residual and of the sum: zero points of every sign, with and without Relu
+JOINS = {"unsigned relu": (("u8", 128, 0.07622), ("u8", 0, 0.04274), ("u8", 0, 0.05397), True),
+         "signed residual": (("u8", 131, 0.05076), ("i8", -3, 0.05087), ("u8", 130, 0.07024), False),
+         "signed": (("i8", -7, 0.07615), ("i8", 5, 0.08084), ("i8", -9, 0.06283), False),
+         "signed sum relu": (("i8", 11, 0.04367), ("u8", 140, 0.0632), ("i8", -20, 0.04647), True),
+         "narrow": (("u8", 3, 0.02), ("i8", 0, 0.9), ("i8", 100, 0.7), False)}  # many sums saturate
+# batch, channels, height, width, filters, kernel, CTA pairs, what the kernel has to say: every kernel and staging depth that takes a join,
+# ragged rows and channel tiles
+JOIN_SHAPES = [(1, 64, 9, 7, 96, 1, "auto", "small"), (1, 512, 7, 7, 160, 1, "auto", "small"), (1, 128, 13, 11, 64, 3, "auto", "small"),
+               (1, 64, 61, 43, 288, 1, "always", "cta-pair"), (1, 512, 61, 43, 544, 1, "always", "cta-pair"), (2, 64, 30, 31, 256, 3, "always", "cta-pair"),
+               (1, 64, 139, 137, 256, 1, "never", "residual-buffers=4"), (1, 512, 137, 137, 384, 1, "never", "residual-buffers=3"),
+               (1, 1024, 137, 137, 256, 1, "never", "residual-buffers=2"), (2, 64, 139, 137, 32, 3, "never", "residual-buffers")]
+
+
+@pytest.mark.parametrize("shape", JOIN_SHAPES, ids=str)
+@pytest.mark.parametrize("join", JOINS)
+def test_quantised_joins_in_the_epilogue_are_the_separate_nodes(shape, join):
+    n, c, h, w, oc, k, pairs, says = shape
+    (a_st, a_z, a_s), (b_st, b_z, b_s), (y_st, y_z, y_s), relu = JOINS[join]
+    rng = np.random.default_rng([n, c, h, oc, k])
+    kinds = {"u8": np.uint8, "i8": np.int8}
+    peak = min(127, (1 << 24) // (300 * c * k * k))  # accumulators that convert exactly
+    weights = {"w": rng.integers(-peak, peak + 1, (oc, c, k, k)).astype(np.float32), "wz": np.int8([0]), "xs": np.float32([0.02]), "xz": np.uint8([121 if k == 1 else 0]),
+               "bias": rng.integers(-1000, 1001, oc).astype(np.float32), "one": np.float32([1]), "rz": kinds[b_st]([128 if b_st == "u8" else 0]),
+               "as": np.float32([a_s]), "az": kinds[a_st]([a_z]), "bs": np.float32([b_s]), "bz": kinds[b_st]([b_z]), "ys": np.float32([y_s]), "yz": kinds[y_st]([y_z])}
+    # a standard deviation of about sixty lanes in front of the first saturation
+    spread = 60 / (50 * peak / np.sqrt(3) * np.sqrt(c * k * k))
+    weights["ws"] = (rng.uniform(0.7, 1.4, oc) * spread * a_s / 0.02).astype(np.float32)
+    nodes = [Node("QuantizeLinear", "qx", ["x", "xs", "xz"], ["xq"], {}), Node("QuantizeLinear", "qr", ["r", "one", "rz"], ["rq"], {}),
+             Node("QLinearConv", "conv", ["xq", "xs", "xz", "w", "ws", "wz", "as", "az", "bias"], ["aq"], {"pads": [k // 2] * 4}),
+             Node("DequantizeLinear", "da", ["aq", "as", "az"], ["a"], {}), Node("DequantizeLinear", "db", ["rq", "bs", "bz"], ["b"], {}),
+             Node("Add", "add", ["a", "b"], ["sum"], {})]
+    if relu:
+        nodes.append(Node("Relu", "relu", ["sum"], ["s"], {}))
+    nodes += [Node("QuantizeLinear", "qy", ["s" if relu else "sum", "ys", "yz"], ["yq"], {}), Node("DequantizeLinear", "dy", ["yq", "ys", "yz"], ["y"], {})]
+    graph = Graph(nodes=nodes, input_names=["x", "r"], output_names=["y"])
+    feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32),
+             "r": (rng.integers(0, 256, (n, oc, h, w)) - 128).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds, cta_pairs=pairs)
+    assert any(s.endswith("+join") and says in s for s in kernels), kernels
+    want, apart = _run(graph, weights, feeds, cta_pairs=pairs, keep_intermediates=True)
+    assert not any("+join" in s for s in apart)
+    assert np.array_equal(got["y"], want["y"])
+    assert np.unique(want["y"]).size > 20  # not only the ends of the range
+
+
 def test_side_by_side_products_are_one_launch():
     rng = np.random.default_rng(5)
     weights, nodes, outs = {}, [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {})], []
