@@ -754,8 +754,11 @@ void Planner::link_chains() {
     while (j < chain_links_.size() && j - i < 4 && chain_links_[j].step == chain_links_[j - 1].step + 1 && chain_links_[j].rows == chain_links_[i].rows &&
            chain_links_[j].layer.x == chain_links_[j - 1].layer.out && chain_links_[j].layer.K == chain_links_[j - 1].layer.N)
       ++j;
-    // Weights above 4 MB stream faster through the layers' own kernels, which overlap their prologues (1024-4096-4096-1024:
-    // 41 us a pass against 47 with 64 rows, 57 against 66 with one); a few small layers cost less as one launch.
+    // Weights above 4 MB stream faster through the layers' own kernels, which overlap their prologues.  So do fewer, as the
+    // small-problem kernel stands: a call with device-bound ends and 64 rows takes, as a chain against layer by layer,
+    // 256-512-512-128 37.1 / 25.8 us, 512-2048-512 30.7 / 24.0, 1024-1024-1024-1024 37.8 / 31.1, 1024-2048-1024 31.0 /
+    // 25.6, 2048-2048-1024 31.6 / 28.7, 1024-4096-4096-1024 42.0 / 37.7, and one row the same 4 to 10 us more.  The line
+    // is where it was drawn before that kernel; no chain at all would be the faster rule.
     size_t weight_bytes = 0;
     for (size_t t = i; t < j; ++t) weight_bytes += (size_t)chain_links_[t].layer.K * chain_links_[t].layer.N;
     if (j - i >= 2 && weight_bytes <= (4u << 20)) {

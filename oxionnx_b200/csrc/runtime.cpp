@@ -931,9 +931,12 @@ void Session::clear_bindings() {
 }
 
 // Between a bound buffer and the session's own: up to 1 MB by a kernel that takes part in the dependent launches, above it
-// at the rate of the driver's copy (64 rows through a 1024-wide MLP: 41.2 -> 39.2 us a call).
+// at the rate of the driver's copy.  A call that binds an output of 64 KB / 256 KB / 512 KB / 1 MB, kernel against driver:
+// 28.7 / 29.4 / 22.9 / 23.9 against 30.8 / 32.5 / 25.6 / 26.2 us.  To an address that is not 16-byte aligned the kernel
+// moves bytes: 28.9 / 31.1 / 26.4 / 29.9 against 30.8 / 32.1 / 25.6 / 29.8 us, so there the line is 256 KB.
 static void copy_on_device(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  if (bytes <= (1u << 20)) k::copy_bytes(dst, src, bytes, s);
+  const bool aligned = (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
+  if (bytes <= (aligned ? 1u << 20 : 256u << 10)) k::copy_bytes(dst, src, bytes, s);
   else OXB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s));
 }
 

@@ -156,3 +156,22 @@ def test_a_plan_made_while_the_default_stream_is_busy(kind):
     assert any({"split_k": "splitK", "dynamic_quantize": "dynamic_quantize", "chain": "chain"}[kind] in k and "small" not in k for k in kernels), kernels
     got, _ = first_run(True)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 255, 256, 257])  # 4 KB a row: both copies' ranges on either side of their ends
+@pytest.mark.parametrize("offset", [0, 4, 12, 16])
+def test_bound_outputs_of_any_size_and_word_alignment(rows, offset):
+    import torch
+    weights = {"z": np.zeros(1, np.float32)}
+    graph = Graph(nodes=[Node("Add", "a", ["x", "z"], ["y"], {})], input_names=["x"], output_names=["y"])
+    x = np.random.default_rng(rows).standard_normal((rows, 1024)).astype(np.float32)
+    session = Session.builder().build_from_graph(graph, weights)
+    session.ensure_planned({"x": x})
+    out = torch.full((x.size + 16,), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    session.bind_output_device("y", out.data_ptr() + offset, x.size)
+    session.run_with_binding({"x": x}, fetch=False)
+    got, skip = out.cpu().numpy(), offset // 4
+    assert np.array_equal(got[skip:skip + x.size], x.ravel())
+    assert np.all(got[:skip] == 7.0) and np.all(got[skip + x.size:] == 7.0)
+    session.close()
