@@ -74,7 +74,8 @@ def kernel_source_sha():
     from another version of the kernel is not reported for this one."""
     h = hashlib.sha256()
     csrc = os.path.join(ROOT, "oxionnx_b200", "csrc")
-    for name in ("umma_kernel.cuh", "umma_launch.cuh", "kernels_umma.cu", "umma_i8.cu", "umma_tf32.cu", "umma_f16.cu"):
+    for name in ("umma_kernel.cuh", "umma_launch.cuh", "kernels_umma.cu", "umma_i8.cu", "umma_tf32.cu", "umma_f16.cu", "umma_small.cuh", "umma_small_i8.cu",
+                 "umma_small_float.cu"):
         with open(os.path.join(csrc, name), "rb") as fh:
             h.update(fh.read())
     return h.hexdigest()[:16]
@@ -344,7 +345,8 @@ def measure(args, key, batch, local_rank, world, dist, torch, lib, flush_l2, bar
                 fam0 = s["kernel"].split()[0]
                 umma_kernels.add("umma_chain_kernel (cooperative tcgen05 chain of quantised linears)" if fam0 == "umma_i8_chain" else
                                  ("umma_attention_kernel (tcgen05 scores + softmax + context)" if fam0 == "umma_attention" else
-                                  "umma_conv_kernel (tcgen05 implicit GEMM)"))
+                                  ("umma_small_kernel (tcgen05, one tile or K slice per CTA)" if " small" in s["kernel"] else
+                                   "umma_conv_kernel (tcgen05 implicit GEMM)")))
                 conv_ms += s["ms"]
                 conv_ops += s["work"]
                 conv_launches += 1
