@@ -330,9 +330,10 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   {
     const double k_bytes = (double)cs.K() * es;
     const double k_steps = k_bytes / 32.0;
-    // epilogue: per output 0.07 ns requantised / 0.03 ns float, plus about 0.5 us per tile whatever its width (the
-    // per-tile handshakes and address arithmetic of the epilogue warps: a 1x1 64 -> 256 layer at M = 802816 takes
-    // 3.0 us per round of 128 x 256 tiles, 1.05 us per round of 128 x 64 tiles, 0.84 us per round of 128 x 32)
+    // epilogue: per output 0.07 ns requantised / 0.03 ns float, plus about 0.5 us per tile whatever its width (what a
+    // tile costs the producer and issuer warps, whose 0.7 us a tile of little K only partly overlap: a 1x1 64 -> 256 layer
+    // at M = 802816 takes 3.0 us per round of 128 x 256 tiles, 1.05 us per round of 128 x 64 tiles, 0.84 us per round of
+    // 128 x 32)
     const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : 0.07e-9;
     const double t_tile_fixed = 0.5e-6;
     const int max_split = tune.split_k_max > 0 ? tune.split_k_max : 8;
