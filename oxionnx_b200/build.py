@@ -19,23 +19,15 @@ LIB = os.path.join(OUT_DIR, "liboxb200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fast-math", "--fmad=false"]
 # --fmad=false everywhere except the tensor-core kernel file, whose float epilogue is one add
-SOURCES = {
-    "kernels_glue.cu": COMMON,
-    "kernels_simt.cu": [f for f in COMMON if f != "--fmad=false"],
-    "kernels_umma.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_i8.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_tf32.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_f16.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_small_i8.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_small_float.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_probe.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_chain.cu": [f for f in COMMON if f != "--fmad=false"],
-    "umma_attention.cu": [f for f in COMMON if f != "--fmad=false"],
-    "runtime.cpp": COMMON,
-    "planner.cpp": COMMON,
-    "abi.cpp": COMMON,
-    "onnx_model.cpp": COMMON,
-    "model_abi.cpp": COMMON,
+KERNEL = [f for f in COMMON if f != "--fmad=false"]
+# object -> (source, flags); the integer contraction kernel is compiled once per tile width, side by side
+OBJECTS = {
+    "kernels_glue": ("kernels_glue.cu", COMMON),
+    **{name: (name + ".cu", KERNEL) for name in ("kernels_simt", "kernels_umma", "umma_i8", "umma_tf32", "umma_f16", "umma_small_i8", "umma_small_float",
+                                                  "umma_probe", "umma_chain", "umma_attention")},
+    **{f"umma_i8_{tile}": ("umma_i8_tile.cu", KERNEL + [f"-DOXB_TILE={bn}", f"-DOXB_PAIR={pair}"])
+       for tile, bn, pair in (("32", 32, "false"), ("64", 64, "false"), ("128", 128, "false"), ("256", 256, "false"), ("pair", 256, "true"))},
+    **{name: (name + ".cpp", COMMON) for name in ("runtime", "planner", "abi", "onnx_model", "model_abi")},
 }
 HEADERS = ["common.hpp", "kernels.hpp", "runtime.hpp", "umma_kernel.cuh", "umma_launch.cuh", "umma_small.cuh", "pdl.cuh", "umma_chain.cuh", "model.hpp", "abi_internal.hpp", os.path.join("..", "..", "include", "oxb200.h")]
 
@@ -60,9 +52,9 @@ def build(force=False, verbose=False):
     nvcc = _nvcc()
     jobs = []
     objs = []
-    for src, flags in SOURCES.items():
+    for name, (src, flags) in OBJECTS.items():
         path = os.path.join(CSRC, src)
-        obj = os.path.join(OBJ_DIR, src + ".o")
+        obj = os.path.join(OBJ_DIR, name + ".o")
         objs.append(obj)
         if force or _stale(obj, [path] + headers):
             cmd = [nvcc] + ARCH + flags + ["-x", "cu", "-c", path, "-o", obj]

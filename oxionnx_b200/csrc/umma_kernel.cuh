@@ -45,6 +45,8 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "kernels.hpp"
 
 namespace oxb {
@@ -212,7 +214,7 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorM
       "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
       : "memory");
 }
-// The same two loads issued by a CTA of a pair: the data lands in the issuing CTA's shared memory, the bytes are
+// The same loads issued by a CTA of a pair: the data lands in the issuing CTA's shared memory, the bytes are
 // counted on `bar`, a shared::cluster address that names the even CTA's barrier.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
@@ -238,39 +240,41 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// The MMAs of one K block (1, 2 or 4 instructions of 32 bytes of K each) in one asm block: the
-// 64-bit descriptors are assembled from a 32-bit low word that advances by 2 (16-byte units) per
-// instruction and a constant high word, so the issuing thread spends a handful of integer
-// instructions per K block.
-#define OXB_MMA_BLOCK(GROUP, KINDSTR)                                                                       \
-  asm volatile(                                                                                             \
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t.reg .b32 la, lb;\n\t"                                 \
-      "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, 1, 0;\n\t"                                                   \
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"                                                  \
-      "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], da, db, %4, p;\n\t"                         \
-      "setp.lt.u32 p, %6, 2;\n\t@p bra DONE_%=;\n\t"                                                        \
-      "add.u32 la, %1, 2;\n\tadd.u32 lb, %2, 2;\n\tmov.b64 da, {la, %3};\n\tmov.b64 db, {lb, %3};\n\t"     \
-      "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], da, db, %4, q;\n\t"                         \
-      "setp.lt.u32 p, %6, 4;\n\t@p bra DONE_%=;\n\t"                                                        \
-      "add.u32 la, %1, 4;\n\tadd.u32 lb, %2, 4;\n\tmov.b64 da, {la, %3};\n\tmov.b64 db, {lb, %3};\n\t"     \
-      "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], da, db, %4, q;\n\t"                         \
-      "add.u32 la, %1, 6;\n\tadd.u32 lb, %2, 6;\n\tmov.b64 da, {la, %3};\n\tmov.b64 db, {lb, %3};\n\t"     \
-      "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], da, db, %4, q;\n\t"                         \
-      "DONE_%=:\n\t}" ::"r"(tmem_d),                                                                        \
-      "r"(lo_a), "r"(lo_b), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(mmas)                            \
-      : "memory")
-
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// One MMA of 32 bytes of K from two complete descriptors (43 cycles each when issued back to back by one thread;
+// assembling them inside the asm block, as tc_mma_block does, takes 70).
+template <int KIND, bool PAIR = false>
+__device__ __forceinline__ void tc_mma_one(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+#define OXB_MMA_ONE(GROUP, KINDSTR)                                                                                                        \
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], %1, %2, %3, p;\n\t}" ::"r"( \
+                   tmem_d),                                                                                                               \
+               "l"(da), "l"(db), "r"(idesc), "r"(accumulate)                                                                              \
+               : "memory")
+  if (PAIR) {
+    if (KIND == KIND_I8) OXB_MMA_ONE("2", "i8");
+    else if (KIND == KIND_TF32) OXB_MMA_ONE("2", "tf32");
+    else OXB_MMA_ONE("2", "f16");
+  } else {
+    if (KIND == KIND_I8) OXB_MMA_ONE("1", "i8");
+    else if (KIND == KIND_TF32) OXB_MMA_ONE("1", "tf32");
+    else OXB_MMA_ONE("1", "f16");
+  }
+#undef OXB_MMA_ONE
+}
+// The MMAs of one K block (1, 2 or 4 of 32 bytes of K each) from the two words of its descriptors.
 template <int KIND, bool PAIR>
 __device__ __forceinline__ void tc_mma_block(uint32_t tmem_d, uint32_t lo_a, uint32_t lo_b, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate,
                                              uint32_t mmas) {
-  if (PAIR) {
-    if (KIND == KIND_I8) OXB_MMA_BLOCK("2", "i8");
-    else if (KIND == KIND_TF32) OXB_MMA_BLOCK("2", "tf32");
-    else OXB_MMA_BLOCK("2", "f16");
-  } else {
-    if (KIND == KIND_I8) OXB_MMA_BLOCK("1", "i8");
-    else if (KIND == KIND_TF32) OXB_MMA_BLOCK("1", "tf32");
-    else OXB_MMA_BLOCK("1", "f16");
+  const uint64_t hi = (uint64_t)desc_hi << 32, da = hi | lo_a, db = hi | lo_b;
+  tc_mma_one<KIND, PAIR>(tmem_d, da, db, idesc, accumulate);
+  if (mmas >= 2) tc_mma_one<KIND, PAIR>(tmem_d, da + 2, db + 2, idesc, 1u);
+  if (mmas >= 4) {
+    tc_mma_one<KIND, PAIR>(tmem_d, da + 4, db + 4, idesc, 1u);
+    tc_mma_one<KIND, PAIR>(tmem_d, da + 6, db + 6, idesc, 1u);
   }
 }
 
@@ -865,6 +869,31 @@ struct TileWalk {
   }
 };
 
+// The first output pixel of an im2col tile, carried from tile to tile without divisions the same way: `step` pixels are
+// split once into columns, rows and images.
+struct PixelStep {
+  int q, p, n;
+  __device__ __forceinline__ PixelStep(int m, int Q, int P) {
+    q = m % Q;
+    const int rest = m / Q;
+    p = rest % P;
+    n = rest / P;
+  }
+  __device__ __forceinline__ void add(const PixelStep& d, int Q, int P) {
+    q += d.q;
+    p += d.p;
+    n += d.n;
+    if (q >= Q) {
+      q -= Q;
+      ++p;
+    }
+    if (p >= P) {
+      p -= P;
+      ++n;
+    }
+  }
+};
+
 // How the epilogue warps of a block share tiles (see the file header).
 template <int BN, int EW>
 struct EpiShape {
@@ -1221,123 +1250,146 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // The producer and the MMA issuer run their loops with the whole warp (every lane polls the
-  // barrier, one lane issues): a lone lane looping while its 31 siblings sit at the teardown
-  // barrier gets only a fraction of the warp's issue slots.
+  // The producer and the MMA issuer are one elected thread each; the other lanes of its warp wait at the warp's own
+  // barrier (at the block's, they would take issue slots).  These two threads bound every layer of small K blocks, so
+  // nothing in their loops is warp-wide, decided per block or divided per tile, and an MMA gets complete descriptors.
+  // Against warp-wide loops with a vote per step, a choice of load per block and two divisions per tile: i8 3x3 64 -> 64 at
+  // M = 1605632 234 -> 145 us, the 64-channel stem at M = 6422528 389 -> 266 us, 3x3 128 -> 128 at M = 401408 94 -> 81 us;
+  // TF32 3x3 64 -> 64 at M = 100352 45 -> 32 us, 3x3 256 -> 128 at M = 65536 107 -> 84 us.
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     uint32_t stage = 0, phase = 0;  // ring position, carried across tiles
     bool ok = true;
     // a pair's copies are counted on the even CTA's barrier, which alone announces the bytes of both
     const uint32_t tx_per_kb = PAIR ? 2u * kb_bytes : kb_bytes;
-    if (b_res && tile0 < total_tiles && lane == 0) {
-      // the whole weight matrix of the (only) channel tile, once: K block i at b_res_base + i * b_bytes
-      mbar_expect_tx(smem_u32(&bar_b_resident), p.b_resident_bytes);
-      for (int i = 0; i < k_iters; ++i) tma_load_2d(b_res_base + (uint32_t)i * b_bytes, &p.tmB, smem_u32(&bar_b_resident), i * p.cb_elems, 0);
-    }
-    __syncwarp();
     const bool plain = !p.batched && p.splits == 1;
-    TileWalk walk(tile0, tile_step, p.n_tiles);
-    for (int t = tile0; t < total_tiles && ok; t += tile_step, walk.next()) {
-      int tt = t, a_row0 = 0, a_col0 = 0, b_row0 = 0, b_col0 = 0;
-      int it_begin = 0, it_end = k_iters;
-      if (p.batched) {
-        const int per = p.m_tiles * p.n_tiles, item = t / per;
-        tt = t - item * per;
-        const int outer = item / p.items_inner, inner = item - outer * p.items_inner;
-        a_row0 = outer * p.a_rb + inner * p.a_rh;
-        a_col0 = inner * p.a_ch;
-        b_row0 = outer * p.b_rb + inner * p.b_rh;
-        b_col0 = inner * p.b_ch;
-      } else if (p.splits > 1) {
-        tt = t / p.splits;
-        it_begin = (t - tt * p.splits) * p.k_per;
-        it_end = min(k_iters, it_begin + p.k_per);
-      }
-      const int tile_n = plain ? walk.n : tt % p.n_tiles, tile_m = plain ? walk.m : tt / p.n_tiles;
-      const int m0 = tile_m * (PAIR ? 2 * BLOCK_M : BLOCK_M) + (PAIR ? pair_rank * BLOCK_M : 0);
-      const int oc0 = tile_n * BN + (PAIR ? pair_rank * B_ROWS : 0);
-      int q0 = 0, p0 = 0, n0 = 0;
-      if (p.a_im2col) {
-        q0 = m0 % p.Q;
-        int rest = m0 / p.Q;
-        p0 = rest % p.P;
-        n0 = rest / p.P;
-      }
-      const int w_base = q0 * p.sw - p.pl, h_base = p0 * p.sh - p.pt;
-      int cb = it_begin % p.cblocks, sx = (it_begin / p.cblocks) % p.S, r = (it_begin / p.cblocks) / p.S;
-      // A barrier round trip, an expect_tx and each TMA instruction cost the issuing thread on the
-      // order of a hundred cycles, whatever the box size: a stage carries several K blocks when
-      // they are small, so that those costs are paid once per stage.
-      for (int it = it_begin; it < it_end; it += p.kpb) {
-        bool got = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp);
-        if (!__all_sync(0xffffffffu, got)) {
-          if (lane == 0 && !*abortp) {
-            *abortp = 1;
-            atomicExch(p.err_flag, 1);
-          }
-          ok = false;
-          break;
+    // One copy of the loop per form of the two loads.  B_FORM: 0 resident, 1 through the ring.
+    auto produce = [&](auto im2col_c, auto b_form_c) {
+      constexpr bool IM2COL = decltype(im2col_c)::value;
+      constexpr int B_FORM = decltype(b_form_c)::value;
+      const int kpb = p.kpb, cblocks = p.cblocks, cb_elems = p.cb_elems, taps_s = p.S, stages = p.stages;
+      constexpr int M_STEP = PAIR ? 2 * BLOCK_M : BLOCK_M;
+      TileWalk walk(tile0, tile_step, p.n_tiles);
+      PixelStep pixel(IM2COL ? walk.m * M_STEP + (PAIR ? pair_rank * BLOCK_M : 0) : 0, p.Q, p.P);
+      const PixelStep by_step(IM2COL ? walk.dm * M_STEP : 0, p.Q, p.P), by_tile(IM2COL ? M_STEP : 0, p.Q, p.P);
+      auto next_tile = [&]() {
+        const int m = walk.m;
+        walk.next();
+        if (IM2COL) {
+          pixel.add(by_step, p.Q, p.P);
+          if (walk.m - m != walk.dm) pixel.add(by_tile, p.Q, p.P);
         }
-        const int blocks = min(p.kpb, it_end - it);
-        const uint32_t full_local = smem_u32(&bar_full[stage]);
-        const uint32_t full = PAIR ? mapa(full_local, 0) : full_local;
-        if (lane == 0 && leader) mbar_expect_tx(full_local, tx_per_kb * (uint32_t)blocks);
-        uint32_t a_dst = tiles_base + stage * stage_bytes;
-        for (int g = 0; g < blocks; ++g, a_dst += kb_bytes) {
-          if (lane == 0) {  // one thread issues: every operand of the copies is warp-uniform
-            const int c_off = cb * p.cb_elems;
+      };
+      for (int t = tile0; t < total_tiles && ok; t += tile_step, next_tile()) {
+        int tt = t, a_row0 = 0, a_col0 = 0, b_row0 = 0, b_col0 = 0;
+        int it_begin = 0, it_end = k_iters;
+        if (p.batched) {
+          const int per = p.m_tiles * p.n_tiles, item = t / per;
+          tt = t - item * per;
+          const int outer = item / p.items_inner, inner = item - outer * p.items_inner;
+          a_row0 = outer * p.a_rb + inner * p.a_rh;
+          a_col0 = inner * p.a_ch;
+          b_row0 = outer * p.b_rb + inner * p.b_rh;
+          b_col0 = inner * p.b_ch;
+        } else if (p.splits > 1) {
+          tt = t / p.splits;
+          it_begin = (t - tt * p.splits) * p.k_per;
+          it_end = min(k_iters, it_begin + p.k_per);
+        }
+        const int tile_n = plain ? walk.n : tt % p.n_tiles, tile_m = plain ? walk.m : tt / p.n_tiles;
+        const int m0 = tile_m * M_STEP + (PAIR ? pair_rank * BLOCK_M : 0);
+        const int oc0 = tile_n * BN + (PAIR ? pair_rank * B_ROWS : 0);
+        const int b_row = b_row0 + oc0;
+        if (IM2COL && !plain) pixel = PixelStep(m0, p.Q, p.P);
+        const int w_base = pixel.q * p.sw - p.pl, h_base = pixel.p * p.sh - p.pt, n0 = pixel.n;
+        int cb = 0, sx = 0, r = 0;
+        if (it_begin > 0) cb = it_begin % cblocks, sx = (it_begin / cblocks) % taps_s, r = (it_begin / cblocks) / taps_s;
+        // A barrier round trip, an expect_tx and each TMA instruction cost the issuing thread on the
+        // order of a hundred cycles, whatever the box size: a stage carries several K blocks when
+        // they are small, so that those costs are paid once per stage.
+        for (int it = it_begin; it < it_end; it += kpb) {
+          if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp)) {
+            if (!*abortp) {
+              *abortp = 1;
+              atomicExch(p.err_flag, 1);
+            }
+            ok = false;
+            break;
+          }
+          const int blocks = min(kpb, it_end - it);
+          const uint32_t full_local = smem_u32(&bar_full[stage]);
+          const uint32_t full = PAIR ? mapa(full_local, 0) : full_local;
+          if (leader) mbar_expect_tx(full_local, tx_per_kb * (uint32_t)blocks);
+          uint32_t a_dst = tiles_base + stage * stage_bytes;
+          for (int g = 0; g < blocks; ++g, a_dst += kb_bytes) {
+            const int c_off = cb * cb_elems;
             if (PAIR) {
-              if (p.a_im2col) tma_load_im2col_4d_pair(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
+              if (IM2COL) tma_load_im2col_4d_pair(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
               else tma_load_2d_pair(a_dst, &p.tmA, full, a_col0 + c_off, a_row0 + m0);
-              tma_load_2d_pair(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * p.cb_elems, b_row0 + oc0);
+              tma_load_2d_pair(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * cb_elems, b_row);
             } else {
-              if (p.a_im2col) tma_load_im2col_4d(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
+              if (IM2COL) tma_load_im2col_4d(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
               else tma_load_2d(a_dst, &p.tmA, full, a_col0 + c_off, a_row0 + m0);
-              if (!b_res) tma_load_2d(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * p.cb_elems, b_row0 + oc0);
+              if (B_FORM == 1) tma_load_2d(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * cb_elems, b_row);
+            }
+            if (++cb == cblocks) {
+              cb = 0;
+              if (++sx == taps_s) {
+                sx = 0;
+                ++r;
+              }
             }
           }
-          if (++cb == p.cblocks) {
-            cb = 0;
-            if (++sx == p.S) {
-              sx = 0;
-              ++r;
-            }
+          if (++stage == (uint32_t)stages) {
+            stage = 0;
+            phase ^= 1u;
           }
         }
-        __syncwarp();
+      }
+    };
+    auto with_b = [&](auto im2col_c) {
+      if constexpr (!PAIR) {
+        if (b_res) return produce(im2col_c, std::integral_constant<int, 0>());
+      }
+      produce(im2col_c, std::integral_constant<int, 1>());
+    };
+    if (elect_one()) {
+      if (b_res && tile0 < total_tiles) {
+        // the whole weight matrix of the (only) channel tile, once: K block i at b_res_base + i * b_bytes
+        mbar_expect_tx(smem_u32(&bar_b_resident), p.b_resident_bytes);
+        for (int i = 0; i < k_iters; ++i) {
+          const uint32_t dst = b_res_base + (uint32_t)i * b_bytes;
+          tma_load_2d(dst, &p.tmB, smem_u32(&bar_b_resident), i * p.cb_elems, 0);
+        }
+      }
+      if (p.a_im2col) with_b(std::true_type());
+      else with_b(std::false_type());
+      // Tail: every stage this CTA filled has been consumed and its release has arrived here, so no arrival is
+      // still on its way to this CTA's shared memory when the CTA ends.
+      for (int i = 0; i < p.stages && ok; ++i) {
+        if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp)) break;  // another role has recorded the cause
         if (++stage == (uint32_t)p.stages) {
           stage = 0;
           phase ^= 1u;
         }
       }
     }
-    // Tail: every stage this CTA filled has been consumed and its release has arrived here, so no arrival is
-    // still on its way to this CTA's shared memory when the CTA ends.
-    for (int i = 0; i < p.stages && ok; ++i) {
-      bool got = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abortp);
-      if (!__all_sync(0xffffffffu, got)) break;  // another role has recorded the cause
-      if (++stage == (uint32_t)p.stages) {
-        stage = 0;
-        phase ^= 1u;
-      }
-    }
+    __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer (the even CTA of a pair issues for both) ----------------
-    if (leader) {
-      const uint32_t mmas = (uint32_t)(swz / 32);
-      const uint64_t desc_rest = make_smem_desc(0, swz);
-      const uint32_t desc_hi = (uint32_t)(desc_rest >> 32), desc_lo = (uint32_t)desc_rest;
+    if (leader && elect_one()) {
+      // descriptors differ between K blocks and steps only in the 16-byte granular start address
+      const uint64_t desc = make_smem_desc(0, swz);
       const uint32_t idesc = p.idesc;
+      const int kpb = p.kpb, stages = p.stages;
       const uint32_t ring16 = tiles_base >> 4, stage16 = stage_bytes >> 4, kb16 = kb_bytes >> 4, a16_bytes = a_bytes >> 4;
       uint32_t stage = 0, phase = 0, a16 = ring16;
       uint32_t local = 0;
       bool ok = true;
       const uint32_t bres16 = b_res_base >> 4, b16_bytes = b_bytes >> 4;
       if (b_res && tile0 < total_tiles) {  // the resident weights have landed
-        const bool got = mbar_wait(smem_u32(&bar_b_resident), 0u, abortp);
-        if (!__all_sync(0xffffffffu, got)) {
-          if (lane == 0 && !*abortp) {
+        if (!mbar_wait(smem_u32(&bar_b_resident), 0u, abortp)) {
+          if (!*abortp) {
             *abortp = 1;
             atomicExch(p.err_flag, 5);
           }
@@ -1349,9 +1401,8 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         const uint32_t buf = local % (uint32_t)ES::NACC;
         const uint32_t acc_phase = (local / (uint32_t)ES::NACC) & 1u;
         // the epilogue must have drained this accumulator (free on its first use)
-        bool got = mbar_wait(smem_u32(&bar_acc_empty[buf]), acc_phase ^ 1u, abortp);
-        if (!__all_sync(0xffffffffu, got)) {
-          if (lane == 0 && !*abortp) {
+        if (!mbar_wait(smem_u32(&bar_acc_empty[buf]), acc_phase ^ 1u, abortp)) {
+          if (!*abortp) {
             *abortp = 1;
             atomicExch(p.err_flag, 4);
           }
@@ -1364,10 +1415,9 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
           it_begin = (t % p.splits) * p.k_per;
           it_end = min(k_iters, it_begin + p.k_per);
         }
-        for (int it = it_begin; it < it_end; it += p.kpb) {
-          got = mbar_wait(smem_u32(&bar_full[stage]), phase, abortp);
-          if (!__all_sync(0xffffffffu, got)) {
-            if (lane == 0 && !*abortp) {
+        for (int it = it_begin; it < it_end; it += kpb) {
+          if (!mbar_wait(smem_u32(&bar_full[stage]), phase, abortp)) {
+            if (!*abortp) {
               *abortp = 1;
               atomicExch(p.err_flag, 2);
             }
@@ -1375,32 +1425,34 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
-            // descriptors differ between K blocks only in the 16-byte granular start address
-            const int blocks = min(p.kpb, it_end - it);
-            uint32_t b16 = a16;
-            for (int g = 0; g < blocks; ++g, b16 += kb16) {
-              const uint32_t w16 = b_res ? bres16 + (uint32_t)(it + g) * b16_bytes : b16 + a16_bytes;
-              tc_mma_block<KIND, PAIR>(tmem_d, desc_lo | (b16 & 0x3fffu), desc_lo | (w16 & 0x3fffu), desc_hi, idesc, (it + g) > it_begin ? 1u : 0u, mmas);
-            }
-            // frees the stage, in both CTAs of a pair, once these MMAs have read it
-            const uint32_t e = smem_u32(&bar_empty[stage]);
-            if (PAIR) {
-              tc_commit<true>(mapa(e, 0));
-              tc_commit<true>(mapa(e, 1));
-            } else {
-              tc_commit<false>(e);
+          const int blocks = min(kpb, it_end - it);
+          uint32_t x16 = a16, w16 = b_res ? bres16 + (uint32_t)it * b16_bytes : a16 + a16_bytes;
+          const uint32_t w_step = b_res ? b16_bytes : kb16;
+          for (int g = 0; g < blocks; ++g, x16 += kb16, w16 += w_step) {
+            const uint64_t da = desc | (x16 & 0x3fffu), db = desc | (w16 & 0x3fffu);
+            tc_mma_one<KIND, PAIR>(tmem_d, da, db, idesc, (it + g) > it_begin ? 1u : 0u);
+            if (swz >= 64) tc_mma_one<KIND, PAIR>(tmem_d, da + 2, db + 2, idesc, 1u);
+            if (swz == 128) {
+              tc_mma_one<KIND, PAIR>(tmem_d, da + 4, db + 4, idesc, 1u);
+              tc_mma_one<KIND, PAIR>(tmem_d, da + 6, db + 6, idesc, 1u);
             }
           }
-          __syncwarp();
+          // frees the stage, in both CTAs of a pair, once these MMAs have read it
+          const uint32_t e = smem_u32(&bar_empty[stage]);
+          if (PAIR) {
+            tc_commit<true>(mapa(e, 0));
+            tc_commit<true>(mapa(e, 1));
+          } else {
+            tc_commit<false>(e);
+          }
           a16 += stage16;
-          if (++stage == (uint32_t)p.stages) {
+          if (++stage == (uint32_t)stages) {
             stage = 0;
             phase ^= 1u;
             a16 = ring16;
           }
         }
-        if (ok && lane == 0) {  // accumulator complete
+        if (ok) {  // accumulator complete
           const uint32_t f = smem_u32(&bar_acc_full[buf]);
           if (PAIR) {
             tc_commit<true>(mapa(f, 0));
@@ -1409,9 +1461,9 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
             tc_commit<false>(f);
           }
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else {
     // ---------------- epilogue ----------------
     const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));

@@ -81,24 +81,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   }
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) { asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)m) : "memory"); }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
-  return p != 0;
-}
-// One MMA of 32 bytes of K from two complete descriptors (43 cycles each when issued back to back by one thread;
-// assembling them inside the asm block, as tc_mma_block does, takes 70).
-template <int KIND>
-__device__ __forceinline__ void tc_mma_one(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-#define OXB_MMA_ONE(KINDSTR)                                                                                                                             \
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::" KINDSTR " [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d), \
-               "l"(da), "l"(db), "r"(idesc), "r"(accumulate)                                                                                             \
-               : "memory")
-  if (KIND == KIND_I8) OXB_MMA_ONE("i8");
-  else if (KIND == KIND_TF32) OXB_MMA_ONE("tf32");
-  else OXB_MMA_ONE("f16");
-#undef OXB_MMA_ONE
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
                "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
