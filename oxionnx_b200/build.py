@@ -29,7 +29,7 @@ OBJECTS = {
        for tile, bn, pair in (("32", 32, "false"), ("64", 64, "false"), ("128", 128, "false"), ("256", 256, "false"), ("pair", 256, "true"))},
     **{name: (name + ".cpp", COMMON) for name in ("runtime", "planner", "abi", "onnx_model", "model_abi")},
 }
-HEADERS = ["common.hpp", "kernels.hpp", "runtime.hpp", "umma_kernel.cuh", "umma_launch.cuh", "umma_small.cuh", "pdl.cuh", "umma_chain.cuh", "model.hpp", "abi_internal.hpp", os.path.join("..", "..", "include", "oxb200.h")]
+HEADERS = ["common.hpp", "kernels.hpp", "runtime.hpp", "umma_kernel.cuh", "umma_epilogue8.cuh", "umma_launch.cuh", "umma_small.cuh", "pdl.cuh", "umma_chain.cuh", "model.hpp", "abi_internal.hpp", os.path.join("..", "..", "include", "oxb200.h")]
 
 
 def _nvcc():

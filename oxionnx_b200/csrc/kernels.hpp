@@ -80,6 +80,9 @@ void residual_requant_prepare(ResidualParams& rp, DT a_dt, DT b_dt);
 struct JoinConstants {
   float ca = 0.f, cb = 0.f, cc = 0.f;
   int lo = 0, hi = 255;
+  // the same with the requantised lane scaled to [0, 1]: lane = clamp(rne(fma(rne((a - a_lo) * d), a8, fma(b, b8, c8))), lo,
+  // hi), a_lo the lowest value of a's type; d == 0 when no constants were found
+  float d = 0.f, a8 = 0.f, b8 = 0.f, c8 = 0.f;
 };
 bool residual_join_constants(const ResidualParams& rp, DT a_dt, DT b_dt, JoinConstants* out);
 void residual_requant(const void* a, DT a_dt, const void* b, DT b_dt, void* y, DT y_dt, int64_t n, const ResidualParams& rp, cudaStream_t s);
@@ -213,6 +216,7 @@ struct Epilogue {
   // out = clamp(rne(lane * join_a + residual * join_b + join_c), join_lo, join_hi); lo / hi / y_zp stay the lane's own
   int join = 0, join_signed = 0, join_lo = 0, join_hi = 255;
   float join_a = 0.f, join_b = 0.f, join_c = 0.f;
+  float join_d = 0.f, join_a8 = 0.f, join_b8 = 0.f, join_c8 = 0.f;  // JoinConstants::d .. c8
   // integer modes.  Direct kernels subtract zero points per element; the tensor-core kernel
   // computes raw = sum(x*w) and applies acc = raw + bias_i[oc] - x_zp * wsum[oc].
   const int32_t* bias_i = nullptr;

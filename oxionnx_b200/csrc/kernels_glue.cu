@@ -2252,32 +2252,42 @@ bool residual_join_constants(const ResidualParams& rp, DT a_dt, DT b_dt, JoinCon
   };
   static const int order[] = {0, 1, -1, 2, -2, 3, -3, 4, -4};
   int hint = 0;  // the pair that refuted the last candidate is tried first
-  for (int sa = 0; sa < 3; ++sa)
-    for (int sb = 0; sb < 3; ++sb)
-      for (int sc : order) {
-        JoinConstants k;
-        k.ca = step((float)ca, order[sa]), k.cb = step((float)cb, order[sb]);
-        k.cc = step((float)((double)rp.y_zp - (double)rp.a_zp * k.ca - (double)rp.b_zp * k.cb), sc);
-        k.lo = (int)lo_eff, k.hi = (int)rp.hi;
-        auto holds = [&](int pair) {
-          const float a = (float)((pair >> 8) + a_lo), b = (float)((pair & 255) + b_lo);
-          const float t = std::fmaf(a, k.ca, std::fmaf(b, k.cb, k.cc));
-          volatile float m = t + magic;
-          const float r = m - magic;
-          return std::fabs(r) <= 32000.f && std::fmin(std::fmax(r, lo_eff), rp.hi) == (float)want[pair];
-        };
-        bool ok = holds(hint);
-        for (int pair = 0; pair < 65536 && ok; ++pair)
-          if (!holds(pair)) {
-            ok = false;
-            hint = pair;
+  // Constants for a's lane times `unit` (rounded to a float of its own), a's lowest value moved to `from`.
+  auto search = [&](double unit, int from, float* fa, float* fb, float* fc) {
+    float lane[256];
+    for (int i = 0; i < 256; ++i) lane[i] = unit == 1.0 ? (float)(i + a_lo - from) : std::fmin((float)(i * unit), 1.0f);  // the scaled lane saturates at 1
+    for (int sa = 0; sa < 3; ++sa)
+      for (int sb = 0; sb < 3; ++sb)
+        for (int sc : order) {
+          const float ka = step((float)(ca / unit), order[sa]), kb = step((float)cb, order[sb]);
+          const float kc = step((float)((double)rp.y_zp - ((double)rp.a_zp - from) * unit * ka - (double)rp.b_zp * kb), sc);
+          auto holds = [&](int pair) {
+            const float t = std::fmaf(lane[pair >> 8], ka, std::fmaf((float)((pair & 255) + b_lo), kb, kc));
+            volatile float m = t + magic;
+            const float r = m - magic;
+            return std::fabs(r) <= 32000.f && std::fmin(std::fmax(r, lo_eff), rp.hi) == (float)want[pair];
+          };
+          bool ok = holds(hint);
+          for (int pair = 0; pair < 65536 && ok; ++pair)
+            if (!holds(pair)) {
+              ok = false;
+              hint = pair;
+            }
+          if (ok) {
+            *fa = ka, *fb = kb, *fc = kc;
+            return true;
           }
-        if (ok) {
-          *out = k;
-          return true;
         }
-      }
-  return false;
+    return false;
+  };
+  JoinConstants k;
+  k.lo = (int)lo_eff, k.hi = (int)rp.hi;
+  if (!search(1.0, 0, &k.ca, &k.cb, &k.cc)) return false;
+  // 1 / 255 rounded up to 21 bits: its product with 1.5 * 2^23 is exact, and 255 of it is at least 1
+  const float d = (float)std::ldexp(std::ceil(std::ldexp(1.0 / 255.0, 28)), -28);
+  if (search((double)d, a_lo, &k.a8, &k.b8, &k.c8)) k.d = d;
+  *out = k;
+  return true;
 }
 
 void s2d_pack(const TensorRef& src, void* dst, DT dst_dt, int c_pad, int sub, cudaStream_t s) {

@@ -187,7 +187,8 @@ void layout_smem(KParams& kp, int bn, int kind, bool pair, size_t* smem_total) {
   const size_t resident = kp.b_resident_bytes;
   const size_t kb_bytes = (size_t)(BLOCK_M + (resident ? 0 : (pair ? bn / 2 : bn))) * kp.swizzle_bytes;
   const size_t stage_bytes = kb_bytes * kp.kpb;
-  const size_t staging = kp.out_tma ? (size_t)ew * 32 * kp.out_row_bytes * std::max(kp.res_bufs, 1) : 0;
+  const size_t staging = kp.b_perm ? ew * (kp.res_bufs * (size_t)B8_RES_BYTES + B8_PARAM_BYTES)
+                                   : (kp.out_tma ? (size_t)ew * 32 * kp.out_row_bytes * std::max(kp.res_bufs, 1) : 0);
   // one persistent CTA per SM: the ring may use most of the shared memory and runs on across tiles
   const size_t budget = std::min<size_t>(192 * 1024, kSmemBudget - staging) - resident;
   int stages = (int)(budget / stage_bytes);
@@ -452,15 +453,6 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     rc = g_encode_tiled(&kp.tmB, dtype, 3, const_cast<void*>(w_packed), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return fail("weight tensor map rejected by the driver");
-  } else {
-    const int64_t ktot = cs.K();
-    cuuint64_t gdim[2] = {(cuuint64_t)ktot, (cuuint64_t)cs.OC};
-    cuuint64_t gstr[1] = {(cuuint64_t)ktot * es};
-    cuuint32_t box[2] = {(cuuint32_t)cb, (cuuint32_t)(pair ? bn / 2 : bn)};  // a CTA of a pair stages its half of the channel tile
-    cuuint32_t estr[2] = {1, 1};
-    rc = g_encode_tiled(&kp.tmB, dtype, 2, const_cast<void*>(w_packed), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) return fail("weight tensor map rejected by the driver");
   }
   {
     // output tile store through TMA when rows are 16-byte granular
@@ -534,37 +526,6 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // the staged row was sized for one run per store; the unsplit loop stores a warp's whole share at once
     if (!have_ws && kp.out_tma && (int)warp_row_bytes(bn, kind, dt_size(e.out_dt), false) != kp.out_row_bytes) kp.out_tma = 0;
   }
-  if (small.bn > 0) {
-    kp.small_bn = bn;
-    kp.a_rows = a_rows;
-    kp.splits = small.splits;
-    kp.k_per = small.k_per;
-    kp.kpb = small.kpb;
-    kp.stages = small.stages;
-    kp.stage_off = (uint32_t)(small.stages * small.stage_bytes);
-    pl->smem = small.smem;
-  } else {
-    // A residual is fetched through the staging rows of the store it is combined for: four buffers per epilogue warp
-    // where the ring keeps three stages beside them, else three or two.
-    if (e.residual && kp.out_tma && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0) {
-      const size_t oes = dt_size(e.out_dt);
-      cuuint64_t gdim[2] = {(cuuint64_t)cs.OC, (cuuint64_t)M};
-      cuuint64_t gstr[1] = {(cuuint64_t)cs.OC * oes};
-      cuuint32_t box[2] = {(cuuint32_t)(kp.out_row_bytes / oes), 32};
-      cuuint32_t estr[2] = {1, 1};
-      if (g_encode_tiled(&kp.tmR, output_map_type(e.out_dt), 2, const_cast<void*>(e.residual), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         swizzle_enum(kp.out_row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
-        const size_t per_buf = (size_t)epi_warps(kind) * 32 * kp.out_row_bytes;
-        auto fits = [&](int bufs, int stages) { return kSmemBudget >= bufs * per_buf + kp.b_resident_bytes + stages * kb_bytes * kp.kpb; };
-        while (kp.kpb > 1 && !fits(3, 2)) kp.kpb /= 2;
-        // From 1 KB of K a row on, the mainloop hides the epilogue but wants the ring: two buffers and three stages instead
-        // (TF32 1x1 512 -> 2048 with a residual, M=1568: 29.0 -> 24.9 us).
-        const bool long_k = (int64_t)cs.K() * es >= 1024;
-        kp.res_bufs = fits(4, 3) ? 4 : (long_k && fits(2, 3) ? 2 : (fits(3, 2) ? 3 : (fits(2, 2) ? 2 : 0)));
-      }
-    }
-    layout_smem(kp, bn, kind, pair, &pl->smem);
-  }
   kp.mode = e.mode;
   if (e.join) kp.variant = V_JOIN;
   else if (e.mode == EPI_F32) kp.variant = (e.residual ? V_F32_RES : V_F32_BASE) + e.act * 2 + (e.round_tf32 ? 1 : 0);
@@ -578,10 +539,78 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   }
   else if (e.mode == EPI_DEQUANT) kp.variant = V_DEQUANT + (e.x_zp_dev ? 1 : 0) + 2 * e.dq_act;
   else kp.variant = e.x_zp_dev ? V_INT32_DYN : V_INT32;
+  kp.lo = (e.relu_fused && e.lo < 0) ? 0 : e.lo;
+  kp.hi = e.hi;
+  if (small.bn > 0) {
+    kp.small_bn = bn;
+    kp.a_rows = a_rows;
+    kp.splits = small.splits;
+    kp.k_per = small.k_per;
+    kp.kpb = small.kpb;
+    kp.stages = small.stages;
+    kp.stage_off = (uint32_t)(small.stages * small.stage_bytes);
+    pl->smem = small.smem;
+  } else {
+    // 8-bit outputs of whole groups of 64 channels take the fragment epilogue (umma_epilogue8.cuh) wherever its arithmetic
+    // is allowed: it is the faster one at every K (the figures stand there).
+    const bool bytes_ok = kind == KIND_I8 && bn >= 64 && cs.OC % 64 == 0 && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0;
+    const bool join_ok = kp.variant == V_JOIN && e.join_d > 0.f && kp.hi - kp.lo == 255;
+    const int perm = bytes_ok && (kp.variant == V_REQUANT_PACKED || join_ok) ? 64 : 0;
+    kp.b_perm = perm;
+    if (perm > 0) {
+      kp.out_tma = 0;
+      kp.out_row_bytes = 64;
+    }
+    // A residual is fetched ahead through buffers per epilogue warp, those of the stores it is combined for or, in the
+    // fragment epilogue, buffers of the same size: four where the ring keeps three stages beside them, else three or two.
+    bool staged = perm > 0 && e.residual;
+    if (perm == 0 && e.residual && kp.out_tma && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0) {
+      const size_t oes = dt_size(e.out_dt);
+      cuuint64_t gdim[2] = {(cuuint64_t)cs.OC, (cuuint64_t)M};
+      cuuint64_t gstr[1] = {(cuuint64_t)cs.OC * oes};
+      cuuint32_t box[2] = {(cuuint32_t)(kp.out_row_bytes / oes), 32};
+      cuuint32_t estr[2] = {1, 1};
+      staged = g_encode_tiled(&kp.tmR, output_map_type(e.out_dt), 2, const_cast<void*>(e.residual), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              swizzle_enum(kp.out_row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    if (staged) {
+      const size_t per_buf = (size_t)epi_warps(kind) * 32 * kp.out_row_bytes;
+      const size_t extra = perm > 0 ? epi_warps(kind) * (size_t)B8_PARAM_BYTES : 0;
+      auto fits = [&](int bufs, int stages) { return kSmemBudget >= extra + bufs * per_buf + kp.b_resident_bytes + stages * kb_bytes * kp.kpb; };
+      while (kp.kpb > 1 && !fits(3, 2)) kp.kpb /= 2;
+      // From 1 KB of K a row on, the mainloop hides the epilogue but wants the ring: two buffers and three stages instead
+      // (TF32 1x1 512 -> 2048 with a residual, M=1568: 29.0 -> 24.9 us).
+      const bool long_k = (int64_t)cs.K() * es >= 1024;
+      kp.res_bufs = fits(4, 3) ? 4 : (long_k && fits(2, 3) ? 2 : (fits(3, 2) ? 3 : (fits(2, 2) ? 2 : 0)));
+      if (perm > 0 && kp.res_bufs == 0) return fail("no room for the residual's buffers");
+    }
+    layout_smem(kp, bn, kind, pair, &pl->smem);
+    const int64_t ktot = cs.K();
+    const cuuint64_t k_bytes = (cuuint64_t)ktot * es;
+    const cuuint32_t b_rows = (cuuint32_t)(pair ? bn / 2 : bn);  // a CTA of a pair stages its half of the channel tile
+    if (perm > 0) {
+      // [group][8 g + 2 q + e] -> channel (perm / 4) q + 2 g + e of the group
+      cuuint64_t gdim[5] = {(cuuint64_t)ktot, 2, 4, (cuuint64_t)perm / 8, (cuuint64_t)cs.OC / perm};
+      cuuint64_t gstr[4] = {k_bytes, k_bytes * (perm / 4), k_bytes * 2, k_bytes * perm};
+      cuuint32_t box[5] = {(cuuint32_t)cb, 2, 4, (cuuint32_t)perm / 8, b_rows / perm};
+      cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+      rc = g_encode_tiled(&kp.tmB, dtype, 5, const_cast<void*>(w_packed), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    } else {
+      cuuint64_t gdim[2] = {(cuuint64_t)ktot, (cuuint64_t)cs.OC};
+      cuuint64_t gstr[1] = {k_bytes};
+      cuuint32_t box[2] = {(cuuint32_t)cb, b_rows};
+      cuuint32_t estr[2] = {1, 1};
+      rc = g_encode_tiled(&kp.tmB, dtype, 2, const_cast<void*>(w_packed), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_enum(swz),
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+    if (rc != CUDA_SUCCESS) return fail("weight tensor map rejected by the driver");
+  }
   kp.bias_f = e.bias_f;
   kp.slope = e.slope;
   kp.residual = e.residual;
   kp.join_a = e.join_a, kp.join_b = e.join_b, kp.join_c = e.join_c;
+  kp.join_d = e.join_d, kp.join_a8 = e.join_a8, kp.join_b8 = e.join_b8, kp.join_c8 = e.join_c8;
   kp.join_lo = e.join_lo, kp.join_hi = e.join_hi, kp.join_flip = e.join_signed;
   kp.dq_w_scale = e.dq_w_scale;
   kp.dq_x_scale = e.dq_x_scale_dev;
@@ -596,8 +625,6 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   kp.x_zp_dev = e.x_zp_dev;
   kp.combined = e.combined;
   kp.y_zp = e.y_zp;
-  kp.lo = (e.relu_fused && e.lo < 0) ? 0 : e.lo;
-  kp.hi = e.hi;
   kp.out_dt = (int)e.out_dt;
   kp.out = out;
   kp.minmax_keys = e.out_dt == DT::F32 ? e.minmax_keys : nullptr;
@@ -628,7 +655,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   if (kp.splits > 1) snprintf(split_note, sizeof split_note, " splitK=%d", kp.splits);
   else if (kp.res_bufs > 0) snprintf(split_note, sizeof split_note, " residual-buffers=%d", kp.res_bufs);
   snprintf(pl->desc, sizeof pl->desc, "umma_%s M=%lld N=%d K=%lld tile=%dx%dx%dB stages=%dx%d %s%s%s", kname, (long long)M, cs.OC, (long long)cs.K(),
-           pair ? 256 : a_rows, bn, swz, kp.stages, kp.kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? " cta-pair" : (pl->small ? " small" : ""));
+           pair ? 256 : a_rows, bn, swz, kp.stages, kp.kpb, gemm_like ? "tiled" : "im2col", split_note, pair ? (kp.b_perm ? " cta-pair fragments" : " cta-pair") : (pl->small ? " small" : (kp.b_perm ? " fragments" : "")));
   if (pl->small) pl->alone = umma_group_create(&pl, 1);
   return pl;
 }

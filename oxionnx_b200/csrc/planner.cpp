@@ -1254,6 +1254,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       for (int i : c.join_nodes) skipped_[i] = 1;
       epi.join = 1;
       epi.join_a = jc.ca, epi.join_b = jc.cb, epi.join_c = jc.cc, epi.join_lo = jc.lo, epi.join_hi = jc.hi;
+      epi.join_d = jc.d, epi.join_a8 = jc.a8, epi.join_b8 = jc.b8, epi.join_c8 = jc.c8;
       epi.join_signed = V(c.join_other).dt == DT::I8 ? 1 : 0;
       epi.out_dt = c.join_rp.lo < 0.f ? DT::I8 : DT::U8;
       c.res_vi = c.join_other;

@@ -99,6 +99,9 @@ struct alignas(64) KParams {
   // > 0: the layer has one channel tile and its whole packed weight matrix (this many bytes) stays in shared memory
   // in front of the ring for the life of the CTA; ring stages then hold activation blocks only
   uint32_t b_resident_bytes;
+  // > 0: tmB is five-dimensional and brings the weights' rows in the order of the fragment epilogues: of every b_perm
+  // output channels, TMEM column 8 g + 2 q + e holds channel (b_perm / 4) q + 2 g + e
+  int b_perm;
   int small_bn, a_rows;  // small-problem kernel only: the tile's channels, the rows of an activation box
   // epilogue
   int mode;
@@ -112,6 +115,8 @@ struct alignas(64) KParams {
   // even, bounds join_lo .. join_hi; join_flip: the residual's lanes are signed
   float join_a, join_b, join_c;
   int join_lo, join_hi, join_flip;
+  // the same constants for a requantised lane that is scaled to [0, 1] by join_d (see bytes_word)
+  float join_d, join_a8, join_b8, join_c8;
   const float* slope;     // PRelu: per-channel slope, padded like the bias
   int act;
   float clip_lo, clip_hi;
@@ -214,11 +219,21 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const CUtensorM
       "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+               "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+               : "memory");
+}
 // The same loads issued by a CTA of a pair: the data lands in the issuing CTA's shared memory, the bytes are
 // counted on `bar`, a shared::cluster address that names the even CTA's barrier.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
                "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1)
+               : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile("cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+               "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
                : "memory");
 }
 __device__ __forceinline__ void tma_load_im2col_4d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c, int w, int h, int n, uint16_t off_w,
@@ -1176,6 +1191,16 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
   }
 }
 
+}  // namespace umma
+}  // namespace k
+}  // namespace oxb
+
+#include "umma_epilogue8.cuh"
+
+namespace oxb {
+namespace k {
+namespace umma {
+
 // ---- the kernel ---------------------------------------------------------------------------
 // Persistent: one CTA per SM (one pair per two SMs) walks the tile list (channel tile fastest, so
 // CTAs that share an activation tile run together and meet in L2).  The shared-memory ring and the
@@ -1263,7 +1288,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
     // a pair's copies are counted on the even CTA's barrier, which alone announces the bytes of both
     const uint32_t tx_per_kb = PAIR ? 2u * kb_bytes : kb_bytes;
     const bool plain = !p.batched && p.splits == 1;
-    // One copy of the loop per form of the two loads.  B_FORM: 0 resident, 1 through the ring.
+    // One copy of the loop per form of the two loads.  B_FORM: 0 resident, 1 rows in order, 2 in the order of b_perm.
     auto produce = [&](auto im2col_c, auto b_form_c) {
       constexpr bool IM2COL = decltype(im2col_c)::value;
       constexpr int B_FORM = decltype(b_form_c)::value;
@@ -1299,7 +1324,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         const int tile_n = plain ? walk.n : tt % p.n_tiles, tile_m = plain ? walk.m : tt / p.n_tiles;
         const int m0 = tile_m * M_STEP + (PAIR ? pair_rank * BLOCK_M : 0);
         const int oc0 = tile_n * BN + (PAIR ? pair_rank * B_ROWS : 0);
-        const int b_row = b_row0 + oc0;
+        const int b_row = B_FORM == 2 ? oc0 / p.b_perm : b_row0 + oc0;
         if (IM2COL && !plain) pixel = PixelStep(m0, p.Q, p.P);
         const int w_base = pixel.q * p.sw - p.pl, h_base = pixel.p * p.sh - p.pt, n0 = pixel.n;
         int cb = 0, sx = 0, r = 0;
@@ -1326,11 +1351,13 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
             if (PAIR) {
               if (IM2COL) tma_load_im2col_4d_pair(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
               else tma_load_2d_pair(a_dst, &p.tmA, full, a_col0 + c_off, a_row0 + m0);
-              tma_load_2d_pair(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * cb_elems, b_row);
+              if (B_FORM == 2) tma_load_5d_pair(a_dst + a_bytes, &p.tmB, full, (it + g) * cb_elems, 0, 0, 0, b_row);
+              else tma_load_2d_pair(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * cb_elems, b_row);
             } else {
               if (IM2COL) tma_load_im2col_4d(a_dst, &p.tmA, full, c_off, w_base, h_base, n0, (uint16_t)(sx * p.dw), (uint16_t)(r * p.dh));
               else tma_load_2d(a_dst, &p.tmA, full, a_col0 + c_off, a_row0 + m0);
               if (B_FORM == 1) tma_load_2d(a_dst + a_bytes, &p.tmB, full, b_col0 + (it + g) * cb_elems, b_row);
+              else if (B_FORM == 2) tma_load_5d(a_dst + a_bytes, &p.tmB, full, (it + g) * cb_elems, 0, 0, 0, b_row);
             }
             if (++cb == cblocks) {
               cb = 0;
@@ -1348,6 +1375,9 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
       }
     };
     auto with_b = [&](auto im2col_c) {
+      if constexpr (KIND == KIND_I8 && BN >= 64) {
+        if (p.b_perm && !b_res) return produce(im2col_c, std::integral_constant<int, 2>());
+      }
       if constexpr (!PAIR) {
         if (b_res) return produce(im2col_c, std::integral_constant<int, 0>());
       }
@@ -1359,7 +1389,8 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         mbar_expect_tx(smem_u32(&bar_b_resident), p.b_resident_bytes);
         for (int i = 0; i < k_iters; ++i) {
           const uint32_t dst = b_res_base + (uint32_t)i * b_bytes;
-          tma_load_2d(dst, &p.tmB, smem_u32(&bar_b_resident), i * p.cb_elems, 0);
+          if (p.b_perm) tma_load_5d(dst, &p.tmB, smem_u32(&bar_b_resident), i * p.cb_elems, 0, 0, 0, 0);
+          else tma_load_2d(dst, &p.tmB, smem_u32(&bar_b_resident), i * p.cb_elems, 0);
         }
       }
       if (p.a_im2col) with_b(std::true_type());
@@ -1466,14 +1497,31 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
     __syncwarp();
   } else {
     // ---------------- epilogue ----------------
-    const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));
+    const uint32_t warp_bytes = p.b_perm ? (uint32_t)p.res_bufs * B8_RES_BYTES + B8_PARAM_BYTES : (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));
+    const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * warp_bytes;
     const bool split = !p.batched && p.splits > 1;
 #define OXB_EPI(V)                                                                                                                                    \
   case V:                                                                                                                                             \
     if (!PAIR && split) epilogue_role<BN, KIND, V, !PAIR, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, bar_res[warp - 2], stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
     else epilogue_role<BN, KIND, V, false, PAIR>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, bar_res[warp - 2], stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank); \
     break;
-    if constexpr (KIND == KIND_I8) {
+    bool fragment = false;
+    if constexpr (KIND == KIND_I8 && BN >= 64) {
+      fragment = p.b_perm == 64;
+#define OXB_BYTES(F) epilogue_bytes<BN, PAIR, F>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank)
+      if (fragment) {
+        if (p.variant == V_JOIN) {
+          if (p.join_lo == 0) OXB_BYTES(B8_JOIN_RELU);
+          else OXB_BYTES(B8_JOIN);
+        } else {
+          if (p.lo == 0) OXB_BYTES(B8_REQUANT_RELU);
+          else OXB_BYTES(B8_REQUANT);
+        }
+      }
+#undef OXB_BYTES
+    }
+    if (fragment) {
+    } else if constexpr (KIND == KIND_I8) {
       switch (p.variant) {
         OXB_EPI(V_REQUANT)
         OXB_EPI(V_REQUANT_DYN)

@@ -1,0 +1,49 @@
+"""The fragment epilogues of the persistent integer kernel (csrc/umma_epilogue8.cuh): every tile width, ragged rows and
+channel tiles, weights in the ring and resident, every bound of the saturation.  The same layers through the general
+epilogue are the reference; joins with a residual are covered by test_gpu_small_problems.py."""
+import numpy as np
+import pytest
+
+from oxionnx_b200.graph import Graph, Node
+from oxionnx_b200.session import Session
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(graph, weights, feeds, **tuning):
+    sess = Session.builder().with_tuning(**tuning).build_from_graph(graph, weights)
+    out = sess.run(feeds)
+    kernels = [s["kernel"] for s in sess.steps()]
+    sess.close()
+    return out, kernels
+
+
+# batch, channels, height, width, filters, kernel, CTA pairs: one to five channel tiles, the last of them ragged, few and many K blocks
+SHAPES = [(1, 64, 211, 199, 64, 1, "never"), (1, 32, 211, 199, 64, 3, "never"), (1, 256, 150, 151, 128, 1, "never"), (1, 64, 150, 151, 192, 1, "never"),
+          (1, 64, 139, 137, 256, 1, "never"), (1, 128, 139, 137, 320, 1, "never"), (1, 64, 100, 101, 1088, 1, "never"), (2, 64, 61, 43, 320, 3, "always"),
+          (1, 512, 61, 43, 448, 1, "always")]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+@pytest.mark.parametrize("relu, y_zp", [(True, 0), (False, -3), (False, 131)])
+def test_fragment_requantisation_is_the_general_epilogues(shape, relu, y_zp):
+    n, c, h, w, oc, k, pairs = shape
+    rng = np.random.default_rng([n, c, h, oc, k, y_zp + 3])
+    weights = {"w": rng.integers(-127, 128, (oc, c, k, k)).astype(np.float32), "wz": np.zeros(oc, np.float32), "b": rng.integers(-1000, 1001, oc).astype(np.float32),
+               "xs": np.float32([0.02]), "z0": np.float32([0]), "yz": np.int8([y_zp]) if y_zp < 0 else np.uint8([y_zp]), "ys": np.float32([0.35])}
+    # a standard deviation of some sixty lanes: ties, saturation on both sides and everything between
+    spread = 60 * 0.35 / (0.02 * 70 * 40 * np.sqrt(c * k * k))
+    weights["ws"] = (spread * rng.uniform(0.7, 1.4, oc)).astype(np.float32)
+    nodes = [Node("QuantizeLinear", "q", ["x", "xs", "z0"], ["xq"], {}),
+             Node("QLinearConv", "conv", ["xq", "xs", "z0", "w", "ws", "wz", "ys", "yz", "b"], ["yq"], {"pads": [k // 2] * 4})]
+    if relu:
+        nodes.append(Node("Relu", "r", ["yq"], ["yr"], {}))
+    nodes.append(Node("DequantizeLinear", "dq", ["yr" if relu else "yq", "ys", "yz"], ["y"], {}))
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["y"])
+    feeds = {"x": np.abs(rng.standard_normal((n, c, h, w))).astype(np.float32)}
+    got, kernels = _run(graph, weights, feeds, cta_pairs=pairs)
+    assert any("fragments" in s and ("cta-pair" in s) == (pairs == "always") for s in kernels), kernels
+    want, general = _run(graph, weights, feeds, cta_pairs=pairs, requant_f64=1)
+    assert not any("fragments" in s for s in general), general
+    assert np.array_equal(got["y"], want["y"]), f"{np.sum(got['y'] != want['y'])} of {want['y'].size} lanes differ"
+    assert np.unique(want["y"]).size > 100, "degenerate test vector"
