@@ -3494,10 +3494,9 @@ void Planner::match_join(Contraction& c) {
     }
     return true;
   };
-  // A short K over a tensor that does not stay in L2 keeps the join a pass of its own: that pass runs at the memory's
-  // rate, while here the join doubles the instructions of an epilogue that already bounds the layer (1x1 64 -> 256 at
-  // M = 3211264: 788 us joined, 334 + 407 apart; 1x1 128 -> 512 at M = 802816: 352 joined, 178 + 207 apart).
-  if (c.cs.K() < 128 && prod(c.out_shape) > (64ll << 20)) return;
+  // Taken at every K and size: with the fragment epilogue the join costs a layer less than its own pass over memory even
+  // where both are bound by their epilogue and nothing stays in L2 (1x1 64 -> 256 at M = 3211264: 497 us joined, 228 + 413
+  // apart; at M = 802816 129 joined, 62 + 105 apart).
   k::ResidualParams rp{};
   bool has_zp;
   const int dq_i = only_consumer(c.out_name);
