@@ -187,7 +187,7 @@ void layout_smem(KParams& kp, int bn, int kind, bool pair, size_t* smem_total) {
   const size_t resident = kp.b_resident_bytes;
   const size_t kb_bytes = (size_t)(BLOCK_M + (resident ? 0 : (pair ? bn / 2 : bn))) * kp.swizzle_bytes;
   const size_t stage_bytes = kb_bytes * kp.kpb;
-  const size_t staging = kp.b_perm ? ew * (kp.res_bufs * (size_t)B8_RES_BYTES + B8_PARAM_BYTES)
+  const size_t staging = kp.b_perm ? ew * (kp.res_bufs * (size_t)B8_RES_BYTES + FRAG_PARAM_BYTES)
                                    : (kp.out_tma ? (size_t)ew * 32 * kp.out_row_bytes * std::max(kp.res_bufs, 1) : 0);
   // one persistent CTA per SM: the ring may use most of the shared memory and runs on across tiles
   const size_t budget = std::min<size_t>(192 * 1024, kSmemBudget - staging) - resident;
@@ -238,10 +238,10 @@ void layout_small(SmallShape& c, int swz) {
 
 // Tile width and slices by a model fitted to sweeps of both over sixteen layer shapes: 3 us from one layer to the next,
 // 0.12 us per K block that the ring holds, 1.7 us over the ring's depth per block beyond it, 0.7 us per further
-// 32-channel run a warp finishes, 1.1 us for the slices' meeting.  Clusters are placed whole, beside those of the layer
+// 32-channel run a warp finishes (run_us), 1.1 us for the slices' meeting.  Clusters are placed whole, beside those of the layer
 // before and behind: with more than 148 / 128 / 64 CTAs in clusters of 2 / 4 / 8 some wait for a place (3x3 512 at 7x7,
 // i8: 5.9 us with 64 CTAs in clusters of 4, 15.6 us with 128 in clusters of 8).
-SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, int max_split) {
+SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, int max_split, double run_us) {
   SmallShape best;
   const int64_t m_tiles = ceil_div(M, BLOCK_M);
   for (int bn : {32, 64, 128}) {
@@ -263,7 +263,7 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
       const double ring = c.stages * c.kpb;
       const double share = ctas > sms ? 2.0 : 1.0;  // CTAs of this layer on one SM
       c.us = 3.0 + share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring)) +
-             0.7 * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
+             run_us * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (run_us - 0.7) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
       if (best.bn == 0 || c.us < best.us) best = c;
     }
   }
@@ -335,7 +335,10 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // tile costs the producer and issuer warps, whose 0.7 us a tile of little K only partly overlap: a 1x1 64 -> 256 layer
     // at M = 802816 takes 3.0 us per round of 128 x 256 tiles, 1.05 us per round of 128 x 64 tiles, 0.84 us per round of
     // 128 x 32)
-    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : 0.07e-9;
+    // with a Gelu behind it 0.2 ns (and 2.5 us for a run of the small-problem kernel), which moves M = 8192 N = 3072 K = 768
+    // from 6 rounds of 256 columns to 11 of 128 (61.5 -> 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us)
+    const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
+    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.07e-9);
     const double t_tile_fixed = 0.5e-6;
     const int max_split = tune.split_k_max > 0 ? tune.split_k_max : 8;
     double best = 1e30;
@@ -361,7 +364,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
     // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
     if (tune.cta_pairs != 2) {
-      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split);
+      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split, gelu ? 2.5 : 0.7);
       if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
       if (small.bn > 0) {
         bn = small.bn;
@@ -551,11 +554,12 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     kp.stage_off = (uint32_t)(small.stages * small.stage_bytes);
     pl->smem = small.smem;
   } else {
-    // 8-bit outputs of whole groups of 64 channels take the fragment epilogue (umma_epilogue8.cuh) wherever its arithmetic
-    // is allowed: it is the faster one at every K (the figures stand there).
-    const bool bytes_ok = kind == KIND_I8 && bn >= 64 && cs.OC % 64 == 0 && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0;
+    // Whole groups of 64 channels, as 8-bit outputs or dequantised, take the fragment epilogues (umma_epilogue8.cuh) wherever
+    // their arithmetic is allowed: they are the faster ones at every K (the figures stand there).
+    const bool frag_ok = kind == KIND_I8 && bn >= 64 && cs.OC % 64 == 0 && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0;
     const bool join_ok = kp.variant == V_JOIN && e.join_d > 0.f && kp.hi - kp.lo == 255;
-    const int perm = bytes_ok && (kp.variant == V_REQUANT_PACKED || join_ok) ? 64 : 0;
+    const bool floats_ok = kp.variant >= V_DEQUANT && kp.variant < V_DEQUANT + 4;  // not the tanh form of Gelu
+    const int perm = !frag_ok ? 0 : (kp.variant == V_REQUANT_PACKED || join_ok ? 64 : (floats_ok ? 16 : 0));
     kp.b_perm = perm;
     if (perm > 0) {
       kp.out_tma = 0;
@@ -575,7 +579,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     }
     if (staged) {
       const size_t per_buf = (size_t)epi_warps(kind) * 32 * kp.out_row_bytes;
-      const size_t extra = perm > 0 ? epi_warps(kind) * (size_t)B8_PARAM_BYTES : 0;
+      const size_t extra = perm > 0 ? epi_warps(kind) * (size_t)FRAG_PARAM_BYTES : 0;
       auto fits = [&](int bufs, int stages) { return kSmemBudget >= extra + bufs * per_buf + kp.b_resident_bytes + stages * kb_bytes * kp.kpb; };
       while (kp.kpb > 1 && !fits(3, 2)) kp.kpb /= 2;
       // From 1 KB of K a row on, the mainloop hides the epilogue but wants the ring: two buffers and three stages instead

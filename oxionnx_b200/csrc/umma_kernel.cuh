@@ -340,6 +340,19 @@ __device__ __forceinline__ uint32_t float_order_key(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// Merges what the threads of a warp have written into the ordered keys of the output's extrema.
+__device__ __forceinline__ void merge_extrema(const KParams& p, int lane, float seen_min, float seen_max) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    seen_min = fminf(seen_min, __shfl_xor_sync(0xffffffffu, seen_min, off));
+    seen_max = fmaxf(seen_max, __shfl_xor_sync(0xffffffffu, seen_max, off));
+  }
+  if (lane == 0) {
+    if (seen_min != INFINITY) atomicMin(p.minmax_keys, float_order_key(seen_min));
+    if (seen_max != -INFINITY) atomicMax(p.minmax_keys + 1, float_order_key(seen_max));
+  }
+}
+
 // ---- fused epilogue math ------------------------------------------------------------------
 // One variant per (mode, activation, rounding) combination, chosen once per kernel, so that
 // the 32 per-channel computations inside are straight-line code with full instruction-level
@@ -1178,17 +1191,7 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
     }
   }
   if (p.out_tma && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  if (track) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      seen_min = fminf(seen_min, __shfl_xor_sync(0xffffffffu, seen_min, off));
-      seen_max = fmaxf(seen_max, __shfl_xor_sync(0xffffffffu, seen_max, off));
-    }
-    if (lane == 0) {
-      if (seen_min != INFINITY) atomicMin(p.minmax_keys, float_order_key(seen_min));
-      if (seen_max != -INFINITY) atomicMax(p.minmax_keys + 1, float_order_key(seen_max));
-    }
-  }
+  if (track) merge_extrema(p, lane, seen_min, seen_max);
 }
 
 }  // namespace umma
@@ -1497,7 +1500,7 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
     __syncwarp();
   } else {
     // ---------------- epilogue ----------------
-    const uint32_t warp_bytes = p.b_perm ? (uint32_t)p.res_bufs * B8_RES_BYTES + B8_PARAM_BYTES : (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));
+    const uint32_t warp_bytes = p.b_perm ? (uint32_t)p.res_bufs * B8_RES_BYTES + FRAG_PARAM_BYTES : (uint32_t)(32 * p.out_row_bytes * (p.res_bufs > 0 ? p.res_bufs : 1));
     const uint32_t stage_addr = ((smem_u32(smem_raw) + 1023u) & ~1023u) + p.stage_off + (uint32_t)(warp - 2) * warp_bytes;
     const bool split = !p.batched && p.splits > 1;
 #define OXB_EPI(V)                                                                                                                                    \
@@ -1519,6 +1522,17 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         }
       }
 #undef OXB_BYTES
+#define OXB_FLOATS(D, G) epilogue_floats<BN, PAIR, D, G>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank)
+      if (p.b_perm == 16) {
+        fragment = true;
+        switch (p.variant) {
+          case V_DEQUANT: OXB_FLOATS(false, false); break;
+          case V_DEQUANT + 1: OXB_FLOATS(true, false); break;
+          case V_DEQUANT + 2: OXB_FLOATS(false, true); break;
+          default: OXB_FLOATS(true, true); break;
+        }
+      }
+#undef OXB_FLOATS
     }
     if (fragment) {
     } else if constexpr (KIND == KIND_I8) {

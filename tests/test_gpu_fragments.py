@@ -47,3 +47,32 @@ def test_fragment_requantisation_is_the_general_epilogues(shape, relu, y_zp):
     assert not any("fragments" in s for s in general), general
     assert np.array_equal(got["y"], want["y"]), f"{np.sum(got['y'] != want['y'])} of {want['y'].size} lanes differ"
     assert np.unique(want["y"]).size > 100, "degenerate test vector"
+
+
+# rows, K, outputs
+LINEARS = [(20001, 64, 192, False), (4099, 256, 1088, True), (9001, 768, 320, False), (20001, 32, 64, True), (20001, 768, 256, False)]
+
+
+@pytest.mark.parametrize("rows, k, n, gelu", LINEARS)
+@pytest.mark.parametrize("pairs", ["never", "always"])
+def test_fragment_dequantisation_is_the_separate_nodes(rows, k, n, gelu, pairs):
+    if pairs == "always" and n < 256:
+        pytest.skip("a pair shares a 256-wide tile")
+    rng = np.random.default_rng([rows, k, n])
+    w = {"w": np.clip(np.rint(rng.standard_normal((k, n)) * 40.0), -127, 127).astype(np.float32),
+         "ws": rng.uniform(0.0005, 0.002, n).astype(np.float32), "bias": (rng.standard_normal(n) * 0.5 + 0.8).astype(np.float32)}
+    nodes = [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {}),
+             Node("MatMulInteger", "mmi", ["xq", "w", "xz"], ["acc"], {}), Node("Cast", "cast", ["acc"], ["accf"], {"to": 1}),
+             Node("Mul", "scales", ["xs", "ws"], ["sc"], {}), Node("Mul", "rescale", ["accf", "sc"], ["scaled"], {}),
+             Node("Add", "addb", ["scaled", "bias"], ["lin"], {})]
+    if gelu:
+        nodes.append(Node("Gelu", "act", ["lin"], ["act_out"], {}))
+    last = nodes[-1].outputs[0]
+    nodes.append(Node("DynamicQuantizeLinear", "q1", [last], ["yq", "ys", "yz"], {}))
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=[last, "yq", "ys", "yz"])
+    feeds = {"x": (rng.standard_normal((rows, k)) * 2 + 0.3).astype(np.float32)}
+    got, kernels = _run(graph, w, feeds, cta_pairs=pairs)
+    assert any("fragments +dequant" in s and ("cta-pair" in s) == (pairs == "always") for s in kernels), kernels
+    want, _ = _run(graph, w, feeds, keep_intermediates=True)
+    for name in graph.output_names:
+        assert np.array_equal(got[name], want[name]), name
