@@ -262,7 +262,11 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
       if (ctas > sms && c.smem > 112 * 1024) continue;
       const double ring = c.stages * c.kpb;
       const double share = ctas > sms ? 2.0 : 1.0;  // CTAs of this layer on one SM
-      c.us = 3.0 + share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring)) +
+      double k_us = share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring));
+      // with most SMs at it L2 feeds one no faster than in the persistent kernel (i8 M = 7252 N = 256 K = 2304: 20.6 us here,
+      // 17 us there)
+      if (ctas > 96) k_us = std::max(k_us, share * c.k_per * (c.a_rows + bn) * swz / 110e3);
+      c.us = 3.0 + k_us +
              run_us * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (run_us - 0.7) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
       if (best.bn == 0 || c.us < best.us) best = c;
     }
@@ -311,16 +315,18 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   if (e.join && (!e.residual || !e.bias_if || dt_size(e.out_dt) != 1 || cs.OC % 32 != 0)) return no("the join needs an 8-bit residual, the float bias and whole channel runs");
   if (e.mode == EPI_F32 && e.act == 4 && e.slope == nullptr) return no("the PRelu epilogue needs a (padded) slope vector");
 
-  // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles
-  // of the tensor pipe but cannot be issued faster than one per ~56 cycles; one SM fills its
-  // shared memory from L2 at about 95 GB/s when all SMs do so; the fused epilogue costs about
-  // 0.07 ns per output for requantisation and 0.03 ns for the float variants, plus a fixed cost per tile.  The three overlap
-  // (ring of stages, two accumulators), so a tile takes the longest of them, the kernel runs
-  // ceil(tiles / SMs) rounds of tiles, and the last tile's epilogue is not hidden.  Pick the
-  // width that minimises that estimate; ties go to the wider tile (fewer re-reads of the activations).
-  // Split K: when even the narrowest useful tiling leaves most SMs without a tile and K is long, `splits`
-  // CTAs share a (wider) tile, each running a slice of K; the slices meet in an L2-resident workspace.  It is
-  // only considered when every slice gets its own SM in one round and at least eight K blocks.
+  // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles of the tensor pipe but
+  // cannot be issued faster than one per ~56 cycles; one SM fills its shared memory from L2 at about 110 GB/s when all
+  // SMs do so; the epilogue has its cost per output and a tile one of its own (below).  The three overlap (ring of stages,
+  // two accumulators), so a tile takes the longest of them, the kernel runs ceil(tiles / SMs) rounds of tiles, and the
+  // last tile's epilogue is not hidden.  Pick the width that minimises that estimate; ties go to the wider tile (fewer
+  // re-reads of the activations).  Fitted to sweeps of width and slices over some thirty layer shapes, where the choice
+  // is within 1 us of the best one but for two of them.
+  // Split K: when few tiles leave most SMs without one and K is long, `splits` CTAs share a tile, each running a slice of
+  // K; the slices meet in an L2-resident workspace, for 1 us and 0.35 us per MB of it (TF32 M = 1568 N = 512 K = 2048:
+  // four slices of 256 columns 3 us faster than 104 tiles of 64; K = 4608: five slices 14 us faster than 52 tiles of 128).
+  // Only with an SM of its own for every slice, at least eight K blocks each, and some SMs to spare: 147 slices on 148 SMs
+  // met 10 us later than that (M = 6272 N = 256, K = 1024 and 2304 alike).
   const int device = current_device();
   const int sms = sm_count(device);
   const int64_t m_tiles = ceil_div(M, BLOCK_M);
@@ -331,28 +337,23 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   {
     const double k_bytes = (double)cs.K() * es;
     const double k_steps = k_bytes / 32.0;
-    // epilogue: per output 0.07 ns requantised / 0.03 ns float, plus about 0.5 us per tile whatever its width (what a
-    // tile costs the producer and issuer warps, whose 0.7 us a tile of little K only partly overlap: a 1x1 64 -> 256 layer
-    // at M = 802816 takes 3.0 us per round of 128 x 256 tiles, 1.05 us per round of 128 x 64 tiles, 0.84 us per round of
-    // 128 x 32)
+    // epilogue: per output 0.045 ns for integers, 0.03 ns float, plus 0.25 us per tile whatever its width;
     // with a Gelu behind it 0.2 ns (and 2.5 us for a run of the small-problem kernel), which moves M = 8192 N = 3072 K = 768
     // from 6 rounds of 256 columns to 11 of 128 (61.5 -> 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us)
     const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
-    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.07e-9);
-    const double t_tile_fixed = 0.5e-6;
+    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.045e-9);
+    const double t_tile_fixed = 0.25e-6;
     const int max_split = tune.split_k_max > 0 ? tune.split_k_max : 8;
     double best = 1e30;
     for (int cand = bn_max; cand >= 32; cand /= 2) {
       const double tiles = (double)m_tiles * (double)ceil_div(cs.OC, cand);
       for (int sp = 1; sp <= max_split; ++sp) {
-        if (sp > 1 && (tiles * sp > sms || k_iters_host / sp < 8)) break;
+        if (sp > 1 && (tiles * sp > 0.92 * sms || k_iters_host / sp < 8)) break;
         const double rounds = std::ceil(tiles * sp / sms);
         const double t_mma = k_steps * std::max(56.0, cand / 2.0) / 1.965e9 / sp;
-        const double t_feed = (double)(BLOCK_M + cand) * k_bytes / 95e9 / sp;
+        const double t_feed = (double)(BLOCK_M + cand) * k_bytes / 110e9 / sp;
         const double t_epi = (double)BLOCK_M * cand * ns_out + t_tile_fixed;
-        // measured: a split launch costs about 10 us more than an unsplit one before its first K block pays
-        // back (the slices' accumulators go through the workspace, and the finishing epilogues are not overlapped)
-        const double t_split = sp > 1 ? 10e-6 : 0.0;
+        const double t_split = sp > 1 ? 1e-6 + 0.35e-12 * tiles * sp * BLOCK_M * cand * 4.0 : 0.0;
         const double t = rounds * std::max(t_mma, std::max(t_feed, t_epi)) + t_epi + t_split;
         if (t < best * 0.97) {
           best = t;
@@ -364,7 +365,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
     // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
     if (tune.cta_pairs != 2) {
-      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split, gelu ? 2.5 : 0.7);
+      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split, gelu && M > 32 ? 2.5 : 0.7);
       if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
       if (small.bn > 0) {
         bn = small.bn;

@@ -88,8 +88,8 @@ struct alignas(64) KParams {
   int a_rb, a_rh, a_ch, b_rb, b_rh, b_ch, o_rb, o_rh, o_ch;
   // split K (few output tiles, long K): work item t is (tile t / splits, slice t % splits); slice s runs K
   // blocks [s * k_per, (s + 1) * k_per) and leaves its raw accumulators in ws[tile][s][128 x BN]; per run of an
-  // epilogue warp, the slice that arrives last (ws_count) adds the slices in order 0 .. splits-1 and runs the
-  // fused epilogue.  Nobody waits for anybody, and the sum does not depend on the arrival order.  Counters are
+  // epilogue warp, the run's owner or the slice that arrives last (ws_count) adds the slices in order 0 .. splits-1 and
+  // runs the fused epilogue.  Nobody waits for anybody, and the sum does not depend on the arrival order.  Counters are
   // kept per tile, epilogue warp and 32-channel run.
   int splits, k_per;
   uint32_t* ws;
@@ -1107,50 +1107,94 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
       continue;
     }
     if constexpr (SPLIT) {
-      // Runs are taken in an order rotated by the slice index and each run has its own arrival counter, so the
-      // slices of a tile finish different runs last and share the summing and the fused epilogue between them.
+      // Every run of the tile has an owner among the slices.  A slice first publishes the runs it does not own (all of them
+      // behind one fence, then one arrival at each run's counter), then turns to its own: when every other slice has
+      // published such a run by then, it adds them to its own accumulators straight from tensor memory; after a short
+      // patience it publishes the run itself instead, and whoever arrives last finishes it.  So nobody waits for a slice
+      // that may not be running, but slices that end together share the finishing and write no more than they must.
       constexpr bool kFloatAcc = VARIANT < V_REQUANT;
       const int split = t - tt * p.splits;
       // workspace of one slice: [lane quarter][run][16-byte piece j][lane], so that every store and load of a
       // warp covers 512 contiguous bytes (only warps with the same index in the other slices read it back)
       const uint4* tile_ws = reinterpret_cast<const uint4*>(p.ws + (size_t)tt * p.splits * (BLOCK_M * BN)) + (size_t)quarter * (BN / 32) * 256 + lane;
       constexpr size_t kSlice = (size_t)BLOCK_M * BN / 4;  // 16-byte pieces per slice
-      uint4* mine = const_cast<uint4*>(tile_ws) + (size_t)split * kSlice;
       unsigned int* counters = p.ws_count + ((size_t)tt * EW + ew) * 4;
       const int runs = end - first;
-      for (int i = 0; i < runs; ++i) {
-        const int c = first + (i + split) % runs;
+      auto own = [&](int c) { return (c + quarter) % p.splits == split; };
+      const bool counts = lane < runs, counts_own = counts && own(first + lane);
+      auto publish = [&](int c) {
+        uint4* mine = const_cast<uint4*>(tile_ws) + (size_t)split * kSlice + c * 256;
         tmem_ld32_nowait(taddr + (uint32_t)c * 32u, va);
-        tmem_ld_wait();
-        if (i == runs - 1) release();
+        tmem_ld_wait_for(va);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) __stcg(mine + (c * 8 + j) * 32, make_uint4(va[4 * j], va[4 * j + 1], va[4 * j + 2], va[4 * j + 3]));
+        for (int j = 0; j < 8; ++j) __stcg(mine + j * 32, make_uint4(va[4 * j], va[4 * j + 1], va[4 * j + 2], va[4 * j + 3]));
+      };
+      // what has been published before is visible before the arrival; the runs of `who` for which this slice is the last
+      auto arrive = [&](bool who) -> uint32_t {
         __threadfence();
         __syncwarp();
-        unsigned int arrived = 0;
-        if (lane == 0) arrived = atomicAdd(counters + (c - first), 1u);
-        arrived = __shfl_sync(0xffffffffu, arrived, 0);
-        if (arrived != (unsigned int)p.splits - 1u) continue;  // a later slice finishes this run
-        if (lane == 0) counters[c - first] = 0u;               // ready for the next launch
-        __threadfence();
-        for (int sl = 0; sl < p.splits; ++sl) {
-          const uint4* src = tile_ws + (size_t)sl * kSlice + c * 256;
-          uint4 xv[8];  // the eight loads of a slice are issued together
+        const bool last = who && atomicAdd(counters + lane, 1u) == (unsigned int)p.splits - 1u;
+        return __ballot_sync(0xffffffffu, last);
+      };
+      auto finish = [&](int c, bool from_tmem) {
+        auto add = [&](const uint32_t(&xv)[32], bool begin) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) xv[j] = __ldcg(src + j * 32);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t xs[4] = {xv[j].x, xv[j].y, xv[j].z, xv[j].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if (sl == 0) va[4 * j + e] = xs[e];
-              else if (kFloatAcc) va[4 * j + e] = __float_as_uint(__fadd_rn(__uint_as_float(va[4 * j + e]), __uint_as_float(xs[e])));
-              else va[4 * j + e] += xs[e];
-            }
+          for (int j = 0; j < 32; ++j) {
+            if (begin) va[j] = xv[j];
+            else if (kFloatAcc) va[j] = __float_as_uint(__fadd_rn(__uint_as_float(va[j]), __uint_as_float(xv[j])));
+            else va[j] += xv[j];
           }
+        };
+        auto fetch = [&](int sl, uint32_t(&xv)[32]) {
+          if (from_tmem && sl == split) {
+            tmem_ld32_nowait(taddr + (uint32_t)c * 32u, xv);
+            tmem_ld_wait_for(xv);
+            return;
+          }
+          const uint4* src = tile_ws + (size_t)sl * kSlice + c * 256;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {  // the loads of a slice are issued together
+            const uint4 x = __ldcg(src + j * 32);
+            xv[4 * j] = x.x, xv[4 * j + 1] = x.y, xv[4 * j + 2] = x.z, xv[4 * j + 3] = x.w;
+          }
+        };
+        // in the order 0 .. splits - 1 whoever finishes; the float kinds have the registers for two slices at a time
+        constexpr int AT_ONCE = KIND == KIND_I8 ? 1 : 2;
+#pragma unroll 1
+        for (int sl = 0; sl < p.splits; sl += AT_ONCE) {
+          uint32_t xv[32], yv[32];
+          const bool second = AT_ONCE == 2 && sl + 1 < p.splits;
+          fetch(sl, xv);
+          if (second) fetch(sl + 1, yv);
+          add(xv, sl == 0);
+          if (second) add(yv, false);
         }
         emit(va, c);
+      };
+#pragma unroll 1
+      for (int c = first; c < end; ++c)
+        if (!own(c)) publish(c);
+      uint32_t to_finish = arrive(counts && !counts_own);
+      uint32_t owned = __ballot_sync(0xffffffffu, counts_own), ready = 0u;
+#pragma unroll 1
+      for (int patience = 0; patience < 32 && ready != owned; ++patience) {
+        unsigned int seen = 0u;
+        if (counts_own) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counters + lane) : "memory");
+        ready = __ballot_sync(0xffffffffu, counts_own && seen == (unsigned int)p.splits - 1u);
       }
+      owned &= ~ready;
+      if (owned != 0u) {
+#pragma unroll 1
+        for (int c = first; c < end; ++c)
+          if ((owned >> (c - first)) & 1u) publish(c);
+        to_finish |= arrive(counts && ((owned >> lane) & 1u) != 0u);
+      }
+      __threadfence();
+      if (counts && (((to_finish | ready) >> lane) & 1u) != 0u) counters[lane] = 0u;  // nobody arrives there any more: ready for the next launch
+#pragma unroll 1
+      for (int c = first; c < end; ++c)
+        if (((to_finish | ready) >> (c - first)) & 1u) finish(c, ((ready >> (c - first)) & 1u) != 0u);
+      release();
     } else {
       // One copy of the run's code in the loop, each run reading its own accumulator columns first.  Starting the
       // next run's TMEM read under this run's store was measured and is slower (102.6 us against 96.7 us on a 1x1
