@@ -10,8 +10,10 @@
 // have left; the second product reads it from there.  Q and K are column windows of their [B * S, H * D]
 // matrices, V arrives transposed per head ([B * H * D, S]), the context is stored by TMA straight into its (possibly
 // head-merged) matrix.  One warp loads and issues; sixteen warps do the rows, four threads per row (32 scores each,
-// the row's maximum and sum meet in shared memory behind two mbarriers); a CTA walks the (batch, head) items and
-// loads the next item's operands as soon as the current product has read them.  Every wait is bounded.
+// the row's maximum and sum meet in shared memory behind two mbarriers of those four warps); a CTA walks the (batch, head) items and
+// loads the next item's operands as soon as the current product has read them.  The scores of the next item and the context
+// of the one before are computed while the row warps are at an item (two tiles of each in TMEM), so that an item costs the
+// row warps' own work and not the chain of both products, their barriers and the store.  Every wait is bounded.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -46,7 +48,7 @@ struct alignas(64) AttnParams {
 
 __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_qk, bar_v, bar_s, bar_p, bar_o, bar_max, bar_sum;
+  __shared__ __align__(8) uint64_t bar_qk, bar_v, bar_s[2], bar_p, bar_o, bar_max[4], bar_sum[4];
   __shared__ float row_max[4][ATT_S], row_sum[4][ATT_S];  // per column block of 32 scores
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
@@ -58,22 +60,26 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
     abort_flag = 0;
     mbar_init(smem_u32(&bar_qk), 1);
     mbar_init(smem_u32(&bar_v), 1);
-    mbar_init(smem_u32(&bar_s), 1);
-    mbar_init(smem_u32(&bar_p), 32 * ATT_ROW_WARPS);
+    mbar_init(smem_u32(&bar_s[0]), 1);
+    mbar_init(smem_u32(&bar_s[1]), 1);
+    mbar_init(smem_u32(&bar_p), ATT_ROW_WARPS);  // one arrival per warp: 512 on one word take longer than the exponentials
     mbar_init(smem_u32(&bar_o), 1);
-    mbar_init(smem_u32(&bar_max), 32 * ATT_ROW_WARPS);
-    mbar_init(smem_u32(&bar_sum), 32 * ATT_ROW_WARPS);
+    for (int q = 0; q < 4; ++q) {  // the four warps that share 32 rows
+      mbar_init(smem_u32(&bar_max[q]), 4);
+      mbar_init(smem_u32(&bar_sum[q]), 4);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == ATT_ROW_WARPS) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(256) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_s = tmem_base_slot, tmem_o = tmem_base_slot + 128u;
+  // two score tiles and two contexts: item i of a CTA uses number i & 1 of each
+  const uint32_t tmem_s = tmem_base_slot, tmem_o = tmem_base_slot + 256u;
   pdl_enter();
   auto give_up = [&](int code) {
     if (!*abortp) {
@@ -96,58 +102,57 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
       mbar_expect_tx(smem_u32(&bar_v), 32768u);
       for (int kb = 0; kb < 4; ++kb) tma_load_2d(base + ATT_V_OFF + (uint32_t)kb * 8192u, &p.tmV, smem_u32(&bar_v), kb * 32, item * ATT_D);
     };
-    if (lane == 0 && (int)blockIdx.x < p.items) {
+    // One elected thread.  While the row warps are at item i, the scores of item i + 1 are computed into the other tile; the
+    // barriers' phases cannot run away from a waiter: scores i + 2 follow the probabilities of item i, which every row warp
+    // hands over after it has seen scores i, and context i follows the row warps' wait for context i - 1.
+    if (elect_one() && (int)blockIdx.x < p.items) {
+      const uint64_t desc = make_smem_desc(0, 128);
+      auto wait = [&](uint64_t& bar, uint32_t parity, int code) {
+        if (mbar_wait(smem_u32(&bar), parity, abortp)) return true;
+        give_up(code);
+        return false;
+      };
+      auto product = [&](uint32_t d, uint32_t a_off, uint32_t b_off, uint32_t b_block, int blocks, uint32_t idesc) {
+        for (int kb = 0; kb < blocks; ++kb) {
+          const uint64_t da = desc | (((base + a_off + (uint32_t)kb * 16384u) >> 4) & 0x3fffu), db = desc | (((base + b_off + (uint32_t)kb * b_block) >> 4) & 0x3fffu);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) tc_mma_one<KIND_TF32>(d, da + 2 * k, db + 2 * k, idesc, kb + k > 0 ? 1u : 0u);
+        }
+      };
       load_qk((int)blockIdx.x);
       load_v((int)blockIdx.x);
-    }
-    __syncwarp();
-    const uint64_t desc_rest = make_smem_desc(0, 128);
-    const uint32_t desc_hi = (uint32_t)(desc_rest >> 32), desc_lo = (uint32_t)desc_rest;
-    uint32_t phase = 0;
-    for (int item = (int)blockIdx.x; item < p.items; item += (int)gridDim.x, phase ^= 1u) {
-      const int next = item + (int)gridDim.x;
-      bool got = mbar_wait(smem_u32(&bar_qk), phase, abortp);
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) give_up(31);
-        break;
+      bool ok = wait(bar_qk, 0u, 31);
+      if (ok) {
+        tc_fence_after();
+        product(tmem_s, ATT_Q_OFF, ATT_K_OFF, 16384u, 2, p.idesc_s);
+        tc_commit<false>(smem_u32(&bar_s[0]));
       }
-      tc_fence_after();
-      if (lane == 0) {
-        for (int kb = 0; kb < 2; ++kb)
-          tc_mma_block<KIND_TF32, false>(tmem_s, desc_lo | (((base + ATT_Q_OFF + (uint32_t)kb * 16384u) >> 4) & 0x3fffu),
-                                         desc_lo | (((base + ATT_K_OFF + (uint32_t)kb * 16384u) >> 4) & 0x3fffu), desc_hi, p.idesc_s, kb > 0 ? 1u : 0u, 4u);
-        tc_commit<false>(smem_u32(&bar_s));
-      }
-      __syncwarp();
-      got = mbar_wait(smem_u32(&bar_s), phase, abortp);  // Q and K have been read
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) give_up(32);
-        break;
-      }
-      if (lane == 0 && next < p.items) load_qk(next);
-      __syncwarp();
-      got = mbar_wait(smem_u32(&bar_p), phase, abortp);  // the probabilities are in shared memory
-      got = mbar_wait(smem_u32(&bar_v), phase, abortp) && got;
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) give_up(33);
-        break;
-      }
-      tc_fence_after();
-      if (lane == 0) {
-        for (int kb = 0; kb < 4; ++kb)
-          tc_mma_block<KIND_TF32, false>(tmem_o, desc_lo | (((base + ATT_P_OFF + (uint32_t)kb * 16384u) >> 4) & 0x3fffu),
-                                         desc_lo | (((base + ATT_V_OFF + (uint32_t)kb * 8192u) >> 4) & 0x3fffu), desc_hi, p.idesc_o, kb > 0 ? 1u : 0u, 4u);
+      uint32_t i = 0;
+      for (int item = (int)blockIdx.x; item < p.items && ok; item += (int)gridDim.x, ++i) {
+        const int next = item + (int)gridDim.x;
+        ok = wait(bar_s[i & 1u], (i >> 1) & 1u, 32);  // Q and K have been read
+        if (!ok) break;
+        if (next < p.items) load_qk(next);
+        if (i > 0) {
+          ok = wait(bar_o, (i - 1u) & 1u, 34);  // V and the probabilities of the item before have been read
+          if (!ok) break;
+          load_v(item);
+        }
+        if (next < p.items) {
+          ok = wait(bar_qk, (i + 1u) & 1u, 31);
+          if (!ok) break;
+          tc_fence_after();
+          product(tmem_s + 128u * ((i + 1u) & 1u), ATT_Q_OFF, ATT_K_OFF, 16384u, 2, p.idesc_s);
+          tc_commit<false>(smem_u32(&bar_s[(i + 1u) & 1u]));
+        }
+        ok = wait(bar_p, i & 1u, 33) && wait(bar_v, i & 1u, 33);  // the probabilities are in shared memory
+        if (!ok) break;
+        tc_fence_after();
+        product(tmem_o + 64u * (i & 1u), ATT_P_OFF, ATT_V_OFF, 8192u, 4, p.idesc_o);
         tc_commit<false>(smem_u32(&bar_o));
       }
-      __syncwarp();
-      got = mbar_wait(smem_u32(&bar_o), phase, abortp);  // V and the probabilities have been read
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) give_up(34);
-        break;
-      }
-      if (lane == 0 && next < p.items) load_v(next);
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // ---------------- 32 scores of one row per thread; four threads share a row through shared memory ----------------
     const int quarter = warp & 3, cb = warp >> 2;
@@ -158,19 +163,59 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
     // context staging of this warp (the warps of column blocks 0 and 1 write the context): 32 rows x 128 bytes
     const uint32_t stage = base + ATT_O_OFF + (uint32_t)((cb & 1) * 4 + quarter) * 4096u;
     uint8_t* stage_ptr = base_ptr + ATT_O_OFF + ((cb & 1) * 4 + quarter) * 4096;
-    uint32_t phase = 0;
-    for (int item = (int)blockIdx.x; item < p.items; item += (int)gridDim.x, phase ^= 1u) {
+    // 32 context lanes of the row of item number i, done: staged (swizzled as the store's tensor map expects), stored by TMA
+    auto store_context = [&](int item, uint32_t i) {
       const int b = item / p.heads, h = item - b * p.heads;
-      bool got = mbar_wait(smem_u32(&bar_s), phase, abortp);
+      uint32_t r[32];
+      tmem_ld32_nowait(tmem_o + 64u * (i & 1u) + lane_base + (uint32_t)cb * 32u, r);
+      tmem_ld_wait_for(r);
+      tc_fence_before();
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous store has read the staging rows
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        *reinterpret_cast<uint4*>(stage_ptr + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+        if (p.minmax_keys) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            seen_min = fminf(seen_min, __uint_as_float(r[4 * c + e]));
+            seen_max = fmaxf(seen_max, __uint_as_float(r[4 * c + e]));
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&p.tmO, stage, h * p.o_ch + cb * 32, b * p.o_rb + h * p.o_rh + quarter * 32);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      }
+    };
+    auto wait_context = [&](uint32_t i) {
+      const bool got = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_o), i & 1u, abortp));
+      if (!got && lane == 0) give_up(38);
+      tc_fence_after();
+      return got;
+    };
+    auto warp_arrive = [&](uint64_t& bar) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar));
+    };
+    uint32_t phase = 0, i = 0;
+    int before = -1;  // the item whose context is still to be stored
+    bool whole = true;
+    for (int item = (int)blockIdx.x; item < p.items; item += (int)gridDim.x, phase ^= 1u, ++i) {
+      const int b = item / p.heads;
+      bool got = mbar_wait(smem_u32(&bar_s[i & 1u]), (i >> 1) & 1u, abortp);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) give_up(35);
+        whole = false;
         break;
       }
       tc_fence_after();
       float v[32];
       {
         uint32_t r[32];
-        tmem_ld32_nowait(tmem_s + lane_base + (uint32_t)cb * 32u, r);
+        tmem_ld32_nowait(tmem_s + 128u * (i & 1u) + lane_base + (uint32_t)cb * 32u, r);
         tmem_ld_wait_for(r);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
@@ -193,10 +238,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
         }
       }
       row_max[cb][row] = mx;
-      mbar_arrive(smem_u32(&bar_max));
-      got = mbar_wait(smem_u32(&bar_max), phase, abortp);
+      warp_arrive(bar_max[quarter]);
+      got = mbar_wait(smem_u32(&bar_max[quarter]), phase, abortp);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) give_up(36);
+        whole = false;
         break;
       }
       mx = fmaxf(fmaxf(row_max[0][row], row_max[1][row]), fmaxf(row_max[2][row], row_max[3][row]));
@@ -208,13 +254,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
         part[j & 1] = __fadd_rn(part[j & 1], v[j]);
       }
       row_sum[cb][row] = __fadd_rn(part[0], part[1]);
-      mbar_arrive(smem_u32(&bar_sum));
-      got = mbar_wait(smem_u32(&bar_sum), phase, abortp);
+      warp_arrive(bar_sum[quarter]);
+      got = mbar_wait(smem_u32(&bar_sum[quarter]), phase, abortp);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) give_up(37);
+        whole = false;
         break;
       }
       const float inv = __frcp_rn(__fadd_rn(__fadd_rn(row_sum[0][row], row_sum[1][row]), __fadd_rn(row_sum[2][row], row_sum[3][row])));
+      if (before >= 0 && !wait_context(i - 1u)) {  // the product before has read its probabilities
+        whole = false;
+        break;
+      }
       // this thread's 32 lanes are K block `cb` of the row: 16-byte piece c sits at row * 128 + ((c ^ (row & 7)) << 4)
       uint8_t* prow = base_ptr + ATT_P_OFF + cb * 16384 + row * 128;
 #pragma unroll
@@ -228,40 +279,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
         *reinterpret_cast<float4*>(prow + ((c ^ (row & 7)) << 4)) = make_float4(o[0], o[1], o[2], o[3]);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the second product reads the rows through the async proxy
-      mbar_arrive(smem_u32(&bar_p));
-      got = mbar_wait(smem_u32(&bar_o), phase, abortp);
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) give_up(38);
-        break;
-      }
-      if (cb < 2) {
-        // 32 context lanes of the row: staged (swizzled as the store's tensor map expects) and stored by TMA
-        tc_fence_after();
-        uint32_t r[32];
-        tmem_ld32_nowait(tmem_o + lane_base + (uint32_t)cb * 32u, r);
-        tmem_ld_wait_for(r);
-        tc_fence_before();
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous store has read the staging rows
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          *reinterpret_cast<uint4*>(stage_ptr + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
-          if (p.minmax_keys) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              seen_min = fminf(seen_min, __uint_as_float(r[4 * c + e]));
-              seen_max = fmaxf(seen_max, __uint_as_float(r[4 * c + e]));
-            }
-          }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&p.tmO, stage, h * p.o_ch + cb * 32, b * p.o_rb + h * p.o_rh + quarter * 32);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-      }
+      warp_arrive(bar_p);
+      // the context before leaves while the product of this item runs
+      if (before >= 0 && cb < 2) store_context(before, i - 1u);
+      before = item;
     }
+    if (whole && before >= 0 && wait_context(i - 1u) && cb < 2) store_context(before, i - 1u);
     if (cb < 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (p.minmax_keys && cb < 2) {
 #pragma unroll
@@ -287,7 +310,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) umma_attention_kernel(const __
     }
   }
   __syncthreads();
-  if (warp == ATT_ROW_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_slot), "r"(256) : "memory");
+  if (warp == ATT_ROW_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_slot), "r"(512) : "memory");
 }
 
 }  // namespace umma
