@@ -209,6 +209,8 @@ struct Epilogue {
   int act = 0;
   float clip_lo = 0.f, clip_hi = 0.f;
   int round_tf32 = 0;
+  // EPI_DEQUANT, where umma_can_transpose says so: sequences of this many rows leave transposed, [sequence][channel][row]
+  int out_seq = 0;
   // EPI_F32 with a fused residual: out = act((acc + bias_f[oc]) + residual[m * OC + oc]); the two
   // additions round as the separate Conv and Add nodes do
   const void* residual = nullptr;
@@ -308,6 +310,8 @@ void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s);
 // all small ones of one kind.  The group keeps what it needs of the plans.
 struct UmmaGroup;
 constexpr int kGroupMax = 3;
+// Whether a dequantising contraction of this shape can write its rows transposed within sequences of `seq` rows (out_seq).
+bool umma_can_transpose(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int seq);
 bool umma_plans_group(const UmmaPlan* a, const UmmaPlan* b);  // may the two be members of one group?
 UmmaGroup* umma_group_create(UmmaPlan* const* plans, int n);
 void umma_group_destroy(UmmaGroup* g);

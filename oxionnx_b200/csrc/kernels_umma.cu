@@ -274,7 +274,112 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
   return best;
 }
 
+// How a contraction is cut into tiles, and which kernel runs it.
+struct TileChoice {
+  int bn = 0, splits = 1;
+  bool pair = false;
+  SmallShape small;  // bn > 0: the small-problem kernel
+};
+TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int cb, int sms) {
+  // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles of the tensor pipe but
+  // cannot be issued faster than one per ~56 cycles; one SM fills its shared memory from L2 at about 110 GB/s when all
+  // SMs do so; the epilogue has its cost per output and a tile one of its own (below).  The three overlap (ring of stages,
+  // two accumulators), so a tile takes the longest of them, the kernel runs ceil(tiles / SMs) rounds of tiles, and the
+  // last tile's epilogue is not hidden.  Pick the width that minimises that estimate; ties go to the wider tile (fewer
+  // re-reads of the activations).  Fitted to sweeps of width and slices over some thirty layer shapes, where the choice
+  // is within 1 us of the best one but for two of them.
+  // Split K: when few tiles leave most SMs without one and K is long, `splits` CTAs share a tile, each running a slice of
+  // K; the slices meet in an L2-resident workspace, for 1 us and 0.35 us per MB of it (TF32 M = 1568 N = 512 K = 2048:
+  // four slices of 256 columns 3 us faster than 104 tiles of 64; K = 4608: five slices 14 us faster than 52 tiles of 128).
+  // Only with an SM of its own for every slice, at least eight K blocks each, and some SMs to spare: 147 slices on 148 SMs
+  // met 10 us later than that (M = 6272 N = 256, K = 1024 and 2304 alike).
+  const int es = umma_elem_bytes(kind);
+  const int64_t M = cs.M(), m_tiles = ceil_div(M, BLOCK_M);
+  const int bn_max = cs.OC <= 32 ? 32 : (cs.OC <= 64 ? 64 : (cs.OC <= 128 ? 128 : 256));
+  const int64_t k_iters_host = (int64_t)cs.R * cs.S * (cs.C / cb);
+  TileChoice t;
+  int &bn = t.bn, &splits = t.splits;
+  SmallShape& small = t.small;
+  bn = bn_max, splits = 1;
+  {
+    const double k_bytes = (double)cs.K() * es;
+    const double k_steps = k_bytes / 32.0;
+    // epilogue: per output 0.045 ns for integers, 0.03 ns float, plus 0.25 us per tile whatever its width;
+    // with a Gelu behind it 0.2 ns (and 2.5 us for a run of the small-problem kernel), which moves M = 8192 N = 3072 K = 768
+    // from 6 rounds of 256 columns to 11 of 128 (61.5 -> 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us)
+    const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
+    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.045e-9);
+    const double t_tile_fixed = 0.25e-6;
+    const int max_split = tune.split_k_max > 0 ? tune.split_k_max : 8;
+    double best = 1e30;
+    for (int cand = bn_max; cand >= 32; cand /= 2) {
+      const double tiles = (double)m_tiles * (double)ceil_div(cs.OC, cand);
+      for (int sp = 1; sp <= max_split; ++sp) {
+        if (sp > 1 && (tiles * sp > 0.92 * sms || k_iters_host / sp < 8)) break;
+        const double rounds = std::ceil(tiles * sp / sms);
+        const double t_mma = k_steps * std::max(56.0, cand / 2.0) / 1.965e9 / sp;
+        const double t_feed = (double)(BLOCK_M + cand) * k_bytes / 110e9 / sp;
+        const double t_epi = (double)BLOCK_M * cand * ns_out + t_tile_fixed;
+        const double t_split = sp > 1 ? 1e-6 + 0.35e-12 * tiles * sp * BLOCK_M * cand * 4.0 : 0.0;
+        const double time = rounds * std::max(t_mma, std::max(t_feed, t_epi)) + t_epi + t_split;
+        if (time < best * 0.97) {
+          best = time;
+          bn = cand;
+          splits = sp;
+        }
+      }
+    }
+    // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
+    // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
+    if (tune.cta_pairs != 2) {
+      small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu && M > 32 ? 2.5 : 0.7);
+      if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
+      if (small.bn > 0) {
+        bn = small.bn;
+        splits = 1;
+      }
+    }
+  }
+  // CTA pairs: two CTAs share a 256 x 256 tile and each stages 128 rows of A and 128 rows of B per K block (32 KB
+  // at 128-byte K blocks instead of the 48 KB of a lone CTA's 128 x 256 tile), which relieves both the L2 -> shared
+  // memory feed and the shared-memory bandwidth the MMAs and the incoming copies compete for.  Worth it where the
+  // operand feed bounds the tile (long K) and there are enough 256-row tiles to keep every pair busy.
+  bool& pair = t.pair;
+  if (tune.cta_pairs == 2 && cs.OC >= 256) {  // forced (tests, comparisons): the pair form wherever the shape allows it
+    bn = 256;
+    splits = 1;
+  }
+  if (tune.cta_pairs != 1 && small.bn == 0 && bn == 256 && splits == 1 && cs.OC >= 256) {
+    const int64_t pair_tiles = ceil_div(M, 2 * BLOCK_M) * ceil_div(cs.OC, 256);
+    const double k_bytes = (double)cs.K() * es;
+    // Measured: with 2 KB of K or more per row a pair wins once every pair has at least two tiles (3x3 256->256,
+    // i8, M=100352: 57.7 us against 65.9 us for lone CTAs); from 8 KB of K it also wins with a single partial wave
+    // (TF32 3x3 256->256 at M=25088: 61.9 us against 78.2 us); below 2 KB the extra barrier traffic of a pair costs
+    // more than the halved operand feed saves (1x1 1024->256, i8, M=12544: 18.6 us against 16.7 us).
+    const int64_t pairs_resident = sms / 2;
+    // A single wave that pairs do not lengthen gains too (TF32 3x3 1024->1024 at M=4096, 64 pair tiles: 145.7 us -> 108.8 us).
+    const bool same_waves = ceil_div(pair_tiles, pairs_resident) <= ceil_div(m_tiles * ceil_div(cs.OC, 256), (int64_t)sms);
+    const bool feed_bound =
+        k_bytes >= 2048.0 && (pair_tiles >= 2 * pairs_resident || (k_bytes >= 8192.0 && (pair_tiles >= pairs_resident || (same_waves && 2 * pair_tiles >= pairs_resident))));
+    if (tune.cta_pairs == 2) pair = true;
+    else pair = feed_bound;
+  }
+  return t;
+}
+
+// The variants that the fragment epilogue for f32 lanes takes, over whole groups of 64 channels.
+bool takes_float_fragments(const ConvShape& cs, const Epilogue& e, int kind, const TileChoice& t, int splits) {
+  return kind == KIND_I8 && e.mode == EPI_DEQUANT && e.dq_act < 2 && t.small.bn == 0 && t.bn >= 64 && cs.OC % 64 == 0 && splits == 1 && !e.residual;  // not the tanh form of Gelu
+}
+
 }  // namespace
+
+bool umma_can_transpose(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int seq) {
+  const int cb = umma_channel_block(cs.C, kind);
+  if (cb == 0 || cs.M() <= 0 || e.dq_act != 0 || seq % 32 != 0 || cs.M() % seq != 0) return false;
+  const TileChoice t = choose_tile(cs, e, kind, tune, cb, sm_count(current_device()));
+  return takes_float_fragments(cs, e, kind, t, t.splits);
+}
 
 UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt, void* out, const ConvShape& cs, const Epilogue& e, int kind,
                            const UmmaTuning& tune, std::string* why) {
@@ -315,88 +420,13 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   if (e.join && (!e.residual || !e.bias_if || dt_size(e.out_dt) != 1 || cs.OC % 32 != 0)) return no("the join needs an 8-bit residual, the float bias and whole channel runs");
   if (e.mode == EPI_F32 && e.act == 4 && e.slope == nullptr) return no("the PRelu epilogue needs a (padded) slope vector");
 
-  // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles of the tensor pipe but
-  // cannot be issued faster than one per ~56 cycles; one SM fills its shared memory from L2 at about 110 GB/s when all
-  // SMs do so; the epilogue has its cost per output and a tile one of its own (below).  The three overlap (ring of stages,
-  // two accumulators), so a tile takes the longest of them, the kernel runs ceil(tiles / SMs) rounds of tiles, and the
-  // last tile's epilogue is not hidden.  Pick the width that minimises that estimate; ties go to the wider tile (fewer
-  // re-reads of the activations).  Fitted to sweeps of width and slices over some thirty layer shapes, where the choice
-  // is within 1 us of the best one but for two of them.
-  // Split K: when few tiles leave most SMs without one and K is long, `splits` CTAs share a tile, each running a slice of
-  // K; the slices meet in an L2-resident workspace, for 1 us and 0.35 us per MB of it (TF32 M = 1568 N = 512 K = 2048:
-  // four slices of 256 columns 3 us faster than 104 tiles of 64; K = 4608: five slices 14 us faster than 52 tiles of 128).
-  // Only with an SM of its own for every slice, at least eight K blocks each, and some SMs to spare: 147 slices on 148 SMs
-  // met 10 us later than that (M = 6272 N = 256, K = 1024 and 2304 alike).
   const int device = current_device();
   const int sms = sm_count(device);
-  const int64_t m_tiles = ceil_div(M, BLOCK_M);
-  const int bn_max = cs.OC <= 32 ? 32 : (cs.OC <= 64 ? 64 : (cs.OC <= 128 ? 128 : 256));
-  const int64_t k_iters_host = (int64_t)cs.R * cs.S * (cs.C / cb);
-  int bn = bn_max, splits = 1;
-  SmallShape small;
-  {
-    const double k_bytes = (double)cs.K() * es;
-    const double k_steps = k_bytes / 32.0;
-    // epilogue: per output 0.045 ns for integers, 0.03 ns float, plus 0.25 us per tile whatever its width;
-    // with a Gelu behind it 0.2 ns (and 2.5 us for a run of the small-problem kernel), which moves M = 8192 N = 3072 K = 768
-    // from 6 rounds of 256 columns to 11 of 128 (61.5 -> 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us)
-    const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
-    const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.045e-9);
-    const double t_tile_fixed = 0.25e-6;
-    const int max_split = tune.split_k_max > 0 ? tune.split_k_max : 8;
-    double best = 1e30;
-    for (int cand = bn_max; cand >= 32; cand /= 2) {
-      const double tiles = (double)m_tiles * (double)ceil_div(cs.OC, cand);
-      for (int sp = 1; sp <= max_split; ++sp) {
-        if (sp > 1 && (tiles * sp > 0.92 * sms || k_iters_host / sp < 8)) break;
-        const double rounds = std::ceil(tiles * sp / sms);
-        const double t_mma = k_steps * std::max(56.0, cand / 2.0) / 1.965e9 / sp;
-        const double t_feed = (double)(BLOCK_M + cand) * k_bytes / 110e9 / sp;
-        const double t_epi = (double)BLOCK_M * cand * ns_out + t_tile_fixed;
-        const double t_split = sp > 1 ? 1e-6 + 0.35e-12 * tiles * sp * BLOCK_M * cand * 4.0 : 0.0;
-        const double t = rounds * std::max(t_mma, std::max(t_feed, t_epi)) + t_epi + t_split;
-        if (t < best * 0.97) {
-          best = t;
-          bn = cand;
-          splits = sp;
-        }
-      }
-    }
-    // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
-    // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
-    if (tune.cta_pairs != 2) {
-      small = choose_small(M, cs.OC, k_iters_host, swz, sms, max_split, gelu && M > 32 ? 2.5 : 0.7);
-      if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
-      if (small.bn > 0) {
-        bn = small.bn;
-        splits = 1;
-      }
-    }
-  }
-  // CTA pairs: two CTAs share a 256 x 256 tile and each stages 128 rows of A and 128 rows of B per K block (32 KB
-  // at 128-byte K blocks instead of the 48 KB of a lone CTA's 128 x 256 tile), which relieves both the L2 -> shared
-  // memory feed and the shared-memory bandwidth the MMAs and the incoming copies compete for.  Worth it where the
-  // operand feed bounds the tile (long K) and there are enough 256-row tiles to keep every pair busy.
-  bool pair = false;
-  if (tune.cta_pairs == 2 && cs.OC >= 256) {  // forced (tests, comparisons): the pair form wherever the shape allows it
-    bn = 256;
-    splits = 1;
-  }
-  if (tune.cta_pairs != 1 && small.bn == 0 && bn == 256 && splits == 1 && cs.OC >= 256) {
-    const int64_t pair_tiles = ceil_div(M, 2 * BLOCK_M) * ceil_div(cs.OC, 256);
-    const double k_bytes = (double)cs.K() * es;
-    // Measured: with 2 KB of K or more per row a pair wins once every pair has at least two tiles (3x3 256->256,
-    // i8, M=100352: 57.7 us against 65.9 us for lone CTAs); from 8 KB of K it also wins with a single partial wave
-    // (TF32 3x3 256->256 at M=25088: 61.9 us against 78.2 us); below 2 KB the extra barrier traffic of a pair costs
-    // more than the halved operand feed saves (1x1 1024->256, i8, M=12544: 18.6 us against 16.7 us).
-    const int64_t pairs_resident = sms / 2;
-    // A single wave that pairs do not lengthen gains too (TF32 3x3 1024->1024 at M=4096, 64 pair tiles: 145.7 us -> 108.8 us).
-    const bool same_waves = ceil_div(pair_tiles, pairs_resident) <= ceil_div(m_tiles * ceil_div(cs.OC, 256), (int64_t)sms);
-    const bool feed_bound =
-        k_bytes >= 2048.0 && (pair_tiles >= 2 * pairs_resident || (k_bytes >= 8192.0 && (pair_tiles >= pairs_resident || (same_waves && 2 * pair_tiles >= pairs_resident))));
-    if (tune.cta_pairs == 2) pair = true;
-    else pair = feed_bound;
-  }
+  const int64_t m_tiles = ceil_div(M, BLOCK_M), k_iters_host = (int64_t)cs.R * cs.S * (cs.C / cb);
+  const TileChoice choice = choose_tile(cs, e, kind, tune, cb, sms);
+  const int bn = choice.bn, splits = choice.splits;
+  const bool pair = choice.pair;
+  const SmallShape& small = choice.small;
   const int64_t n_tiles = ceil_div(cs.OC, bn);
   if (m_tiles * n_tiles > 0x7fffffffLL) return no("grid too large");
 
@@ -545,6 +575,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   else kp.variant = e.x_zp_dev ? V_INT32_DYN : V_INT32;
   kp.lo = (e.relu_fused && e.lo < 0) ? 0 : e.lo;
   kp.hi = e.hi;
+  if (e.out_seq > 0 && small.bn > 0) return fail("transposed rows need the fragment epilogue");
   if (small.bn > 0) {
     kp.small_bn = bn;
     kp.a_rows = a_rows;
@@ -559,8 +590,9 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // their arithmetic is allowed: they are the faster ones at every K (the figures stand there).
     const bool frag_ok = kind == KIND_I8 && bn >= 64 && cs.OC % 64 == 0 && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0;
     const bool join_ok = kp.variant == V_JOIN && e.join_d > 0.f && kp.hi - kp.lo == 255;
-    const bool floats_ok = kp.variant >= V_DEQUANT && kp.variant < V_DEQUANT + 4;  // not the tanh form of Gelu
-    const int perm = !frag_ok ? 0 : (kp.variant == V_REQUANT_PACKED || join_ok ? 64 : (floats_ok ? 16 : 0));
+    const int perm = takes_float_fragments(cs, e, kind, choice, kp.splits) ? 16 : (frag_ok && (kp.variant == V_REQUANT_PACKED || join_ok) ? 64 : 0);
+    if (e.out_seq > 0 && perm != 16) return fail("transposed rows need the fragment epilogue");
+    kp.out_seq = e.out_seq;
     kp.b_perm = perm;
     if (perm > 0) {
       kp.out_tma = 0;

@@ -556,6 +556,13 @@ class Planner {
     int step;
     k::UmmaPlan* plan;
   };
+  struct DequantStep {
+    k::ConvShape cs;
+    k::Epilogue epi;
+    int kind;
+  };
+  std::map<int, DequantStep> dequant_steps_;  // dequantising contractions by the value they write
+  bool transposed_at_source(int root_vi, int64_t seq, int heads_node, int reader);
   std::vector<PlanStep> plan_steps_;  // contractions on the tensor cores, in launch order
   void link_independent();
   struct LastAdd {
@@ -1372,6 +1379,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       if (res_vi >= 0) e.residual = V(res_vi).ptr;
       if (dq_vi >= 0) e.dq_x_scale_dev = (const float*)V(dq_vi).ptr;
       e.minmax_keys = (unsigned int*)V(out_vi).minmax_keys;
+      e.out_seq = V(out_vi).out_seq;
       std::string why2;
       k::UmmaTuning tune;
       tune.requant_f64 = C.cfg().requant_f64;
@@ -1416,6 +1424,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       };
     };
     (void)stp;
+    if (epi.mode == k::EPI_DEQUANT) dequant_steps_[out_vi] = {cs, epi, kind};
     return;
   }
 
@@ -3197,7 +3206,11 @@ bool Planner::try_plan_fused_attention(const NodeDef& n, int qi, int ki) {
   const float* dscale = (const float*)C.resident_form(mul.inputs[s_slot], "raw_f32", 4, [sc](void* p) { std::memcpy(p, sc->data.data(), 4); },
                                                       cacheable_const(mul.inputs[s_slot]));
   int vt = -1;
-  if (!simt) {
+  const bool at_source = !simt && transposed_at_source(hv.root_vi, Sq, hv.node, av_i);
+  if (at_source) {
+    vt = hv.root_vi;
+    V(vt).out_seq = (int)Sq;
+  } else if (!simt) {
     vt = add_value(V(hv.src_vi).name + "@heads_t", {B, H, D, Sq}, DT::F32, Layout::PLAIN);
     emit_transpose(nodes_[hv.node], hv.src_vi, {0, 2, 3, 1}, vt);
   }
@@ -3258,6 +3271,35 @@ bool Planner::try_plan_fused_attention(const NodeDef& n, int qi, int ki) {
     };
   };
   return true;
+}
+
+// V's linear may write its rows transposed per sequence, which is the layout the attention kernel reads V in, when it is a
+// dequantising contraction of the persistent kernel and nothing but views stand between it and the one product that reads it
+// (encoder of 64x128 tokens: 12 us a layer for the transpose by a launch of its own).
+bool Planner::transposed_at_source(int root_vi, int64_t seq, int heads_node, int reader) {
+  auto it = dequant_steps_.find(root_vi);
+  if (it == dequant_steps_.end() || V(root_vi).is_graph_output) return false;
+  auto sole_reader = [&](const std::string& name, int node) {
+    auto c = consumers_.find(name);
+    return !graph_outputs_.count(name) && c != consumers_.end() && c->second.size() == 1 && c->second[0].first == node;
+  };
+  if (!sole_reader(nodes_[heads_node].outputs[0], reader)) return false;
+  for (int node = heads_node;;) {
+    const std::string name = in_name(nodes_[node], 0);
+    auto vi = S.index_.find(name);
+    if (vi == S.index_.end() || !sole_reader(name, node)) return false;
+    if (vi->second == root_vi) break;
+    int from = -1;  // the view that made it
+    for (int j = 0; j < (int)nodes_.size() && from < 0; ++j)
+      if (nodes_[j].op == "Reshape" && !nodes_[j].outputs.empty() && nodes_[j].outputs[0] == name) from = j;
+    if (from < 0 || V(vi->second).alias_of < 0) return false;
+    node = from;
+  }
+  k::UmmaTuning tune;
+  tune.requant_f64 = C.cfg().requant_f64;
+  tune.split_k_max = C.cfg().split_k_max;
+  tune.cta_pairs = C.cfg().cta_pairs;
+  return k::umma_can_transpose(it->second.cs, it->second.epi, it->second.kind, tune, (int)seq);
 }
 
 // Softmax over the last axis (nn/normalization.rs softmax_into); other axes are declined.

@@ -87,6 +87,7 @@ struct Value {
   // keys (the scratch of the DynamicQuantizeLinear that reads it, which then skips its own first pass)
   void* minmax_keys = nullptr;
   int dq_src = -1, dq_step = -1;
+  int out_seq = 0;  // > 0: the contraction that produces it writes its rows transposed within sequences of this many
   float dq_scale = 1.f, dq_zp = 0.f;
   int64_t numel() const { return prod(shape); }
 };

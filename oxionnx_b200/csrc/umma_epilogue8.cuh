@@ -281,6 +281,8 @@ __device__ __forceinline__ void epilogue_floats(const KParams& p, int warp, int 
     tc_fence_after();
     const int m = walk.m * M_STEP + row;
     float* const out = (float*)p.out + ((size_t)m * p.OC + oc + 4 * (lane & 3));
+    float* out_t = nullptr;  // transposed: a warp's 32 rows are in one sequence, eight rows of a channel are 32 contiguous bytes
+    if (!GELU && p.out_seq > 0) out_t = (float*)p.out + (((size_t)(m / p.out_seq) * p.OC + oc + 4 * (lane & 3)) * p.out_seq + m % p.out_seq);
     const int rows = mine ? p.M - m : 0;  // of this thread's rows 0, 8, 16 and 24 those below this bound are written
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * (uint32_t)BN + (uint32_t)col0;
     constexpr int STEPS = 4 / GROUPS;  // bodies of a half
@@ -323,7 +325,12 @@ __device__ __forceinline__ void epilogue_floats(const KParams& p, int warp, int 
           }
           const int r = 16 * h + 8 * s;
           if (r < rows) {
-            *reinterpret_cast<float4*>(out + (size_t)r * p.OC + 16 * (g0 + g)) = make_float4(y[0], y[1], y[2], y[3]);
+            if (!GELU && out_t) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) out_t[(size_t)(16 * (g0 + g) + j) * p.out_seq + r] = y[j];
+            } else {
+              *reinterpret_cast<float4*>(out + (size_t)r * p.OC + 16 * (g0 + g)) = make_float4(y[0], y[1], y[2], y[3]);
+            }
             if (track) {
               seen_min = fminf(seen_min, fminf(fminf(y[0], y[1]), fminf(y[2], y[3])));
               seen_max = fmaxf(seen_max, fmaxf(fmaxf(y[0], y[1]), fmaxf(y[2], y[3])));

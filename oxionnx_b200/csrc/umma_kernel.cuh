@@ -131,6 +131,7 @@ struct alignas(64) KParams {
   const float* dq_bias;      // per-channel f32 bias
   int y_zp, lo, hi;
   int out_dt;
+  int out_seq;  // > 0: rows leave transposed within sequences of this many, [sequence][channel][row] (epilogue_floats only)
   void* out;
   // f32 outputs only, or null: two ordered keys (see float_order_key) into which the kernel merges the minimum and
   // the maximum of everything it writes, for a DynamicQuantizeLinear that reads the output next

@@ -76,3 +76,23 @@ def test_fragment_dequantisation_is_the_separate_nodes(rows, k, n, gelu, pairs):
     want, _ = _run(graph, w, feeds, keep_intermediates=True)
     for name in graph.output_names:
         assert np.array_equal(got[name], want[name]), name
+
+
+def test_values_transposed_by_their_linear():
+    """V leaves its linear in the layout that the attention kernel reads, unless somebody else reads it too.  Copies of two
+    sentences have the extrema of the two, so every copy is the small batch's, where V is transposed by a launch of its own."""
+    from oxionnx_b200 import models
+    rng = np.random.default_rng(5)
+    ids, mask = rng.integers(0, 500, (2, 128)).astype(np.float32), np.ones((2, 128), np.float32)
+    mask[1, 90:] = 0
+    out = {}
+    for batch, other_reader in ((2, False), (42, False), (42, True)):
+        graph, weights, _, _ = models.build_bert_dynamic_int8(batch=batch, seq=128, hidden=768, heads=12, ffn=768, layers=2, vocab=500)
+        if other_reader:
+            graph = Graph(nodes=graph.nodes, input_names=graph.input_names, output_names=graph.output_names + ["l0_v_out"])
+        got, kernels = _run(graph, weights, {"input_ids": np.tile(ids, (batch // 2, 1)), "attention_mask": np.tile(mask, (batch // 2, 1))})
+        assert sum("umma_attention" in s for s in kernels) == 2, kernels
+        assert sum(s.startswith("transpose") for s in kernels) == (2 if batch == 2 else int(other_reader)), kernels
+        out[batch, other_reader] = got["hidden"].reshape(batch // 2, 2, 128, 768)
+    for copies in ((42, False), (42, True)):
+        assert all(np.array_equal(c, out[2, False][0]) for c in out[copies]), copies
