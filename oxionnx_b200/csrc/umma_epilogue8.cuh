@@ -237,7 +237,7 @@ __device__ __forceinline__ void epilogue_bytes(const KParams& p, int warp, int l
 // eight outputs so that the loop stays in the instruction cache (sixteen: 1 % slower over an encoder).
 // Measured, general epilogue -> this one: M = 8192, N = 768, K = 768 22.6 -> 16.5 us, with extrema 24.9 -> 18.5 us, K = 3072
 // 43.2 -> 31.0 us; N = 3072, K = 768 with Gelu 70.1 -> 59.8 us; an encoder of 64x128 tokens 3480 -> 2949 us.
-template <int BN, bool PAIR, bool DYN, bool GELU>
+template <int BN, bool PAIR, bool DYN, bool GELU, bool TRANSPOSED>
 __device__ __forceinline__ void epilogue_floats(const KParams& p, int warp, int lane, uint32_t tmem_base, uint64_t* bar_acc_full, uint64_t* bar_acc_empty,
                                                 uint32_t params, volatile int* abortp, int total_tiles, int tile0, int tile_step, int pair_rank) {
   using ES = EpiShape<BN, epi_warps(KIND_I8)>;
@@ -282,7 +282,7 @@ __device__ __forceinline__ void epilogue_floats(const KParams& p, int warp, int 
     const int m = walk.m * M_STEP + row;
     float* const out = (float*)p.out + ((size_t)m * p.OC + oc + 4 * (lane & 3));
     float* out_t = nullptr;  // transposed: a warp's 32 rows are in one sequence, eight rows of a channel are 32 contiguous bytes
-    if (!GELU && p.out_seq > 0) out_t = (float*)p.out + (((size_t)(m / p.out_seq) * p.OC + oc + 4 * (lane & 3)) * p.out_seq + m % p.out_seq);
+    if (TRANSPOSED) out_t = (float*)p.out + (((size_t)(m / p.out_seq) * p.OC + oc + 4 * (lane & 3)) * p.out_seq + m % p.out_seq);
     const int rows = mine ? p.M - m : 0;  // of this thread's rows 0, 8, 16 and 24 those below this bound are written
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * (uint32_t)BN + (uint32_t)col0;
     constexpr int STEPS = 4 / GROUPS;  // bodies of a half
@@ -325,7 +325,7 @@ __device__ __forceinline__ void epilogue_floats(const KParams& p, int warp, int 
           }
           const int r = 16 * h + 8 * s;
           if (r < rows) {
-            if (!GELU && out_t) {
+            if (TRANSPOSED) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) out_t[(size_t)(16 * (g0 + g) + j) * p.out_seq + r] = y[j];
             } else {

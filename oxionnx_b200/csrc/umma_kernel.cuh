@@ -1567,14 +1567,20 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
         }
       }
 #undef OXB_BYTES
-#define OXB_FLOATS(D, G) epilogue_floats<BN, PAIR, D, G>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank)
+#define OXB_FLOATS(D, G, T) epilogue_floats<BN, PAIR, D, G, T>(p, warp, lane, tmem_base, bar_acc_full, bar_acc_empty, stage_addr, abortp, total_tiles, tile0, tile_step, pair_rank)
       if (p.b_perm == 16) {
         fragment = true;
         switch (p.variant) {
-          case V_DEQUANT: OXB_FLOATS(false, false); break;
-          case V_DEQUANT + 1: OXB_FLOATS(true, false); break;
-          case V_DEQUANT + 2: OXB_FLOATS(false, true); break;
-          default: OXB_FLOATS(true, true); break;
+          case V_DEQUANT:
+            if (p.out_seq > 0) OXB_FLOATS(false, false, true);
+            else OXB_FLOATS(false, false, false);
+            break;
+          case V_DEQUANT + 1:
+            if (p.out_seq > 0) OXB_FLOATS(true, false, true);
+            else OXB_FLOATS(true, false, false);
+            break;
+          case V_DEQUANT + 2: OXB_FLOATS(false, true, false); break;
+          default: OXB_FLOATS(true, true, false); break;
         }
       }
 #undef OXB_FLOATS
