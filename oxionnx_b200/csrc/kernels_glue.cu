@@ -1815,7 +1815,12 @@ __global__ void softmax_rows_reg_kernel(const float4* __restrict__ x, float4* __
 // query rows of one head, so that short batches still fill the chip; a thread holds RM x 4 results, which takes one
 // 16-byte read of each operand per RM x 4 FMAs, and K is kept transposed so that both are conflict free.  The
 // block's score rows stay in shared memory.  A layer of 2 x 77 positions, 12 heads: 60 us in eight launches -> 18 us.
-template <int TM>
+// A warp takes four rows of the softmax side by side (encoder of 2x77 tokens 978 -> 951 us, of 64x40 1738 -> 1682 us).  Where
+// several tiles follow one another and there are blocks enough, they are fetched ahead (20x300 5756 -> 5442 us, 64x77 2998
+// -> 2909 us); the registers for that cost more than they bring over a single tile (64x40 1682 -> 1729 us) and where a
+// block of 16 rows has an SM to itself (2x77 951 -> 986 us, 3x180 the same).  64 rows and 8 x 8 results a thread, with one
+// block an SM, took 20x300 to 6910 us.
+template <int TM, bool AHEAD>
 __global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ kk, const float* __restrict__ v,
                                                             float* __restrict__ out, int S, int H, const float* __restrict__ scale,
                                                             const float* __restrict__ mask, unsigned int* minmax_keys) {
@@ -1834,19 +1839,53 @@ __global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restr
   const float* kb = kk + (int64_t)b * S * ld + h * D;
   const float* vb = v + (int64_t)b * S * ld + h * D;
   const int rows = min(TM, S - row0);
+  // AHEAD: the next tile of K or V is on its way into registers while the one in shared memory is worked on
+  float4 next[8];
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto fetch_k = [&](int k0) {  // 16 keys x 32 bytes per warp and pass
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = tid + 128 * j, key = k0 + (i & 15) + ((i >> 8) << 4), d4 = ((i >> 4) & 15) * 4;
+      next[j] = key < S ? *reinterpret_cast<const float4*>(kb + (int64_t)key * ld + d4) : zero4;
+    }
+  };
+  auto fetch_v = [&](int k0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = tid + 128 * j, key = k0 + (i >> 4), d4 = (i & 15) * 4;
+      next[j] = key < S ? *reinterpret_cast<const float4*>(vb + (int64_t)key * ld + d4) : zero4;
+    }
+  };
+  auto store_v = [&]() {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(kv + (tid + 128 * j) * 4) = next[j];
+  };
+  if (AHEAD) fetch_k(0);
   for (int i = tid; i < TM * 16; i += 128) {  // 16 rows x 32 bytes per warp and pass
     const int r = (i & 15) + ((i >> 8) << 4), d4 = ((i >> 4) & 15) * 4;
-    const float4 t = r < rows ? *reinterpret_cast<const float4*>(qb + (int64_t)r * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 t = r < rows ? *reinterpret_cast<const float4*>(qb + (int64_t)r * ld + d4) : zero4;
     qs[(d4 + 0) * QP + r] = t.x, qs[(d4 + 1) * QP + r] = t.y, qs[(d4 + 2) * QP + r] = t.z, qs[(d4 + 3) * QP + r] = t.w;
   }
   const int kg = (tid & 15) * 4, rg = (tid >> 4) * RM;  // this thread's four keys (or lanes) and RM rows
   for (int k0 = 0; k0 < S; k0 += 64) {
-    for (int i = tid; i < 64 * 16; i += 128) {
+    auto store_k = [&](int i, const float4& t) {
       const int key = (i & 15) + ((i >> 8) << 4), d4 = ((i >> 4) & 15) * 4;
-      const float4 t = k0 + key < S ? *reinterpret_cast<const float4*>(kb + (int64_t)(k0 + key) * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
       kv[(d4 + 0) * KP + key] = t.x, kv[(d4 + 1) * KP + key] = t.y, kv[(d4 + 2) * KP + key] = t.z, kv[(d4 + 3) * KP + key] = t.w;
+    };
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) store_k(tid + 128 * j, next[j]);
+    } else {
+      for (int i = tid; i < 64 * 16; i += 128) {
+        const int key = k0 + (i & 15) + ((i >> 8) << 4);
+        store_k(i, key < S ? *reinterpret_cast<const float4*>(kb + (int64_t)key * ld + ((i >> 4) & 15) * 4) : zero4);
+      }
     }
     __syncthreads();
+    if (AHEAD) {
+      if (k0 + 64 < S) fetch_k(k0 + 64);
+      else fetch_v(0);
+    }
     float acc[RM][4];
 #pragma unroll
     for (int r = 0; r < RM; ++r)
@@ -1870,28 +1909,49 @@ __global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restr
     for (int r = 0; r < RM; ++r) *reinterpret_cast<float4*>(ps + (rg + r) * pitch + k0 + kg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     __syncthreads();
   }
+  if (AHEAD) {
+    store_v();  // K has been read
+    if (64 < S) fetch_v(64);
+  }
   const float sc = scale ? scale[0] : 1.f;
   const float* pm = mask ? mask + (int64_t)b * S : nullptr;
-  for (int r = warp; r < TM; r += 4) {
+  constexpr int AT_ONCE = 4;  // rows of a warp side by side: their chains of exponentials and shuffles overlap
+  for (int r = warp * AT_ONCE; r < TM; r += 4 * AT_ONCE) {
     float* row = ps + r * pitch;
-    float mx = -INFINITY;
+    float mx[AT_ONCE], sum[AT_ONCE], inv[AT_ONCE];
+#pragma unroll
+    for (int a = 0; a < AT_ONCE; ++a) mx[a] = -INFINITY, sum[a] = 0.f;
     for (int k = lane; k < S; k += 32) {
-      float x = row[k];
-      if (scale) x = __fmul_rn(x, sc);
-      if (pm) x = __fadd_rn(x, pm[k]);
-      row[k] = x;
-      mx = fmaxf(mx, x);
+      const float m = pm ? pm[k] : 0.f;
+#pragma unroll
+      for (int a = 0; a < AT_ONCE; ++a) {
+        float x = row[a * pitch + k];
+        if (scale) x = __fmul_rn(x, sc);
+        if (pm) x = __fadd_rn(x, m);
+        row[a * pitch + k] = x;
+        mx[a] = fmaxf(mx[a], x);
+      }
     }
-    mx = warp_max(mx);
-    float sum = 0.f;
+#pragma unroll
+    for (int a = 0; a < AT_ONCE; ++a) mx[a] = warp_max(mx[a]);
     for (int k = lane; k < S; k += 32) {
-      const float e = expf(__fsub_rn(row[k], mx));
-      row[k] = e;
-      sum += e;
+#pragma unroll
+      for (int a = 0; a < AT_ONCE; ++a) {
+        const float e = expf(__fsub_rn(row[a * pitch + k], mx[a]));
+        row[a * pitch + k] = e;
+        sum[a] += e;
+      }
     }
-    const float inv = __frcp_rn(warp_sum(sum));
-    for (int k = lane; k < S; k += 32) row[k] = round_tf32(__fmul_rn(row[k], inv));  // the probabilities feed a contraction
-    for (int k = S + lane; k < pitch; k += 32) row[k] = 0.f;
+#pragma unroll
+    for (int a = 0; a < AT_ONCE; ++a) inv[a] = __frcp_rn(warp_sum(sum[a]));
+    for (int k = lane; k < S; k += 32) {
+#pragma unroll
+      for (int a = 0; a < AT_ONCE; ++a) row[a * pitch + k] = round_tf32(__fmul_rn(row[a * pitch + k], inv[a]));  // the probabilities feed a contraction
+    }
+    for (int k = S + lane; k < pitch; k += 32) {
+#pragma unroll
+      for (int a = 0; a < AT_ONCE; ++a) row[a * pitch + k] = 0.f;
+    }
   }
   float acc[RM][4];
 #pragma unroll
@@ -1899,14 +1959,20 @@ __global__ void __launch_bounds__(128) attention_f32_kernel(const float* __restr
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
   for (int k0 = 0; k0 < S; k0 += 64) {
-    __syncthreads();
-    const int n = min(64, S - k0);
-    for (int i = tid; i < 64 * 16; i += 128) {
-      const int key = i >> 4, d4 = (i & 15) * 4;
-      *reinterpret_cast<float4*>(kv + key * D + d4) =
-          key < n ? *reinterpret_cast<const float4*>(vb + (int64_t)(k0 + key) * ld + d4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!AHEAD || k0 > 0) {
+      __syncthreads();  // the tile before has been read
+      if constexpr (AHEAD) {
+        store_v();
+        if (k0 + 64 < S) fetch_v(k0 + 64);
+      } else {
+        for (int i = tid; i < 64 * 16; i += 128) {
+          const int key = k0 + (i >> 4);
+          *reinterpret_cast<float4*>(kv + i * 4) = key < S ? *reinterpret_cast<const float4*>(vb + (int64_t)key * ld + (i & 15) * 4) : zero4;
+        }
+      }
     }
     __syncthreads();
+    const int n = min(64, S - k0);
 #pragma unroll 2
     for (int k4 = 0; k4 < n; k4 += 4) {  // lanes past the last position multiply zeros, as the padded slabs of the plain product do
       float pf[RM][4];
@@ -2643,7 +2709,7 @@ size_t attention_f32_smem(int S) {
   return (size_t)(64 * (TM + 4) + 64 * 68 + TM * (((S + 63) & ~63) + 4)) * sizeof(float);
 }
 
-template <int TM>
+template <int TM, bool AHEAD>
 void attention_f32_launch(const FusedAttention& a, cudaStream_t s) {
   // the opt-in for more than 48 KB of dynamic shared memory is a per-device property of the kernel
   static std::mutex mu;
@@ -2653,19 +2719,20 @@ void attention_f32_launch(const FusedAttention& a, cudaStream_t s) {
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!have[device & 63]) {
-      OXB_CUDA(cudaFuncSetAttribute(attention_f32_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_f32_smem<TM>(kAttentionF32MaxS)));
+      OXB_CUDA(cudaFuncSetAttribute(attention_f32_kernel<TM, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attention_f32_smem<TM>(kAttentionF32MaxS)));
       have[device & 63] = true;
     }
   }
-  launch(attention_f32_kernel<TM>, dim3((unsigned)ceil_div(a.S, TM), (unsigned)(a.B * a.H)), 128, attention_f32_smem<TM>(a.S), s, a.q, a.k, a.v, a.out, a.S, a.H,
+  launch(attention_f32_kernel<TM, AHEAD>, dim3((unsigned)ceil_div(a.S, TM), (unsigned)(a.B * a.H)), 128, attention_f32_smem<TM>(a.S), s, a.q, a.k, a.v, a.out, a.S, a.H,
          a.scale, a.mask, a.minmax_keys);
 }
 }  // namespace
 
 // 16 query rows per block while 32 would leave SMs without two (2 sequences of 77: 120 blocks instead of 72).
 void attention_f32(const FusedAttention& a, cudaStream_t s) {
-  if ((int64_t)a.B * a.H * ceil_div(a.S, 32) < 2 * 148) attention_f32_launch<16>(a, s);
-  else attention_f32_launch<32>(a, s);
+  if ((int64_t)a.B * a.H * ceil_div(a.S, 32) < 2 * 148) attention_f32_launch<16, false>(a, s);
+  else if (a.S <= 64) attention_f32_launch<32, false>(a, s);
+  else attention_f32_launch<32, true>(a, s);
 }
 
 void layer_norm_rows(const float* x, float* y, int64_t rows, int64_t n, const float* scale, const float* bias, float eps, cudaStream_t s,
