@@ -23,8 +23,11 @@
 //    that lands in its own TMEM.  The pair's loads signal the even CTA's barrier; its commits
 //    free the ring stage and publish the accumulator in both CTAs.
 //  * Epilogue warps (sixteen for the integer kind, eight for the float kinds) read the
-//    accumulator with tcgen05.ld (one output pixel per thread, 32 channels per load), apply the
-//    fused epilogue in registers and hand the tile to TMA stores through swizzled staging rows.
+//    accumulator with tcgen05.ld, apply the fused epilogue in registers and write the tile.  Integer
+//    layers of whole groups of 64 channels take the fragment epilogues (umma_epilogue8.cuh: four or
+//    sixteen consecutive channels of two pixels per thread, stored directly); the others and the float
+//    kinds hold one output pixel per thread, 32 channels per load, and hand the tile to TMA stores
+//    through swizzled staging rows.
 //    A warp may only read the TMEM lanes 32 * (warp % 4) .. + 31, so the warps of a lane
 //    quarter split a tile's channel runs, at least two runs per warp; when that leaves warps
 //    over (tiles narrower than 256 channels) the warps form groups, each group drains a tile of
