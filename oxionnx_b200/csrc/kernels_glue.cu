@@ -2460,7 +2460,9 @@ void dynamic_quantize_linear(const TensorRef& x, const TensorRef& y, float* para
   }
   const int64_t cap = 148 * 8;
   const int64_t b_mm = std::min<int64_t>(cap, std::max<int64_t>(1, (n / 4 + kThreads * 4 - 1) / (kThreads * 4)));
-  const int64_t b_ap = std::min<int64_t>(cap, std::max<int64_t>(1, (n / 4 + (kThreads / 32) * 128 - 1) / ((kThreads / 32) * 128)));
+  // The second pass takes one wave of blocks: five fit an SM, a sixth waits for a place, and each block ends with an arrival
+  // at one counter (25 MB: 14.4 -> 12.4 us, 100 MB: 30.8 -> 29.0 us against eight per SM; three per SM 12.9 and 35.1).
+  const int64_t b_ap = std::min<int64_t>(148 * 4, std::max<int64_t>(1, (n / 4 + (kThreads / 32) * 128 - 1) / ((kThreads / 32) * 128)));
   if (!have_minmax) launch(minmax_wide_kernel, (int)b_mm, kThreads, 0, s, (const float*)x.ptr, n, keys);
   launch(dynq_apply_wide_kernel, (int)b_ap, kThreads, 0, s, (const float*)x.ptr, (uint8_t*)y.ptr, keys, params, n);
 }
