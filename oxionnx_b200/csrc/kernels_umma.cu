@@ -263,9 +263,9 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
       const double ring = c.stages * c.kpb;
       const double share = ctas > sms ? 2.0 : 1.0;  // CTAs of this layer on one SM
       double k_us = share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring));
-      // with most SMs at it L2 feeds one no faster than in the persistent kernel (i8 M = 7252 N = 256 K = 2304: 20.6 us here,
-      // 17 us there)
-      if (ctas > 96) k_us = std::max(k_us, share * c.k_per * (c.a_rows + bn) * swz / 110e3);
+      // with most SMs at it and slices longer than the ring, L2 feeds an SM no faster than in the persistent kernel (i8
+      // M = 7252 N = 256 K = 2304: 20.6 us here, 17 us there)
+      if (ctas > 96 && c.k_per > ring) k_us = std::max(k_us, share * c.k_per * (c.a_rows + bn) * swz / 110e3);
       c.us = 3.0 + k_us +
              run_us * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (run_us - 0.7) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
       if (best.bn == 0 || c.us < best.us) best = c;
@@ -330,10 +330,11 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
       }
     }
     // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
-    // estimate above does not count the 3.5 us that the persistent kernel takes to get going).
+    // estimate above does not count the 3.6 us that the persistent kernel takes to get going; at 3.5 the f32 stem of one
+    // frame moves there and the frame takes 2 us more, at 2.5 half of the INT8 frame does, 253 -> 307 us).
     if (tune.cta_pairs != 2) {
       small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu && M > 32 ? 2.5 : 0.7);
-      if (small.bn > 0 && small.us * 1e-6 > best + 3.5e-6) small = SmallShape();
+      if (small.bn > 0 && small.us * 1e-6 > best + 3.6e-6) small = SmallShape();
       if (small.bn > 0) {
         bn = small.bn;
         splits = 1;
