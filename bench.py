@@ -74,7 +74,7 @@ def kernel_source_sha():
     from another version of the kernel is not reported for this one."""
     h = hashlib.sha256()
     csrc = os.path.join(ROOT, "oxionnx_b200", "csrc")
-    for name in ("umma_kernel.cuh", "umma_launch.cuh", "kernels_umma.cu", "umma_i8.cu", "umma_tf32.cu", "umma_f16.cu", "umma_small.cuh", "umma_small_i8.cu",
+    for name in ("umma_kernel.cuh", "umma_epilogue8.cuh", "umma_launch.cuh", "kernels_umma.cu", "umma_i8.cu", "umma_i8_tile.cu", "umma_tf32.cu", "umma_f16.cu", "umma_small.cuh", "umma_small_i8.cu",
                  "umma_small_float.cu"):
         with open(os.path.join(csrc, name), "rb") as fh:
             h.update(fh.read())
