@@ -1133,10 +1133,11 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
 #pragma unroll
         for (int j = 0; j < 8; ++j) __stcg(mine + j * 32, make_uint4(va[4 * j], va[4 * j + 1], va[4 * j + 2], va[4 * j + 3]));
       };
-      // what has been published before is visible before the arrival; the runs of `who` for which this slice is the last
+      // What every lane has published before is ordered before the arrivals: the warp meets, then the lanes that arrive
+      // fence, which carries the others' stores along.  Returns the runs of `who` for which this slice is the last.
       auto arrive = [&](bool who) -> uint32_t {
-        __threadfence();
         __syncwarp();
+        __threadfence();
         const bool last = who && atomicAdd(counters + lane, 1u) == (unsigned int)p.splits - 1u;
         return __ballot_sync(0xffffffffu, last);
       };
@@ -1193,7 +1194,10 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
           if ((owned >> (c - first)) & 1u) publish(c);
         to_finish |= arrive(counts && ((owned >> lane) & 1u) != 0u);
       }
+      // The other way round: the lanes that have seen the arrivals fence, then the warp meets, and every lane may read what
+      // the other slices have published (a ballot alone orders no memory between lanes).
       __threadfence();
+      __syncwarp();
       if (counts && (((to_finish | ready) >> lane) & 1u) != 0u) counters[lane] = 0u;  // nobody arrives there any more: ready for the next launch
 #pragma unroll 1
       for (int c = first; c < end; ++c)

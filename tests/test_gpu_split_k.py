@@ -31,3 +31,44 @@ def test_slices_meet_in_the_order_of_their_index(shape, precision):
         out[most] = runs[0]
     # the same exact products, added in f32 in another order: K additions of terms of 1 / sqrt(K), 2^-24 each
     assert np.max(np.abs(out[0] - out[1])) <= 4 * np.sqrt(c * k * k) * 2.0**-24 * np.abs(out[1]).max()
+
+
+# batch, channels, height, filters: slices of the persistent kernel behind a 3x3 filter of 81 K blocks and more, where the small-problem
+# kernel takes no slice; whole and ragged channel tiles, ragged rows
+INTEGER_SHAPES = [(32, 1152, 7, 256), (11, 1280, 13, 160), (29, 1152, 7, 512)]
+
+
+@pytest.mark.parametrize("shape", INTEGER_SHAPES, ids=str)
+@pytest.mark.parametrize("behind", ["requantisation", "join"])
+def test_integer_slices_are_the_unsplit_sum(shape, behind):
+    n, c, h, oc = shape
+    rng = np.random.default_rng([n, c, h, oc])
+    peak = (1 << 24) // (300 * c * 9)  # accumulators that convert exactly
+    weights = {"w": rng.integers(-peak, peak + 1, (oc, c, 3, 3)).astype(np.float32), "wz": np.int8([0]), "xs": np.float32([0.02]), "z0": np.uint8([0]),
+               "bias": rng.integers(-1000, 1001, oc).astype(np.float32), "as": np.float32([0.07]), "az": np.uint8([128]), "one": np.float32([1]), "ys": np.float32([0.06])}
+    # a standard deviation of about thirty lanes, so that no accumulator can leave the int16 range
+    weights["ws"] = (rng.uniform(0.7, 1.4, oc) * 30 / (40 * peak / np.sqrt(3) * np.sqrt(9 * c)) * 0.07 / 0.02).astype(np.float32)
+    nodes = [Node("QuantizeLinear", "qx", ["x", "xs", "z0"], ["xq"], {}),
+             Node("QLinearConv", "conv", ["xq", "xs", "z0", "w", "ws", "wz", "as", "az", "bias"], ["aq"], {"pads": [1] * 4})]
+    feeds = {"x": np.abs(rng.standard_normal((n, c, h, h))).astype(np.float32)}
+    if behind == "join":
+        nodes += [Node("QuantizeLinear", "qr", ["r", "one", "az"], ["rq"], {}), Node("DequantizeLinear", "da", ["aq", "as", "az"], ["a"], {}),
+                  Node("DequantizeLinear", "db", ["rq", "as", "az"], ["b"], {}), Node("Add", "add", ["a", "b"], ["sum"], {}), Node("Relu", "relu", ["sum"], ["s"], {}),
+                  Node("QuantizeLinear", "qy", ["s", "ys", "z0"], ["yq"], {}), Node("DequantizeLinear", "dy", ["yq", "ys", "z0"], ["y"], {})]
+        # the residual's producer stands in front of the convolution
+        nodes.insert(0, nodes.pop(2))
+        feeds["r"] = (rng.integers(0, 256, (n, oc, h, h)) - 128).astype(np.float32)
+    else:
+        nodes.append(Node("DequantizeLinear", "dy", ["aq", "as", "az"], ["y"], {}))
+    graph = Graph(nodes=nodes, input_names=list(feeds), output_names=["y"])
+    out = {}
+    for most in (0, 1):
+        session = Session.builder().with_tuning(split_k_max=most).build_from_graph(graph, weights)
+        runs = [session.run(feeds)["y"].copy() for _ in range(4)]
+        assert all(np.array_equal(r, runs[0]) for r in runs)
+        kernel = [s["kernel"] for s in session.steps() if s["node"] == "conv" and s["kernel"].startswith("umma")][0]
+        assert ("splitK" in kernel) == (most == 0) and "small" not in kernel and kernel.endswith("+join") == (behind == "join"), kernel
+        session.close()
+        out[most] = runs[0]
+    assert np.array_equal(out[0], out[1])
+    assert np.unique(out[0]).size > 60
