@@ -699,7 +699,14 @@ void Session::fetch_value(const std::string& name, oxb200_result* out) {
   else d = k::Dims4{n, 1, 1, 1};
   k::TensorRef src{v->ptr, v->dt, v->shape.size() == 4 ? v->layout : Layout::PLAIN, d};
   k::TensorRef dst{tmp, DT::F32, Layout::PLAIN, d};
-  k::convert(src, dst, ctx_->stream());
+  const Value* root = v;
+  while (root->alias_of >= 0) root = &values_[root->alias_of];
+  if (root->out_seq > 0) {  // f32 rows that their linear left transposed within sequences: [sequence][channel][row]
+    const int64_t seq = root->out_seq, ch = root->shape.back();
+    k::transpose_perm(v->ptr, tmp, k::Dims4{1, n / (seq * ch), seq, ch}, k::Dims4{0, seq * ch, 1, seq}, ctx_->stream());
+  } else {
+    k::convert(src, dst, ctx_->stream());
+  }
   OXB_CUDA(cudaMemcpyAsync(out->lanes, tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx_->stream()));
   sync();
   ctx_->free_device(tmp);

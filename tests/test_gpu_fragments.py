@@ -96,3 +96,24 @@ def test_values_transposed_by_their_linear():
         out[batch, other_reader] = got["hidden"].reshape(batch // 2, 2, 128, 768)
     for copies in ((42, False), (42, True)):
         assert all(np.array_equal(c, out[2, False][0]) for c in out[copies]), copies
+
+
+def test_transposed_values_are_fetched_in_order():
+    """A value that its linear left transposed is handed out in its logical order, by its own name and by a view's."""
+    from oxionnx_b200 import models
+    rng = np.random.default_rng(6)
+    graph, weights, _, _ = models.build_bert_dynamic_int8(batch=42, seq=128, hidden=768, heads=12, ffn=768, layers=1, vocab=500)
+    upto = [n.name for n in graph.nodes].index("l0_ctx_merge") + 1
+    graph = Graph(nodes=graph.nodes[:upto], input_names=graph.input_names, output_names=["l0_ctx"])
+    feeds = {"input_ids": rng.integers(0, 500, (42, 128)).astype(np.float32), "attention_mask": np.ones((42, 128), np.float32)}
+    got = {}
+    for keep in (False, True):
+        sess = Session.builder().with_keep_intermediates(keep).build_from_graph(graph, weights)
+        sess.run(feeds)
+        assert any(s["kernel"].startswith("transpose") for s in sess.steps()) == keep
+        got[keep] = [sess.fetch_value(name) for name in ("l0_v_out", "l0_v4r")]
+        sess.close()
+    for plain, kept in zip(got[False], got[True]):
+        assert plain.shape == kept.shape and np.unique(kept).size > 1000
+        # the lanes that a TF32 product reads are rounded to eleven bits by their producer where it knows of the product
+        assert np.all(np.abs(plain - kept) <= 2.0**-11 * np.abs(kept))
