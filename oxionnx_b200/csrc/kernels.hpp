@@ -291,14 +291,21 @@ struct UmmaPlan;
 // Choices a context may override (oxb200_config): `requant_f64` 1 keeps the two-pass f64 requantisation even where
 // the one-FMA form is proven, 2 keeps the one-FMA form without the packed 16-bit saturation; `split_k_max` bounds the slices of a split reduction (0: the default of 8, 1: never
 // split); `cta_pairs` 0 lets the tile model decide, 1 never pairs CTAs, 2 pairs them wherever the shape allows.
-// `alloc` gives the device memory of workspaces, null when there is none (the plan then does without).
+// `workspace`, of `workspace_bytes`, is where the slices of a split reduction meet: one for all the plans of a session, whose
+// launches follow one another on its stream (umma_workspace_bytes says what a layer needs).  `alloc` gives the device memory
+// of a plan's arrival counters.  Without either the plan does not split.  `may_split` false says so from the start.
 typedef std::function<void*(size_t)> DeviceAlloc;
 struct UmmaTuning {
   int requant_f64 = 0;
   int split_k_max = 0;
   int cta_pairs = 0;
   DeviceAlloc alloc;
+  void* workspace = nullptr;
+  size_t workspace_bytes = 0;
+  bool may_split = true;  // false: there was no memory for the workspace
 };
+// What umma_plan_create will want of `tune.workspace` for this layer; 0 when it will not split.
+size_t umma_workspace_bytes(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune);
 UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt, void* out, const ConvShape& cs, const Epilogue& e, int kind,
                            const UmmaTuning& tune, std::string* why);
 void umma_plan_destroy(UmmaPlan* p);

@@ -140,8 +140,7 @@ struct UmmaPlan {
   int device;
   size_t smem;
   char desc[176];
-  void* ws = nullptr;        // split-K workspace and arrival counters, owned by the plan
-  void* ws_count = nullptr;
+  void* ws_count = nullptr;  // split K: the arrival counters, owned by the plan
 };
 
 bool umma_available() {
@@ -280,7 +279,7 @@ struct TileChoice {
   bool pair = false;
   SmallShape small;  // bn > 0: the small-problem kernel
 };
-TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int cb, int sms) {
+TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int cb, int sms, bool may_split) {
   // Tile width.  Measured on B200 (1.965 GHz): a tcgen05.mma of 32 bytes of K takes N/2 cycles of the tensor pipe but
   // cannot be issued faster than one per ~56 cycles; one SM fills its shared memory from L2 at about 110 GB/s when all
   // SMs do so; the epilogue has its cost per output and a tile one of its own (below).  The three overlap (ring of stages,
@@ -314,7 +313,7 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
     double best = 1e30;
     for (int cand = bn_max; cand >= 32; cand /= 2) {
       const double tiles = (double)m_tiles * (double)ceil_div(cs.OC, cand);
-      for (int sp = 1; sp <= max_split; ++sp) {
+      for (int sp = 1; sp <= (may_split ? max_split : 1); ++sp) {
         if (sp > 1 && (tiles * sp > 0.92 * sms || k_iters_host / sp < 8)) break;
         const double rounds = std::ceil(tiles * sp / sms);
         const double t_mma = k_steps * std::max(56.0, cand / 2.0) / 1.965e9 / sp;
@@ -368,6 +367,32 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
   return t;
 }
 
+// K blocks a ring stage carries: up to four small ones share a barrier round trip, as long as a stage stays within 64 KB
+// (the ring then still has three stages).
+int blocks_per_stage(size_t kb_bytes, int64_t k_iters) {
+  int kpb = 1;
+  while (kpb < 4 && (size_t)(kpb * 2) * kb_bytes <= 64 * 1024 && kpb * 2 <= k_iters) kpb *= 2;
+  return kpb;
+}
+
+// Slices of K: whole stages each, none empty.  choose_tile leaves a slice at least eight blocks and a stage carries at most
+// four, so there are at least two.
+struct Slices {
+  int count = 1;
+  int64_t k_per = 0;
+  size_t workspace = 0;  // bytes
+};
+Slices cut_slices(const TileChoice& t, int64_t m_tiles, int OC, int64_t k_iters, int swz) {
+  Slices s;
+  s.k_per = k_iters;
+  if (t.splits <= 1) return s;
+  const int kpb = blocks_per_stage((size_t)(BLOCK_M + t.bn) * swz, k_iters);
+  s.k_per = ceil_div(ceil_div(k_iters, (int64_t)t.splits), (int64_t)kpb) * kpb;
+  s.count = (int)ceil_div(k_iters, s.k_per);
+  s.workspace = (size_t)m_tiles * ceil_div(OC, t.bn) * s.count * BLOCK_M * t.bn * 4;
+  return s;
+}
+
 // The variants that the fragment epilogue for f32 lanes takes, over whole groups of 64 channels.
 bool takes_float_fragments(const ConvShape& cs, const Epilogue& e, int kind, const TileChoice& t, int splits) {
   return kind == KIND_I8 && e.mode == EPI_DEQUANT && e.dq_act < 2 && t.small.bn == 0 && t.bn >= 64 && cs.OC % 64 == 0 && splits == 1 && !e.residual;  // not the tanh form of Gelu
@@ -378,8 +403,18 @@ bool takes_float_fragments(const ConvShape& cs, const Epilogue& e, int kind, con
 bool umma_can_transpose(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int seq) {
   const int cb = umma_channel_block(cs.C, kind);
   if (cb == 0 || cs.M() <= 0 || e.dq_act != 0 || seq % 32 != 0 || cs.M() % seq != 0) return false;
-  const TileChoice t = choose_tile(cs, e, kind, tune, cb, sm_count(current_device()));
-  return takes_float_fragments(cs, e, kind, t, t.splits);
+  for (bool may_split : {true, false}) {  // whether there will be a workspace is not known yet
+    const TileChoice t = choose_tile(cs, e, kind, tune, cb, sm_count(current_device()), may_split);
+    if (!takes_float_fragments(cs, e, kind, t, t.splits)) return false;
+  }
+  return true;
+}
+
+size_t umma_workspace_bytes(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune) {
+  const int cb = umma_channel_block(cs.C, kind);
+  if (cb == 0 || cs.M() <= 0) return 0;
+  const TileChoice t = choose_tile(cs, e, kind, tune, cb, sm_count(current_device()), true);
+  return cut_slices(t, ceil_div(cs.M(), BLOCK_M), cs.OC, (int64_t)cs.R * cs.S * (cs.C / cb), cb * umma_elem_bytes(kind)).workspace;
 }
 
 UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt, void* out, const ConvShape& cs, const Epilogue& e, int kind,
@@ -424,18 +459,32 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   const int device = current_device();
   const int sms = sm_count(device);
   const int64_t m_tiles = ceil_div(M, BLOCK_M), k_iters_host = (int64_t)cs.R * cs.S * (cs.C / cb);
-  const TileChoice choice = choose_tile(cs, e, kind, tune, cb, sms);
-  const int bn = choice.bn, splits = choice.splits;
+  TileChoice choice = choose_tile(cs, e, kind, tune, cb, sms, tune.may_split);
+  Slices slices = cut_slices(choice, m_tiles, cs.OC, k_iters_host, swz);
+  void* ws_count = nullptr;
+  if (slices.count > 1) {
+    const size_t cnt = (size_t)m_tiles * ceil_div(cs.OC, choice.bn) * epi_warps(kind) * 4 * sizeof(unsigned int);
+    const bool fits = slices.workspace <= tune.workspace_bytes;
+    if (fits) ws_count = tune.alloc(cnt);
+    if (!ws_count || !zero_now(ws_count, cnt)) {  // no memory for the counters: the tiles of an unsplit run
+      (void)cudaGetLastError();
+      if (ws_count) cudaFree(ws_count);
+      ws_count = nullptr;
+      choice = choose_tile(cs, e, kind, tune, cb, sms, false);
+      slices = cut_slices(choice, m_tiles, cs.OC, k_iters_host, swz);
+    }
+  }
+  const int bn = choice.bn, splits = slices.count;
   const bool pair = choice.pair;
   const SmallShape& small = choice.small;
   const int64_t n_tiles = ceil_div(cs.OC, bn);
-  if (m_tiles * n_tiles > 0x7fffffffLL) return no("grid too large");
+  if (m_tiles * n_tiles > 0x7fffffffLL) return no("grid too large");  // far above a grid that is split
 
   UmmaPlan* pl = new UmmaPlan();
+  pl->ws_count = ws_count;
   pl->kp = KParams();
   KParams& kp = pl->kp;
   auto fail = [&](const char* msg) -> UmmaPlan* {
-    if (pl->ws) cudaFree(pl->ws);
     if (pl->ws_count) cudaFree(pl->ws_count);
     delete pl;
     return no(msg);
@@ -524,8 +573,6 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
   kp.n_tiles = (int)n_tiles;
   kp.m_tiles = pair ? (int)ceil_div(M, 2 * BLOCK_M) : (int)m_tiles;
   kp.idesc = make_idesc(kind, x_dt == DT::I8, w_dt == DT::I8, bn, pair ? 2 * BLOCK_M : BLOCK_M);
-  // K blocks per stage: up to four small ones share a barrier round trip, as long as a stage stays
-  // within 64 KB (the ring then still has three stages)
   // A layer with one channel tile whose packed weights fit beside the ring keeps them in shared memory for the
   // life of the CTA: every tile after a CTA's first then fetches activation rows only.
   {
@@ -534,32 +581,12 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     if (!pair && small.bn == 0 && splits == 1 && n_tiles == 1 && b_total <= 48 * 1024 && m_tiles >= 2 * sms) kp.b_resident_bytes = (uint32_t)b_total;
   }
   const size_t kb_bytes = (size_t)(BLOCK_M + (kp.b_resident_bytes ? 0 : (pair ? bn / 2 : bn))) * swz;
-  int kpb = 1;
-  while (kpb < 4 && (size_t)(kpb * 2) * kb_bytes <= 64 * 1024 && kpb * 2 <= k_iters_host) kpb *= 2;
-  kp.kpb = kpb;
-  // slices of K: whole stages each, none empty
-  kp.splits = 1;
-  kp.k_per = (int)k_iters_host;
+  kp.kpb = blocks_per_stage(kb_bytes, k_iters_host);
+  kp.splits = splits;
+  kp.k_per = (int)slices.k_per;
   if (splits > 1) {
-    const int64_t k_per = ceil_div(ceil_div(k_iters_host, (int64_t)splits), (int64_t)kpb) * kpb;
-    const int64_t eff = ceil_div(k_iters_host, k_per);
-    bool have_ws = false;
-    if (eff > 1) {
-      const size_t ws_words = (size_t)m_tiles * n_tiles * eff * BLOCK_M * bn;
-      const size_t cnt = (size_t)m_tiles * n_tiles * epi_warps(kind) * 4;
-      if ((pl->ws = tune.alloc(ws_words * 4)) && (pl->ws_count = tune.alloc(cnt * sizeof(unsigned int))) &&
-          zero_now(pl->ws_count, cnt * sizeof(unsigned int))) {
-        kp.splits = (int)eff;
-        kp.k_per = (int)k_per;
-        kp.ws = (uint32_t*)pl->ws;
-        kp.ws_count = (unsigned int*)pl->ws_count;
-        have_ws = true;
-      } else {
-        (void)cudaGetLastError();  // no workspace: run unsplit
-      }
-    }
-    // the staged row was sized for one run per store; the unsplit loop stores a warp's whole share at once
-    if (!have_ws && kp.out_tma && (int)warp_row_bytes(bn, kind, dt_size(e.out_dt), false) != kp.out_row_bytes) kp.out_tma = 0;
+    kp.ws = (uint32_t*)tune.workspace;
+    kp.ws_count = (unsigned int*)ws_count;
   }
   kp.mode = e.mode;
   if (e.join) kp.variant = V_JOIN;
@@ -780,9 +807,7 @@ UmmaPlan* umma_plan_create_batched(const BatchedGemm& g, std::string* why) {
   kp.o_rb = g.o_rb, kp.o_rh = g.o_rh, kp.o_ch = g.o_ch;
   kp.idesc = make_idesc(KIND_TF32, false, false, bn, BLOCK_M);
   const size_t kb_bytes = (size_t)(BLOCK_M + bn) * swz;
-  int kpb = 1;
-  while (kpb < 4 && (size_t)(kpb * 2) * kb_bytes <= 64 * 1024 && kpb * 2 <= kp.cblocks) kpb *= 2;
-  kp.kpb = kpb;
+  kp.kpb = blocks_per_stage(kb_bytes, kp.cblocks);
   layout_smem(kp, bn, KIND_TF32, false, &pl->smem);
   kp.mode = EPI_F32;
   kp.variant = g.round_tf32 ? 1 : 0;
@@ -797,14 +822,13 @@ UmmaPlan* umma_plan_create_batched(const BatchedGemm& g, std::string* why) {
   pl->small = 0;
   pl->device = current_device();
   pl->grid = (int)std::min<int64_t>(items * m_tiles * n_tiles, sm_count(pl->device));
-  snprintf(pl->desc, sizeof pl->desc, "umma_tf32 batched %lldx(M=%d N=%d K=%d) tile=128x%dx%dB stages=%dx%d", (long long)items, g.M, g.N, g.K, bn, swz, kp.stages, kpb);
+  snprintf(pl->desc, sizeof pl->desc, "umma_tf32 batched %lldx(M=%d N=%d K=%d) tile=128x%dx%dB stages=%dx%d", (long long)items, g.M, g.N, g.K, bn, swz, kp.stages, kp.kpb);
   return pl;
 }
 
 void umma_plan_destroy(UmmaPlan* p) {
   if (!p) return;
   umma_group_destroy(p->alone);
-  if (p->ws) cudaFree(p->ws);
   if (p->ws_count) cudaFree(p->ws_count);
   delete p;
 }

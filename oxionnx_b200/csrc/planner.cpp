@@ -564,6 +564,15 @@ class Planner {
   std::map<int, DequantStep> dequant_steps_;  // dequantising contractions by the value they write
   bool transposed_at_source(int root_vi, int64_t seq, int heads_node, int reader);
   std::vector<PlanStep> plan_steps_;  // contractions on the tensor cores, in launch order
+  DeviceBuffer split_workspace_{nullptr, 0};  // as large as the layer that wants most of it; the session owns it
+  bool may_split_ = true;
+  k::UmmaTuning tuning() const {
+    k::UmmaTuning t;
+    t.requant_f64 = C.cfg().requant_f64;
+    t.split_k_max = C.cfg().split_k_max;
+    t.cta_pairs = C.cfg().cta_pairs;
+    return t;
+  }
   void link_independent();
   struct LastAdd {
     int step = -1, a = -1, b = -1, y = -1;
@@ -667,6 +676,13 @@ void Planner::run(const std::vector<std::pair<std::string, std::vector<int64_t>>
 
   drop_unread_slices();
   finalize_lifetimes_and_arena();
+  // One workspace for the split reductions of all layers, which run one after the other like everything in the arena: a
+  // layer's slices are at most 136 tiles of 128 KB, so at most 17.8 MB.  When there is no memory the layers run unsplit.
+  if (split_workspace_.bytes > 0) {
+    split_workspace_.ptr = C.try_alloc_device(split_workspace_.bytes);
+    if (split_workspace_.ptr) S.owned_.push_back(split_workspace_);
+    else may_split_ = false;
+  }
   for (auto& st : S.steps_)
     if (st.finalize) st.finalize();
   link_chains();
@@ -1381,11 +1397,11 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       e.minmax_keys = (unsigned int*)V(out_vi).minmax_keys;
       e.out_seq = V(out_vi).out_seq;
       std::string why2;
-      k::UmmaTuning tune;
-      tune.requant_f64 = C.cfg().requant_f64;
-      tune.split_k_max = C.cfg().split_k_max;
-      tune.cta_pairs = C.cfg().cta_pairs;
+      k::UmmaTuning tune = tuning();
       tune.alloc = [this](size_t bytes) { return C.try_alloc_device(bytes); };
+      tune.workspace = split_workspace_.ptr;
+      tune.workspace_bytes = split_workspace_.ptr ? split_workspace_.bytes : 0;
+      tune.may_split = may_split_;
       k::UmmaPlan* plan = k::umma_plan_create(V(x_vi).ptr, xdt, wdev, wdt, V(out_vi).ptr, cs, e, kind, tune, &why2);
       if (!plan) OXB_FAIL("%s '%s': tensor-core plan rejected after selection: %s", n.op.c_str(), n.name.c_str(), why2.c_str());
       S.umma_plans_.push_back(plan);
@@ -1424,6 +1440,7 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
       };
     };
     (void)stp;
+    split_workspace_.bytes = std::max(split_workspace_.bytes, k::umma_workspace_bytes(cs, epi, kind, tuning()));
     if (epi.mode == k::EPI_DEQUANT) dequant_steps_[out_vi] = {cs, epi, kind};
     return;
   }
@@ -3295,11 +3312,7 @@ bool Planner::transposed_at_source(int root_vi, int64_t seq, int heads_node, int
     if (from < 0 || V(vi->second).alias_of < 0) return false;
     node = from;
   }
-  k::UmmaTuning tune;
-  tune.requant_f64 = C.cfg().requant_f64;
-  tune.split_k_max = C.cfg().split_k_max;
-  tune.cta_pairs = C.cfg().cta_pairs;
-  return k::umma_can_transpose(it->second.cs, it->second.epi, it->second.kind, tune, (int)seq);
+  return k::umma_can_transpose(it->second.cs, it->second.epi, it->second.kind, tuning(), (int)seq);
 }
 
 // Softmax over the last axis (nn/normalization.rs softmax_into); other axes are declined.

@@ -72,3 +72,28 @@ def test_integer_slices_are_the_unsplit_sum(shape, behind):
         out[most] = runs[0]
     assert np.array_equal(out[0], out[1])
     assert np.unique(out[0]).size > 60
+
+
+def test_layers_of_a_session_share_one_workspace():
+    """Two and ten layers of the same filters, each of whose slices fill a workspace of several MB: the longer session holds no more of them."""
+    import torch
+    rng = np.random.default_rng(3)
+    weights = {"w": (rng.standard_normal((512, 512, 3, 3)) / np.sqrt(9 * 512)).astype(np.float32), "b": np.zeros(512, np.float32)}
+    feeds = {"x": rng.standard_normal((32, 512, 7, 7)).astype(np.float32)}
+    held = {}
+    for layers in (2, 10):
+        nodes = [Node("Relu", "pre", ["x"], ["x0"], {})]
+        nodes += [Node("Conv", f"c{i}", [f"x{i}", "w", "b"], [f"x{i + 1}"], {"pads": [1] * 4, "activation": "relu"}) for i in range(layers)]
+        graph = Graph(nodes=nodes, input_names=["x"], output_names=[f"x{layers}"])
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        session = Session.builder().build_from_graph(graph, weights)
+        session.run(feeds)
+        held[layers] = before - torch.cuda.mem_get_info()[0]
+        split = [s["kernel"] for s in session.steps() if "splitK" in s["kernel"]]
+        session.close()
+        assert len(split) == layers and not any("small" in s for s in split), split
+    tile = [int(v) for v in split[0].split("tile=")[1].split("x")[:2]]
+    workspace = -(-32 * 49 // tile[0]) * (512 // tile[1]) * int(split[0].split("splitK=")[1].split()[0]) * tile[0] * tile[1] * 4
+    assert workspace >= 4 << 20
+    assert held[10] - held[2] < 2 * workspace, (held, workspace)
