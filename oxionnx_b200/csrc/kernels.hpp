@@ -317,6 +317,8 @@ void umma_launch(const UmmaPlan* p, int* err_flag, cudaStream_t s);
 // all small ones of one kind.  The group keeps what it needs of the plans.
 struct UmmaGroup;
 constexpr int kGroupMax = 3;
+// Whether a join (Epilogue::join and its constants set) is one that the fragment epilogue takes.
+bool umma_join_takes_fragments(const ConvShape& cs, const Epilogue& e);
 // Whether a dequantising contraction of this shape can write its rows transposed within sequences of `seq` rows (out_seq).
 bool umma_can_transpose(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int seq);
 bool umma_plans_group(const UmmaPlan* a, const UmmaPlan* b);  // may the two be members of one group?

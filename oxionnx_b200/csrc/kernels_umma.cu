@@ -400,6 +400,13 @@ bool takes_float_fragments(const ConvShape& cs, const Epilogue& e, int kind, con
 
 }  // namespace
 
+// Whole groups of 64 channels, a lane that spans its type (the saturating fma clamps to nothing narrower) and constants for
+// the scaled lane.
+bool umma_join_takes_fragments(const ConvShape& cs, const Epilogue& e) {
+  const int lo = (e.relu_fused && e.lo < 0) ? 0 : e.lo;
+  return e.join && e.join_d > 0.f && e.hi - lo == 255 && cs.OC % 64 == 0;
+}
+
 bool umma_can_transpose(const ConvShape& cs, const Epilogue& e, int kind, const UmmaTuning& tune, int seq) {
   const int cb = umma_channel_block(cs.C, kind);
   if (cb == 0 || cs.M() <= 0 || e.dq_act != 0 || seq % 32 != 0 || cs.M() % seq != 0) return false;
@@ -617,7 +624,7 @@ UmmaPlan* umma_plan_create(const void* x, DT x_dt, const void* w_packed, DT w_dt
     // Whole groups of 64 channels, as 8-bit outputs or dequantised, take the fragment epilogues (umma_epilogue8.cuh) wherever
     // their arithmetic is allowed: they are the faster ones at every K (the figures stand there).
     const bool frag_ok = kind == KIND_I8 && bn >= 64 && cs.OC % 64 == 0 && kp.splits == 1 && ((uintptr_t)e.residual & 15) == 0;
-    const bool join_ok = kp.variant == V_JOIN && e.join_d > 0.f && kp.hi - kp.lo == 255;
+    const bool join_ok = kp.variant == V_JOIN && umma_join_takes_fragments(cs, e);
     const int perm = takes_float_fragments(cs, e, kind, choice, kp.splits) ? 16 : (frag_ok && (kp.variant == V_REQUANT_PACKED || join_ok) ? 64 : 0);
     if (e.out_seq > 0 && perm != 16) return fail("transposed rows need the fragment epilogue");
     kp.out_seq = e.out_seq;

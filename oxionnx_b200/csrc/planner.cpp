@@ -1274,6 +1274,15 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
     take = take && (double)acc_abs_bound * cmax * 1.0001 + std::fabs((double)epi.y_zp) + 1.0 < 32000.0;
     if (take) take = k::residual_join_constants(c.join_rp, epi.out_dt, V(c.join_other).dt, &jc);
     if (take) {
+      // With the fragment epilogue the join costs a layer less than its own pass over memory at every K and size, also where
+      // both are bound by their epilogue and nothing stays in L2 (1x1 64 -> 256 at M = 3211264: 497 us joined, 228 + 413
+      // apart; at M = 802816 129 joined, 62 + 105 apart).  The general epilogue bounds a layer of short K by itself, and the
+      // join doubles its instructions: over a tensor that does not stay in L2 the pass of its own is the faster one.
+      k::Epilogue joined = epi;
+      joined.join = 1, joined.join_d = jc.d;
+      take = k::umma_join_takes_fragments(cs, joined) || cs.K() >= 128 || prod(c.out_shape) <= (64ll << 20);
+    }
+    if (take) {
       for (int i : c.join_nodes) skipped_[i] = 1;
       epi.join = 1;
       epi.join_a = jc.ca, epi.join_b = jc.cb, epi.join_c = jc.cc, epi.join_lo = jc.lo, epi.join_hi = jc.hi;
@@ -3549,9 +3558,6 @@ void Planner::match_join(Contraction& c) {
     }
     return true;
   };
-  // Taken at every K and size: with the fragment epilogue the join costs a layer less than its own pass over memory even
-  // where both are bound by their epilogue and nothing stays in L2 (1x1 64 -> 256 at M = 3211264: 497 us joined, 228 + 413
-  // apart; at M = 802816 129 joined, 62 + 105 apart).
   k::ResidualParams rp{};
   bool has_zp;
   const int dq_i = only_consumer(c.out_name);

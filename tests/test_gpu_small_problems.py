@@ -266,6 +266,34 @@ def test_quantised_joins_in_the_epilogue_are_the_separate_nodes(shape, join):
     assert np.unique(want["y"]).size > 20  # not only the ends of the range
 
 
+# a 1x1 filter of 32 channels whose outputs are a few more, or a few fewer, than 64 Mi: images, filters, a Relu on the lane itself, joined or not
+SHORT_JOINS = [(56, 96, False, False), (55, 96, False, True), (84, 64, False, True), (84, 64, True, False), (83, 64, True, True)]
+
+
+@pytest.mark.parametrize("images, oc, lane_relu, joins", SHORT_JOINS)
+def test_short_joins_past_l2_are_fused_where_the_fragments_take_them(images, oc, lane_relu, joins):
+    rng = np.random.default_rng([images, oc])
+    weights = {"xs": np.float32([0.02]), "xz": np.uint8([0]), "as": np.float32([0.07615]), "az": np.int8([0]), "bs": np.float32([0.08084]), "bz": np.int8([5]),
+               "ys": np.float32([0.06283]), "yz": np.int8([-9]), "z0": np.float32([0])}
+    nodes = [Node("QuantizeLinear", "qx", ["x", "xs", "xz"], ["xq"], {})]
+    for name, scale, zp in (("b", "bs", "bz"), ("a", "as", "az")):
+        weights[name + "w"] = rng.integers(-127, 128, (oc, 32, 1, 1)).astype(np.float32)
+        weights[name + "ws"] = (rng.uniform(0.7, 1.4, oc) * 0.003).astype(np.float32)
+        weights[name + "bias"] = rng.integers(-1000, 1001, oc).astype(np.float32)
+        nodes.append(Node("QLinearConv", "conv_" + name, ["xq", "xs", "xz", name + "w", name + "ws", "z0", scale, zp, name + "bias"], [name + "q"], {}))
+    if lane_relu:
+        nodes.append(Node("Relu", "lane", ["aq"], ["ar"], {}))
+    nodes += [Node("DequantizeLinear", "da", ["ar" if lane_relu else "aq", "as", "az"], ["a"], {}), Node("DequantizeLinear", "db", ["bq", "bs", "bz"], ["b"], {}),
+              Node("Add", "add", ["a", "b"], ["sum"], {}), Node("QuantizeLinear", "qy", ["sum", "ys", "yz"], ["yq"], {}),
+              Node("DequantizeLinear", "dy", ["yq", "ys", "yz"], ["y"], {}), Node("GlobalAveragePool", "gap", ["y"], ["z"], {})]
+    graph = Graph(nodes=nodes, input_names=["x"], output_names=["z"])
+    feeds = {"x": np.abs(rng.standard_normal((images, 32, 112, 112), dtype=np.float32))}
+    got, kernels = _run(graph, weights, feeds)
+    assert any(s.endswith("+join") for s in kernels) == joins and any(s.startswith("residual_requant") for s in kernels) != joins, kernels
+    want, _ = _run(graph, weights, feeds, keep_intermediates=True)
+    assert np.array_equal(got["z"], want["z"])
+
+
 def test_side_by_side_products_are_one_launch():
     rng = np.random.default_rng(5)
     weights, nodes, outs = {}, [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {})], []
