@@ -1276,11 +1276,15 @@ void Planner::emit_contraction(const NodeDef& n, Contraction& c) {
     if (take) {
       // With the fragment epilogue the join costs a layer less than its own pass over memory at every K and size, also where
       // both are bound by their epilogue and nothing stays in L2 (1x1 64 -> 256 at M = 3211264: 497 us joined, 228 + 413
-      // apart; at M = 802816 129 joined, 62 + 105 apart).  The general epilogue bounds a layer of short K by itself, and the
-      // join doubles its instructions: over a tensor that does not stay in L2 the pass of its own is the faster one.
+      // apart; at M = 802816 121 joined, 66 + 107 apart).  The general epilogue bounds a layer of 64 lanes of K by itself, and
+      // the join doubles its instructions: over a tensor that does not stay in L2 the pass of its own is the faster one
+      // (M = 802816: 256 filters with a Relu of their own 217 us joined, 171 apart; 96 filters 115 and 97, 160 189 and 152, 288
+      // 285 and 247).  From 32 lanes of K it makes no such difference (96 filters 99 and 97, 224 179 and 187), and a tile of
+      // 32 channels has one run a warp (32 filters at M = 2207744: 103 and 119).
       k::Epilogue joined = epi;
       joined.join = 1, joined.join_d = jc.d;
-      take = k::umma_join_takes_fragments(cs, joined) || cs.K() >= 128 || prod(c.out_shape) <= (64ll << 20);
+      const bool epilogue_bound = cs.K() > 32 && cs.K() < 128 && cs.OC > 32 && prod(c.out_shape) > (64ll << 20);
+      take = k::umma_join_takes_fragments(cs, joined) || !epilogue_bound;
     }
     if (take) {
       for (int i : c.join_nodes) skipped_[i] = 1;

@@ -231,7 +231,12 @@ JOINS = {"unsigned relu": (("u8", 128, 0.07622), ("u8", 0, 0.04274), ("u8", 0, 0
 JOIN_SHAPES = [(1, 64, 9, 7, 96, 1, "auto", "small"), (1, 512, 7, 7, 160, 1, "auto", "small"), (1, 128, 13, 11, 64, 3, "auto", "small"),
                (1, 64, 61, 43, 288, 1, "always", "cta-pair"), (1, 512, 61, 43, 544, 1, "always", "cta-pair"), (2, 64, 30, 31, 256, 3, "always", "cta-pair"),
                (1, 64, 139, 137, 256, 1, "never", "residual-buffers=4"), (1, 512, 137, 137, 384, 1, "never", "residual-buffers=3"),
-               (1, 1024, 137, 137, 256, 1, "never", "residual-buffers=2"), (2, 64, 139, 137, 32, 3, "never", "residual-buffers")]
+               (1, 1024, 137, 137, 256, 1, "never", "residual-buffers=2"), (2, 64, 139, 137, 32, 3, "never", "residual-buffers"),
+               # whole groups of 64 filters (the fragment epilogue) with a ragged last channel tile in a CTA pair, and 32 more than that (the
+               # general epilogue) at every depth of the staging
+               (1, 64, 61, 43, 320, 1, "always", "cta-pair fragments"), (1, 512, 61, 43, 448, 1, "always", "cta-pair fragments"),
+               (1, 64, 139, 137, 288, 1, "never", "residual-buffers=4"), (1, 512, 137, 137, 352, 1, "never", "residual-buffers=3"),
+               (1, 1024, 137, 137, 224, 1, "never", "residual-buffers=2")]
 
 
 @pytest.mark.parametrize("shape", JOIN_SHAPES, ids=str)
@@ -259,25 +264,28 @@ def test_quantised_joins_in_the_epilogue_are_the_separate_nodes(shape, join):
     feeds = {"x": rng.standard_normal((n, c, h, w)).astype(np.float32),
              "r": (rng.integers(0, 256, (n, oc, h, w)) - 128).astype(np.float32)}
     got, kernels = _run(graph, weights, feeds, cta_pairs=pairs)
-    assert any(s.endswith("+join") and says in s for s in kernels), kernels
+    joined = [s for s in kernels if s.endswith("+join")]
+    assert len(joined) == 1 and says in joined[0], kernels
+    # the persistent kernel joins whole groups of 64 filters in its fragment epilogue, everything else in its general one
+    assert ("fragments" in joined[0]) == (says != "small" and oc % 64 == 0), joined
     want, apart = _run(graph, weights, feeds, cta_pairs=pairs, keep_intermediates=True)
     assert not any("+join" in s for s in apart)
     assert np.array_equal(got["y"], want["y"])
     assert np.unique(want["y"]).size > 20  # not only the ends of the range
 
 
-# a 1x1 filter of 32 channels whose outputs are a few more, or a few fewer, than 64 Mi: images, filters, a Relu on the lane itself, joined or not
-SHORT_JOINS = [(56, 96, False, False), (55, 96, False, True), (84, 64, False, True), (84, 64, True, False), (83, 64, True, True)]
+# a 1x1 filter whose outputs are a few more, or a few fewer, than 64 Mi: images, channels, filters, a Relu on the lane itself, joined or not
+SHORT_JOINS = [(56, 64, 96, False, False), (55, 64, 96, False, True), (56, 32, 96, False, True), (84, 64, 64, False, True), (84, 64, 64, True, False), (83, 64, 64, True, True)]
 
 
-@pytest.mark.parametrize("images, oc, lane_relu, joins", SHORT_JOINS)
-def test_short_joins_past_l2_are_fused_where_the_fragments_take_them(images, oc, lane_relu, joins):
+@pytest.mark.parametrize("images, c, oc, lane_relu, joins", SHORT_JOINS)
+def test_short_joins_past_l2_are_fused_where_the_fragments_take_them(images, c, oc, lane_relu, joins):
     rng = np.random.default_rng([images, oc])
     weights = {"xs": np.float32([0.02]), "xz": np.uint8([0]), "as": np.float32([0.07615]), "az": np.int8([0]), "bs": np.float32([0.08084]), "bz": np.int8([5]),
                "ys": np.float32([0.06283]), "yz": np.int8([-9]), "z0": np.float32([0])}
     nodes = [Node("QuantizeLinear", "qx", ["x", "xs", "xz"], ["xq"], {})]
     for name, scale, zp in (("b", "bs", "bz"), ("a", "as", "az")):
-        weights[name + "w"] = rng.integers(-127, 128, (oc, 32, 1, 1)).astype(np.float32)
+        weights[name + "w"] = rng.integers(-127, 128, (oc, c, 1, 1)).astype(np.float32)
         weights[name + "ws"] = (rng.uniform(0.7, 1.4, oc) * 0.003).astype(np.float32)
         weights[name + "bias"] = rng.integers(-1000, 1001, oc).astype(np.float32)
         nodes.append(Node("QLinearConv", "conv_" + name, ["xq", "xs", "xz", name + "w", name + "ws", "z0", scale, zp, name + "bias"], [name + "q"], {}))
@@ -287,7 +295,7 @@ def test_short_joins_past_l2_are_fused_where_the_fragments_take_them(images, oc,
               Node("Add", "add", ["a", "b"], ["sum"], {}), Node("QuantizeLinear", "qy", ["sum", "ys", "yz"], ["yq"], {}),
               Node("DequantizeLinear", "dy", ["yq", "ys", "yz"], ["y"], {}), Node("GlobalAveragePool", "gap", ["y"], ["z"], {})]
     graph = Graph(nodes=nodes, input_names=["x"], output_names=["z"])
-    feeds = {"x": np.abs(rng.standard_normal((images, 32, 112, 112), dtype=np.float32))}
+    feeds = {"x": np.abs(rng.standard_normal((images, c, 112, 112), dtype=np.float32))}
     got, kernels = _run(graph, weights, feeds)
     assert any(s.endswith("+join") for s in kernels) == joins and any(s.startswith("residual_requant") for s in kernels) != joins, kernels
     want, _ = _run(graph, weights, feeds, keep_intermediates=True)
