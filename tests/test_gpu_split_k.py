@@ -10,6 +10,8 @@ pytestmark = pytest.mark.gpu
 # batch, channels, height, filters, kernel: two to eight slices of 128 and 256 columns, ragged rows, a ragged channel tile
 SHAPES = [(32, 256, 14, 256, 3), (8, 512, 7, 512, 3), (32, 512, 7, 512, 3), (29, 2048, 7, 480, 1), (7, 512, 7, 200, 3)]
 
+UNSPLIT_16 = [SHAPES[0]]  # half the K blocks in 16 bits: whole sums there; the others meet in the workspace (SHAPES[2]) or within a cluster
+
 
 @pytest.mark.parametrize("shape", SHAPES, ids=str)
 @pytest.mark.parametrize("precision", ["tf32", "bf16"])
@@ -25,8 +27,8 @@ def test_slices_meet_in_the_order_of_their_index(shape, precision):
         runs = [session.run(feeds)["y"].copy() for _ in range(4)]
         assert all(np.array_equal(r, runs[0]) for r in runs), "the sum depends on who arrived when"
         kernels = [s["kernel"] for s in session.steps()]
-        if precision == "tf32":
-            assert any("splitK" in s for s in kernels) == (most == 0), kernels
+        split = most == 0 and not (precision == "bf16" and shape in UNSPLIT_16)
+        assert any("splitK" in s for s in kernels) == split, kernels
         session.close()
         out[most] = runs[0]
     # the same exact products, added in f32 in another order: K additions of terms of 1 / sqrt(K), 2^-24 each
@@ -45,15 +47,16 @@ def test_integer_slices_are_the_unsplit_sum(shape, behind):
     rng = np.random.default_rng([n, c, h, oc])
     peak = (1 << 24) // (300 * c * 9)  # accumulators that convert exactly
     weights = {"w": rng.integers(-peak, peak + 1, (oc, c, 3, 3)).astype(np.float32), "wz": np.int8([0]), "xs": np.float32([0.02]), "z0": np.uint8([0]),
-               "bias": rng.integers(-1000, 1001, oc).astype(np.float32), "as": np.float32([0.07]), "az": np.uint8([128]), "one": np.float32([1]), "ys": np.float32([0.06])}
+               "bias": rng.integers(-1000, 1001, oc).astype(np.float32), "as": np.float32([0.07622]), "az": np.uint8([128]), "one": np.float32([1]),
+               "bs": np.float32([0.04274]), "ys": np.float32([0.05397])}
     # a standard deviation of about thirty lanes, so that no accumulator can leave the int16 range
-    weights["ws"] = (rng.uniform(0.7, 1.4, oc) * 30 / (40 * peak / np.sqrt(3) * np.sqrt(9 * c)) * 0.07 / 0.02).astype(np.float32)
+    weights["ws"] = (rng.uniform(0.7, 1.4, oc) * 30 / (40 * peak / np.sqrt(3) * np.sqrt(9 * c)) * 0.07622 / 0.02).astype(np.float32)
     nodes = [Node("QuantizeLinear", "qx", ["x", "xs", "z0"], ["xq"], {}),
              Node("QLinearConv", "conv", ["xq", "xs", "z0", "w", "ws", "wz", "as", "az", "bias"], ["aq"], {"pads": [1] * 4})]
     feeds = {"x": np.abs(rng.standard_normal((n, c, h, h))).astype(np.float32)}
     if behind == "join":
         nodes += [Node("QuantizeLinear", "qr", ["r", "one", "az"], ["rq"], {}), Node("DequantizeLinear", "da", ["aq", "as", "az"], ["a"], {}),
-                  Node("DequantizeLinear", "db", ["rq", "as", "az"], ["b"], {}), Node("Add", "add", ["a", "b"], ["sum"], {}), Node("Relu", "relu", ["sum"], ["s"], {}),
+                  Node("DequantizeLinear", "db", ["rq", "bs", "z0"], ["b"], {}), Node("Add", "add", ["a", "b"], ["sum"], {}), Node("Relu", "relu", ["sum"], ["s"], {}),
                   Node("QuantizeLinear", "qy", ["s", "ys", "z0"], ["yq"], {}), Node("DequantizeLinear", "dy", ["yq", "ys", "z0"], ["y"], {})]
         # the residual's producer stands in front of the convolution
         nodes.insert(0, nodes.pop(2))
