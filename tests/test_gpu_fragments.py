@@ -1,6 +1,7 @@
 """The fragment epilogues of the persistent integer kernel (csrc/umma_epilogue8.cuh): every tile width, ragged rows and
-channel tiles, weights in the ring and resident, every bound of the saturation.  The same layers through the general
-epilogue are the reference; joins with a residual are covered by test_gpu_small_problems.py."""
+channel tiles, weights in the ring and resident, every bound of the saturation, activations with a zero point and without.
+The same layers through the general epilogue, or their nodes one by one, are the reference.  Joins with a residual are covered
+by test_quantised_joins_in_the_epilogue_are_the_separate_nodes, which says for each which epilogue it takes."""
 import numpy as np
 import pytest
 
@@ -55,14 +56,15 @@ LINEARS = [(20001, 64, 192, False), (4099, 256, 1088, True), (9001, 768, 320, Fa
 
 @pytest.mark.parametrize("rows, k, n, gelu", LINEARS)
 @pytest.mark.parametrize("pairs", ["never", "always"])
-def test_fragment_dequantisation_is_the_separate_nodes(rows, k, n, gelu, pairs):
+@pytest.mark.parametrize("zero_point", [True, False])
+def test_fragment_dequantisation_is_the_separate_nodes(rows, k, n, gelu, pairs, zero_point):
     if pairs == "always" and n < 256:
         pytest.skip("a pair shares a 256-wide tile")
     rng = np.random.default_rng([rows, k, n])
     w = {"w": np.clip(np.rint(rng.standard_normal((k, n)) * 40.0), -127, 127).astype(np.float32),
          "ws": rng.uniform(0.0005, 0.002, n).astype(np.float32), "bias": (rng.standard_normal(n) * 0.5 + 0.8).astype(np.float32)}
     nodes = [Node("DynamicQuantizeLinear", "q0", ["x"], ["xq", "xs", "xz"], {}),
-             Node("MatMulInteger", "mmi", ["xq", "w", "xz"], ["acc"], {}), Node("Cast", "cast", ["acc"], ["accf"], {"to": 1}),
+             Node("MatMulInteger", "mmi", ["xq", "w"] + ["xz"] * zero_point, ["acc"], {}), Node("Cast", "cast", ["acc"], ["accf"], {"to": 1}),
              Node("Mul", "scales", ["xs", "ws"], ["sc"], {}), Node("Mul", "rescale", ["accf", "sc"], ["scaled"], {}),
              Node("Add", "addb", ["scaled", "bias"], ["lin"], {})]
     if gelu:
@@ -78,7 +80,9 @@ def test_fragment_dequantisation_is_the_separate_nodes(rows, k, n, gelu, pairs):
         assert np.array_equal(got[name], want[name]), name
 
 
-def test_values_transposed_by_their_linear():
+@pytest.mark.parametrize("pairs", ["never", "always"])
+@pytest.mark.parametrize("zero_point", [True, False])
+def test_values_transposed_by_their_linear(pairs, zero_point):
     """V leaves its linear in the layout that the attention kernel reads, unless somebody else reads it too.  Copies of two
     sentences have the extrema of the two, so every copy is the small batch's, where V is transposed by a launch of its own."""
     from oxionnx_b200 import models
@@ -88,9 +92,17 @@ def test_values_transposed_by_their_linear():
     out = {}
     for batch, other_reader in ((2, False), (42, False), (42, True)):
         graph, weights, _, _ = models.build_bert_dynamic_int8(batch=batch, seq=128, hidden=768, heads=12, ffn=768, layers=2, vocab=500)
+        if not zero_point:
+            for node in graph.nodes:
+                if node.name in ("l0_v_mmi", "l1_v_mmi"):
+                    node.inputs = node.inputs[:2]
         if other_reader:
             graph = Graph(nodes=graph.nodes, input_names=graph.input_names, output_names=graph.output_names + ["l0_v_out"])
-        got, kernels = _run(graph, weights, {"input_ids": np.tile(ids, (batch // 2, 1)), "attention_mask": np.tile(mask, (batch // 2, 1))})
+        got, kernels = _run(graph, weights, {"input_ids": np.tile(ids, (batch // 2, 1)), "attention_mask": np.tile(mask, (batch // 2, 1))},
+                            cta_pairs=pairs if batch > 2 else "never")
+        if batch > 2:
+            values = [s for s in kernels if s.endswith("fragments +dequant") and "N=768 K=768" in s]
+            assert values and all(("cta-pair" in s) == (pairs == "always") for s in values), kernels
         assert sum("umma_attention" in s for s in kernels) == 2, kernels
         assert sum(s.startswith("transpose") for s in kernels) == (2 if batch == 2 else int(other_reader)), kernels
         out[batch, other_reader] = got["hidden"].reshape(batch // 2, 2, 128, 768)
