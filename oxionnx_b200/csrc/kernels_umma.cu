@@ -263,7 +263,9 @@ SmallShape choose_small(int64_t M, int OC, int64_t k_iters, int swz, int sms, in
       const double share = ctas > sms ? 2.0 : 1.0;  // CTAs of this layer on one SM
       double k_us = share * (0.12 * std::min<double>(c.k_per, ring) + 1.7 / ring * std::max(0.0, c.k_per - ring));
       // with most SMs at it and slices longer than the ring, L2 feeds an SM no faster than in the persistent kernel (i8
-      // M = 7252 N = 256 K = 2304: 20.6 us here, 17 us there)
+      // M = 7252 N = 256 K = 2304: 20.6 us here, 17 us there).  "Most" is two thirds: over 30 networks of few items (f32 and
+      // INT8 residual networks of 1 - 3 images of 160 - 256, encoders, MLPs) the mean is 0.5 % worse without the term, and the
+      // same within 0.3 % from half the SMs (two f32 networks 4 % faster, encoder of 2x77 tokens 1 % slower) to four fifths.
       if (ctas > 96 && c.k_per > ring) k_us = std::max(k_us, share * c.k_per * (c.a_rows + bn) * swz / 110e3);
       c.us = 3.0 + k_us +
              run_us * (share * std::ceil((bn / 32) / (double)sp) - 1.0) + (run_us - 0.7) + (sp > 1 ? 1.1 + 0.2 * (bn / 32) : 0.0);
@@ -303,9 +305,15 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
   {
     const double k_bytes = (double)cs.K() * es;
     const double k_steps = k_bytes / 32.0;
-    // epilogue: per output 0.045 ns for integers, 0.03 ns float, plus 0.25 us per tile whatever its width;
-    // with a Gelu behind it 0.2 ns (and 2.5 us for a run of the small-problem kernel), which moves M = 8192 N = 3072 K = 768
-    // from 6 rounds of 256 columns to 11 of 128 (61.5 -> 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us)
+    // epilogue: per output 0.045 ns for integers, 0.03 ns float, plus 0.25 us per tile whatever its width.  These are the
+    // fragment epilogue's; the layers that it does not take need no others: over 26 of them (QLinearConv of 96 - 480 filters,
+    // int32 outputs, M = 2048 - 401408, K = 64 - 1152) the choice is at most 2.1 us from the best width, 10.5 us in sum, and
+    // with 0.07 ns and 0.5 us, the general epilogue's before the roles of one thread, 2.1 and 10.3.
+    // With a Gelu behind it 0.2 ns, which moves M = 8192 N = 3072 K = 768 from 6 rounds of 256 columns to 11 of 128 (61.5 ->
+    // 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us), and 2 us for a run of the small-problem kernel:
+    // whatever the rows (1 - 400), its tiles of 32 / 64 / 128 channels take 0 - 2 / 2 - 4 / 4 - 6 us more than without one.
+    // From 1 to 2.5 us a run the choice is the best of its neighbours but once (M = 300 N = 2048 K = 512: 14.5 us up to 2 us a
+    // run, 16.4 from there on); at 3 us few rows leave that kernel.
     const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
     const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.045e-9);
     const double t_tile_fixed = 0.25e-6;
@@ -328,12 +336,13 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
         }
       }
     }
-    // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one (the
-    // estimate above does not count the 3.6 us that the persistent kernel takes to get going; at 3.5 the f32 stem of one
-    // frame moves there and the frame takes 2 us more, at 2.5 half of the INT8 frame does, 253 -> 307 us).
+    // A problem of at most a wave of tiles: the small-problem kernel where its estimate is the shorter one, counting the
+    // 4 us that the persistent kernel takes to get going.  Over the 30 networks above the mean is flat from 3.7 to 4.5 us
+    // (within 0.2 %); at 3.2 it is 1 % worse (INT8 network of 3 images of 192 302 us instead of 291, f32 of 2 of 224 495 instead of
+    // 490) and at 2.5 10 % (one INT8 frame 308 instead of 255).
     if (tune.cta_pairs != 2) {
-      small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu && M > 32 ? 2.5 : 0.7);
-      if (small.bn > 0 && small.us * 1e-6 > best + 3.6e-6) small = SmallShape();
+      small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu ? 2.0 : 0.7);
+      if (small.bn > 0 && small.us * 1e-6 > best + 4e-6) small = SmallShape();
       if (small.bn > 0) {
         bn = small.bn;
         splits = 1;
