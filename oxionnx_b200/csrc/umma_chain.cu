@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1) umma_chain_kernel(const __gr
             const uint32_t desc_hi = (uint32_t)(desc_rest >> 32), desc_lo = (uint32_t)desc_rest;
             const uint32_t w16 = (base + L.w_off) >> 4, x16 = (base + p.x_off) >> 4;
             for (int i = 0; i < L.kb; ++i)
-              tc_mma_block<KIND_I8, false>(tmem_base, desc_lo | ((w16 + (uint32_t)i * (CHAIN_W_TILE >> 4)) & 0x3fffu),
-                                           desc_lo | ((x16 + (uint32_t)i * (CHAIN_X_TILE >> 4)) & 0x3fffu), desc_hi, L.idesc, i > 0 ? 1u : 0u, 4u);
+              tc_mma_block<KIND_I8>(tmem_base, desc_lo | ((w16 + (uint32_t)i * (CHAIN_W_TILE >> 4)) & 0x3fffu),
+                                    desc_lo | ((x16 + (uint32_t)i * (CHAIN_X_TILE >> 4)) & 0x3fffu), desc_hi, L.idesc, i > 0 ? 1u : 0u);
             tc_commit<false>(smem_u32(&bar_mma));
           }
           __syncwarp();

@@ -264,8 +264,8 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
   return p != 0;
 }
-// One MMA of 32 bytes of K from two complete descriptors (43 cycles each when issued back to back by one thread;
-// assembling them inside the asm block, as tc_mma_block does, takes 70).
+// One MMA of 32 bytes of K from two complete descriptors (43 cycles each when issued back to back by one thread; with the
+// descriptors assembled from 32-bit words inside the asm block it was 70).
 template <int KIND, bool PAIR = false>
 __device__ __forceinline__ void tc_mma_one(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
 #define OXB_MMA_ONE(GROUP, KINDSTR)                                                                                                        \
@@ -284,17 +284,13 @@ __device__ __forceinline__ void tc_mma_one(uint32_t tmem_d, uint64_t da, uint64_
   }
 #undef OXB_MMA_ONE
 }
-// The MMAs of one K block (1, 2 or 4 of 32 bytes of K each) from the two words of its descriptors.
-template <int KIND, bool PAIR>
-__device__ __forceinline__ void tc_mma_block(uint32_t tmem_d, uint32_t lo_a, uint32_t lo_b, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate,
-                                             uint32_t mmas) {
+// The four MMAs of one K block of 128 bytes from the two words of its descriptors (chain and probe kernels).
+template <int KIND>
+__device__ __forceinline__ void tc_mma_block(uint32_t tmem_d, uint32_t lo_a, uint32_t lo_b, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
   const uint64_t hi = (uint64_t)desc_hi << 32, da = hi | lo_a, db = hi | lo_b;
-  tc_mma_one<KIND, PAIR>(tmem_d, da, db, idesc, accumulate);
-  if (mmas >= 2) tc_mma_one<KIND, PAIR>(tmem_d, da + 2, db + 2, idesc, 1u);
-  if (mmas >= 4) {
-    tc_mma_one<KIND, PAIR>(tmem_d, da + 4, db + 4, idesc, 1u);
-    tc_mma_one<KIND, PAIR>(tmem_d, da + 6, db + 6, idesc, 1u);
-  }
+  tc_mma_one<KIND>(tmem_d, da, db, idesc, accumulate);
+#pragma unroll
+  for (int k = 2; k < 8; k += 2) tc_mma_one<KIND>(tmem_d, da + k, db + k, idesc, 1u);
 }
 
 // Shared-memory matrix descriptor, K-major operand, swizzled rows of `swz` bytes: start
@@ -328,8 +324,7 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[3
         "=r"(r[31])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// The same wait, naming the registers a pending read lands in: nothing that uses them may be scheduled above it.
+// The wait for a pending read, naming the registers it lands in: nothing that uses them may be scheduled above it.
 // Neither this nor the read itself is a compiler barrier for memory: the per-channel parameter loads of the run's
 // math may be started above the wait, so that their latency (the top stall of the short-K layers) overlaps it.
 __device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[32]) {
@@ -1113,8 +1108,8 @@ __device__ __forceinline__ void epilogue_role(const KParams& p, int warp, int la
     if constexpr (SPLIT) {
       // Every run of the tile has an owner among the slices.  A slice first publishes the runs it does not own (all of them
       // behind one fence, then one arrival at each run's counter), then turns to its own: when every other slice has
-      // published such a run by then, it adds them to its own accumulators straight from tensor memory; after a short
-      // patience it publishes the run itself instead, and whoever arrives last finishes it.  So nobody waits for a slice
+      // published such a run by then, it adds them to its own accumulators straight from tensor memory; after 32 looks at the
+      // counters (12400 cycles, 6.3 us) it publishes the run itself instead, and whoever arrives last finishes it.  So nobody waits for a slice
       // that may not be running, but slices that end together share the finishing and write no more than they must.
       constexpr bool kFloatAcc = VARIANT < V_REQUANT;
       const int split = t - tt * p.splits;
@@ -1332,7 +1327,9 @@ __global__ void __launch_bounds__(64 + 32 * epi_warps(KIND), 1) umma_conv_kernel
 
   // The producer and the MMA issuer are one elected thread each; the other lanes of its warp wait at the warp's own
   // barrier (at the block's, they would take issue slots).  These two threads bound every layer of small K blocks, so
-  // nothing in their loops is warp-wide, decided per block or divided per tile, and an MMA gets complete descriptors.
+  // nothing in their loops is warp-wide, the producer's form of load is chosen once, pixels advance without a division (a
+  // tile of reordered weights divides its channel by b_perm, and slices of K and batched items divide their tile number;
+  // the issuer compares the swizzle per block), and an MMA gets complete descriptors.
   // Against warp-wide loops with a vote per step, a choice of load per block and two divisions per tile: i8 3x3 64 -> 64 at
   // M = 1605632 234 -> 145 us, the 64-channel stem at M = 6422528 389 -> 266 us, 3x3 128 -> 128 at M = 401408 94 -> 81 us;
   // TF32 3x3 64 -> 64 at M = 100352 45 -> 32 us, 3x3 256 -> 128 at M = 65536 107 -> 84 us.

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(128, 1) probe_kernel(int groups, uint32_t ides
       const uint32_t a16 = base >> 4, b16 = (base + 16384u) >> 4;
       // four instructions (one 128-byte K block) per group, two accumulators in turn
       for (int g = 0; g < groups; ++g)
-        tc_mma_block<KIND, false>(tm + (uint32_t)(g & 1) * 256u, desc_lo | (a16 & 0x3fffu), desc_lo | (b16 & 0x3fffu), desc_hi, idesc, g >= 2 ? 1u : 0u, 4u);
+        tc_mma_block<KIND>(tm + (uint32_t)(g & 1) * 256u, desc_lo | (a16 & 0x3fffu), desc_lo | (b16 & 0x3fffu), desc_hi, idesc, g >= 2 ? 1u : 0u);
       tc_commit<false>(smem_u32(&bar));
       const long long start = clock64();
       while (!mbar_try_wait(smem_u32(&bar), 0)) {
