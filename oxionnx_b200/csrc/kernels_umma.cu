@@ -310,10 +310,11 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
     // int32 outputs, M = 2048 - 401408, K = 64 - 1152) the choice is at most 2.1 us from the best width, 10.5 us in sum, and
     // with 0.07 ns and 0.5 us, the general epilogue's before the roles of one thread, 2.1 and 10.3.
     // With a Gelu behind it 0.2 ns, which moves M = 8192 N = 3072 K = 768 from 6 rounds of 256 columns to 11 of 128 (61.5 ->
-    // 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us), and 2 us for a run of the small-problem kernel:
-    // whatever the rows (1 - 400), its tiles of 32 / 64 / 128 channels take 0 - 2 / 2 - 4 / 4 - 6 us more than without one.
-    // From 1 to 2.5 us a run the choice is the best of its neighbours but once (M = 300 N = 2048 K = 512: 14.5 us up to 2 us a
-    // run, 16.4 from there on); at 3 us few rows leave that kernel.
+    // 57.5 us) and M = 300 to tiles of 32 (encoder of 5x60 1043 -> 1022 us), and 2 us for a run of the small-problem kernel,
+    // whose tiles of 32 / 64 / 128 channels take 0 - 2 / 2 - 4 / 4 - 6 us more than without one.  Not so with one lane quarter
+    // of rows alone (M <= 32, one epilogue warp of a tile at work): M = 2 N = 30000 K = 768 20.5 us there and 22.6 - 30.8 in the
+    // persistent kernel.  From 33 rows, at 2 against 2.5 us a run: M = 33 N = 8192 K = 64 14.4 and 16.4, M = 300 N = 2048
+    // K = 512 14.5 and 16.4, N = 16384 and 30000 the same; at 0.7: M = 64 N = 16384 18.5 instead of 16.4.
     const bool gelu = e.mode == EPI_DEQUANT && e.dq_act != 0;
     const double ns_out = e.mode == EPI_F32 ? 0.03e-9 : (gelu ? 0.2e-9 : 0.045e-9);
     const double t_tile_fixed = 0.25e-6;
@@ -341,7 +342,7 @@ TileChoice choose_tile(const ConvShape& cs, const Epilogue& e, int kind, const U
     // (within 0.2 %); at 3.2 it is 1 % worse (INT8 network of 3 images of 192 302 us instead of 291, f32 of 2 of 224 495 instead of
     // 490) and at 2.5 10 % (one INT8 frame 308 instead of 255).
     if (tune.cta_pairs != 2) {
-      small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu ? 2.0 : 0.7);
+      small = choose_small(M, cs.OC, k_iters_host, cb * es, sms, max_split, gelu && M > 32 ? 2.0 : 0.7);
       if (small.bn > 0 && small.us * 1e-6 > best + 4e-6) small = SmallShape();
       if (small.bn > 0) {
         bn = small.bn;
